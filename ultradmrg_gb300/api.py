@@ -48,6 +48,12 @@ class Context:
         call("udmrg_ctx_tc_tuning", self.h, C.byref(t), C.byref(c))
         return t.value, c.value
 
+    def set_gemm_form(self, form: int = -1):
+        """FP64-accurate grouped GEMMs of plans built afterwards: 0 FP64 (or
+        double-word) FMAs, 1 digit slices on the tensor cores, -1 the one the
+        cost rule expects to be faster (default)."""
+        call("udmrg_ctx_set_gemm_form", self.h, int(form))
+
     def set_gemm_tiles(self, policy: int = -1):
         """Tile policy of a matvec plan's FP64-accurate grouped GEMMs: 0 least
         padding, 1 fewer 32 x 32 tiles, -1 the autotuner (default)."""

@@ -81,6 +81,10 @@ struct Ctx {
   int gemm_policy = -1;
   std::map<std::array<int64_t, 4>, int> gemm_tuned;
   int64_t gemm_trials = 0;
+  // Form of the FP64-accurate grouped GEMMs: -1 the faster one by the cost
+  // rule (contract.cpp), 0 FP64 (or double-word) FMAs, 1 digit slices on the
+  // tensor cores wherever they can express the GEMM
+  int gemm_form = -1;
   // C-ABI lifetime: live tensor / plan handles on this context; a context
   // whose destroy was requested is deleted when the last handle goes
   int64_t live_handles = 0;

@@ -141,6 +141,13 @@ int udmrg_ctx_tc_tuning(udmrg_ctx *c, int64_t *trials, int64_t *classes) {
   });
 }
 
+int udmrg_ctx_set_gemm_form(udmrg_ctx *c, int form) {
+  return guarded([&] {
+    UDMRG_REQUIRE(c && form >= -1 && form <= 1, "gemm form: -1, 0 or 1");
+    c->ctx.gemm_form = form;
+  });
+}
+
 int udmrg_ctx_set_gemm_tiles(udmrg_ctx *c, int policy) {
   return guarded([&] {
     UDMRG_REQUIRE(c && policy >= -1 && policy <= 1, "gemm tile policy: -1, 0 or 1");

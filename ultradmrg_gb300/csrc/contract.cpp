@@ -26,6 +26,7 @@ void GemmPlan::upload() {
   d_segs = upload_vec(ctx, segs);
   d_probs = upload_vec(ctx, probs);
   for (int c = 0; c < kNumCfg; ++c) d_tiles[c] = upload_vec(ctx, tiles[c]);
+  if (sl) sl->upload();
   // host vectors stay: the descriptors are read before the upload completes
   ctx->sync();
 }
@@ -96,6 +97,320 @@ void add_tiles(GemmPlan &g, int32_t pid, int64_t M, int64_t N, int policy) {
 }  // namespace
 
 static void sort_tiles(GemmPlan &g);
+
+namespace {
+
+constexpr int64_t up8(int64_t x) { return (x + 7) & ~(int64_t)7; }
+
+// Estimated time of a plan's FP64 tiles: multiply-adds of the padded tiles at
+// 0.5e12 per second (80% of the FP64 pipe), four per complex one.
+double fp64_seconds(const GemmPlan &g, bool cplx) {
+  std::vector<double> k(g.probs.size(), 0.0);
+  for (size_t p = 0; p < g.probs.size(); ++p)
+    for (int s = 0; s < g.probs[p].nseg; ++s)
+      k[p] += (double)((g.segs[g.probs[p].seg0 + s].K + 15) / 16 * 16);
+  double macs = 0;
+  for (int c = 0; c < kNumCfg; ++c)
+    for (const GTile &t : g.tiles[c]) macs += k[t.prob] * kCfgBM[c] * kCfgBN[c];
+  return 4e-6 + macs * (cplx ? 4.0 : 1.0) / 0.5e12;
+}
+
+// Below this estimate the sliced form's three launches and its passes over
+// the operands cannot pay, and its tables are not built.
+constexpr double kSliceMin = 50e-6;
+
+// Contractions over an MPO tensor's few channels stay on the FMAs: their K
+// fills one or two steps, and packing the large operand costs more than its
+// products.
+constexpr double kSliceMinK = 28;
+double mean_k(const GemmPlan &g) {  // mean summed K, weighted with the work
+  double w = 0, wk = 0;
+  for (const GProb &p : g.probs) {
+    double k = 0;
+    for (int s = 0; s < p.nseg; ++s) k += g.segs[p.seg0 + s].K;
+    w += k * p.M * p.N;
+    wk += k * k * p.M * p.N;
+  }
+  return w > 0 ? wk / w : 0.0;
+}
+
+// Sub-dimensions (extent, stride in doubles) of a block over some axes,
+// row-major, merged where contiguous; false: more than four remain.
+bool op_dims(const BTensor &T, int64_t b, const int64_t *st, const std::vector<int> &axes, int es,
+             int32_t *ext, int64_t *str, int32_t *n) {
+  int m = 0;
+  int64_t e[kMaxRank], s[kMaxRank];
+  for (int ax : axes) {
+    const int64_t d = T.dim_of(b, ax);
+    if (d == 1) continue;
+    if (m > 0 && s[m - 1] == d * st[ax] * es) {
+      e[m - 1] *= d;
+      s[m - 1] = st[ax] * es;
+    } else {
+      e[m] = d;
+      s[m++] = st[ax] * es;
+    }
+  }
+  if (m > 4) return false;
+  for (int i = 0; i < m; ++i) {
+    ext[i] = (int32_t)e[i];
+    str[i] = s[i];
+  }
+  *n = m;
+  return true;
+}
+
+// The ops of one operand block (or strided matrix): `base` real; complex data
+// [re | im] along K for operand A, rows (re, im) interleaved for operand B:
+// [[re, -im], [im, re]], so that the real product is the interleaved complex
+// one.  kh: K columns of the real half.
+void add_ops(SlicePlan &sp, int group, SlOp base, bool cplx, int32_t kh) {
+  if (!cplx) {
+    base.rstep = 1;
+    sp.add_op(group, base);
+    return;
+  }
+  auto part = [&](int im, int32_t r0, int32_t rstep, int32_t k0, int neg) {
+    SlOp o = base;
+    o.src_off = base.src_off + im;
+    o.r0 = base.r0 * rstep + r0;
+    o.rstep = rstep;
+    o.k0 = base.k0 + k0;
+    o.neg = neg;
+    sp.add_op(group, o);
+  };
+  if (base.src == 0) {
+    part(0, 0, 1, 0, 0);
+    part(1, 0, 1, kh, 0);
+  } else {
+    part(0, 0, 2, 0, 0);
+    part(1, 0, 2, kh, 1);
+    part(1, 1, 2, 0, 0);
+    part(0, 1, 2, kh, 0);
+  }
+}
+
+// Lines of C's rows (blk, m) and columns (blk, n, block width; two per complex
+// column).
+void push_rows(std::vector<SlLine> &v, int blk, int64_t M) {
+  for (int64_t m = 0; m < M; ++m) v.push_back({blk, (int32_t)m, 0, 0});
+}
+void push_cols(std::vector<SlLine> &v, int blk, int64_t N, int es) {
+  for (int64_t n = 0; n < N * es; ++n) v.push_back({blk, (int32_t)n, (int32_t)(N * es), 0});
+}
+
+// The sliced form of gemm_add_simple's problems: one group each.
+std::unique_ptr<SlicePlan> slice_simple(const GemmPlan &g, bool cplx, bool upper) {
+  auto sp = std::make_unique<SlicePlan>();
+  sp->ctx = g.ctx;
+  const int es = cplx ? 2 : 1;
+  for (const GProb &p : g.probs) {
+    const GSeg &s = g.segs[p.seg0];
+    const int64_t kh = up8(s.K);
+    std::vector<SlLine> rows, cols;
+    push_rows(rows, 0, p.M);
+    push_cols(cols, 0, p.N, es);
+    const int id = sp->add_group({p.M, (int64_t)p.N * es, kh * es}, rows, cols, {p.c_off * es},
+                                 upper);
+    for (int side = 0; side < 2; ++side) {
+      SlOp o{};
+      o.src = side;
+      o.src_off = (side ? s.b_off : s.a_off) * es;
+      o.rows = side ? p.N : p.M;
+      o.cols = s.K;
+      o.nr = o.nk = 1;
+      o.re[0] = o.rows;
+      o.ke[0] = o.cols;
+      o.rs[0] = (side ? s.b_ns[0] : s.a_ms[0]) * es;
+      o.ks[0] = (side ? s.b_ks[0] : s.a_ks[0]) * es;
+      if (o.cols) add_ops(*sp, id, o, cplx, (int32_t)kh);
+    }
+  }
+  sp->finalize();
+  return sp;
+}
+
+// The sliced form of a block contraction: blocks that share contracted
+// sectors, directly or through others, form one dense group (with abelian
+// charges: one quantum-number flow), its rows the A blocks' free sectors, its
+// columns the B blocks', its K their common contracted sectors, each padded
+// to a multiple of 8.  matches sorted by (output key, a, b); output o's block
+// starts at coff[o].
+std::unique_ptr<SlicePlan> slice_contract(const BTensor &A, const BTensor &B,
+                                          const std::vector<int> &ca, const std::vector<int> &cb,
+                                          const std::vector<int> &fa, const std::vector<int> &fb,
+                                          const std::vector<Match> &matches,
+                                          const std::vector<size_t> &mstart,
+                                          const std::vector<int64_t> &coff) {
+  const bool cplx = A.dtype == kC128;
+  const int es = cplx ? 2 : 1;
+  auto key_of = [](const BTensor &T, int64_t b, const std::vector<int> &axes) {
+    Key128 k = 0;
+    for (int ax : axes) k = (k << 16) | (Key128)T.key(b)[ax];
+    return k;
+  };
+  // ids of the contracted keys, A's and B's free keys (ascending keys), over
+  // the blocks that have a partner
+  std::vector<char> ahit(A.nblocks(), 0), bhit(B.nblocks(), 0);
+  for (const Match &m : matches) ahit[m.a] = bhit[m.b] = 1;
+  struct Ids {
+    std::vector<Key128> keys;
+    void close() {
+      std::sort(keys.begin(), keys.end());
+      keys.erase(std::unique(keys.begin(), keys.end()), keys.end());
+    }
+    int at(Key128 k) const {
+      return (int)(std::lower_bound(keys.begin(), keys.end(), k) - keys.begin());
+    }
+    int n() const { return (int)keys.size(); }
+  } kk, ki, kj;
+  for (int64_t a = 0; a < A.nblocks(); ++a)
+    if (ahit[a]) {
+      kk.keys.push_back(key_of(A, a, ca));
+      ki.keys.push_back(key_of(A, a, fa));
+    }
+  for (int64_t b = 0; b < B.nblocks(); ++b)
+    if (bhit[b]) kj.keys.push_back(key_of(B, b, fb));
+  kk.close();
+  ki.close();
+  kj.close();
+  std::vector<int> a_k(A.nblocks()), a_i(A.nblocks()), b_k(B.nblocks()), b_j(B.nblocks());
+  // connected components over the contracted keys
+  const int nodes = kk.n() + ki.n() + kj.n();
+  std::vector<int> root(nodes);
+  for (int i = 0; i < nodes; ++i) root[i] = i;
+  auto find = [&](int x) {
+    while (root[x] != x) x = root[x] = root[root[x]];
+    return x;
+  };
+  for (int64_t a = 0; a < A.nblocks(); ++a)
+    if (ahit[a]) {
+      a_k[a] = kk.at(key_of(A, a, ca));
+      a_i[a] = ki.at(key_of(A, a, fa));
+      root[find(a_k[a])] = find(kk.n() + a_i[a]);
+    }
+  for (int64_t b = 0; b < B.nblocks(); ++b)
+    if (bhit[b]) {
+      b_k[b] = kk.at(key_of(B, b, cb));
+      b_j[b] = kj.at(key_of(B, b, fb));
+      root[find(b_k[b])] = find(kk.n() + ki.n() + b_j[b]);
+    }
+  // members of each component with their sizes and offsets
+  std::vector<int64_t> ksz(kk.n(), 0), isz(ki.n(), 0), jsz(kj.n(), 0);
+  auto prod = [](const BTensor &T, int64_t b, const std::vector<int> &axes) {
+    int64_t p = 1;
+    for (int ax : axes) p *= T.dim_of(b, ax);
+    return p;
+  };
+  for (int64_t a = 0; a < A.nblocks(); ++a)
+    if (ahit[a]) {
+      ksz[a_k[a]] = prod(A, a, ca);
+      isz[a_i[a]] = prod(A, a, fa);
+    }
+  for (int64_t b = 0; b < B.nblocks(); ++b)
+    if (bhit[b]) jsz[b_j[b]] = prod(B, b, fb);
+  std::vector<int> comp(nodes, -1);  // component of a root
+  int nc = 0;
+  auto comp_of = [&](int node) {
+    const int r = find(node);
+    if (comp[r] < 0) comp[r] = nc++;
+    return comp[r];
+  };
+  struct Comp {
+    std::vector<SlLine> rows, cols;
+    int64_t M = 0, N = 0, K = 0;
+    int ni = 0, nj = 0, nk = 0;
+    int64_t na = 0, nb = 0;
+    std::vector<int64_t> blocks;
+    int id = 0;
+  };
+  std::vector<Comp> cs;
+  auto at = [&](int c) -> Comp & {
+    if ((int)cs.size() <= c) cs.resize(c + 1);
+    return cs[c];
+  };
+  std::vector<int64_t> k0(kk.n()), r0(ki.n()), c0(kj.n());
+  std::vector<int> iloc(ki.n()), jloc(kj.n());
+  for (int k = 0; k < kk.n(); ++k) {
+    Comp &c = at(comp_of(k));
+    k0[k] = c.K;
+    c.K += up8(ksz[k]);
+    c.nk++;
+  }
+  for (int i = 0; i < ki.n(); ++i) {
+    Comp &c = at(comp_of(kk.n() + i));
+    r0[i] = c.M;
+    iloc[i] = c.ni++;
+    push_rows(c.rows, iloc[i], isz[i]);
+    c.M += isz[i];
+  }
+  for (int j = 0; j < kj.n(); ++j) {
+    Comp &c = at(comp_of(kk.n() + ki.n() + j));
+    c0[j] = c.N;
+    jloc[j] = c.nj++;
+    push_cols(c.cols, jloc[j], jsz[j], es);
+    c.N += jsz[j];
+  }
+  for (Comp &c : cs) {
+    if (c.M >= (1 << 30) || c.N >= (1 << 29) || c.K >= (1 << 29)) return nullptr;
+    c.blocks.assign((size_t)c.ni * c.nj, -1);
+  }
+  for (size_t o = 0; o + 1 < mstart.size(); ++o) {
+    const Match &m = matches[mstart[o]];
+    Comp &c = cs[comp_of(kk.n() + a_i[m.a])];
+    c.blocks[(size_t)iloc[a_i[m.a]] * c.nj + jloc[b_j[m.b]]] = coff[o] * es;
+  }
+  auto sp = std::make_unique<SlicePlan>();
+  sp->ctx = A.ctx;
+  for (Comp &c : cs)
+    c.id = sp->add_group({c.M, c.N * es, c.K * es}, c.rows, c.cols, c.blocks, false);
+  int64_t st[kMaxRank];
+  for (int side = 0; side < 2; ++side) {
+    const BTensor &T = side ? B : A;
+    for (int64_t b = 0; b < T.nblocks(); ++b) {
+      if (!(side ? bhit : ahit)[b]) continue;
+      const int k = side ? b_k[b] : a_k[b];
+      Comp &c = cs[comp_of(k)];
+      (side ? c.nb : c.na)++;
+      SlOp o{};
+      o.src = side;
+      o.src_off = T.offs[b] * es;
+      o.rows = (int32_t)(side ? jsz[b_j[b]] : isz[a_i[b]]);
+      o.cols = (int32_t)ksz[k];
+      o.r0 = (int32_t)(side ? c0[b_j[b]] : r0[a_i[b]]);
+      o.k0 = (int32_t)k0[k];
+      block_strides(T, b, st);
+      if (!op_dims(T, b, st, side ? fb : fa, es, o.re, o.rs, &o.nr) ||
+          !op_dims(T, b, st, side ? cb : ca, es, o.ke, o.ks, &o.nk))
+        return nullptr;
+      add_ops(*sp, c.id, o, cplx, (int32_t)c.K);
+    }
+  }
+  for (const Comp &c : cs)  // sub-matrices without a block
+    if (c.na != (int64_t)c.ni * c.nk || c.nb != (int64_t)c.nj * c.nk) sp->holes = true;
+  sp->finalize();
+  return sp;
+}
+
+// The form rule: the sliced plan where its estimate is below the FP64 tiles'.
+// Both are sums over padded work, so ragged sectors, short K and narrow blocks
+// (the MPO tensors' few channels) stay on the FMAs.
+template <typename Build>
+std::unique_ptr<SlicePlan> slice_worth(const GemmPlan &g, bool cplx, Build build) {
+  const int form = g.ctx ? g.ctx->gemm_form : 0;
+  if (form == 0 || !g.may_slice || g.probs.empty()) return nullptr;
+  double t64 = 0.0;
+  if (form < 0) {
+    if (mean_k(g) < kSliceMinK) return nullptr;
+    t64 = fp64_seconds(g, cplx);
+    if (t64 < kSliceMin) return nullptr;
+  }
+  auto sp = build();
+  if (sp && form < 0 && sp->seconds() >= t64) sp.reset();
+  return sp;
+}
+
+}  // namespace
 
 static std::unique_ptr<ContractPlan> plan_impl(const BTensor &A, const BTensor &B,
                                                const std::vector<int> &ca,
@@ -311,10 +626,15 @@ static std::unique_ptr<ContractPlan> plan_impl(const BTensor &A, const BTensor &
     add_tiles(g, (int32_t)g.probs.size(), M, N, g.policy);
     g.probs.push_back(p);
   }
-  if (upload)
-    gemm_finalize(g);
-  else
-    sort_tiles(g);
+  sort_tiles(g);
+  if (!ca.empty()) {
+    std::vector<int64_t> coff(nout);
+    for (size_t o = 0; o < nout; ++o) coff[o] = C->offs[dest[o]];
+    g.sl = slice_worth(g, A.dtype == kC128, [&] {
+      return slice_contract(A, B, ca, cb, fa, fb, matches, mstart, coff);
+    });
+  }
+  if (upload) g.upload();
   plan->out = std::move(out);
   return plan;
 }
@@ -361,24 +681,20 @@ static void sort_tiles(GemmPlan &g) {
     });
 }
 
-void gemm_finalize(GemmPlan &g) {
+void gemm_finalize(GemmPlan &g, bool cplx, bool upper) {
+  if (upper)
+    for (int c = 0; c < kNumCfg; ++c) {
+      auto &t = g.tiles[c];
+      t.erase(std::remove_if(t.begin(), t.end(),
+                             [&](const GTile &x) { return x.m0 > x.n0 + kCfgBN[c] - 1; }),
+              t.end());
+    }
   sort_tiles(g);
+  g.sl = slice_worth(g, cplx, [&] { return slice_simple(g, cplx, upper); });
   g.upload();
 }
 
 void gemm_upload(GemmPlan &g) { g.upload(); }
-
-void gemm_keep_upper(GemmPlan &g) {
-  for (int c = 0; c < kNumCfg; ++c) {
-    auto &t = g.tiles[c];
-    t.erase(std::remove_if(t.begin(), t.end(),
-                           [&](const GTile &x) { return x.m0 > x.n0 + kCfgBN[c] - 1; }),
-            t.end());
-    g.ctx->free(g.d_tiles[c]);
-    g.d_tiles[c] = upload_vec(g.ctx, t);
-  }
-  g.ctx->sync();
-}
 
 void gemm_retile(GemmPlan &g, int policy) {
   if (policy == g.policy) return;

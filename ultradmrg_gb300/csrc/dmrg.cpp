@@ -121,6 +121,10 @@ static void tune_gemm_tiles(Ctx &ctx, MatvecPlan &mv) {
     gp.push_back(&mv.p2->gemm);
     if (mv.p3) gp.push_back(&mv.p3->gemm);
   }
+  // a plan in the sliced form runs no tiles
+  gp.erase(std::remove_if(gp.begin(), gp.end(), [](GemmPlan *g) { return g->sl != nullptr; }),
+           gp.end());
+  if (gp.empty()) return;
   auto retile = [&](int pol) {
     for (GemmPlan *g : gp) gemm_retile(*g, pol);
   };
@@ -920,7 +924,18 @@ LocalUpdate two_site_update_local(Ctx &ctx, const BTensor &lenv, const BTensor &
                                   const SketchHint *hint, BondSpectra *spectra) {
   UDMRG_REQUIRE(dir == 'r' || dir == 'l', "dir must be 'r' or 'l'");
   const double t0 = now();
-  auto init_state = contract_axes(ctx, mps_l, mps_r, {2}, {0});
+  // The mixed Krylov run follows the last bit of its start vector, so the
+  // two-site state is formed by the FP64 kernels in either form of the solve.
+  TensorPtr init_state;
+  {
+    struct FmaForm {
+      Ctx &c;
+      const int form;
+      explicit FmaForm(Ctx &x) : c(x), form(x.gemm_form) { c.gemm_form = 0; }
+      ~FmaForm() { c.gemm_form = form; }
+    } fma(ctx);
+    init_state = contract_axes(ctx, mps_l, mps_r, {2}, {0});
+  }
   auto mv = plan_matvec2(ctx, lenv, mpo_l, mpo_r, renv, *init_state, p.lancz.precision);
   const double tplan = now() - t0;
   auto lres = lanczos_gs(ctx, *mv, *init_state, p.lancz);

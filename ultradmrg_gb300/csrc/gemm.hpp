@@ -11,6 +11,7 @@
 #pragma once
 
 #include "btensor.hpp"
+#include "slice_gemm.hpp"
 
 namespace udmrg {
 
@@ -49,6 +50,10 @@ struct GemmPlan {
   std::vector<GTile> tiles[kNumCfg];
   double flops = 0;  // algorithmic: sum 2*M*N*K (x4 for complex data)
   int policy = 0;    // tile policy (add_tiles): 0 least padded work, 1 fewer 32 x 32 tiles
+  // the digit-sliced tensor-core form of the same problems, where it is the
+  // faster one (slice_worth); the tiles then only run on operands outside its range
+  std::unique_ptr<SlicePlan> sl;
+  bool may_slice = true;  // false: C = alpha A B + beta C with beta != 0
   // device copies
   GSeg *d_segs = nullptr;
   GProb *d_probs = nullptr;
@@ -72,16 +77,15 @@ void gemm_add_simple(GemmPlan &g, int64_t c_off, int64_t M, int64_t N, int64_t K
                      int64_t a_ms, int64_t a_ks, int64_t b_off, int64_t b_ks, int64_t b_ns,
                      bool cplx);
 // Sort tiles (largest K first) and upload the descriptors.
-void gemm_finalize(GemmPlan &g);
+// cplx: element type of the data (the sliced form's choice depends on it).
+// upper: square problems whose result is symmetric (Hermitian): only the tiles
+// that reach the diagonal or lie above it (the caller mirrors the upper triangle).
+void gemm_finalize(GemmPlan &g, bool cplx = false, bool upper = false);
 // the descriptors of a plan made with upload = false onto the device
 void gemm_upload(GemmPlan &g);
 // The same problems tiled under another policy (results are bit-identical:
 // every output element sums its segments and K in the same order).
 void gemm_retile(GemmPlan &g, int policy);
-// Square problems whose result is symmetric (Hermitian): drop the tiles
-// entirely below the diagonal (the caller mirrors the upper triangle).
-void gemm_keep_upper(GemmPlan &g);
-
 // Run C = alpha * A*B (+ beta * C) for every problem of the plan.
 void run_gemm(Ctx &ctx, const GemmPlan &plan, DType dt, const double *a, const double *b,
               double *c, double alpha, double beta);

@@ -1352,6 +1352,7 @@ void sym_eig_vectors(Ctx &ctx, DeviceScratch &scratch, const std::vector<EigJob>
       double *S = ns.get<double>(stot), *Zc = ns.get<double>(ztot);
       GemmPlan gs, gz, gc;
       gs.ctx = gz.ctx = gc.ctx = &ctx;
+      gz.may_slice = false;  // accumulates into Zc
       for (int q = 0; q < nj; ++q) {
         if (k[q] == 0) continue;
         const int64_t n = jobs[q].n, kk = k[q];

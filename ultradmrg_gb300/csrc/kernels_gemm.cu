@@ -147,7 +147,9 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
     grouped_gemm_kernel(const GTile *__restrict__ tiles, int ntiles,
                         const GProb *__restrict__ probs, const GSeg *__restrict__ segs,
                         const In *__restrict__ A, const In *__restrict__ B, In *__restrict__ C,
-                        double alpha, double beta) {
+                        double alpha, double beta, const int *__restrict__ gate) {
+  // gate: the sliced form's flags; the tiles run only where it did not apply
+  if (gate && gate[0] == 0 && gate[1] == 0) return;
   constexpr int NT = (BM / TM) * (BN / TN);
   // rows padded by one element: the staging stores of a warp walk K (the
   // rows) when K is the operand's contiguous direction, and unpadded rows of
@@ -244,7 +246,7 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 
 template <typename T, typename In, int BM, int BN, int TM, int TN, int BK>
 void launch_cfg(Ctx &ctx, const GemmPlan &plan, int cfg, const In *a, const In *b, In *c,
-                double alpha, double beta) {
+                double alpha, double beta, const int *gate) {
   const int ntiles = (int)plan.tiles[cfg].size();
   if (ntiles == 0) return;
   constexpr int NT = (BM / TM) * (BN / TN);
@@ -253,7 +255,7 @@ void launch_cfg(Ctx &ctx, const GemmPlan &plan, int cfg, const In *a, const In *
       &per_sm, grouped_gemm_kernel<T, In, BM, BN, TM, TN, BK>, NT, 0));
   const int grid = std::min(ntiles, std::max(1, per_sm) * ctx.num_sms);
   grouped_gemm_kernel<T, In, BM, BN, TM, TN, BK><<<grid, NT, 0, ctx.stream>>>(
-      plan.d_tiles[cfg], ntiles, plan.d_probs, plan.d_segs, a, b, c, alpha, beta);
+      plan.d_tiles[cfg], ntiles, plan.d_probs, plan.d_segs, a, b, c, alpha, beta, gate);
   UDMRG_CHECK_CUDA(cudaGetLastError());
   ctx.launches++;
 }
@@ -261,12 +263,17 @@ void launch_cfg(Ctx &ctx, const GemmPlan &plan, int cfg, const In *a, const In *
 template <typename T, typename In>
 void run_typed(Ctx &ctx, const GemmPlan &plan, const In *a, const In *b, In *c, double alpha,
                double beta) {
+  const int *gate = nullptr;
+  if (plan.sl && alpha == 1.0 && beta == 0.0) {
+    run_slice(ctx, *plan.sl, (const double *)a, (const double *)b, (double *)c);
+    gate = plan.sl->scale;
+  }
   // K chunk: 16 for 8-byte operands, 8 for complex (keeps static shared memory < 48 KB)
   constexpr int BK = sizeof(T) == 8 ? 16 : 8;
-  launch_cfg<T, In, 64, 64, 4, 4, BK>(ctx, plan, kCfg64x64, a, b, c, alpha, beta);
-  launch_cfg<T, In, 256, 16, 4, 4, BK>(ctx, plan, kCfg256x16, a, b, c, alpha, beta);
-  launch_cfg<T, In, 16, 256, 4, 4, BK>(ctx, plan, kCfg16x256, a, b, c, alpha, beta);
-  launch_cfg<T, In, 32, 32, 2, 2, BK>(ctx, plan, kCfg32x32, a, b, c, alpha, beta);
+  launch_cfg<T, In, 64, 64, 4, 4, BK>(ctx, plan, kCfg64x64, a, b, c, alpha, beta, gate);
+  launch_cfg<T, In, 256, 16, 4, 4, BK>(ctx, plan, kCfg256x16, a, b, c, alpha, beta, gate);
+  launch_cfg<T, In, 16, 256, 4, 4, BK>(ctx, plan, kCfg16x256, a, b, c, alpha, beta, gate);
+  launch_cfg<T, In, 32, 32, 2, 2, BK>(ctx, plan, kCfg32x32, a, b, c, alpha, beta, gate);
 }
 
 }  // namespace

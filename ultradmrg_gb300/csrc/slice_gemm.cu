@@ -1,0 +1,552 @@
+// Digit-sliced FP64-accurate grouped GEMM (see slice_gemm.hpp): scale pass,
+// digit pack, tcgen05 GEMM.
+#include "slice_gemm.hpp"
+
+#include <algorithm>
+
+#include "tc_roles.cuh"
+
+namespace udmrg {
+
+namespace {
+
+constexpr int kPackThreads = 256;
+constexpr int kLoExp = 1023 - 500, kHiExp = 1023 + 500;  // biased exponents of the sliced range
+
+__device__ __forceinline__ int64_t sl_off(int64_t i, const int32_t *ext, const int64_t *str, int n) {
+  int64_t off = 0;
+  for (int j = n - 1; j > 0; --j) {
+    const int32_t e = ext[j];
+    const int32_t q = (int32_t)i / e;
+    off += (int64_t)((int32_t)i - q * e) * str[j];
+    i = q;
+  }
+  return n > 0 ? off + i * str[0] : 0;
+}
+
+// Offsets of the tile's 32 rows and 64 columns (one division chain each, by
+// 96 threads); -1 past the op's edge.
+__device__ __forceinline__ void tile_offsets(const SlOp &op, const SlItem &it, int64_t *roff,
+                                             int64_t *koff) {
+  const int t = threadIdx.x;
+  if (t < 32) {
+    const int r = it.r0 + t;
+    roff[t] = r < op.rows ? op.src_off + sl_off(r, op.re, op.rs, op.nr) : -1;
+  } else if (t < 96) {
+    const int k = it.k0 + t - 32;
+    koff[t - 32] = k < op.cols ? sl_off(k, op.ke, op.ks, op.nk) : -1;
+  }
+}
+
+// scale[line] = max over the line's elements of the high word of |x| (bit 0
+// set where the low word alone is nonzero): its exponent bounds the line.
+// HBM bound: 8 B per element, read once; lanes walk the contiguous direction.
+__global__ void __launch_bounds__(kPackThreads)
+    slice_scale_kernel(const SlOp *__restrict__ ops, const SlItem *__restrict__ items, int nitems,
+                       const double *__restrict__ a, const double *__restrict__ b,
+                       int *__restrict__ scale) {
+  __shared__ int64_t roff[32], koff[64];
+  __shared__ int mx[32];
+  const int tid = threadIdx.x;
+  for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
+    const SlItem it = items[w];
+    const SlOp &op = ops[it.op];
+    const double *src = op.src ? b : a;
+    const bool rows_fast = op.rows_fast != 0;
+    __syncthreads();
+    tile_offsets(op, it, roff, koff);
+    if (tid < 32) mx[tid] = 0;
+    __syncthreads();
+    int best[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int e = tid + q * kPackThreads;
+      const int r = rows_fast ? e & 31 : e >> 6, k = rows_fast ? e >> 5 : e & 63;
+      int v = 0;
+      if (roff[r] >= 0 && koff[k] >= 0) {
+        const uint64_t d = (uint64_t)__double_as_longlong(__ldg(src + roff[r] + koff[k]));
+        v = (int)((uint32_t)(d >> 32) & 0x7FFFFFFFu) | ((uint32_t)d ? 1 : 0);
+      }
+      best[q] = v;
+    }
+    if (rows_fast) {  // a thread's eight elements share its row
+      int v = 0;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v = max(v, best[q]);
+      if (v) atomicMax(&mx[tid & 31], v);
+    } else {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int v = __reduce_max_sync(0xffffffffu, best[q]);
+        if ((tid & 31) == 0 && v) atomicMax(&mx[(tid + q * kPackThreads) >> 6], v);
+      }
+    }
+    __syncthreads();
+    if (tid < 32 && mx[tid]) {
+      atomicMax(scale + 2 + op.sc0 + op.r0 + (int64_t)(it.r0 + tid) * op.rstep, mx[tid]);
+    }
+  }
+}
+
+// x 2^(62 - e) rounded to an integer, e the line's exponent (|x| < 2^e), plus
+// 128 in each of its seven lower base-256 digits: byte d of the result is the
+// digit's value + 128 (balanced digits, -128 .. 127), its top byte the signed
+// leading digit (-64 .. 64).  Integer instructions only.
+__device__ __forceinline__ int64_t slice_bits(double x, int be, bool neg) {
+  const uint64_t d = (uint64_t)__double_as_longlong(x);
+  const int s = be - (int)((d >> 52) & 0x7FF);  // 0 for the line's largest binade
+  const uint64_t m = (d & 0xFFFFFFFFFFFFFull) | (1ull << 52);
+  int64_t v = 0;
+  if (s <= 9)
+    v = (int64_t)(m << (9 - s));
+  else if (s < 64)
+    v = (int64_t)((m + (1ull << (s - 10))) >> (s - 9));
+  if (((d >> 63) != 0) != neg) v = -v;
+  return v + 0x80808080808080ll;
+}
+
+// Digits of the operands into their images.  A work item is 32 rows x 64
+// columns of one op, staged in shared memory along the source's contiguous
+// direction; then a thread cuts one row's 8 consecutive columns into eight
+// 16-byte plane segments (a byte of slice_bits becomes a float by the
+// 2^23 + byte pattern: one byte permute and one FP32 add per digit), and the
+// 32 rows of a warp fill 512 contiguous bytes per plane.  HBM bound: 8 B read
+// and 16 B written per element.  Ops start at columns that are multiples of 8; the
+// columns from an op's edge to the next one are written as zeros.  A line whose
+// largest element is non-finite or outside the sliced range raises the flag.
+__global__ void __launch_bounds__(kPackThreads)
+    slice_pack_kernel(const SlOp *__restrict__ ops, const SlItem *__restrict__ items, int nitems,
+                      const double *__restrict__ a, const double *__restrict__ b,
+                      int *__restrict__ scale, uint8_t *__restrict__ img) {
+  __shared__ int64_t roff[32], koff[64];
+  __shared__ double tile[64][33];
+  const int tid = threadIdx.x;
+  for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
+    const SlItem it = items[w];
+    const SlOp &op = ops[it.op];
+    const double *src = op.src ? b : a;
+    const bool rows_fast = op.rows_fast != 0;
+    __syncthreads();
+    tile_offsets(op, it, roff, koff);
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int e = tid + q * kPackThreads;
+      const int r = rows_fast ? e & 31 : e >> 6, k = rows_fast ? e >> 5 : e & 63;
+      tile[k][r] = roff[r] >= 0 && koff[k] >= 0 ? __ldg(src + roff[r] + koff[k]) : 0.0;
+    }
+    __syncthreads();
+    const int r = tid & 31, g = tid >> 5;
+    const int rs = it.r0 + r, ks = it.k0 + g * 8;
+    if (rs >= op.rows || ks >= op.cols) continue;
+    const int row = op.r0 + rs * op.rstep, col = op.k0 + ks;
+    const int sc = scale[2 + op.sc0 + row];
+    const int be = sc == 0 ? 0x7FF : sc >> 20;  // a line of zeros: every digit zero
+    if (sc != 0 && (be < kLoExp || be > kHiExp)) atomicExch(scale, 1);
+    const int tr = op.tr, ts = tr == kSlU ? 7 : 6;
+    const int64_t plane = (int64_t)tr * kSlK * 2;
+    const int64_t tbase = op.img_off + (int64_t)(row >> ts) * op.kc * kSlDigits * plane;
+    const int rin = row & (tr - 1);
+    const int n = min(8, op.cols - ks);
+    float f[kSlDigits][8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int64_t v = j < n ? slice_bits(tile[g * 8 + j][r], be, op.neg != 0)
+                              : 0x80808080808080ll;
+      const uint32_t lo = (uint32_t)v, hi = (uint32_t)(v >> 32);
+      f[0][j] = __uint_as_float(0x4B000000u + 128u + (uint32_t)((int32_t)hi >> 24)) - 8388736.0f;
+      f[1][j] = __uint_as_float(__byte_perm(hi, 0x4B000000u, 0x7652)) - 8388736.0f;
+      f[2][j] = __uint_as_float(__byte_perm(hi, 0x4B000000u, 0x7651)) - 8388736.0f;
+      f[3][j] = __uint_as_float(__byte_perm(hi, 0x4B000000u, 0x7650)) - 8388736.0f;
+      f[4][j] = __uint_as_float(__byte_perm(lo, 0x4B000000u, 0x7653)) - 8388736.0f;
+      f[5][j] = __uint_as_float(__byte_perm(lo, 0x4B000000u, 0x7652)) - 8388736.0f;
+      f[6][j] = __uint_as_float(__byte_perm(lo, 0x4B000000u, 0x7651)) - 8388736.0f;
+      f[7][j] = __uint_as_float(__byte_perm(lo, 0x4B000000u, 0x7650)) - 8388736.0f;
+    }
+    uint8_t *o = img + tbase + (int64_t)(col >> 4) * kSlDigits * plane +
+                 canon_off(rin, col & 15, tr);
+#pragma unroll
+    for (int p = 0; p < kSlDigits; ++p)
+      *(uint4 *)(o + p * plane) =
+          make_uint4(__byte_perm(__float_as_uint(f[p][0]), __float_as_uint(f[p][1]), 0x7632),
+                     __byte_perm(__float_as_uint(f[p][2]), __float_as_uint(f[p][3]), 0x7632),
+                     __byte_perm(__float_as_uint(f[p][4]), __float_as_uint(f[p][5]), 0x7632),
+                     __byte_perm(__float_as_uint(f[p][6]), __float_as_uint(f[p][7]), 0x7632));
+  }
+}
+
+// ---- the GEMM ----
+//
+// Warp-specialised persistent kernel over the tile list (t = blockIdx.x + i *
+// gridDim.x): warp 0 stages the two operands' K steps by bulk copies (four
+// stages of 48 KB), warp 1 issues 36 tcgen05.mma (M 128, N 64, K 16) per step
+// into eight 64-column accumulators (all 512 TMEM columns), warps 2 .. 9 drain
+// them after every kSlChunk steps.  An epilogue thread owns 32 outputs of one
+// lane; it adds the levels into two 64-bit integers per output and frees the
+// accumulators before it rounds and stores, so the next chunk's products
+// overlap the rounding.  Every wait is bounded.
+constexpr int kSlThreads = 320;
+constexpr int kSlStages = 4;
+constexpr int kSlStageBytes = (int)(kSlUnitU + kSlUnitV);
+constexpr int kSlBarOffset = kSlStages * kSlStageBytes + kPadBytes;
+constexpr int kSlSmem = kSlBarOffset + 1024;
+static_assert(kSlSmem <= 227 * 1024, "sliced GEMM: shared memory budget");
+static_assert(kSlLevels * kSlV == 512, "sliced GEMM: the accumulators fill TMEM");
+
+struct SlBars {
+  uint64_t full[kSlStages], empty[kSlStages], tfull, tempty, fin;
+  uint32_t tmem;
+  volatile int abort;
+};
+
+__device__ __forceinline__ void sl_fail(SlBars *b, int *flags) {
+  atomicExch(flags + 1, 1);
+  b->abort = 1;
+}
+
+// 32 lanes x 32 bit, 4 consecutive columns per thread
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(taddr)
+               : "memory");
+}
+
+// (hi 2^32 + lo) 2^(e - 68) rounded to nearest FP64; |hi| < 2^62, the sum of
+// the level products with the lowest level's unit 2^-68
+__device__ __forceinline__ double sl_round(int64_t hi, int64_t lo, int e) {
+  hi += lo >> 32;
+  uint32_t w0 = (uint32_t)lo;
+  const bool neg = hi < 0;
+  uint64_t h = (uint64_t)hi;
+  if (neg) {
+    h = ~h + (w0 == 0 ? 1 : 0);
+    w0 = 0u - w0;
+  }
+  uint32_t w2 = (uint32_t)(h >> 32), w1 = (uint32_t)h;
+  int ex = 1023 + 95 - 68 + e;
+  if (w2 == 0) {
+    w2 = w1;
+    w1 = w0;
+    w0 = 0;
+    ex -= 32;
+    if (w2 == 0) {
+      w2 = w1;
+      w1 = 0;
+      ex -= 32;
+    }
+  }
+  if (w2 == 0) return 0.0;
+  const int c = __clz(w2);
+  ex -= c;
+  const uint32_t m1 = __funnelshift_l(w1, w2, c), m0 = __funnelshift_l(w0, w1, c);
+  const uint64_t m = ((uint64_t)m1 << 32) | m0;
+  uint64_t r = ((uint64_t)ex << 52) + ((m >> 11) & 0xFFFFFFFFFFFFFull) + ((m >> 10) & 1);
+  r |= (uint64_t)neg << 63;
+  return __longlong_as_double((long long)r);
+}
+
+__global__ void __launch_bounds__(kSlThreads, 1)
+    slice_gemm_kernel(const SlTile *__restrict__ tiles, int ntiles,
+                      const SlGroup *__restrict__ groups, const SlLine *__restrict__ lines,
+                      const int64_t *__restrict__ cblk, const int *__restrict__ scale,
+                      const uint8_t *__restrict__ img, double *__restrict__ C, int *flags) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  SlBars *b = (SlBars *)(smem + kSlBarOffset);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (scale[0]) return;  // the sliced form does not apply (uniform over the grid)
+  if (tid == 0) {
+    for (int s = 0; s < kSlStages; ++s) {
+      tc::mbar_init(&b->full[s], 1);
+      tc::mbar_init(&b->empty[s], 1);
+    }
+    tc::mbar_init(&b->tfull, 1);
+    tc::mbar_init(&b->tempty, 8);  // one arrival per epilogue warp
+    tc::mbar_init(&b->fin, 1);
+    b->abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    tc::tmem_alloc(&b->tmem, 512);
+    tc::tmem_relinquish();
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = b->tmem;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      uint32_t G = 0;
+      for (int t = blockIdx.x; t < ntiles && !b->abort; t += gridDim.x) {
+        const SlTile tile = tiles[t];
+        const SlGroup g = groups[tile.group];
+        const uint8_t *u = img + g.u_img + (int64_t)tile.ut * g.kc * kSlUnitU;
+        const uint8_t *v = img + g.v_img + (int64_t)tile.vt * g.kc * kSlUnitV;
+        for (int c = 0; c < g.kc; ++c, ++G) {
+          const uint32_t s = G % kSlStages;
+          if (G >= kSlStages && !wait_phase(&b->empty[s], ((G / kSlStages) - 1) & 1)) {
+            sl_fail(b, flags);
+            break;
+          }
+          uint8_t *st = smem + s * kSlStageBytes;
+          tc::mbar_expect_tx(&b->full[s], (uint32_t)kSlStageBytes);
+          tc::bulk_g2s(st, u + (int64_t)c * kSlUnitU, (uint32_t)kSlUnitU, &b->full[s]);
+          tc::bulk_g2s(st + kSlUnitU, v + (int64_t)c * kSlUnitV, (uint32_t)kSlUnitV, &b->full[s]);
+        }
+      }
+      // no copy is in flight when the block ends
+      for (uint32_t k = G < kSlStages ? 0 : G - kSlStages; k < G; ++k)
+        if (!wait_phase(&b->full[k % kSlStages], (k / kSlStages) & 1)) sl_fail(b, flags);
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = tc::idesc_bf16_f32(kSlU, kSlV);
+      uint32_t G = 0, n = 0;  // K steps, chunks so far
+      bool ok = true;
+      for (int t = blockIdx.x; t < ntiles && ok && !b->abort; t += gridDim.x) {
+        const int kc = groups[tiles[t].group].kc;
+        for (int c = 0; c < kc && ok; ++c, ++G) {
+          const bool first = c % kSlChunk == 0;
+          if (first) {
+            if (n > 0 && !wait_phase(&b->tempty, (n - 1) & 1)) {
+              ok = false;
+              break;
+            }
+            ++n;
+          }
+          const uint32_t s = G % kSlStages;
+          if (!wait_phase(&b->full[s], (G / kSlStages) & 1)) {
+            ok = false;
+            break;
+          }
+          tc::fence_after_sync();
+          const uint32_t su = tc::smem_u32(smem + s * kSlStageBytes);
+          const uint32_t sv = su + (uint32_t)kSlUnitU;
+          constexpr uint32_t planeU = kSlU * kSlK * 2, planeV = kSlV * kSlK * 2;
+#pragma unroll
+          for (int i = 0; i < kSlDigits; ++i) {
+            const uint64_t ad =
+                tc::make_desc(su + i * planeU, (kSlU / 8) * 128, 128);
+#pragma unroll
+            for (int j = 0; j < kSlDigits; ++j) {
+              if (i + j >= kSlLevels) break;
+              const uint64_t bd =
+                  tc::make_desc(sv + j * planeV, (kSlV / 8) * 128, 128);
+              // digit pair (0, l) is the first product of level l
+              tc::mma_bf16(tmem + (i + j) * kSlV, ad, bd, idesc, first && i == 0 ? 0u : 1u);
+            }
+          }
+          tc::mma_commit(&b->empty[s]);
+          if (c % kSlChunk == kSlChunk - 1 || c == kc - 1) tc::mma_commit(&b->tfull);
+        }
+      }
+      if (!ok) sl_fail(b, flags);
+      tc::mma_commit(&b->fin);  // every MMA of this CTA has completed
+      if (!wait_phase(&b->fin, 0)) sl_fail(b, flags);
+    }
+  } else {
+    const int q = warp & 3, half = (warp - 2) >> 2;
+    uint32_t n = 0;  // chunks so far
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+      const SlTile tile = tiles[t];
+      const SlGroup g = groups[tile.group];
+      int64_t hi[32], lo[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) hi[j] = lo[j] = 0;
+      bool ok = true;
+      for (int c0 = 0; c0 < g.kc; c0 += kSlChunk, ++n) {
+        if (b->abort || !wait_phase(&b->tfull, n & 1)) {
+          ok = false;
+          break;
+        }
+        tc::fence_after_sync();
+        const uint32_t base = tmem + ((uint32_t)(q * 32) << 16) + half * 32;
+#pragma unroll
+        for (int cb = 0; cb < 8; ++cb) {
+          uint32_t r[kSlLevels][4];
+#pragma unroll
+          for (int l = 0; l < kSlLevels; ++l) tmem_ld4(base + l * kSlV + cb * 4, r[l]);
+          tc::tmem_wait_ld();
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            int v[kSlLevels];
+#pragma unroll
+            for (int l = 0; l < kSlLevels; ++l) v[l] = __float2int_rn(__uint_as_float(r[l][j]));
+            hi[cb * 4 + j] += (int64_t)v[0] * (1 << 24) + (int64_t)v[1] * (1 << 16) +
+                              (int64_t)v[2] * (1 << 8) + (int64_t)v[3];
+            lo[cb * 4 + j] += (int64_t)v[4] * (1 << 24) + (int64_t)v[5] * (1 << 16) +
+                              (int64_t)v[6] * (1 << 8) + (int64_t)v[7];
+          }
+        }
+        tc::fence_before_sync();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&b->tempty);
+      }
+      if (!ok) {
+        if (lane == 0) sl_fail(b, flags);
+        break;
+      }
+      const int64_t ui = (int64_t)tile.ut * kSlU + q * 32 + lane;
+      const bool uok = ui < g.nu;
+      const SlLine ul = uok ? lines[g.u0 + ui] : SlLine{0, 0, 0, 0};
+      // a line without nonzero elements has scale 0: its sums are zero
+      const int ue = uok ? (scale[2 + g.u0 + ui] >> 20) - 1022 : 0;
+      int64_t cb = -1;
+      int blk = -1;
+      const int64_t vi0 = (int64_t)tile.vt * kSlV + half * 32;
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        const int64_t vi = vi0 + j;
+        if (vi >= g.nv) break;
+        const SlLine vl = lines[g.v0 + vi];
+        const int ve = (scale[2 + g.v0 + vi] >> 20) - 1022;
+        if (vl.blk != blk) {
+          blk = vl.blk;
+          cb = !uok ? -1
+                    : cblk[g.cb0 + (g.lanes_n ? (int64_t)vl.blk * g.ncb + ul.blk
+                                              : (int64_t)ul.blk * g.ncb + vl.blk)];
+        }
+        if (cb < 0) continue;
+        const int64_t at = cb + (g.lanes_n ? (int64_t)vl.loc * ul.w + ul.loc
+                                           : (int64_t)ul.loc * vl.w + vl.loc);
+        C[at] = sl_round(hi[j], lo[j], ue + ve);
+      }
+    }
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  if (warp == 0) tc::tmem_dealloc(tmem, 512);
+}
+
+template <typename V>
+V *up(Ctx *ctx, const std::vector<V> &v) {
+  if (v.empty()) return nullptr;
+  V *d = (V *)ctx->alloc(v.size() * sizeof(V));
+  UDMRG_CHECK_CUDA(
+      cudaMemcpyAsync(d, v.data(), v.size() * sizeof(V), cudaMemcpyHostToDevice, ctx->stream));
+  return d;
+}
+
+}  // namespace
+
+SlicePlan::~SlicePlan() {
+  if (!ctx) return;
+  for (void *p : {(void *)d_ops, (void *)d_items, (void *)d_groups, (void *)d_tiles,
+                  (void *)d_lines, (void *)d_cblk, (void *)img, (void *)scale})
+    ctx->free(p);
+}
+
+int SlicePlan::add_group(const Dims &d, const std::vector<SlLine> &rows,
+                         const std::vector<SlLine> &cols, const std::vector<int64_t> &blocks,
+                         bool upper) {
+  auto tiles_of = [](int64_t n, int t) { return (n + t - 1) / t; };
+  SlGroup g{};
+  // the side of 128-row tiles: the one that pads less, C's columns on a tie
+  // (consecutive lanes then store consecutive elements)
+  const int64_t wn = tiles_of(d.N, kSlU) * kSlU * tiles_of(d.M, kSlV) * kSlV;
+  const int64_t wm = tiles_of(d.M, kSlU) * kSlU * tiles_of(d.N, kSlV) * kSlV;
+  g.lanes_n = wn <= wm ? 1 : 0;
+  g.nu = (int32_t)(g.lanes_n ? d.N : d.M);
+  g.nv = (int32_t)(g.lanes_n ? d.M : d.N);
+  g.kc = (int32_t)((d.K + kSlK - 1) / kSlK);
+  g.u0 = (int64_t)lines.size();
+  const std::vector<SlLine> &u = g.lanes_n ? cols : rows, &v = g.lanes_n ? rows : cols;
+  lines.insert(lines.end(), u.begin(), u.end());
+  g.v0 = (int64_t)lines.size();
+  lines.insert(lines.end(), v.begin(), v.end());
+  g.cb0 = (int64_t)cblk.size();
+  int32_t ncb = 0;
+  for (const SlLine &l : cols) ncb = std::max(ncb, l.blk + 1);
+  g.ncb = ncb;
+  cblk.insert(cblk.end(), blocks.begin(), blocks.end());
+  g.upper = upper ? 1 : 0;
+  const int64_t ut = tiles_of(g.nu, kSlU), vt = tiles_of(g.nv, kSlV);
+  g.u_img = img_bytes;
+  img_bytes += ut * g.kc * kSlUnitU;
+  g.v_img = img_bytes;
+  img_bytes += vt * g.kc * kSlUnitV;
+  const int32_t id = (int32_t)groups.size();
+  for (int64_t i = 0; i < ut; ++i)
+    for (int64_t j = 0; j < vt; ++j) {
+      if (upper) {  // rows m, columns n: drop tiles with every n < m
+        const int64_t n1 = (g.lanes_n ? i * kSlU + kSlU - 1 : j * kSlV + kSlV - 1) * d.M / d.N;
+        const int64_t m0 = g.lanes_n ? j * kSlV : i * kSlU;
+        if (m0 > n1) continue;
+      }
+      tiles.push_back({id, (int32_t)i, (int32_t)j, 0});
+    }
+  if (d.K % kSlK) holes = true;
+  groups.push_back(g);
+  return id;
+}
+
+void SlicePlan::add_op(int group, SlOp op) {
+  const SlGroup &g = groups[group];
+  const bool is_u = (op.src == 1) == (g.lanes_n == 1);  // operand B holds C's columns
+  op.img_off = is_u ? g.u_img : g.v_img;
+  op.sc0 = is_u ? g.u0 : g.v0;
+  op.tr = is_u ? kSlU : kSlV;
+  op.kc = g.kc;
+  // lanes walk the source's contiguous direction
+  const bool rf = op.nr > 0 && op.re[op.nr - 1] > 1 && (op.nk == 0 || op.ke[op.nk - 1] == 1 ||
+                                                        op.rs[op.nr - 1] < op.ks[op.nk - 1]);
+  op.rows_fast = rf ? 1 : 0;
+  ops.push_back(op);
+}
+
+void SlicePlan::finalize() {
+  items.clear();
+  for (size_t o = 0; o < ops.size(); ++o)
+    for (int32_t r = 0; r < ops[o].rows; r += 32)
+      for (int32_t k = 0; k < ops[o].cols; k += 64) items.push_back({(int32_t)o, r, k, 0});
+  // largest K first (longest processing time first over the persistent grid)
+  std::stable_sort(tiles.begin(), tiles.end(), [&](const SlTile &x, const SlTile &y) {
+    return groups[x.group].kc > groups[y.group].kc;
+  });
+}
+
+void SlicePlan::upload() {
+  d_ops = up(ctx, ops);
+  d_items = up(ctx, items);
+  d_groups = up(ctx, groups);
+  d_tiles = up(ctx, tiles);
+  d_lines = up(ctx, lines);
+  d_cblk = up(ctx, cblk);
+  img = (uint8_t *)ctx->alloc(std::max<int64_t>(img_bytes, 1));
+  scale = (int *)ctx->alloc((lines.size() + 2) * sizeof(int));
+  if (holes) UDMRG_CHECK_CUDA(cudaMemsetAsync(img, 0, img_bytes, ctx->stream));
+}
+
+size_t SlicePlan::workspace() const {
+  return (size_t)img_bytes + (lines.size() + 2) * sizeof(int);
+}
+
+double SlicePlan::seconds() const {
+  double steps = 0, elems = 0;
+  for (const SlTile &t : tiles) steps += groups[t.group].kc + 2.0;
+  for (const SlOp &o : ops) elems += (double)o.rows * o.cols;
+  return 30e-6 + steps * 0.7e-6 / 152 + elems * 30.0 / 3e12;
+}
+
+void run_slice(Ctx &ctx, const SlicePlan &p, const double *a, const double *b, double *c) {
+  if (p.tiles.empty()) return;
+  UDMRG_CHECK_CUDA(cudaMemsetAsync(p.scale, 0, (p.lines.size() + 2) * sizeof(int), ctx.stream));
+  const int ni = (int)p.items.size();
+  const int pg = std::min(ni, 8 * ctx.num_sms);
+  if (ni) {
+    slice_scale_kernel<<<pg, kPackThreads, 0, ctx.stream>>>(p.d_ops, p.d_items, ni, a, b, p.scale);
+    slice_pack_kernel<<<pg, kPackThreads, 0, ctx.stream>>>(p.d_ops, p.d_items, ni, a, b, p.scale,
+                                                           p.img);
+  }
+  UDMRG_CHECK_CUDA(cudaFuncSetAttribute(slice_gemm_kernel,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize, kSlSmem));
+  const int nt = (int)p.tiles.size();
+  slice_gemm_kernel<<<std::min(nt, ctx.num_sms), kSlThreads, kSlSmem, ctx.stream>>>(
+      p.d_tiles, nt, p.d_groups, p.d_lines, p.d_cblk, p.scale, p.img, c, p.scale);
+  UDMRG_CHECK_CUDA(cudaGetLastError());
+  ctx.launches += ni ? 3 : 1;
+}
+
+}  // namespace udmrg

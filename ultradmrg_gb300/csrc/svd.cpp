@@ -272,7 +272,7 @@ void build_outputs(Ctx &ctx, DeviceScratch &scratch, const BTensor &T, int ldims
         gemm_add_simple(g, coffs[q], sc.rows, kept[q], sc.cols, sc.m_off, sc.cols, 1,
                         iso_off[q], iso_ld[q], 1, cplx);
     }
-    gemm_finalize(g);
+    gemm_finalize(g, cplx);
     if (left)
       (ctx.svd_dw ? run_gemm_dw : run_gemm)(ctx, g, dt, iso_c, Mbuf, Cbuf, 1.0, 0.0);
     else
@@ -419,8 +419,7 @@ SvdResult svd_trunc(Ctx &ctx, const BTensor &T, int ldims, const QN &ldiv, doubl
       gemm_add_simple(g, jobs[q].g_off, x.xr, x.xr, x.xc, x.off, x.sr, x.sc, x.off, x.sc, x.sr,
                       cplx);
     }
-    gemm_finalize(g);
-    gemm_keep_upper(g);  // the eigensolver mirrors the upper triangle
+    gemm_finalize(g, cplx, true);  // the eigensolver mirrors the upper triangle
     run_gemm(ctx, g, cplx ? kC128 : kF64, Mbuf, Mc, G, 1.0, 0.0);
   }
   // at most Dmax states are kept: only the leading eigenvalues of the sectors
