@@ -12,9 +12,9 @@ namespace udmrg {
 static_assert(kSpectrumFloor == kRankSv, "the SVD keeps the spectrum the rank model reads");
 
 TensorPtr contract_axes(Ctx &ctx, const BTensor &A, const BTensor &B, const std::vector<int> &ca,
-                        const std::vector<int> &cb) {
+                        const std::vector<int> &cb, bool dw) {
   auto p = plan_contract_axes(A, B, ca, cb);
-  return run_contract(ctx, *p, A, B);
+  return run_contract(ctx, *p, A, B, dw);
 }
 
 TensorPtr contract_cyclic(Ctx &ctx, const BTensor &A, const BTensor &B, int a_start, int b_start,
@@ -68,6 +68,35 @@ TensorPtr struct_union(const BTensor &a, const BTensor &b) {
   auto t = a.clone_struct();
   t->set_blocks(std::move(flat));
   return t;
+}
+
+// The same blocks with the axes in another order (structure only).
+static TensorPtr permute_struct(const BTensor &t, const std::vector<int> &perm) {
+  auto r = std::make_unique<BTensor>();
+  r->ctx = t.ctx;
+  r->dtype = t.dtype;
+  r->nq = t.nq;
+  for (int ax : perm) r->idx.push_back(t.idx[ax]);
+  std::vector<int32_t> flat;
+  flat.reserve(t.keys.size());
+  for (int64_t b = 0; b < t.nblocks(); ++b)
+    for (int ax : perm) flat.push_back(t.key(b)[ax]);
+  r->set_blocks(sort_keys(flat, t.rank()));
+  return r;
+}
+
+// Structure of T (a, x1, x2, b) contracted with W over W's axes x1, x2, its two
+// others between a and b.
+static TensorPtr mpo_map_struct(const BTensor &T, const BTensor &W, int x1, int x2) {
+  const int y1 = x1 == 0 ? 2 : 0;
+  for (int i = 0; i < 2; ++i) {
+    const Index &it = T.idx[1 + i], &iw = W.idx[i ? x2 : x1];
+    UDMRG_REQUIRE(it.same_space(iw) && it.dir == -iw.dir,
+                  "contract: contracted indexes do not match (sectors or directions)");
+  }
+  UDMRG_REQUIRE(T.dtype == W.dtype, "contract: operands must have the same element type");
+  return permute_struct(*contract_struct(T, W, {1, 2}, {x1, x2}, {0, 3}, {y1, y1 + 1}),
+                        {0, 2, 3, 1});
 }
 
 // keys of b's blocks that a lacks (flat, sorted)
@@ -228,17 +257,20 @@ std::unique_ptr<MatvecPlan> plan_matvec2(Ctx &ctx, const BTensor &L, const BTens
   mv->build_sec[0] = lap();
   mv->precision = precision;
   UDMRG_REQUIRE(precision == kPrecFP64 || precision == kPrecMixed, "matvec: unknown precision");
-  // real tensors: the two MPO steps as one sparse channel map (FP64 form) and
-  // the same fused coefficients for the mixed form
-  const bool real = L.dtype == kF64 && W1.dtype == kF64 && W2.dtype == kF64 &&
-                    R.dtype == kF64 && psi0.dtype == kF64;
+  // real MPO coefficients: the two MPO steps as one sparse channel map, shared
+  // by the FP64 and the mixed form
   const bool mixed = precision == kPrecMixed;
-  std::unique_ptr<FusedMpo> fm, fm_sg;  // host copies of W1 W2 (one per thread)
-  if (real || mixed) {
-    fm = std::make_unique<FusedMpo>(ctx, W1, W2);
-    if (real && mixed) fm_sg = std::make_unique<FusedMpo>(*fm);
-  }
-  FusedMpo *fmx = fm_sg ? fm_sg.get() : fm.get();
+  auto fm = std::make_unique<FusedMpo>(ctx, W1, W2);  // host copy of W1 W2
+  if (mixed && !fm->real)
+    throw Error(kErrInvalid,
+                "mixed-precision matvec: MPO with complex coefficients (use the FP64 form)");
+  const bool map = fm->real;
+  std::unique_ptr<FusedMpo> fm_sg;  // a copy for the mixed tables' thread
+  if (mixed) fm_sg = std::make_unique<FusedMpo>(*fm);
+  FusedMpo *fmx = fm_sg.get();
+  // the channel map writes T3 with b contiguous: (a', s1', s2', w2, b)
+  TensorPtr t3s;
+  if (map) t3s = permute_struct(*s3, {1, 2, 3, 4, 0});
   int bn1 = 0, bn3 = 0;
   const bool sg_known = mixed && sg_tiles_known(ctx, *S, &bn1, &bn3);
   // The host halves of the plans are independent given the closed structure
@@ -254,9 +286,11 @@ std::unique_ptr<MatvecPlan> plan_matvec2(Ctx &ctx, const BTensor &L, const BTens
     run([&] { mv->p2 = plan_contract_cyclic(*s1, W1, 1, 0, 2, false); });
     run([&] { mv->p3 = plan_contract_cyclic(*s2, W2, 4, 0, 2, false); });
     run([&] {
-      mv->p4 = plan_contract_into(*s3, R, ca, cb, fa, fb, *S, &mv->missing, false);
+      mv->p4 = map ? plan_contract_into(*t3s, R, {3, 4}, {1, 2}, {0, 1, 2}, {0}, *S, &mv->missing,
+                                        false)
+                   : plan_contract_into(*s3, R, ca, cb, fa, fb, *S, &mv->missing, false);
     });
-    if (real) run([&] { mv->m64 = build_mpo_step64(*fm, *s1, *s3); });
+    if (map) run([&] { mv->m64 = build_mpo_step64(*fm, *s1, *t3s); });
     if (sg_known) run([&] { mv->sg = plan_sg_tables(L, R, *S, *fmx, bn1, bn3); });
     for (Fut &f : jobs) f.wait();
     for (Fut &f : jobs) f.get();  // the first failure, after every job ended
@@ -266,9 +300,14 @@ std::unique_ptr<MatvecPlan> plan_matvec2(Ctx &ctx, const BTensor &L, const BTens
                     mv->p3->out->keys == s3->keys,
                 "matvec: intermediate block structures differ from the closure's");
   mv->build_sec[1] = lap();
-  for (ContractPlan *cp : {mv->p1.get(), mv->p2.get(), mv->p3.get(), mv->p4.get()})
-    gemm_upload(cp->gemm);
-  if (mv->m64) upload_mpo_step64(ctx, *mv->m64);
+  gemm_upload(mv->p1->gemm);
+  if (mv->m64) {
+    upload_mpo_step64(ctx, *mv->m64);
+  } else {
+    gemm_upload(mv->p2->gemm);
+    gemm_upload(mv->p3->gemm);
+  }
+  gemm_upload(mv->p4->gemm);
   mv->build_sec[2] = lap();
   mv->sstruct = std::move(S);
   mv->flops = mv->p1->gemm.flops + mv->p2->gemm.flops + mv->p3->gemm.flops + mv->p4->gemm.flops;
@@ -320,8 +359,19 @@ std::unique_ptr<MatvecPlan> plan_matvec1(Ctx &ctx, const BTensor &L, const BTens
     UDMRG_REQUIRE(it < 15, "matvec: Krylov block structure did not close");
   }
   mv->p1 = plan_contract_axes(L, *S, {2}, {0});
-  mv->p2 = plan_contract_cyclic(*mv->p1->out, W, 1, 0, 2);
-  mv->p4 = plan_contract_into(*mv->p2->out, R, ca, cb, fa, fb, *S, &mv->missing);
+  mv->p2 = plan_contract_cyclic(*mv->p1->out, W, 1, 0, 2, false);
+  bool real = true;
+  const std::vector<double> wh = mpo_data(ctx, W, &real);
+  if (real) {  // (a', s', w', b)
+    const BTensor &t1 = *mv->p1->out;
+    auto t2 = mpo_map_struct(t1, W, 0, 1);
+    mv->m64 = build_mpo_map(t1, W, wh, 0, 1, *t2);
+    upload_mpo_step64(ctx, *mv->m64);
+    mv->p4 = plan_contract_into(*t2, R, {2, 3}, {1, 2}, {0, 1}, {0}, *S, &mv->missing);
+  } else {
+    gemm_upload(mv->p2->gemm);
+    mv->p4 = plan_contract_into(*mv->p2->out, R, ca, cb, fa, fb, *S, &mv->missing);
+  }
   mv->sstruct = std::move(S);
   mv->flops = mv->p1->gemm.flops + mv->p2->gemm.flops + mv->p4->gemm.flops;
   const int es = elem_doubles(psi0.dtype);
@@ -344,7 +394,7 @@ void MatvecPlan::apply_fp64(const double *in, double *out, bool dw) {
   auto gemm = dw ? run_gemm_dw : run_gemm;
   gemm(*ctx, p1->gemm, dt, L->data, in, t1, 1.0, 0.0);
   if (m64) {
-    run_mpo_step64(*ctx, *m64, t1, t3);
+    run_mpo_step64(*ctx, *m64, t1, sites == 2 ? t3 : t2);
   } else {
     gemm(*ctx, p2->gemm, dt, t1, W1->data, t2, 1.0, 0.0);
     if (sites == 2) gemm(*ctx, p3->gemm, dt, t2, W2->data, t3, 1.0, 0.0);
@@ -755,10 +805,28 @@ ExpmvResult lanczos_expmv(Ctx &ctx, MatvecPlan &mv, const BTensor &init_state, d
 // Environments
 // ---------------------------------------------------------------------------
 
+// T (a, x1, x2, b) through the MPO tensor W: (a, y1, y2, b).  Null where W has
+// imaginary coefficients.
+static TensorPtr mpo_apply(Ctx &ctx, const BTensor &T, const BTensor &W, int x1, int x2) {
+  auto out = mpo_map_struct(T, W, x1, x2);
+  bool real = true;
+  const std::vector<double> wh = mpo_data(ctx, W, &real);
+  if (!real) return nullptr;
+  auto m = build_mpo_map(T, W, wh, x1, x2, *out);
+  upload_mpo_step64(ctx, *m);
+  out->alloc_data();
+  run_mpo_step64(ctx, *m, T.data, out->data);
+  return out;
+}
+
 TensorPtr update_site_lenv(Ctx &ctx, const BTensor &lenv, const BTensor &A, const BTensor &W,
                            bool dw) {
   auto Ad = dag(ctx, A);
-  auto t = contract_cyclic(ctx, lenv, A, 2, 0, 1, dw);
+  auto t = contract_cyclic(ctx, lenv, A, 2, 0, 1, dw);  // (a', w, s, b)
+  if (auto t2 = mpo_apply(ctx, *t, W, 0, 1)) {          // (a', s', w', b)
+    t.reset();
+    return contract_axes(ctx, *Ad, *t2, {0, 1}, {0, 1}, dw);
+  }
   auto t2 = contract_cyclic(ctx, *t, W, 1, 0, 2, dw);
   t.reset();
   return contract_cyclic(ctx, *Ad, *t2, 0, 1, 2, dw);
@@ -767,7 +835,11 @@ TensorPtr update_site_lenv(Ctx &ctx, const BTensor &lenv, const BTensor &A, cons
 TensorPtr update_site_renv(Ctx &ctx, const BTensor &renv, const BTensor &A, const BTensor &W,
                            bool dw) {
   auto Ad = dag(ctx, A);
-  auto t = contract_cyclic(ctx, *Ad, renv, 2, 0, 1, dw);
+  auto t = contract_cyclic(ctx, *Ad, renv, 2, 0, 1, dw);  // (a', s', w, b)
+  if (auto t2 = mpo_apply(ctx, *t, W, 2, 3)) {            // (a', w', s, b)
+    t.reset();
+    return contract_axes(ctx, *t2, A, {2, 3}, {1, 2}, dw);
+  }
   auto t2 = contract_cyclic(ctx, *t, W, 1, 2, 2, dw);
   t.reset();
   return contract_cyclic(ctx, *t2, A, 3, 1, 2, dw);

@@ -14,7 +14,7 @@ enum Precision : int { kPrecFP64 = 0, kPrecMixed = 1 };
 
 // Block-sparse ops built on plan + run.
 TensorPtr contract_axes(Ctx &ctx, const BTensor &A, const BTensor &B, const std::vector<int> &ca,
-                        const std::vector<int> &cb);
+                        const std::vector<int> &cb, bool dw = false);
 TensorPtr contract_cyclic(Ctx &ctx, const BTensor &A, const BTensor &B, int a_start, int b_start,
                           int n, bool dw = false);
 TensorPtr dag(Ctx &ctx, const BTensor &A);
@@ -39,8 +39,8 @@ struct MatvecPlan {
   int precision = kPrecFP64;
   int sites = 2;  // 1: single-site form (L, W1, R; p3 unused)
   std::unique_ptr<SgMatvecPlan> sg;  // the mixed-precision form
-  // real two-site FP64 form: the two MPO steps as one sparse channel map
-  // (p2, p3 then only describe the intermediate structures)
+  // real MPO coefficients: the MPO steps as one sparse channel map (p2, p3 then
+  // only describe the intermediate structures and count their flops)
   std::unique_ptr<MpoStep64> m64;
   // host seconds of the plan's construction: 0 Krylov closure (and the W1 W2
   // download), 1 the host tables built on host threads (contraction plans,

@@ -130,73 +130,72 @@ __global__ void __launch_bounds__(32 * kMpoWarps, 2)
   tc::pdl_launch_dependents();
 }
 
-// FP64 form: the same work units; inputs from T1 and outputs to T3 in their
-// block layouts (b contiguous in T1, strided in T3), FP64 accumulation.
-__global__ void mpo_unit64_kernel(const int64_t *__restrict__ unit0,
-                                  const int32_t *__restrict__ unit_pair, int64_t nunits,
-                                  const MpoPair64 *__restrict__ pairs,
-                                  const MpoIn64 *__restrict__ ins,
-                                  const MpoOut64 *__restrict__ outs,
-                                  const int32_t *__restrict__ rowptr,
-                                  const MpoNz64 *__restrict__ nz,
-                                  const double *__restrict__ t1, double *__restrict__ t3,
-                                  int slice) {
-  extern __shared__ double sm64[];
+// FP64 form.  A warp takes 64 consecutive (a', b) entries of one pair, two per
+// lane, and walks the pair's couplings (32 records held one per lane, handed
+// out by shuffles; the loads of four couplings' two entries in flight).  HBM
+// bound: 8 B read per T1 entry and written per T3 entry, both in contiguous
+// runs of db.
+__global__ void __launch_bounds__(256)
+    mpo_map64_kernel(const MpoTask64 *__restrict__ tasks, int ntasks,
+                     const MpoPair64 *__restrict__ pairs, const MpoOut64 *__restrict__ outs,
+                     const int32_t *__restrict__ rowptr, const MpoNz64 *__restrict__ nz,
+                     const double *__restrict__ t1, double *__restrict__ t3) {
+  constexpr int kB = 4;  // couplings whose loads are in flight together
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nwarp = blockDim.x >> 5;
-  double *X = sm64 + (int64_t)warp * slice;  // slice = max input channels x 32
-  for (int64_t u = (int64_t)blockIdx.x * nwarp + warp; u < nunits;
-       u += (int64_t)gridDim.x * nwarp) {
-    const int lo = __ldg(unit_pair + u);
-    const MpoPair64 pr = pairs[lo];
-    const int nbt = (pr.db + 31) >> 5;
-    const int64_t local = u - __ldg(unit0 + lo);
-    const int a = (int)(local / nbt);
-    const int b = (int)(local - (int64_t)a * nbt) * 32 + lane;
-    const bool col = b < pr.db;
-    for (int i = 0; i < pr.nin; ++i) {
-      const MpoIn64 in = ins[pr.in0 + i];
-      X[(i << 5) + lane] = col ? __ldg(t1 + in.base + (int64_t)a * in.astride + b) : 0.0;
-    }
-    __syncwarp();
-    for (int o = 0; o < pr.nout; ++o) {
-      const int k0 = __ldg(rowptr + pr.row0 + o), k1 = __ldg(rowptr + pr.row0 + o + 1);
-      double acc = 0.0;
-      for (int k = k0; k < k1; ++k) {
-        const MpoNz64 e = nz[k];
-        acc = fma(e.v, X[(e.i << 5) + lane], acc);
+  for (int t = blockIdx.x * 8 + warp; t < ntasks; t += gridDim.x * 8) {
+    const MpoTask64 tk = tasks[t];
+    const MpoPair64 pr = pairs[tk.pair];
+    const int u0 = tk.u0 + lane, u1 = u0 + 32, n = pr.da * pr.db;
+    const bool v0 = u0 < n, v1 = u1 < n;
+    const int a0 = v0 ? u0 / pr.db : 0, b0 = v0 ? u0 - a0 * pr.db : 0;
+    const int a1 = v1 ? u1 / pr.db : 0, b1 = v1 ? u1 - a1 * pr.db : 0;
+    const int kbeg = __ldg(rowptr + pr.row0), kend = __ldg(rowptr + pr.row0 + pr.nout);
+    int o = 0;
+    int next = __ldg(rowptr + pr.row0 + 1);  // end of output channel o's couplings
+    double s0 = 0.0, s1 = 0.0;
+    auto finish = [&]() {  // warp-uniform: write channel o, move to o + 1
+      const MpoOut64 ot = outs[pr.out0 + o];
+      if (v0) t3[ot.base + (int64_t)a0 * ot.astride + b0] = s0;
+      if (v1) t3[ot.base + (int64_t)a1 * ot.astride + b1] = s1;
+      s0 = s1 = 0.0;
+      if (++o < pr.nout) next = __ldg(rowptr + pr.row0 + 1 + o);
+    };
+    for (int kb = kbeg; kb < kend; kb += 32) {
+      const int nb = min(32, kend - kb);
+      MpoNz64 mine{0, 0.0, 0, 0};
+      if (lane < nb) mine = nz[kb + lane];
+      for (int q0 = 0; q0 < nb; q0 += kB) {
+        double x0[kB], x1[kB], c[kB];
+#pragma unroll
+        for (int q = 0; q < kB; ++q) {
+          const long long base = __shfl_sync(kFull, (long long)mine.base, q0 + q);
+          const int as = __shfl_sync(kFull, mine.astride, q0 + q);
+          c[q] = __shfl_sync(kFull, mine.v, q0 + q);
+          const bool ok = q0 + q < nb;
+          x0[q] = ok && v0 ? __ldg(t1 + base + (int64_t)a0 * as + b0) : 0.0;
+          x1[q] = ok && v1 ? __ldg(t1 + base + (int64_t)a1 * as + b1) : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < kB; ++q) {
+          if (q0 + q >= nb) break;
+          while (kb + q0 + q >= next) finish();
+          s0 = fma(c[q], x0[q], s0);
+          s1 = fma(c[q], x1[q], s1);
+        }
       }
-      if (col) {
-        const MpoOut64 ot = outs[pr.out0 + o];
-        t3[ot.base + (int64_t)a * ot.astride + (int64_t)b * ot.bstride] = acc;
-      }
     }
-    __syncwarp();  // X is rewritten by the next unit
+    while (o < pr.nout) finish();  // the last channel and channels without couplings
   }
 }
 
 }  // namespace
 
 void run_mpo_step64(Ctx &ctx, const MpoStep64 &p, const double *t1, double *t3) {
-  if (p.pairs.empty()) return;
-  const int64_t nunits = p.unit0.back();
-  if (nunits == 0) return;
-  const int slice = std::max(1, p.max_nin) * 32;
-  const size_t per_warp = (size_t)slice * sizeof(double);
-  UDMRG_REQUIRE(per_warp <= 200 * 1024, "MPO step: too many input channels in a pair");
-  const int warps = (int)std::max<size_t>(1, std::min<size_t>(8, (96 * 1024) / per_warp));
-  const size_t smem = per_warp * warps;
-  static size_t attr = 0;
-  if (smem > 48 * 1024 && smem > attr) {
-    UDMRG_CHECK_CUDA(cudaFuncSetAttribute(mpo_unit64_kernel,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr = smem;
-  }
-  const int64_t blocks = (nunits + warps - 1) / warps;
-  const int grid = (int)std::min<int64_t>(blocks, 16 * (int64_t)ctx.num_sms);
-  mpo_unit64_kernel<<<grid, 32 * warps, smem, ctx.stream>>>(
-      p.d_unit0, p.d_unit_pair, nunits, p.d_pairs, p.d_ins, p.d_outs, p.d_rowptr, p.d_nz, t1, t3,
-      slice);
+  const int ntasks = (int)p.tasks.size();
+  if (ntasks == 0) return;
+  const int grid = std::min((ntasks + 7) / 8, 16 * ctx.num_sms);
+  mpo_map64_kernel<<<grid, 256, 0, ctx.stream>>>(p.d_tasks, ntasks, p.d_pairs, p.d_outs,
+                                                 p.d_rowptr, p.d_nz, t1, t3);
   UDMRG_CHECK_CUDA(cudaGetLastError());
   ctx.launches++;
 }

@@ -6,26 +6,6 @@ namespace udmrg {
 
 namespace {
 
-// Host copy of a real tensor, or the real parts of a complex one whose
-// imaginary parts are all zero (an MPO made complex by promotion).
-std::vector<double> download_data(Ctx &ctx, const BTensor &t) {
-  const int es = elem_doubles(t.dtype);
-  std::vector<double> h(t.size() * es);
-  if (t.size())
-    UDMRG_CHECK_CUDA(cudaMemcpyAsync(h.data(), t.data, h.size() * sizeof(double),
-                                     cudaMemcpyDeviceToHost, ctx.stream));
-  ctx.sync();
-  if (es == 1) return h;
-  std::vector<double> r(t.size());
-  for (int64_t i = 0; i < t.size(); ++i) {
-    if (h[2 * i + 1] != 0.0)
-      throw Error(kErrInvalid,
-                  "mixed-precision matvec: MPO with complex coefficients (use the FP64 form)");
-    r[i] = h[2 * i];
-  }
-  return r;
-}
-
 template <typename V>
 V *upload(Ctx &ctx, const std::vector<V> &v) {
   if (v.empty()) return nullptr;
@@ -37,9 +17,28 @@ V *upload(Ctx &ctx, const std::vector<V> &v) {
 
 }  // namespace
 
+std::vector<double> mpo_data(Ctx &ctx, const BTensor &t, bool *real) {
+  const int es = elem_doubles(t.dtype);
+  std::vector<double> h(t.size() * es);
+  if (t.size())
+    UDMRG_CHECK_CUDA(cudaMemcpyAsync(h.data(), t.data, h.size() * sizeof(double),
+                                     cudaMemcpyDeviceToHost, ctx.stream));
+  ctx.sync();
+  *real = true;
+  if (es == 1) return h;
+  std::vector<double> r(t.size());
+  for (int64_t i = 0; i < t.size(); ++i) {
+    if (h[2 * i + 1] != 0.0) *real = false;
+    r[i] = h[2 * i];
+  }
+  return r;
+}
+
 FusedMpo::FusedMpo(Ctx &ctx, const BTensor &w1, const BTensor &w2) : W1(w1), W2(w2) {
-  w1h = download_data(ctx, W1);
-  w2h = download_data(ctx, W2);
+  bool r1 = true, r2 = true;
+  w1h = mpo_data(ctx, W1, &r1);
+  w2h = mpo_data(ctx, W2, &r2);
+  real = r1 && r2;
   for (int64_t b = 0; b < W1.nblocks(); ++b) w1_by_s1o[W1.key(b)[2]].push_back(b);
   for (int64_t b = 0; b < W2.nblocks(); ++b)
     w2_by[{W2.key(b)[0], W2.key(b)[2], W2.key(b)[3]}].push_back(b);
@@ -97,110 +96,177 @@ const std::vector<FusedMpo::Entry> &FusedMpo::get(int32_t S1p, int32_t S2p, int3
 
 MpoStep64::~MpoStep64() {
   if (!ctx) return;
-  for (void *p : {(void *)d_pairs, (void *)d_ins, (void *)d_outs, (void *)d_rowptr, (void *)d_nz,
-                  (void *)d_unit0, (void *)d_unit_pair})
+  for (void *p : {(void *)d_pairs, (void *)d_outs, (void *)d_rowptr, (void *)d_nz, (void *)d_tasks})
     ctx->free(p);
 }
+
+namespace {
+
+// One (a, b) sector pair under construction: its channels and couplings.
+struct PairMap {
+  struct In {
+    int64_t base, astride;
+  };
+  struct Nz {
+    int32_t o, i;
+    double v;
+  };
+  std::vector<In> ins;
+  std::vector<MpoOut64> outs;
+  std::vector<Nz> nz;
+};
+
+// Appends the pair in CSR form (couplings of one (o, i) summed, by ascending i).
+void push_pair(MpoStep64 &p, PairMap &m, int64_t da, int64_t db, int es) {
+  MpoPair64 pr{};
+  pr.out0 = (int32_t)p.outs.size();
+  pr.nout = (int32_t)m.outs.size();
+  pr.row0 = (int32_t)(p.rowptr.size() - 1);
+  pr.da = (int32_t)da;
+  pr.db = (int32_t)(db * es);
+  for (MpoOut64 o : m.outs) p.outs.push_back({o.base * es, o.astride * es, 0});
+  std::stable_sort(m.nz.begin(), m.nz.end(), [](const PairMap::Nz &x, const PairMap::Nz &y) {
+    return x.o != y.o ? x.o < y.o : x.i < y.i;
+  });
+  const size_t n0 = p.nz.size();
+  size_t q = 0;
+  for (int o = 0; o < pr.nout; ++o) {
+    for (; q < m.nz.size() && m.nz[q].o == o;) {
+      double v = 0.0;
+      const int i = m.nz[q].i;
+      for (; q < m.nz.size() && m.nz[q].o == o && m.nz[q].i == i; ++q) v += m.nz[q].v;
+      if (v == 0.0) continue;
+      UDMRG_REQUIRE(m.ins[i].astride * es < (1ll << 31), "MPO step: block too large");
+      p.nz.push_back({m.ins[i].base * es, v, (int32_t)(m.ins[i].astride * es), 0});
+    }
+    p.rowptr.push_back((int32_t)p.nz.size());
+  }
+  p.flops += 2.0 * (double)(p.nz.size() - n0) * pr.da * pr.db;
+  UDMRG_REQUIRE((int64_t)pr.da * pr.db < (1ll << 31), "MPO step: block too large");
+  for (int64_t u = 0; u < (int64_t)pr.da * pr.db; u += 64)
+    p.tasks.push_back({(int32_t)p.pairs.size(), (int32_t)u});
+  p.pairs.push_back(pr);
+}
+
+// Blocks grouped by the sectors of their first and last axes.
+std::map<std::pair<int32_t, int32_t>, std::vector<int64_t>> by_ends(const BTensor &t) {
+  std::map<std::pair<int32_t, int32_t>, std::vector<int64_t>> m;
+  for (int64_t b = 0; b < t.nblocks(); ++b)
+    m[{t.key(b)[0], t.key(b)[t.rank() - 1]}].push_back(b);
+  return m;
+}
+
+}  // namespace
 
 std::unique_ptr<MpoStep64> build_mpo_step64(FusedMpo &fm, const BTensor &T1, const BTensor &T3) {
   UDMRG_REQUIRE(T1.rank() == 5 && T3.rank() == 5, "MPO step: rank-5 intermediates expected");
   auto p = std::make_unique<MpoStep64>();
-  // T1 blocks by key (A', W, S1, S2, B)
-  std::map<std::array<int32_t, 5>, int64_t> t1blk;
+  const int es = elem_doubles(T1.dtype);
+  std::map<std::array<int32_t, 5>, int64_t> t1blk;  // (A', W, S1, S2, B)
   for (int64_t b = 0; b < T1.nblocks(); ++b) {
     const int32_t *k = T1.key(b);
     t1blk[{k[0], k[1], k[2], k[3], k[4]}] = b;
   }
-  // T3 blocks (B, A', S1', S2', W2) grouped by (A', B)
-  std::map<std::pair<int32_t, int32_t>, std::vector<int64_t>> by_pair;
-  for (int64_t b = 0; b < T3.nblocks(); ++b) by_pair[{T3.key(b)[1], T3.key(b)[0]}].push_back(b);
   p->rowptr.push_back(0);
-  p->unit0.push_back(0);
-  for (auto &kv : by_pair) {
+  for (auto &kv : by_ends(T3)) {
     const int32_t Ap = kv.first.first, Bs = kv.first.second;
-    MpoPair64 pr{};
-    pr.in0 = (int32_t)p->ins.size();
-    pr.out0 = (int32_t)p->outs.size();
-    pr.row0 = (int32_t)(p->rowptr.size() - 1);
-    pr.da = (int32_t)T3.idx[1].dims[Ap];
-    pr.db = (int32_t)T3.idx[0].dims[Bs];
+    const int64_t da = T3.idx[0].dims[Ap], db = T3.idx[4].dims[Bs];
+    PairMap m;
     std::map<int64_t, int32_t> in_first;  // T1 block -> its first input channel
-    struct Src {
-      int32_t out_first, in_first, nout, nin;
-      const std::vector<double> *coef;
-    };
-    std::vector<Src> srcs;
     for (int64_t ob : kv.second) {
       const int32_t *k = T3.key(ob);
-      const int32_t S1p = k[2], S2p = k[3], W2s = k[4];
-      const int64_t ds1p = T3.idx[2].dims[S1p], ds2p = T3.idx[3].dims[S2p];
-      const int64_t dw2 = T3.idx[4].dims[W2s];
-      const int32_t ofirst = (int32_t)(p->outs.size() - pr.out0);
-      const int32_t nout = (int32_t)(ds1p * ds2p * dw2);
-      for (int64_t s12 = 0; s12 < ds1p * ds2p; ++s12)
-        for (int64_t w2 = 0; w2 < dw2; ++w2)
-          p->outs.push_back({T3.offs[ob] + s12 * dw2 + w2, ds1p * ds2p * dw2,
-                             (int64_t)pr.da * ds1p * ds2p * dw2});
-      for (const FusedMpo::Entry &e : fm.get(S1p, S2p, W2s)) {
+      const int64_t nout =
+          T3.idx[1].dims[k[1]] * T3.idx[2].dims[k[2]] * T3.idx[3].dims[k[3]];
+      const int32_t ofirst = (int32_t)m.outs.size();
+      for (int64_t c = 0; c < nout; ++c)
+        m.outs.push_back({T3.offs[ob] + c * db, (int32_t)(nout * db), 0});
+      for (const FusedMpo::Entry &e : fm.get(k[1], k[2], k[3])) {
         auto tb = t1blk.find({Ap, e.src[0], e.src[1], e.src[2], Bs});
         if (tb == t1blk.end()) continue;
-        const int64_t ib = tb->second;
-        const int64_t dw = T1.idx[1].dims[e.src[0]], ds1 = T1.idx[2].dims[e.src[1]];
-        const int64_t ds2 = T1.idx[3].dims[e.src[2]];
-        auto f = in_first.find(ib);
-        if (f == in_first.end()) {
-          f = in_first.emplace(ib, (int32_t)(p->ins.size() - pr.in0)).first;
-          for (int64_t c = 0; c < dw * ds1 * ds2; ++c)
-            p->ins.push_back({T1.offs[ib] + c * pr.db, dw * ds1 * ds2 * pr.db});
-        }
-        srcs.push_back({ofirst, f->second, nout, (int32_t)(dw * ds1 * ds2), &e.coef});
+        const int64_t nin = T1.idx[1].dims[e.src[0]] * T1.idx[2].dims[e.src[1]] *
+                            T1.idx[3].dims[e.src[2]];
+        auto f = in_first.emplace(tb->second, (int32_t)m.ins.size());
+        if (f.second)
+          for (int64_t c = 0; c < nin; ++c)
+            m.ins.push_back({T1.offs[tb->second] + c * db, nin * db});
+        for (int64_t ic = 0; ic < nin; ++ic)
+          for (int64_t oc = 0; oc < nout; ++oc) {
+            const double v = e.coef[ic * nout + oc];
+            if (v != 0.0)
+              m.nz.push_back({(int32_t)(ofirst + oc), (int32_t)(f.first->second + ic), v});
+          }
       }
     }
-    pr.nin = (int32_t)p->ins.size() - pr.in0;
-    pr.nout = (int32_t)p->outs.size() - pr.out0;
-    UDMRG_REQUIRE(pr.nin <= 512, "MPO step: more than 512 input channels in one sector pair");
-    std::vector<double> C((size_t)pr.nout * std::max(pr.nin, 1), 0.0);
-    for (const Src &s : srcs)
-      for (int ic = 0; ic < s.nin; ++ic)
-        for (int oc = 0; oc < s.nout; ++oc)
-          C[(size_t)(s.out_first + oc) * pr.nin + s.in_first + ic] += (*s.coef)[ic * s.nout + oc];
-    int64_t nnz = 0;
-    for (int o = 0; o < pr.nout; ++o) {
-      for (int i = 0; i < pr.nin; ++i) {
-        const double v = C[(size_t)o * pr.nin + i];
-        if (v != 0.0) p->nz.push_back({v, i, 0});
+    push_pair(*p, m, da, db, es);
+  }
+  return p;
+}
+
+std::unique_ptr<MpoStep64> build_mpo_map(const BTensor &T, const BTensor &W,
+                                         const std::vector<double> &wh, int x1, int x2,
+                                         const BTensor &out) {
+  UDMRG_REQUIRE(T.rank() == 4 && out.rank() == 4 && W.rank() == 4, "MPO map: rank-4 tensors");
+  auto p = std::make_unique<MpoStep64>();
+  const int es = elem_doubles(T.dtype);
+  int y[2], ny = 0;
+  for (int ax = 0; ax < 4; ++ax)
+    if (ax != x1 && ax != x2) y[ny++] = ax;
+  std::map<std::array<int32_t, 4>, int64_t> tblk;
+  for (int64_t b = 0; b < T.nblocks(); ++b) {
+    const int32_t *k = T.key(b);
+    tblk[{k[0], k[1], k[2], k[3]}] = b;
+  }
+  std::map<std::pair<int32_t, int32_t>, std::vector<int64_t>> w_by_y;
+  for (int64_t b = 0; b < W.nblocks(); ++b) w_by_y[{W.key(b)[y[0]], W.key(b)[y[1]]}].push_back(b);
+  p->rowptr.push_back(0);
+  for (auto &kv : by_ends(out)) {
+    const int32_t Ap = kv.first.first, Bs = kv.first.second;
+    const int64_t da = out.idx[0].dims[Ap], db = out.idx[3].dims[Bs];
+    PairMap m;
+    std::map<int64_t, int32_t> in_first;
+    for (int64_t ob : kv.second) {
+      const int32_t *k = out.key(ob);
+      const int64_t d1 = out.idx[1].dims[k[1]], d2 = out.idx[2].dims[k[2]];
+      const int32_t ofirst = (int32_t)m.outs.size();
+      for (int64_t c = 0; c < d1 * d2; ++c)
+        m.outs.push_back({out.offs[ob] + c * db, (int32_t)(d1 * d2 * db), 0});
+      for (int64_t wb : w_by_y[{k[1], k[2]}]) {
+        const int32_t *kw = W.key(wb);
+        auto tb = tblk.find({Ap, kw[x1], kw[x2], Bs});
+        if (tb == tblk.end()) continue;
+        const int64_t e1 = W.idx[x1].dims[kw[x1]], e2 = W.idx[x2].dims[kw[x2]];
+        auto f = in_first.emplace(tb->second, (int32_t)m.ins.size());
+        if (f.second)
+          for (int64_t c = 0; c < e1 * e2; ++c)
+            m.ins.push_back({T.offs[tb->second] + c * db, e1 * e2 * db});
+        int64_t st[4];
+        st[3] = 1;
+        for (int ax = 2; ax >= 0; --ax) st[ax] = st[ax + 1] * W.idx[ax + 1].dims[kw[ax + 1]];
+        for (int64_t i1 = 0; i1 < e1; ++i1)
+          for (int64_t i2 = 0; i2 < e2; ++i2)
+            for (int64_t o1 = 0; o1 < d1; ++o1)
+              for (int64_t o2 = 0; o2 < d2; ++o2) {
+                const double v = wh[W.offs[wb] + i1 * st[x1] + i2 * st[x2] + o1 * st[y[0]] +
+                                    o2 * st[y[1]]];
+                if (v != 0.0)
+                  m.nz.push_back({(int32_t)(ofirst + o1 * d2 + o2),
+                                  (int32_t)(f.first->second + i1 * e2 + i2), v});
+              }
       }
-      nnz += (int64_t)p->nz.size() - p->rowptr.back();
-      p->rowptr.push_back((int32_t)p->nz.size());
     }
-    p->flops += 2.0 * (double)nnz * pr.da * pr.db;
-    p->max_nin = std::max(p->max_nin, (int)pr.nin);
-    const int64_t nu = (int64_t)pr.da * ((pr.db + 31) / 32);
-    p->unit0.push_back(p->unit0.back() + nu);
-    p->unit_pair.insert(p->unit_pair.end(), nu, (int32_t)p->pairs.size());
-    p->pairs.push_back(pr);
+    push_pair(*p, m, da, db, es);
   }
   return p;
 }
 
 void upload_mpo_step64(Ctx &ctx, MpoStep64 &m) {
-  MpoStep64 *p = &m;
-  p->ctx = &ctx;
-  p->d_pairs = upload(ctx, p->pairs);
-  p->d_ins = upload(ctx, p->ins);
-  p->d_outs = upload(ctx, p->outs);
-  p->d_rowptr = upload(ctx, p->rowptr);
-  p->d_nz = upload(ctx, p->nz);
-  p->d_unit0 = upload(ctx, p->unit0);
-  p->d_unit_pair = upload(ctx, p->unit_pair);
+  m.ctx = &ctx;
+  m.d_pairs = upload(ctx, m.pairs);
+  m.d_outs = upload(ctx, m.outs);
+  m.d_rowptr = upload(ctx, m.rowptr);
+  m.d_nz = upload(ctx, m.nz);
+  m.d_tasks = upload(ctx, m.tasks);
   ctx.sync();  // host vectors stay, but the uploads finish before they could move
-}
-
-std::unique_ptr<MpoStep64> plan_mpo_step64(Ctx &ctx, FusedMpo &fm, const BTensor &T1,
-                                           const BTensor &T3) {
-  auto p = build_mpo_step64(fm, T1, T3);
-  upload_mpo_step64(ctx, *p);
-  return p;
 }
 
 }  // namespace udmrg

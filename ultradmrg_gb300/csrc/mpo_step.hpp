@@ -8,7 +8,8 @@
 // tensors are first contracted over their shared bond (FusedMpo, per target
 // sector triple), then every (A', B) sector pair of T1/T3 becomes one small
 // dense channel map: out[o](a', b) = sum_i C[o][i] in[i](a', b), applied per
-// (a', 32 b) work unit by one warp.
+// (a', b) by one warp for 64 of them.  The single MPO tensor of an environment
+// update and of the one-site product is such a map too.
 #pragma once
 
 #include <array>
@@ -22,8 +23,8 @@ namespace udmrg {
 // output sector triple (S1', S2', W2): the contributing input sectors
 // (W, S1, S2) with their dense coefficient matrices coef[ic * nout + oc],
 // ic = (w ds1 + s1) ds2 + s2, oc = (s1' ds2' + s2') dw2 + w2.  Host side;
-// zero matrices are dropped.  Complex MPO tensors are accepted when every
-// imaginary part is zero (an MPO promoted to complex with its state).
+// zero matrices are dropped.  real: every imaginary part of complex MPO tensors
+// is zero (an MPO promoted to complex with its state); only then may get be called.
 struct FusedMpo {
   struct Entry {
     std::array<int32_t, 3> src;  // (W, S1, S2)
@@ -31,6 +32,7 @@ struct FusedMpo {
   };
   const BTensor &W1, &W2;
   std::vector<double> w1h, w2h;
+  bool real = true;
   std::map<int32_t, std::vector<int64_t>> w1_by_s1o;
   std::map<std::array<int32_t, 3>, std::vector<int64_t>> w2_by;  // (wr, s2', w2)
   std::map<std::array<int32_t, 3>, std::vector<Entry>> cache;
@@ -38,54 +40,54 @@ struct FusedMpo {
   const std::vector<Entry> &get(int32_t S1p, int32_t S2p, int32_t W2s);
 };
 
-// FP64 form.  T1 blocks (A', W, S1, S2, B) and T3 blocks (B, A', S1', S2', W2)
-// row-major in their tensors' buffers (the layouts of the grouped-GEMM plans
-// of the first and last steps).
-struct MpoIn64 {
-  int64_t base;     // element offset of channel (w, s1, s2) at (a' = 0, b = 0)
-  int64_t astride;  // elements between consecutive a' (b is contiguous)
+// FP64 form: T1 (A', W, S1, S2, B) to T3 (A', S1', S2', W2, B), both row-major
+// block tensors with b contiguous, so reads, writes and the next step's K runs
+// are contiguous.  The coefficients are real; complex data are moved as twice
+// as many reals.  Offsets and strides in doubles.
+struct MpoNz64 {
+  int64_t base;  // input channel at (a' = 0, b = 0)
+  double v;
+  int32_t astride, pad;  // doubles between consecutive a'
 };
 struct MpoOut64 {
-  int64_t base;     // element offset of channel (s1', s2', w2) at (a' = 0, b = 0)
-  int64_t astride, bstride;
+  int64_t base;
+  int32_t astride, pad;
 };
 struct MpoPair64 {
-  int32_t in0, nin, out0, nout;
-  int32_t row0, da, db, pad;  // row0: first CSR row of the pair
+  int32_t out0, nout;
+  int32_t row0, da, db, pad;  // row0: first CSR row of the pair; db in doubles
 };
-struct MpoNz64 {
-  double v;
-  int32_t i, pad;
+struct MpoTask64 {  // 64 consecutive (a', b) entries of a pair
+  int32_t pair, u0;
 };
 
 struct MpoStep64 {
   Ctx *ctx = nullptr;
   std::vector<MpoPair64> pairs;
-  std::vector<MpoIn64> ins;
   std::vector<MpoOut64> outs;
   std::vector<int32_t> rowptr;
   std::vector<MpoNz64> nz;
-  std::vector<int64_t> unit0;      // first work unit of each pair (+ total)
-  std::vector<int32_t> unit_pair;  // pair of every work unit
+  std::vector<MpoTask64> tasks;
   MpoPair64 *d_pairs = nullptr;
-  MpoIn64 *d_ins = nullptr;
   MpoOut64 *d_outs = nullptr;
   int32_t *d_rowptr = nullptr;
   MpoNz64 *d_nz = nullptr;
-  int64_t *d_unit0 = nullptr;
-  int32_t *d_unit_pair = nullptr;
-  int max_nin = 0;
+  MpoTask64 *d_tasks = nullptr;
   double flops = 0;  // 2 per nonzero coupling and (a', b) entry
   ~MpoStep64();
 };
 
-// T1, T3: the block structures of the two outer steps' intermediate tensors.
-// Every T3 entry is written (zero where no coupling reaches it).
-std::unique_ptr<MpoStep64> plan_mpo_step64(Ctx &ctx, FusedMpo &fm, const BTensor &T1,
-                                           const BTensor &T3);
-// The same in two parts: the host tables (no device call; safe on a host
-// thread with its own FusedMpo), then their upload.
+// The tables (host only: safe on a host thread with its own FusedMpo), for the
+// block structures of the two outer steps' intermediates.  Every T3 entry is
+// written (zero where no coupling reaches it).
 std::unique_ptr<MpoStep64> build_mpo_step64(FusedMpo &fm, const BTensor &T1, const BTensor &T3);
+// One MPO tensor W (data wh, real): T (a, x1, x2, b) to out (a, y1, y2, b) over
+// W's axes x1, x2; y1, y2 are W's two others in ascending order.
+std::unique_ptr<MpoStep64> build_mpo_map(const BTensor &T, const BTensor &W,
+                                         const std::vector<double> &wh, int x1, int x2,
+                                         const BTensor &out);
+// Host copy of an MPO tensor's real parts; *real = no nonzero imaginary part.
+std::vector<double> mpo_data(Ctx &ctx, const BTensor &w, bool *real);
 void upload_mpo_step64(Ctx &ctx, MpoStep64 &p);
 void run_mpo_step64(Ctx &ctx, const MpoStep64 &p, const double *t1, double *t3);
 
