@@ -143,11 +143,13 @@ int udmrg_ctx_host_mapped(const udmrg_ctx *ctx, int *mode);
 int udmrg_ctx_set_tc_tiles(udmrg_ctx *ctx, int bn1, int bn3);
 int udmrg_ctx_tc_tuning(udmrg_ctx *ctx, int64_t *trials, int64_t *classes);
 /* Form of the FP64-accurate grouped GEMMs (matvec, environments, SVD): 0 FP64
- * FMAs (double-word FP32 where a solver asks for it), 1 digit slices on the
+ * FMAs (double-word FP32 where a solver asks for it; an environment update's
+ * MPO tensor as a GEMM too), 1 digit slices on the
  * tensor cores (exact integer products, one rounding), -1 the one a cost rule
  * on the padded work expects to be faster (default).  Plans built afterwards
  * follow it.  No counterpart in the reference. */
 int udmrg_ctx_set_gemm_form(udmrg_ctx *ctx, int form);
+int udmrg_ctx_gemm_form(udmrg_ctx *ctx, int *form);
 /* Tile policy of the grouped FP64 (and double-word) block GEMMs of a
  * two-site matvec plan's FP64-accurate product: 0 least padded work per
  * output block, 1 fewer 32 x 32 tiles (taken only where larger tiles would

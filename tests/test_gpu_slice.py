@@ -106,7 +106,12 @@ def test_block_sparse_forms_agree(ctx, dtype):
     out = {}
     for form in (0, 1):
         ctx.set_gemm_form(form)
-        L, R = api.build_envs(ctx, mpo, mps, 2)
+        ten = [[api.DeviceTensor.from_data(ctx, t) for t in x] for x in (mps, mpo)]
+        L, R = (api.DeviceTensor.from_data(ctx, api.trivial_env_data(mps[i], mpo[i], s))
+                for i, s in ((0, "l"), (5, "r")))
+        for i in (0, 1):
+            L = api.update_site_lenvs(ctx, L, ten[0][i], ten[1][i])
+            R = api.update_site_renvs(ctx, R, ten[0][5 - i], ten[1][5 - i])
         w1, w2 = (api.DeviceTensor.from_data(ctx, mpo[i]) for i in (2, 3))
         psi = api.contract(ctx, api.DeviceTensor.from_data(ctx, mps[2]),
                            api.DeviceTensor.from_data(ctx, mps[3]), [2], [0])

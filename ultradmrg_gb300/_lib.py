@@ -79,6 +79,7 @@ SIGNATURES = {
     "udmrg_ctx_profiler_range": [C.c_void_p, C.c_int],
     "udmrg_ctx_set_gemm_tiles": [C.c_void_p, C.c_int],
     "udmrg_ctx_set_gemm_form": [C.c_void_p, C.c_int],
+    "udmrg_ctx_gemm_form": [C.c_void_p, C.POINTER(C.c_int)],
     "udmrg_ctx_gemm_tuning": [C.c_void_p, c_int64_p, c_int64_p],
     "udmrg_ctx_set_anchor_dw": [C.c_void_p, C.c_int],
     "udmrg_ctx_set_host_mapped": [C.c_void_p, C.c_int],

@@ -54,6 +54,12 @@ class Context:
         cost rule expects to be faster (default)."""
         call("udmrg_ctx_set_gemm_form", self.h, int(form))
 
+    def gemm_form(self) -> int:
+        """The form of the FP64-accurate grouped GEMMs (see set_gemm_form)."""
+        v = C.c_int()
+        call("udmrg_ctx_gemm_form", self.h, C.byref(v))
+        return v.value
+
     def set_gemm_tiles(self, policy: int = -1):
         """Tile policy of a matvec plan's FP64-accurate grouped GEMMs: 0 least
         padding, 1 fewer 32 x 32 tiles, -1 the autotuner (default)."""
@@ -629,7 +635,20 @@ def trivial_env_data(mps_ten: BlockTensorData, mpo_ten: BlockTensorData, side: s
 def build_envs(ctx, mpo: Sequence[BlockTensorData], mps: Sequence[BlockTensorData], l: int,
                normalize: bool = True):
     """Left environment of sites [0, l) and right environment of sites (l+1, N)
-    by device environment updates (each one normalised when ``normalize``)."""
+    by device environment updates (each one normalised when ``normalize``).
+
+    They use the plain FP64 GEMMs, whose summation order is fixed: a mixed
+    Krylov run follows the last bit of the environments it starts from, so
+    these do not depend on the form rule."""
+    form = ctx.gemm_form()
+    ctx.set_gemm_form(0)
+    try:
+        return _grow_envs(ctx, mpo, mps, l, normalize)
+    finally:
+        ctx.set_gemm_form(form)
+
+
+def _grow_envs(ctx, mpo, mps, l, normalize):
     N = len(mps)
     L = DeviceTensor.from_data(ctx, trivial_env_data(mps[0], mpo[0], "l"))
     for i in range(l):

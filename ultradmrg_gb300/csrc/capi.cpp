@@ -148,6 +148,13 @@ int udmrg_ctx_set_gemm_form(udmrg_ctx *c, int form) {
   });
 }
 
+int udmrg_ctx_gemm_form(udmrg_ctx *c, int *form) {
+  return guarded([&] {
+    UDMRG_REQUIRE(c && form, "null argument");
+    *form = c->ctx.gemm_form;
+  });
+}
+
 int udmrg_ctx_set_gemm_tiles(udmrg_ctx *c, int policy) {
   return guarded([&] {
     UDMRG_REQUIRE(c && policy >= -1 && policy <= 1, "gemm tile policy: -1, 0 or 1");

@@ -806,8 +806,9 @@ ExpmvResult lanczos_expmv(Ctx &ctx, MatvecPlan &mv, const BTensor &init_state, d
 // ---------------------------------------------------------------------------
 
 // T (a, x1, x2, b) through the MPO tensor W: (a, y1, y2, b).  Null where W has
-// imaginary coefficients.
+// imaginary coefficients or the context asks for plain FP64 GEMMs.
 static TensorPtr mpo_apply(Ctx &ctx, const BTensor &T, const BTensor &W, int x1, int x2) {
+  if (ctx.gemm_form == 0) return nullptr;
   auto out = mpo_map_struct(T, W, x1, x2);
   bool real = true;
   const std::vector<double> wh = mpo_data(ctx, W, &real);
