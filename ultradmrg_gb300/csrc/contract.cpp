@@ -398,7 +398,7 @@ std::unique_ptr<SlicePlan> slice_contract(const BTensor &A, const BTensor &B,
 template <typename Build>
 std::unique_ptr<SlicePlan> slice_worth(const GemmPlan &g, bool cplx, Build build) {
   const int form = g.ctx ? g.ctx->gemm_form : 0;
-  if (form == 0 || !g.may_slice || g.probs.empty()) return nullptr;
+  if (form == 0 || g.probs.empty()) return nullptr;
   double t64 = 0.0;
   if (form < 0) {
     if (mean_k(g) < kSliceMinK) return nullptr;

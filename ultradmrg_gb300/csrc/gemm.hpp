@@ -53,7 +53,6 @@ struct GemmPlan {
   // the digit-sliced tensor-core form of the same problems, where it is the
   // faster one (slice_worth); the tiles then only run on operands outside its range
   std::unique_ptr<SlicePlan> sl;
-  bool may_slice = true;  // false: C = alpha A B + beta C with beta != 0
   // device copies
   GSeg *d_segs = nullptr;
   GProb *d_probs = nullptr;
@@ -79,7 +78,7 @@ void gemm_add_simple(GemmPlan &g, int64_t c_off, int64_t M, int64_t N, int64_t K
 // Sort tiles (largest K first) and upload the descriptors.
 // cplx: element type of the data (the sliced form's choice depends on it).
 // upper: square problems whose result is symmetric (Hermitian): only the tiles
-// that reach the diagonal or lie above it (the caller mirrors the upper triangle).
+// that reach the diagonal or lie above it.
 void gemm_finalize(GemmPlan &g, bool cplx = false, bool upper = false);
 // the descriptors of a plan made with upload = false onto the device
 void gemm_upload(GemmPlan &g);

@@ -3,9 +3,9 @@
 //
 // FP64 throughput per SM is low on this GPU, so the solver does as little
 // FP64 work as the problem allows:
-//   1. Householder reduction to tridiagonal form (about 2 n^3 flops; one CTA
-//      per matrix held in shared memory, several co-resident CTAs per larger
-//      matrix; the reflectors stay in the matrix's upper triangle);
+//   1. Householder reduction to tridiagonal form (n^3 FMAs; the rows stay in
+//      the shared memory of one CTA, or of several co-resident ones; the
+//      reflectors stay in the matrix's upper triangle);
 //   2. every eigenvalue by Sturm-sequence bisection (O(n) per step and
 //      eigenvalue, all eigenvalues of all matrices in parallel);
 //   3. only the eigenvectors the caller needs, by inverse iteration on the
@@ -14,7 +14,7 @@
 //   4. orthonormalisation by Newton-Schulz steps (grouped GEMMs, host side);
 //   5. back-transformation by the Householder reflectors (one CTA per matrix).
 // These are the textbook methods (Golub & Van Loan ch. 8; Wilkinson's
-// inverse iteration; the Sturm count of Barth, Martin & Wilkinson), written
+// inverse iteration; Givens' Sturm sequence), written
 // for this batch layout.
 #include <algorithm>
 #include <cmath>
@@ -26,166 +26,67 @@ namespace udmrg {
 
 namespace {
 
-constexpr int kTriThreads = 512;
-constexpr int kBackThreads = 256;
+constexpr int kTriThreads = 256;
 
-__device__ double block_sum(double v, double *red) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  const int w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[w] = v;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double s = 0.0;
-    for (int i = 0; i < nw; ++i) s += red[i];
-    red[32] = s;
-  }
-  __syncthreads();
-  return red[32];
+// x 2^k by the exponent field (zero where it would leave the normal range)
+__device__ __forceinline__ double exp_shift(double x, int k) {
+  const int hi = __double2hiint(x), ex = ((hi >> 20) & 0x7FF) + k;
+  return ex > 0 ? __hiloint2double(hi + (k << 20), __double2loint(x)) : 0.0;
 }
 
-// Householder tridiagonalisation of the symmetric n x n matrix of each job
-// that fits in shared memory (row-major at G + g_off; the matrix is first
-// scaled to unit max-abs, the scale goes to scale[job]).  Step j reflects
-// row/column j: v (v_0 = 1) is stored in row j right of the first
-// superdiagonal, tau in tau[lam_off + j], the diagonal in d[lam_off + i] and
-// the off-diagonal in e[lam_off + i].
-__global__ void tridiag_kernel(const EigJob *__restrict__ jobs, double *__restrict__ G_all,
-                               double *__restrict__ d_all, double *__restrict__ e_all,
-                               double *__restrict__ tau_all, double *__restrict__ scale_all,
-                               int *__restrict__ status) {
-  extern __shared__ double sm[];
-  __shared__ double red[33];
-  __shared__ int bad;
-  const EigJob job = jobs[blockIdx.x];
-  const int n = job.n;
-  if (n == 0 || !job.smem) return;  // larger matrices: tridiag_mc_kernel
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const int lane = tid & 31, warp = tid >> 5, nwarp = nt >> 5;
-  double *A = sm;
-  double *v = sm + (int64_t)n * n;
-  double *w = v + n;
-  double *d = d_all + job.lam_off, *e = e_all + job.lam_off, *tau = tau_all + job.lam_off;
-
-  for (int64_t x = tid; x < (int64_t)n * n; x += nt) A[x] = G_all[job.g_off + x];
-  // scale to unit max-abs; non-finite input is reported
-  double mx = 0.0;
-  int nf = 0;
-  if (tid == 0) bad = 0;
-  for (int64_t x = tid; x < (int64_t)n * n; x += nt) {
-    const double g = A[x];
-    nf |= !isfinite(g);
-    mx = fmax(mx, fabs(g));
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    mx = fmax(mx, __shfl_down_sync(0xffffffffu, mx, o));
-    nf |= __shfl_down_sync(0xffffffffu, nf, o);
-  }
-  __syncthreads();
-  if (lane == 0) {
-    red[warp] = mx;
-    if (nf) atomicOr(&bad, 1);
-  }
-  __syncthreads();
-  if (tid == 0) {
-    double m = 0.0;
-    for (int i = 0; i < nwarp; ++i) m = fmax(m, red[i]);
-    red[32] = m;
-  }
-  __syncthreads();
-  if (bad) {
-    if (tid == 0) atomicExch(status, 2);
-    return;
-  }
-  const double scale = red[32];
-  if (tid == 0) scale_all[blockIdx.x] = scale;
-  // scale and symmetrise (a GEMM-made Gram matrix is symmetric only up to rounding)
-  const double inv = scale > 0.0 ? 1.0 / scale : 0.0;
-  for (int64_t x = tid; x < (int64_t)n * n; x += nt) {
-    const int r = (int)(x / n), c = (int)(x - (int64_t)r * n);
-    if (r < c) {
-      const double g = 0.5 * inv * (A[x] + A[(int64_t)c * n + r]);
-      A[x] = g;
-      A[(int64_t)c * n + r] = g;
-    } else if (r == c) {
-      A[x] *= inv;
+// Number of eigenvalues of the tridiagonal (diagonal d, squared off-diagonal
+// e2) below x: sign changes of the leading principal minors p_k(x) = (d_k - x)
+// p_{k-1} - e2_{k-1} p_{k-2} (Givens' Sturm sequence), rescaled by their
+// exponents every four steps.  Three FP64 instructions per entry instead of
+// the fourteen of the quotient form's division, and a chain of one FMA; signs
+// and scaling run on the integer pipes (64 sectors of a D = 2000 bond: 4.6 ->
+// 1.4 ms).  A zero minor counts as a sign change and goes on as -1e-30 of its
+// predecessor.  Up to 32 rows the quotients q_k = d_k - x - e2_{k-1} / q_{k-1}
+// themselves (Barth, Martin and Wilkinson): the chain is short either way, and
+// the few-state sectors of short chains keep their rounding, on whose last bit
+// a noised sweep's adaptation can turn.
+constexpr int kSturmQuotient = 32;
+__device__ __forceinline__ int sturm_count(const double *d, const double *e2, int n, double x) {
+  if (n <= kSturmQuotient) {
+    const double pivmin = 1e-290;
+    int c = 0;
+    double q = 0.0;
+    for (int k = 0; k < n; ++k) {
+      q = k == 0 ? d[0] - x : d[k] - x - e2[k - 1] / q;
+      if (fabs(q) < pivmin) q = -pivmin;
+      c += q < 0.0;
     }
+    return c;
   }
-  __syncthreads();
-
-  for (int j = 0; j + 2 < n; ++j) {
-    const int m = n - j - 1;  // length of the reflected vector (rows j+1 .. n-1)
-    double *rowj = A + (int64_t)j * n;
-    const double alpha = rowj[j + 1];
-    double x2 = 0.0;
-    for (int c = j + 2 + tid; c < n; c += nt) x2 += rowj[c] * rowj[c];
-    x2 = block_sum(x2, red);
-    double t = 0.0, beta = alpha, vs = 0.0;
-    if (x2 > 0.0) {
-      beta = -copysign(sqrt(alpha * alpha + x2), alpha);
-      t = (beta - alpha) / beta;
-      vs = 1.0 / (alpha - beta);
+  double p0 = 1.0, p1 = d[0] - x;
+  int cnt = 0, neg = 0;
+  auto sign = [&]() {  // counts the change from p0 to p1
+    const int hi = __double2hiint(p1);
+    if (((hi << 1) | __double2loint(p1)) == 0) {
+      p1 = p0 * -1e-30;
+      neg ^= 1;
+      ++cnt;
+    } else {
+      const int s = (int)((unsigned)hi >> 31);
+      cnt += s ^ neg;
+      neg = s;
     }
-    for (int r = tid; r < m; r += nt) {
-      const double vr = r == 0 ? 1.0 : rowj[j + 1 + r] * vs;
-      v[r] = t == 0.0 ? (r == 0 ? 1.0 : 0.0) : vr;
-      if (r > 0) rowj[j + 1 + r] = v[r];
+  };
+  sign();
+  for (int k0 = 1; k0 < n; k0 += 4) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int k = k0 + q;
+      if (k < n) {
+        const double p2 = fma(d[k] - x, p1, -(e2[k - 1] * p0));
+        p0 = p1;
+        p1 = p2;
+        sign();
+      }
     }
-    if (tid == 0) {
-      d[j] = rowj[j];
-      e[j] = beta;
-      tau[j] = t;
-    }
-    __syncthreads();
-    if (t == 0.0) continue;
-    // w = t * A_t v, A_t = trailing block rows/cols j+1 .. n-1 (one warp per row)
-    for (int r = warp; r < m; r += nwarp) {
-      const double *ar = A + (int64_t)(j + 1 + r) * n + (j + 1);
-      double s = 0.0;
-      for (int c = lane; c < m; c += 32) s += ar[c] * v[c];
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-      if (lane == 0) w[r] = t * s;
-    }
-    __syncthreads();
-    double wv = 0.0;
-    for (int r = tid; r < m; r += nt) wv += w[r] * v[r];
-    wv = block_sum(wv, red);
-    const double K = -0.5 * t * wv;
-    for (int r = tid; r < m; r += nt) w[r] += K * v[r];
-    __syncthreads();
-    // A_t -= v w^T + w v^T
-    for (int64_t x = tid; x < (int64_t)m * m; x += nt) {
-      const int r = (int)(x / m), c = (int)(x - (int64_t)r * m);
-      A[(int64_t)(j + 1 + r) * n + (j + 1 + c)] -= v[r] * w[c] + w[r] * v[c];
-    }
-    __syncthreads();
-  }
-  if (tid == 0) {
-    if (n >= 2) {
-      d[n - 2] = A[(int64_t)(n - 2) * n + (n - 2)];
-      e[n - 2] = A[(int64_t)(n - 2) * n + (n - 1)];
-      tau[n - 2] = 0.0;
-    }
-    d[n - 1] = A[(int64_t)(n - 1) * n + (n - 1)];
-    e[n - 1] = 0.0;
-    tau[n - 1] = 0.0;
-  }
-  __syncthreads();
-  // the reflectors live in the rows' upper parts
-  for (int64_t x = tid; x < (int64_t)n * n; x += nt) G_all[job.g_off + x] = A[x];
-}
-
-// Number of eigenvalues of the tridiagonal (d, e) below x (Sturm count).
-__device__ __forceinline__ int sturm_count(const double *d, const double *e, int n, double x,
-                                           double pivmin) {
-  int cnt = 0;
-  double q = d[0] - x;
-  if (fabs(q) < pivmin) q = -pivmin;
-  if (q < 0.0) ++cnt;
-  for (int k = 1; k < n; ++k) {
-    q = d[k] - x - e[k - 1] * e[k - 1] / q;
-    if (fabs(q) < pivmin) q = -pivmin;
-    if (q < 0.0) ++cnt;
+    const int m = max(__double2hiint(p0) & 0x7FFFFFFF, __double2hiint(p1) & 0x7FFFFFFF) >> 20;
+    p0 = exp_shift(p0, 1023 - m);
+    p1 = exp_shift(p1, 1023 - m);
   }
   return cnt;
 }
@@ -194,8 +95,10 @@ __device__ __forceinline__ int sturm_count(const double *d, const double *e, int
 // A warp handles kBisectEigs eigenvalues of one job, kBisectLanes lanes each:
 // per step the lanes of an eigenvalue take Sturm counts at the kBisectLanes
 // interior points that cut its interval into kBisectLanes + 1 equal parts,
-// and the part holding the eigenvalue is kept (the division chain of a Sturm
-// count is serial, so points side by side shorten the chain of steps).
+// and the part holding the eigenvalue is kept (a Sturm count is a
+// serial chain, so points side by side shorten the chain of steps; eight lanes
+// per eigenvalue fill the chip's FP64 pipes with one warp each at 2,000
+// eigenvalues).
 // Block b handles eigenvalues i0 .. i0 + kBisectEigs - 1 (ascending index) of
 // job chunk[b].x, i0 = chunk[b].y.
 // With the threshold grid of the leading-eigenvalue path (top, cnt; see
@@ -220,28 +123,28 @@ __global__ void __launch_bounds__(32)
   const int n = job.n;
   if (n == 0) return;
   const int lane = threadIdx.x, grp = lane / kBisectLanes, k = lane % kBisectLanes;
-  double *d = sm, *e = sm + n;
+  double *d = sm, *e = sm + n;  // e: first the off-diagonal, then its squares
   for (int i = lane; i < n; i += 32) {
     d[i] = d_all[job.lam_off + i];
     e[i] = i + 1 < n ? e_all[job.lam_off + i] : 0.0;
   }
   __syncwarp();
-  // Gershgorin interval and the largest off-diagonal (warp reduction)
-  double glo = 1e308, ghi = -1e308, em = 0.0;
+  // Gershgorin interval (warp reduction)
+  double glo = 1e308, ghi = -1e308;
   for (int i = lane; i < n; i += 32) {
     const double r = (i > 0 ? fabs(e[i - 1]) : 0.0) + (i + 1 < n ? fabs(e[i]) : 0.0);
     glo = fmin(glo, d[i] - r);
     ghi = fmax(ghi, d[i] + r);
-    if (i + 1 < n) em = fmax(em, fabs(e[i]));
   }
   for (int o = 16; o > 0; o >>= 1) {
     glo = fmin(glo, __shfl_xor_sync(0xffffffffu, glo, o));
     ghi = fmax(ghi, __shfl_xor_sync(0xffffffffu, ghi, o));
-    em = fmax(em, __shfl_xor_sync(0xffffffffu, em, o));
   }
+  __syncwarp();
+  for (int i = lane; i < n; i += 32) e[i] *= e[i];
+  __syncwarp();
   const double pad = 2.2e-16 * fmax(fabs(glo), fabs(ghi)) * n + 1e-300;
   const double lo0 = glo - pad, hi0 = ghi + pad;
-  const double pivmin = 1e-290 * fmax(1.0, em * em);
   const double scale = scale_all[jb];
   // absolute accuracy far below the eps * |T| the reduction itself achieves
   const double atol = 1e-18 * fmax(fabs(lo0), fabs(hi0));
@@ -267,7 +170,7 @@ __global__ void __launch_bounds__(32)
     if (__all_sync(0xffffffffu, done)) break;
     const double w = (hi - lo) / (kBisectLanes + 1);
     const double x = lo + w * (k + 1);
-    const bool above = !done && x > lo && x < hi && sturm_count(d, e, n, x, pivmin) > i;
+    const bool above = !done && x > lo && x < hi && sturm_count(d, e, n, x) > i;
     const unsigned m = (__ballot_sync(0xffffffffu, above) >> (grp * kBisectLanes)) &
                        ((1u << kBisectLanes) - 1);
     if (!done) {
@@ -329,35 +232,26 @@ __global__ void grid_count_kernel(const EigJob *__restrict__ jobs,
                                   const double *__restrict__ top, int *__restrict__ cnt,
                                   double *__restrict__ tr) {
   extern __shared__ double sm[];
-  __shared__ double pm[2];
+  __shared__ double pm;
   const int q = blockIdx.x;
   const EigJob job = jobs[q];
   const int n = job.n;
   double *d = sm, *e = sm + n;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     d[i] = d_all[job.lam_off + i];
-    e[i] = i + 1 < n ? e_all[job.lam_off + i] : 0.0;
+    const double x = i + 1 < n ? e_all[job.lam_off + i] : 0.0;
+    e[i] = x * x;
   }
   __syncthreads();
   if (threadIdx.x < 32) {
-    double t = 0.0, em = 0.0;
-    for (int i = threadIdx.x; i < n; i += 32) {
-      t += d[i];
-      em = fmax(em, fabs(e[i]));
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      t += __shfl_down_sync(0xffffffffu, t, o);
-      em = fmax(em, __shfl_down_sync(0xffffffffu, em, o));
-    }
-    if (threadIdx.x == 0) {
-      pm[0] = t;
-      pm[1] = em;
-    }
+    double t = 0.0;
+    for (int i = threadIdx.x; i < n; i += 32) t += d[i];
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    if (threadIdx.x == 0) pm = t;
   }
   __syncthreads();
   const double sc = scale_all[q];
-  if (threadIdx.x == 0) tr[q] = sc * pm[0];
-  const double pivmin = 1e-290 * fmax(1.0, pm[1] * pm[1]);  // as in bisect_kernel
+  if (threadIdx.x == 0) tr[q] = sc * pm;
   for (int k = threadIdx.x; k <= kGrid; k += blockDim.x) {
     int c;
     if (k == kGrid || n == 0) {
@@ -365,7 +259,7 @@ __global__ void grid_count_kernel(const EigJob *__restrict__ jobs,
     } else if (sc <= 0.0 || top[0] <= 0.0) {
       c = 0;  // a zero matrix: no eigenvalue reaches x_k > 0
     } else {
-      c = n - sturm_count(d, e, n, grid_point(top[0], k) / sc, pivmin);
+      c = n - sturm_count(d, e, n, grid_point(top[0], k) / sc);
     }
     cnt[(int64_t)q * (kGrid + 1) + k] = c;
   }
@@ -385,23 +279,28 @@ __device__ __forceinline__ double start_entry(uint64_t seed, int i) {
 // orthogonalised against the cluster's earlier vectors (modified
 // Gram-Schmidt).  Vector of position p goes to column p of Z (row-major
 // n x ld at z_off).  Work arrays are interleaved by thread (coalesced).
-__global__ void invit_kernel(const EigCluster *__restrict__ cl, int ncl,
-                             const EigJob *__restrict__ jobs, const double *__restrict__ d_all,
-                             const double *__restrict__ e_all,
-                             const double *__restrict__ scale_all,
-                             const double *__restrict__ lam_all, double *__restrict__ Z,
-                             double *__restrict__ work, int nmax) {
+//
+// Bound: a serial chain of about 40 FP64 instructions per row, 64 clocks each
+// (a few hundred warps cannot fill the chip).  The factors of eight rows are
+// loaded together, ahead of the recurrences that use them, so the chain does
+// not wait for L2; one division per row; the norm is summed in the back
+// substitution and its factor applied by the next pass.
+constexpr int kInvB = 8;
+__global__ void __launch_bounds__(32)
+    invit_kernel(const EigCluster *__restrict__ cl, int ncl, const EigJob *__restrict__ jobs,
+                 const double *__restrict__ d_all, const double *__restrict__ e_all,
+                 const double *__restrict__ scale_all, const double *__restrict__ lam_all,
+                 double *__restrict__ Z, double *__restrict__ work, int nmax) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= ncl) return;
   const EigCluster c = cl[t];
   const EigJob job = jobs[c.job];
   const int n = job.n;
   const double *d = d_all + job.lam_off, *e = e_all + job.lam_off;
-  const int64_t T = ncl;
-  double *l = work + 0 * (int64_t)nmax * T, *u0 = work + 1 * (int64_t)nmax * T;
-  double *u1 = work + 2 * (int64_t)nmax * T, *u2 = work + 3 * (int64_t)nmax * T;
-  double *y = work + 4 * (int64_t)nmax * T, *pv = work + 5 * (int64_t)nmax * T;
-  auto at = [&](double *a, int i) -> double & { return a[(int64_t)i * T + t]; };
+  const int64_t T = ncl, A = (int64_t)nmax * T;
+  // l: multipliers (an interchange in the lowest bit of pv), u0: reciprocal
+  // diagonal of U, u1, u2: its superdiagonals, y: the vector
+  double *l = work + t, *u0 = l + A, *u1 = u0 + A, *u2 = u1 + A, *y = u2 + A, *pv = y + A;
   double tnorm = 0.0;
   for (int i = 0; i < n; ++i)
     tnorm = fmax(tnorm, fabs(d[i]) + (i > 0 ? fabs(e[i - 1]) : 0.0) +
@@ -423,62 +322,100 @@ __global__ void invit_kernel(const EigCluster *__restrict__ cl, int ncl,
       return 1.0 / (fabs(v) > tiny ? v : (v < 0 ? -tiny : tiny));
     };
     double a = d[0] - lam, b = e[0];
+    double sub = e[0], dn = d[1], sup = n > 2 ? e[1] : 0.0;
     for (int i = 0; i + 1 < n; ++i) {
-      const double sub = e[i], dn = d[i + 1] - lam, sup = i + 2 < n ? e[i + 1] : 0.0;
-      if (fabs(a) >= fabs(sub)) {
-        const double piv = a != 0.0 ? a : tiny;
-        const double f = sub / piv;
-        at(u0, i) = rinv(piv);
-        at(u1, i) = b;
-        at(u2, i) = 0.0;
-        at(l, i) = f;
-        at(pv, i) = 0.0;
-        a = dn - f * b;
-        b = sup;
-      } else {
-        const double f = a / sub;
-        at(u0, i) = rinv(sub);
-        at(u1, i) = dn;
-        at(u2, i) = sup;
-        at(l, i) = f;
-        at(pv, i) = 1.0;
-        a = b - f * dn;
-        b = -f * sup;
+      const double s0 = sub, dl = dn - lam, s1 = sup;
+      if (i + 2 < n) {  // the next row's entries
+        sub = s1;
+        dn = d[i + 2];
+        sup = i + 3 < n ? e[i + 2] : 0.0;
       }
+      const bool keep = fabs(a) >= fabs(s0);
+      const double r = rinv(keep ? a : s0);
+      const double f = (keep ? s0 : a) * r;
+      const int64_t at = i * T;
+      u0[at] = r;
+      u1[at] = keep ? b : dl;
+      u2[at] = keep ? 0.0 : s1;
+      l[at] = f;
+      pv[at] = keep ? 0.0 : 1.0;
+      a = keep ? fma(-f, b, dl) : fma(-f, dl, b);
+      b = keep ? s1 : -f * s1;
     }
-    at(u0, n - 1) = rinv(a);
-    for (int i = 0; i < n; ++i) at(y, i) = start_entry(c.seed + 7919ull * (uint64_t)p, i);
+    u0[(n - 1) * T] = rinv(a);
+    const uint64_t seed = c.seed + 7919ull * (uint64_t)p;
+    double fac = 1.0;  // factor of the stored y still to be applied
     for (int it = 0; it < 3; ++it) {
       // forward: apply the interchanges and multipliers
-      for (int i = 0; i + 1 < n; ++i) {
-        if (at(pv, i) != 0.0) {
-          const double tmp = at(y, i);
-          at(y, i) = at(y, i + 1);
-          at(y, i + 1) = tmp - at(l, i) * at(y, i);
-        } else {
-          at(y, i + 1) -= at(l, i) * at(y, i);
+      double cur = it == 0 ? start_entry(seed, 0) : y[0] * fac;
+      for (int i0 = 0; i0 + 1 < n; i0 += kInvB) {
+        double lv[kInvB], pq[kInvB], yv[kInvB];
+#pragma unroll
+        for (int q = 0; q < kInvB; ++q) {
+          const int i = i0 + q;
+          if (i + 1 < n) {
+            lv[q] = l[i * T];
+            pq[q] = pv[i * T];
+            yv[q] = it == 0 ? start_entry(seed, i + 1) : y[(i + 1) * T];
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < kInvB; ++q) {
+          const int i = i0 + q;
+          if (i + 1 < n) {
+            const double nx = it == 0 ? yv[q] : yv[q] * fac;
+            const bool sw = __double2hiint(pq[q]) != 0;
+            const double top = sw ? nx : cur, bot = sw ? cur : nx;
+            y[i * T] = top;
+            cur = fma(-lv[q], top, bot);
+          }
         }
       }
-      // back substitution with U
-      for (int i = n - 1; i >= 0; --i) {
-        double s = at(y, i);
-        if (i + 1 < n) s -= at(u1, i) * at(y, i + 1);
-        if (i + 2 < n) s -= at(u2, i) * at(y, i + 2);
-        at(y, i) = s * at(u0, i);
+      // back substitution with U, summing the norm
+      double y1 = 0.0, y2 = 0.0, nrm = 0.0;
+      y1 = cur * u0[(n - 1) * T];
+      y[(n - 1) * T] = y1;
+      nrm = y1 * y1;
+      for (int i0 = n - 2; i0 >= 0; i0 -= kInvB) {
+        double av[kInvB], bv[kInvB], cv[kInvB], yv[kInvB];
+#pragma unroll
+        for (int q = 0; q < kInvB; ++q) {
+          const int i = i0 - q;
+          if (i >= 0) {
+            av[q] = u0[i * T];
+            bv[q] = u1[i * T];
+            cv[q] = u2[i * T];
+            yv[q] = y[i * T];
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < kInvB; ++q) {
+          const int i = i0 - q;
+          if (i >= 0) {
+            const double s = fma(-cv[q], y2, fma(-bv[q], y1, yv[q])) * av[q];
+            y[i * T] = s;
+            nrm = fma(s, s, nrm);
+            y2 = y1;
+            y1 = s;
+          }
+        }
       }
-      // orthogonalise against the cluster's earlier vectors, normalise
+      // orthogonalise against the cluster's earlier vectors
       for (int q = c.first; q < p; ++q) {
         double s = 0.0;
-        for (int i = 0; i < n; ++i) s += zc[(int64_t)i * c.ld + q] * at(y, i);
-        for (int i = 0; i < n; ++i) at(y, i) -= s * zc[(int64_t)i * c.ld + q];
+        for (int i = 0; i < n; ++i) s += zc[(int64_t)i * c.ld + q] * y[i * T];
+        nrm = 0.0;
+        for (int i = 0; i < n; ++i) {
+          const double v = y[i * T] - s * zc[(int64_t)i * c.ld + q];
+          y[i * T] = v;
+          nrm = fma(v, v, nrm);
+        }
       }
-      double nrm = 0.0;
-      for (int i = 0; i < n; ++i) nrm += at(y, i) * at(y, i);
       nrm = sqrt(nrm);
-      const double f = nrm > 0.0 ? 1.0 / nrm : 0.0;
-      for (int i = 0; i < n; ++i) at(y, i) *= f;
+      fac = nrm > 0.0 ? 1.0 / nrm : 0.0;
     }
-    for (int i = 0; i < n; ++i) zc[(int64_t)i * c.ld + p] = at(y, i);
+#pragma unroll 8
+    for (int i = 0; i < n; ++i) zc[(int64_t)i * c.ld + p] = y[i * T] * fac;
   }
 }
 
@@ -490,67 +427,7 @@ struct BackChunk {
   int64_t z_off, ld;
   int32_t job, c0, cw, pad;
 };
-// Real data: narrow column chunks (W = 8
-// columns per block, 4 for matrices above 3,400 rows), so that the largest
-// sector's columns spread over many SMs: this GPU issues about two FP64 FMAs
-// per clock per SM, and one sector's 4 n^2 k flops on one SM would bound the
-// whole kernel.  The chunk lives in shared memory (n x W doubles) for all
-// reflectors; thread t owns column t % W and the rows congruent to t / W
-// modulo kBackThreads / W.  Per reflector: partial dot products, a reduction
-// over the row groups (shuffles inside a warp, one shared-memory stage across
-// warps), the rank-1 update; two block barriers.
-template <int W>
-__global__ void __launch_bounds__(kBackThreads)
-    backtransform_narrow_kernel(const EigJob *__restrict__ jobs,
-                                const BackChunk *__restrict__ bt,
-                                const double *__restrict__ G_all,
-                                const double *__restrict__ tau_all, double *__restrict__ Z) {
-  constexpr int RG = kBackThreads / W;  // row groups
-  static_assert(RG * W == kBackThreads && W <= 32 && (32 % W) == 0, "back transformation layout");
-  extern __shared__ double zs[];  // n x W
-  __shared__ double part[kBackThreads / 32][W];
-  const BackChunk ch = bt[blockIdx.x];
-  const EigJob job = jobs[ch.job];
-  const int n = job.n;
-  if (n < 3 || ch.cw == 0) return;
-  const int c = threadIdx.x % W, g = threadIdx.x / W;
-  const int warp = threadIdx.x >> 5;
-  double *z = Z + ch.z_off + ch.c0;
-  const bool col = c < ch.cw;
-  for (int r = g; r < n; r += RG) zs[r * W + c] = col ? z[(int64_t)r * ch.ld + c] : 0.0;
-  __syncthreads();
-  const double *A = G_all + job.g_off;
-  for (int j = n - 3; j >= 0; --j) {
-    const double t = tau_all[job.lam_off + j];
-    if (t == 0.0) continue;  // uniform across the block
-    const int m = n - j - 1;
-    const double *vrow = A + (int64_t)j * n + j + 1;  // v[r] for r >= 1; v[0] = 1
-    double *zj = zs + (j + 1) * W + c;
-    double s0 = 0.0, s1 = 0.0;
-    int r = g;
-    for (; r + RG < m; r += 2 * RG) {
-      const double v0 = r == 0 ? 1.0 : __ldg(vrow + r);
-      const double v1 = __ldg(vrow + r + RG);
-      s0 = fma(v0, zj[r * W], s0);
-      s1 = fma(v1, zj[(r + RG) * W], s1);
-    }
-    if (r < m) s0 = fma(r == 0 ? 1.0 : __ldg(vrow + r), zj[r * W], s0);
-    double sum = s0 + s1;
-    // the row groups of this warp, then the warps
-#pragma unroll
-    for (int o = W; o < 32; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if ((threadIdx.x & 31) < W) part[warp][c] = sum;
-    __syncthreads();
-    double w = 0.0;
-#pragma unroll
-    for (int q = 0; q < kBackThreads / 32; ++q) w += part[q][c];
-    w *= t;
-    for (int r2 = g; r2 < m; r2 += RG) zj[r2 * W] -= (r2 == 0 ? 1.0 : __ldg(vrow + r2)) * w;
-    __syncthreads();
-  }
-  if (col)
-    for (int r = g; r < n; r += RG) z[(int64_t)r * ch.ld + c] = zs[r * W + c];
-}
+
 
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
@@ -564,20 +441,29 @@ __device__ __forceinline__ double2 cadd(double2 a, double2 b) {
 
 // ---- Householder tridiagonalisation of one large matrix by several CTAs ----
 //
-// A matrix too large for shared memory is reduced by P co-resident CTAs (a
-// cooperative launch): CTA p owns the rows i with i % P == p.  Step j uses
-// the reflector v_j of row j and w_j = t_j A v_j - K v_j; one fused pass over
-// each CTA's own rows applies the rank-2 update of step j and forms the
-// matrix-vector product of step j + 1, so the trailing block is read and
-// written once per step.  Per step the CTAs meet once, at a counter barrier
-// (every w_j entry and partial sum is written); then every CTA applies step
-// j's update to row j + 1 in its own shared memory (the same arithmetic in
-// every CTA) and forms the next reflector from it.  The barrier gives up
-// after kTriTimeoutNs and sets status 3.  Partial sums are added in CTA
-// order, so the result does not depend on timing.
+// A matrix too large for one SM's shared memory is reduced by P co-resident
+// CTAs (a cooperative launch): CTA p owns the rows i with i % P == p and keeps
+// them in its shared memory (in the global matrix where they do not fit).
+// Step j uses the reflector v_j of row j and w_j = t_j A v_j - K v_j; one fused
+// pass over each CTA's own rows applies the rank-2 update of step j and forms
+// the matrix-vector product of step j + 1, and the owner of the next pivot row
+// publishes it.  Per step the CTAs meet once, at a counter barrier; then every
+// CTA reads w_j's entries, the partial sums and the pivot row together, applies
+// step j's update to that row (the same arithmetic in every CTA) and forms the
+// next reflector.  The barrier gives up after kTriTimeoutNs and sets status 3.
+// Partial sums are added in CTA order, so the result does not depend on timing.
+//
+// Bound: 3 m^2 FP64 FMAs per step at two per clock and SM (n^3 in all, shared
+// out over the CTAs), plus about 5.5 us per step of barrier, L2 and scalar
+// latency.  A warp's FP64 instruction holds its quarter's pipe for
+// 64 clocks, so a warp takes four rows at a time with eight lanes each (their
+// sums reduced by three additions) and nothing scalar is computed by more than
+// one warp.
 struct TriPart {
   int32_t job, p, P, slot;
-  int64_t wb_off;  // 2 n scalars of w buffers (double-buffered by step parity)
+  int64_t wb_off;  // 4 n scalars: w entries and pivot rows (double-buffered by step parity)
+  int64_t part_off;  // slice sums in the w buffer (-1: in shared memory)
+  int32_t resident, pad;  // the own rows are kept in shared memory
 };
 struct TriSlot {  // one per matrix, zeroed before the launch
   unsigned int arrive;
@@ -600,6 +486,32 @@ __device__ __forceinline__ double2 sadd(double2 a, double2 b) { return cadd(a, b
 __device__ __forceinline__ double ssub(double a, double b) { return a - b; }
 __device__ __forceinline__ double2 ssub(double2 a, double2 b) {
   return make_double2(a.x - b.x, a.y - b.y);
+}
+// s + a x and s - a x.  Complex data form the product first: two fused steps
+// would round at s's size twice (measured: a third more error in a ladder SVD).
+__device__ __forceinline__ double smadd(double s, double a, double x) { return fma(a, x, s); }
+__device__ __forceinline__ double2 smadd(double2 s, double2 a, double2 x) {
+  return cadd(s, cmul(a, x));
+}
+__device__ __forceinline__ double smsub(double s, double a, double x) { return fma(-a, x, s); }
+__device__ __forceinline__ double2 smsub(double2 s, double2 a, double2 x) {
+  const double2 p = cmul(a, x);
+  return make_double2(s.x - p.x, s.y - p.y);
+}
+// a - v w - u x, the rank-2 update of one entry.  Complex data form the products'
+// sum first: four fused subtractions would round at a's size four times
+// (measured: twice the error of a ladder SVD's state).
+__device__ __forceinline__ double rank2(double a, double v, double w, double u, double x) {
+  return fma(-u, x, fma(-v, w, a));
+}
+__device__ __forceinline__ double2 rank2(double2 a, double2 v, double2 w, double2 u, double2 x) {
+  const double2 p = cadd(cmul(v, w), cmul(u, x));
+  return make_double2(a.x - p.x, a.y - p.y);
+}
+__device__ __forceinline__ double sinv(double a) { return 1.0 / a; }
+__device__ __forceinline__ double2 sinv(double2 a) {
+  const double dd = a.x * a.x + a.y * a.y;
+  return make_double2(a.x / dd, -a.y / dd);
 }
 __device__ __forceinline__ double sre(double a) { return a; }
 __device__ __forceinline__ double sre(double2 a) { return a.x; }
@@ -628,64 +540,56 @@ __device__ __forceinline__ double2 warp_sum(double2 v) {
   return make_double2(warp_sum(v.x), warp_sum(v.y));
 }
 
+// Sum over each group of eight lanes.
+__device__ __forceinline__ double oct_sum(double v) {
+  v += __shfl_xor_sync(0xffffffffu, v, 4);
+  v += __shfl_xor_sync(0xffffffffu, v, 2);
+  return v + __shfl_xor_sync(0xffffffffu, v, 1);
+}
+__device__ __forceinline__ double2 oct_sum(double2 v) {
+  return make_double2(oct_sum(v.x), oct_sum(v.y));
+}
+
 // All CTAs of the matrix arrive; false (status 3) if the others do not
-// arrive within the time limit.
-__device__ bool tri_barrier(TriSlot *sl, unsigned target, int *status) {
+// arrive within the time limit.  The release of one thread covers the block's
+// writes (ordered before it by the block barrier), the acquire the reads after.
+__device__ bool tri_barrier(TriSlot *sl, int P, unsigned target, int *status) {
   __shared__ int ok;
   __syncthreads();
+  if (P == 1) return true;
   if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(&sl->arrive, 1u);
-    const unsigned long long t0 = global_ns();
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&sl->arrive) : "memory");
     int good = 1;
-    while (*(volatile unsigned *)&sl->arrive < target) {
-      if (global_ns() - t0 > kTriTimeoutNs) {
-        good = 0;
-        atomicExch(status, 3);
-        break;
+    unsigned long long t0 = 0;
+    for (unsigned spin = 0;; ++spin) {
+      unsigned got;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(got) : "l"(&sl->arrive) : "memory");
+      if (got >= target) break;
+      if ((spin & 63) == 63) {
+        const unsigned long long t = global_ns();
+        if (t0 == 0) t0 = t;
+        if (t - t0 > kTriTimeoutNs) {
+          good = 0;
+          atomicExch(status, 3);
+          break;
+        }
       }
-      __nanosleep(64);
     }
-    __threadfence();
     ok = good;
   }
   __syncthreads();
   return ok != 0;
 }
 
-// Reflector of step j from row j, held in shared memory from its diagonal
-// on (row[c - j] = A[j][c]): v (v_0 = 1) into v[0 .. m), returns tau; the CTA
-// with writer set writes d[j], e[j], tau[j].  Same formulas as the
-// single-CTA kernels.
+// Leading dimension of resident rows: four rows by eight lanes of a warp fall
+// into different shared-memory banks where it is 8 modulo 16 doubles.
 template <typename T>
-__device__ T tri_reflector(const T *row, int n, int j, T *v, double *red, bool writer, double *d,
-                           double *e, T *tau) {
-  const T *rowj = row - j;  // rowj[c] = A[j][c], c >= j
-  const int m = n - j - 1;
-  const T alpha = cj(rowj[j + 1]);
-  double x2 = 0.0;
-  for (int c = j + 2 + threadIdx.x; c < n; c += blockDim.x) x2 += sabs2(rowj[c]);
-  x2 = block_sum(x2, red);
-  T t = smake<T>(0.0, 0.0), sc = smake<T>(0.0, 0.0);
-  double beta = sre(alpha);
-  const bool refl = x2 > 0.0 || sim(alpha) != 0.0;
-  if (refl) {
-    beta = -copysign(sqrt(sabs2(alpha) + x2), sre(alpha));
-    t = smake<T>((beta - sre(alpha)) / beta, -sim(alpha) / beta);
-    const double dr = sre(alpha) - beta, di = sim(alpha), dd = dr * dr + di * di;
-    sc = smake<T>(dr / dd, -di / dd);  // 1 / (alpha - beta)
-  }
-  for (int r = threadIdx.x; r < m; r += blockDim.x)
-    v[r] = r == 0 ? smake<T>(1.0, 0.0)
-                  : (refl ? smul(cj(rowj[j + 1 + r]), sc) : smake<T>(0.0, 0.0));
-  if (writer && threadIdx.x == 0) {
-    d[j] = sre(rowj[j]);
-    e[j] = beta;
-    tau[j] = t;
-  }
-  __syncthreads();
-  return t;
+__host__ __device__ constexpr int tri_ld(int n) {
+  return sizeof(T) == 8 ? (n + 7) / 16 * 16 + 8 : (n | 1);
 }
+// Slice sums of the row pass: one per own row of the full rounds, at most eight
+// for each of the 4 x 7 rows left over.
+__host__ __device__ constexpr int tri_parts(int n, int P) { return 224 + (n + P - 1) / P + 4; }
 
 template <typename T>
 __global__ void __launch_bounds__(kTriThreads)
@@ -697,32 +601,39 @@ __global__ void __launch_bounds__(kTriThreads)
                       int *__restrict__ status) {
   extern __shared__ __align__(16) unsigned char tri_sm[];
   __shared__ double red[33];
-  __shared__ T ksum;
+  __shared__ T sh_k, sh_t, sh_sc;
+  __shared__ T wpart[kTriThreads / 32];
   const TriPart pt = parts[blockIdx.x];
   const EigJob job = jobs[pt.job];
   const int n = job.n, p = pt.p, P = pt.P;
   TriSlot *sl = slots + pt.slot;
   T *A = G_all + job.g_off;
-  T *wb = wbuf_all + pt.wb_off;
+  T *wb = wbuf_all + pt.wb_off;      // w entries, two buffers by step parity
+  T *pb = wb + 2 * (int64_t)n;       // published pivot rows, likewise
   T *rd = red_all + (int64_t)pt.slot * 2 * kTriMaxParts;
   double *d = d_all + job.lam_off, *e = e_all + job.lam_off;
   T *tau = tau_all + job.lam_off;
   T *vA = (T *)tri_sm, *vB = vA + n, *wA = vB + n, *rb = wA + n;  // rb: the next pivot row
+  T *part = pt.part_off < 0 ? rb + n : wbuf_all + pt.part_off;
+  const int kown = p < n ? (n - p + P - 1) / P : 0;  // own rows p, p + P, ...
+  T *rows = pt.resident ? rb + n + tri_parts(n, P) : A + (int64_t)p * n;
+  const int64_t rld = pt.resident ? tri_ld<T>(n) : (int64_t)P * n;
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
   const int nwarp = nt >> 5;
   unsigned nbar = 0;
-  // first row >= lo owned by this CTA
-  auto first_own = [&](int lo) { return lo + ((p - lo % P) + P) % P; };
 
-  // 1. max-abs and finiteness of the own rows; partials in the w buffer
+  // 1. max-abs and finiteness of the upper triangle of the own rows; partials
+  //    in the w buffer
   double mx = 0.0;
   int nf = 0;
-  for (int i = first_own(0) + P * warp; i < n; i += P * nwarp)
-    for (int c = lane; c < n; c += 32) {
+  for (int k = warp; k < kown; k += nwarp) {
+    const int i = p + k * P;
+    for (int c = i + lane; c < n; c += 32) {
       const T g = A[(int64_t)i * n + c];
       nf |= !sfinite(g);
       mx = fmax(mx, samax(g));
     }
+  }
   for (int o = 16; o > 0; o >>= 1) {
     mx = fmax(mx, __shfl_down_sync(0xffffffffu, mx, o));
     nf |= __shfl_down_sync(0xffffffffu, nf, o);
@@ -741,7 +652,7 @@ __global__ void __launch_bounds__(kTriThreads)
     pw[p] = m;
     pw[P + p] = bad;
   }
-  if (!tri_barrier(sl, ++nbar * P, status)) return;
+  if (!tri_barrier(sl, P, ++nbar * P, status)) return;
   if (warp == 0) {
     double m = 0.0;
     int bad = 0;
@@ -763,103 +674,222 @@ __global__ void __launch_bounds__(kTriThreads)
   }
   if (tid == 0 && p == 0) scale_all[pt.job] = scale;
   const double inv = scale > 0.0 ? 1.0 / scale : 0.0;
-  // 2. lower triangle of the own rows <- scaled conjugate of the upper triangle
-  //    (exactly Hermitian; the upper triangle is not written in this phase)
-  for (int i = first_own(0) + P * warp; i < n; i += P * nwarp) {
-    T *ar = A + (int64_t)i * n;
+  // 2. own rows scaled, their lower parts the conjugate of the upper triangle
+  //    (exactly Hermitian).  In the global matrix the lower parts come first:
+  //    nobody reads them, and the upper ones are overwritten after a barrier.
+  for (int k = warp; k < kown; k += nwarp) {
+    const int i = p + k * P;
+    T *ar = rows + k * rld;
     for (int c = lane; c < i; c += 32) ar[c] = sscale(inv, cj(__ldcg(&A[(int64_t)c * n + i])));
-    if (lane == 0) ar[i] = smake<T>(inv * sre(ar[i]), 0.0);
   }
-  if (!tri_barrier(sl, ++nbar * P, status)) return;
-  // 3. upper triangle of the own rows scaled
-  for (int i = first_own(0) + P * warp; i < n; i += P * nwarp) {
-    T *ar = A + (int64_t)i * n;
-    for (int c = i + 1 + lane; c < n; c += 32) ar[c] = sscale(inv, ar[c]);
+  if (!pt.resident && !tri_barrier(sl, P, ++nbar * P, status)) return;
+  for (int k = warp; k < kown; k += nwarp) {
+    const int i = p + k * P;
+    T *ar = rows + k * rld;
+    for (int c = i + lane; c < n; c += 32) {
+      const T g = sscale(inv, A[(int64_t)i * n + c]);
+      ar[c] = c == i ? smake<T>(sre(g), 0.0) : g;
+    }
   }
-  if (!tri_barrier(sl, ++nbar * P, status)) return;
+  if (n == 1) {
+    if (tid == 0) {
+      d[0] = sre(rows[0]);
+      e[0] = 0.0;
+      tau[0] = smake<T>(0.0, 0.0);
+    }
+    return;
+  }
+  if (p == 0) {  // row 0 for the first reflector
+    __syncthreads();
+    for (int c = tid; c < n; c += nt) pb[n + c] = rows[c];
+  }
+  // (also: the reflectors overwrite rows of A once every CTA has read them)
+  if (!tri_barrier(sl, P, ++nbar * P, status)) return;
 
-  // Own rows i >= lo: optional rank-2 update with (vA, wA) of step j = lo - 2,
-  // then w[i - lo] = t * (row i, columns lo ..) . vn into wbuf, and the CTA's
-  // partial sum of conj(w_i) vn_i into rd.
-  auto rows_pass = [&](int lo, bool upd, const T *vn, T t, T *wout, T *rout) {
-    const int j = lo - 2;
-    T acc = smake<T>(0.0, 0.0);
-    for (int i = first_own(lo) + P * warp; i < n; i += P * nwarp) {
-      T *ar = A + (int64_t)i * n;
-      T s = smake<T>(0.0, 0.0);
-      if (upd) {
-        const T vi = vA[i - j - 1], wi = wA[i - j - 1];
-        for (int c = lo + lane; c < n; c += 32) {
-          const T a = ssub(ar[c], sadd(smul(vi, cj(wA[c - j - 1])), smul(wi, cj(vA[c - j - 1]))));
-          ar[c] = a;
-          s = sadd(s, smul(a, vn[c - lo]));
-        }
-      } else {
-        for (int c = lo + lane; c < n; c += 32) s = sadd(s, smul(ar[c], vn[c - lo]));
+  // Reflector of step j from the pivot row in rb (rb[c - j] = A[j][c]; its
+  // entries rb[2 ..] already squared into x2): v (v_0 = 1) into v[0 .. m), tau
+  // into sh_t.  Same formulas as the single-CTA kernels.
+  auto reflector = [&](int j, double x2, T *v) {
+    for (int o = 16; o > 0; o >>= 1) x2 += __shfl_down_sync(0xffffffffu, x2, o);
+    if (lane == 0) red[warp] = x2;
+    __syncthreads();
+    const int m = n - j - 1;
+    if (warp == 0) {
+      double s = lane < nwarp ? red[lane] : 0.0;
+      for (int o = kTriThreads / 64; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      const T alpha = cj(rb[1]);
+      const bool refl = s > 0.0 || sim(alpha) != 0.0;
+      double beta = sre(alpha);
+      T t = smake<T>(0.0, 0.0), sc = smake<T>(0.0, 0.0);
+      if (refl) {
+        beta = -copysign(sqrt(sabs2(alpha) + s), sre(alpha));
+        t = smake<T>((beta - sre(alpha)) / beta, -sim(alpha) / beta);
+        sc = sinv(smake<T>(sre(alpha) - beta, sim(alpha)));
       }
-      s = warp_sum(s);
       if (lane == 0) {
-        const T wi = smul(t, s);
-        wout[i - lo] = wi;
-        acc = sadd(acc, smul(cj(wi), vn[i - lo]));
+        sh_t = t;
+        sh_sc = sc;
+        if (p == 0) {
+          d[j] = sre(rb[0]);
+          e[j] = beta;
+          tau[j] = t;
+        }
       }
     }
-    // CTA partial, summed over warps in order
     __syncthreads();
-    T *wp = (T *)(tri_sm + 4 * (size_t)n * sizeof(T));  // nwarp scalars
-    if (lane == 0) wp[warp] = acc;
+    const T sc = sh_sc;  // zero without a reflection
+    for (int r = tid; r < m; r += nt)
+      v[r] = r == 0 ? smake<T>(1.0, 0.0) : smul(cj(rb[1 + r]), sc);
     __syncthreads();
-    if (tid == 0) {
+  };
+
+  // Own rows i >= lo: optional rank-2 update with (vA, wA) of step j = lo - 2,
+  // then w[i - lo] = t * (row i, columns lo ..) . vn into wout, and the CTA's
+  // partial sum of conj(w_i) vn_i into rout; row lo goes to prow.  A warp takes
+  // four rows at a time, eight lanes each (three additions reduce the four
+  // sums); the groups left over after full rounds of all warps are cut into Q
+  // interleaved column slices, so that every warp gets the same number of items.
+  auto rows_pass = [&](int lo, bool upd, const T *vn, T t, T *wout, T *rout, T *prow) {
+    constexpr int W = kTriThreads / 32;
+    const int k0 = lo <= p ? 0 : (lo - p + P - 1) / P;
+    const int cnt = kown - k0, g4 = (cnt + 3) >> 2;
+    const int gfull = g4 / W * W, rem = g4 - gfull;
+    int lq = 0;  // log2 Q: the smallest with rem Q a multiple of the warps
+    while (((rem << lq) & (W - 1)) != 0) ++lq;
+    const int Q = 1 << lq, len = n - lo;
+    const T *va = vA + 1, *wa = wA + 1;  // va[c] belongs to column lo + c
+    for (int it = warp; it < gfull + (rem << lq); it += W) {
+      const bool whole = it < gfull;
+      const int g = whole ? it : gfull + ((it - gfull) >> lq);
+      const int q = whole ? 0 : (it - gfull) & (Q - 1), step = whole ? 8 : 8 << lq;
+      const int k = k0 + 4 * g + (lane >> 3), i = p + k * P;
+      const bool ok = k < kown, first = i == lo;
       T s = smake<T>(0.0, 0.0);
-      for (int q = 0; q < nwarp; ++q) s = sadd(s, wp[q]);
-      rout[p] = s;
+      T *ar = rows + (ok ? k : k0) * rld + lo;
+      if (upd) {
+        const T vi = ok ? va[i - lo] : s, wi = ok ? wa[i - lo] : s;
+#pragma unroll 4
+        for (int c = q * 8 + (lane & 7); c < len; c += step) {
+          const T a = rank2(ar[c], vi, cj(wa[c]), wi, cj(va[c]));
+          if (ok) ar[c] = a;
+          if (first) prow[c] = a;
+          s = smadd(s, a, vn[c]);
+        }
+      } else {
+#pragma unroll 4
+        for (int c = q * 8 + (lane & 7); c < len; c += step) {
+          const T a = ar[c];
+          if (first) prow[c] = a;
+          s = smadd(s, a, vn[c]);
+        }
+      }
+      s = oct_sum(s);
+      if ((lane & 7) == 0) {
+        const int r = k - k0;  // rows of sliced groups hold Q sums each
+        part[whole ? r : 4 * gfull + (r - 4 * gfull) * Q + q] = s;
+      }
+    }
+    __syncthreads();
+    T acc = smake<T>(0.0, 0.0);
+    for (int k = tid; k < cnt; k += nt) {
+      const bool whole = k < 4 * gfull;
+      const T *pk = part + (whole ? k : 4 * gfull + (k - 4 * gfull) * Q);
+      T s = pk[0];
+      if (!whole && Q == 8)
+        s = sadd(sadd(sadd(s, pk[1]), sadd(pk[2], pk[3])),
+                 sadd(sadd(pk[4], pk[5]), sadd(pk[6], pk[7])));
+      else if (!whole && Q == 4)
+        s = sadd(sadd(s, pk[1]), sadd(pk[2], pk[3]));
+      else if (!whole && Q == 2)
+        s = sadd(s, pk[1]);
+      const int r = p + (k0 + k) * P - lo;
+      const T w = smul(t, s);
+      wout[r] = w;
+      acc = sadd(acc, smul(cj(w), vn[r]));
+    }
+    if (cnt <= 32) {
+      if (warp == 0) {
+        acc = warp_sum(acc);
+        if (lane == 0) rout[p] = acc;
+      }
+    } else {
+      acc = warp_sum(acc);
+      if (lane == 0) wpart[warp] = acc;
+      __syncthreads();
+      if (tid == 0) {
+        T s = wpart[0];
+        for (int q = 1; q < nwarp; ++q) s = sadd(s, wpart[q]);
+        rout[p] = s;
+      }
     }
   };
 
   // step 0: reflector and products of the own rows
-  for (int c = tid; c < n; c += nt) rb[c] = __ldcg(&A[c]);
-  __syncthreads();
-  T t = tri_reflector(rb, n, 0, vA, red, p == 0, d, e, tau);
-  rows_pass(1, false, vA, t, wb, rd);
+  {
+    double x2 = 0.0;
+    for (int c = tid; c < n; c += nt) {
+      rb[c] = __ldcg(&pb[n + c]);
+      if (c >= 2) x2 += sabs2(rb[c]);
+    }
+    reflector(0, x2, vA);
+  }
+  T t = sh_t;
+  rows_pass(1, false, vA, t, wb, rd, pb);
   for (int j = 0; j + 1 < n; ++j) {
     const int m = n - j - 1, par = j & 1;
-    if (!tri_barrier(sl, ++nbar * P, status)) return;
-    if (j % P == p)  // reflector storage; every CTA has read row j by now
-      for (int c = j + 2 + tid; c < n; c += nt) A[(int64_t)j * n + c] = vA[c - j - 1];
+    if (!tri_barrier(sl, P, ++nbar * P, status)) return;
+    // w's entries, the pivot row and the partial sums, one L2 round trip
+    const T *wj = wb + par * n, *pj = pb + par * n;
+    constexpr int kPer = 4;  // entries per thread held in registers (n <= 1024)
+    T we[kPer], pe[kPer];
+    const T w0raw = __ldcg(&wj[0]);
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+      const int r = tid + q * nt;
+      if (r < m) {
+        we[q] = __ldcg(&wj[r]);
+        pe[q] = __ldcg(&pj[r]);
+      }
+    }
     if (warp == 0) {  // the P partials: lane q holds q and q + 32, tree sum in lane order
       T s = smake<T>(0.0, 0.0);
       if (lane < P) s = __ldcg(&rd[par * kTriMaxParts + lane]);
       if (lane + 32 < P) s = sadd(s, __ldcg(&rd[par * kTriMaxParts + lane + 32]));
       s = warp_sum(s);
-      if (lane == 0) ksum = smul(sscale(-0.5, t), s);  // K = -t (w^H v) / 2
+      if (lane == 0) sh_k = smul(sscale(-0.5, t), s);  // K = -t (w^H v) / 2
     }
+    if (j % P == p)  // reflector storage
+      for (int c = j + 2 + tid; c < n; c += nt) A[(int64_t)j * n + c] = vA[c - j - 1];
     __syncthreads();
-    const T K = ksum;
-    for (int r = tid; r < m; r += nt) wA[r] = sadd(__ldcg(&wb[par * n + r]), smul(K, vA[r]));
-    __syncthreads();
+    const T K = sh_k;
+    const T w0 = sadd(w0raw, K);  // v_0 = 1
+    // w = w + K v; row j + 1 (updated through step j - 1 by its owner) with
+    // step j's update
+    double x2 = 0.0;
+    auto entry = [&](int r, T wr, T ar) {
+      const T v = vA[r];
+      const T w = smadd(wr, K, v);
+      wA[r] = w;
+      const T a = rank2(ar, smake<T>(1.0, 0.0), cj(w), w0, cj(v));
+      rb[r] = a;
+      if (r >= 2) x2 += sabs2(a);
+    };
+#pragma unroll
+    for (int q = 0; q < kPer; ++q)
+      if (tid + q * nt < m) entry(tid + q * nt, we[q], pe[q]);
+    for (int r = tid + kPer * nt; r < m; r += nt) entry(r, __ldcg(&wj[r]), __ldcg(&pj[r]));
     if (j + 2 == n) {  // the trailing block is the last diagonal entry
-      if ((n - 1) % P == p && tid == 0) {
-        T *a = A + (int64_t)(n - 1) * n + (n - 1);
-        const T v0 = vA[0], w0 = wA[0];
-        const T an = ssub(*a, sadd(smul(v0, cj(w0)), smul(w0, cj(v0))));
-        *a = an;
-        d[n - 1] = sre(an);
+      if (p == 0 && tid == 0) {
+        d[n - 1] = sre(rb[0]);
         e[n - 1] = 0.0;
         tau[n - 1] = smake<T>(0.0, 0.0);
       }
       break;
     }
-    // row j + 1 (updated through step j - 1 by its owner) with step j's update
-    {
-      const T *ar = A + (int64_t)(j + 1) * n;
-      const T v0 = vA[0], w0 = wA[0];
-      for (int c = j + 1 + tid; c < n; c += nt)
-        rb[c - j - 1] =
-            ssub(__ldcg(&ar[c]), sadd(smul(v0, cj(wA[c - j - 1])), smul(w0, cj(vA[c - j - 1]))));
-      __syncthreads();
-    }
-    const T tn = tri_reflector(rb, n, j + 1, vB, red, p == 0, d, e, tau);
-    rows_pass(j + 2, true, vB, tn, wb + (par ^ 1) * n, rd + (par ^ 1) * kTriMaxParts);
+    reflector(j + 1, x2, vB);
+    const T tn = sh_t;
+    rows_pass(j + 2, true, vB, tn, wb + (par ^ 1) * n, rd + (par ^ 1) * kTriMaxParts,
+              pb + (par ^ 1) * n);
     T *x = vA;
     vA = vB;
     vB = x;
@@ -867,296 +897,266 @@ __global__ void __launch_bounds__(kTriThreads)
   }
 }
 
-// Complex Hermitian version of tridiag_kernel.  Step j (0 <= j <= n-2)
-// reflects the column x = A[j+1.., j] (read as conj of row j) with
-// H = I - tau v v^H, v_0 = 1, beta real, so that H^H x = beta e_0 and the
-// tridiagonal matrix is real; v (r >= 1) is stored in row j at column j+1+r,
-// tau (complex) in tau[lam_off + j].
-__global__ void tridiag_c_kernel(const EigJob *__restrict__ jobs, double2 *__restrict__ G_all,
-                                 double *__restrict__ d_all, double *__restrict__ e_all,
-                                 double2 *__restrict__ tau_all, double *__restrict__ scale_all,
-                                 int *__restrict__ status) {
-  extern __shared__ double2 smc[];
-  __shared__ double red[33];
-  __shared__ double redi[33];
-  __shared__ int bad;
-  const EigJob job = jobs[blockIdx.x];
-  const int n = job.n;
-  if (n == 0 || !job.smem) return;  // larger matrices: tridiag_mc_kernel
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const int lane = tid & 31, warp = tid >> 5, nwarp = nt >> 5;
-  double2 *A = smc;
-  double2 *v = smc + (int64_t)n * n;
-  double2 *w = v + n;
-  double *d = d_all + job.lam_off, *e = e_all + job.lam_off;
-  double2 *tau = tau_all + job.lam_off;
-
-  for (int64_t x = tid; x < (int64_t)n * n; x += nt) A[x] = G_all[job.g_off + x];
-  double mx = 0.0;
-  int nf = 0;
-  if (tid == 0) bad = 0;
-  for (int64_t x = tid; x < (int64_t)n * n; x += nt) {
-    const double2 g = A[x];
-    nf |= !isfinite(g.x) || !isfinite(g.y);
-    mx = fmax(mx, fmax(fabs(g.x), fabs(g.y)));
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    mx = fmax(mx, __shfl_down_sync(0xffffffffu, mx, o));
-    nf |= __shfl_down_sync(0xffffffffu, nf, o);
-  }
-  __syncthreads();
-  if (lane == 0) {
-    red[warp] = mx;
-    if (nf) atomicOr(&bad, 1);
-  }
-  __syncthreads();
-  if (tid == 0) {
-    double m = 0.0;
-    for (int i = 0; i < nwarp; ++i) m = fmax(m, red[i]);
-    red[32] = m;
-  }
-  __syncthreads();
-  if (bad) {
-    if (tid == 0) atomicExch(status, 2);
-    return;
-  }
-  const double scale = red[32];
-  if (tid == 0) scale_all[blockIdx.x] = scale;
-  // scale and make exactly Hermitian
-  const double inv = scale > 0.0 ? 1.0 / scale : 0.0;
-  for (int64_t x = tid; x < (int64_t)n * n; x += nt) {
-    const int r = (int)(x / n), c = (int)(x - (int64_t)r * n);
-    if (r < c) {
-      const double2 a = A[x], b = A[(int64_t)c * n + r];
-      const double2 g = make_double2(0.5 * inv * (a.x + b.x), 0.5 * inv * (a.y - b.y));
-      A[x] = g;
-      A[(int64_t)c * n + r] = make_double2(g.x, -g.y);
-    } else if (r == c) {
-      A[x] = make_double2(A[x].x * inv, 0.0);
-    }
-  }
-  __syncthreads();
-
-  for (int j = 0; j + 1 < n; ++j) {
-    const int m = n - j - 1;
-    double2 *rowj = A + (int64_t)j * n;
-    const double2 alpha = make_double2(rowj[j + 1].x, -rowj[j + 1].y);  // x_0
-    double x2 = 0.0;
-    for (int c = j + 2 + tid; c < n; c += nt) x2 += rowj[c].x * rowj[c].x + rowj[c].y * rowj[c].y;
-    x2 = block_sum(x2, red);
-    double2 t = make_double2(0.0, 0.0), sc = make_double2(0.0, 0.0);
-    double beta = alpha.x;
-    if (x2 > 0.0 || alpha.y != 0.0) {
-      beta = -copysign(sqrt(alpha.x * alpha.x + alpha.y * alpha.y + x2), alpha.x);
-      t = make_double2((beta - alpha.x) / beta, -alpha.y / beta);
-      const double2 den = make_double2(alpha.x - beta, alpha.y);  // 1 / (alpha - beta)
-      const double dd = den.x * den.x + den.y * den.y;
-      sc = make_double2(den.x / dd, -den.y / dd);
-    }
-    const bool refl = t.x != 0.0 || t.y != 0.0;
-    for (int r = tid; r < m; r += nt) {
-      double2 vr;
-      if (r == 0)
-        vr = make_double2(1.0, 0.0);
-      else if (!refl)
-        vr = make_double2(0.0, 0.0);
-      else
-        vr = cmul(make_double2(rowj[j + 1 + r].x, -rowj[j + 1 + r].y), sc);
-      v[r] = vr;
-      if (r > 0) rowj[j + 1 + r] = vr;
-    }
-    if (tid == 0) {
-      d[j] = rowj[j].x;
-      e[j] = beta;
-      tau[j] = t;
-    }
-    __syncthreads();
-    if (!refl) continue;
-    // w = t * A_t v (one warp per row)
-    for (int r = warp; r < m; r += nwarp) {
-      const double2 *ar = A + (int64_t)(j + 1 + r) * n + (j + 1);
-      double2 acc = make_double2(0.0, 0.0);
-      for (int c = lane; c < m; c += 32) acc = cadd(acc, cmul(ar[c], v[c]));
-      for (int o = 16; o > 0; o >>= 1) {
-        acc.x += __shfl_down_sync(0xffffffffu, acc.x, o);
-        acc.y += __shfl_down_sync(0xffffffffu, acc.y, o);
-      }
-      if (lane == 0) w[r] = cmul(t, acc);
-    }
-    __syncthreads();
-    // K = -1/2 t (w^H v); w += K v
-    double kr = 0.0, ki = 0.0;
-    for (int r = tid; r < m; r += nt) {
-      const double2 q = cmulc(w[r], v[r]);
-      kr += q.x;
-      ki += q.y;
-    }
-    kr = block_sum(kr, red);
-    ki = block_sum(ki, redi);
-    const double2 K = cmul(make_double2(-0.5 * t.x, -0.5 * t.y), make_double2(kr, ki));
-    for (int r = tid; r < m; r += nt) w[r] = cadd(w[r], cmul(K, v[r]));
-    __syncthreads();
-    // A_t -= v w^H + w v^H
-    for (int64_t x = tid; x < (int64_t)m * m; x += nt) {
-      const int r = (int)(x / m), c = (int)(x - (int64_t)r * m);
-      const double2 a = cmul(v[r], make_double2(w[c].x, -w[c].y));
-      const double2 b = cmul(w[r], make_double2(v[c].x, -v[c].y));
-      double2 &g = A[(int64_t)(j + 1 + r) * n + (j + 1 + c)];
-      g = make_double2(g.x - a.x - b.x, g.y - a.y - b.y);
-    }
-    __syncthreads();
-  }
-  if (tid == 0) {
-    d[n - 1] = A[(int64_t)(n - 1) * n + (n - 1)].x;
-    e[n - 1] = 0.0;
-    tau[n - 1] = make_double2(0.0, 0.0);
-  }
-  __syncthreads();
-  for (int64_t x = tid; x < (int64_t)n * n; x += nt) G_all[job.g_off + x] = A[x];
+// One warp per chunk of C columns (two real, one complex), held in shared memory
+// for all reflectors; lanes walk the rows.  One pass applies reflector j and
+// forms the products with reflector j - 1, whose vector was copied to shared
+// memory meanwhile (cp.async), so neither L2 nor a block barrier is waited for.
+// FP64 bound: a warp's FP64 instruction holds its quarter's pipe for 64 clocks,
+// four per row of C columns and five additions per reflector.
+template <typename T>
+struct BackShape;
+template <>
+struct BackShape<double> {
+  static constexpr int kCols = 2;
+};
+template <>
+struct BackShape<double2> {
+  static constexpr int kCols = 1;
+};
+// sum of x over the warp in lanes 0 .. 15, of y in lanes 16 .. 31
+__device__ __forceinline__ double pair_sum(double x, double y) {
+  const bool up = threadIdx.x & 16;
+  double v = (up ? y : x) + __shfl_xor_sync(0xffffffffu, up ? x : y, 16);
+  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+__device__ __forceinline__ void back_weights(const double (&s)[2], double t, double (&w)[2]) {
+  const double v = pair_sum(s[0], s[1]) * t;
+  w[0] = __shfl_sync(0xffffffffu, v, 0);
+  w[1] = __shfl_sync(0xffffffffu, v, 16);
+}
+__device__ __forceinline__ void back_weights(const double2 (&s)[1], double2 t, double2 (&w)[1]) {
+  const double v = pair_sum(s[0].x, s[0].y);
+  w[0] = cmul(t, make_double2(__shfl_sync(0xffffffffu, v, 0), __shfl_sync(0xffffffffu, v, 16)));
 }
 
-// Complex back-transformation: Z <- H_0 H_1 ... H_{n-2} Z, H_j = I - tau_j v_j v_j^H.
-__global__ void backtransform_c_kernel(const EigJob *__restrict__ jobs,
-                                       const BackChunk *__restrict__ bt,
-                                       const double2 *__restrict__ G_all,
-                                       const double2 *__restrict__ tau_all,
-                                       double2 *__restrict__ Z) {
-  extern __shared__ double2 smc[];
-  __shared__ double2 part[8][33];
+template <typename T>
+__global__ void __launch_bounds__(32)
+    backtransform_kernel(const EigJob *__restrict__ jobs, const BackChunk *__restrict__ bt,
+                         const T *__restrict__ G_all, const T *__restrict__ tau_all,
+                         T *__restrict__ Z) {
+  constexpr int C = BackShape<T>::kCols;
+  extern __shared__ __align__(16) unsigned char back_sm[];
   const BackChunk ch = bt[blockIdx.x];
   const EigJob job = jobs[ch.job];
-  const int n = job.n;
+  const int n = job.n, lane = threadIdx.x;
   if (n < 2 || ch.cw == 0) return;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  double2 *z = Z + ch.z_off + ch.c0;
-  double2 *v = smc;
-  const double2 *A = G_all + job.g_off;
-  const bool col = tx < ch.cw;
+  // C columns of n, then the reflectors of two consecutive steps (entry r of
+  // row j's vector at index j + 1 + r)
+  T *zs = (T *)back_sm, *vb = zs + C * n;
+  T *z = Z + ch.z_off + ch.c0;
+  const T *A = G_all + job.g_off;
+  const T *tau = tau_all + job.lam_off;
+  auto fetch = [&](int j) {  // the vector of step j
+    T *dst = vb + (j & 1) * n;
+    const T *src = A + (int64_t)j * n;
+    if (lane == 0) dst[j + 1] = smake<T>(1.0, 0.0);
+    for (int c = j + 2 + lane; c < n; c += 32)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
+                       (uint32_t)__cvta_generic_to_shared(dst + c)),
+                   "l"(src + c), "n"(sizeof(T))
+                   : "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int r = lane; r < n; r += 32)
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+      zs[c * n + r] = c < ch.cw ? z[(int64_t)r * ch.ld + c] : smake<T>(0.0, 0.0);
+  fetch(n - 2);
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncwarp();
+  // products with the first reflector: rows n - 1 only
+  T s[C];
+#pragma unroll
+  for (int c = 0; c < C; ++c)
+    s[c] = lane == 0 ? smul(cj(vb[((n - 2) & 1) * n + n - 1]), zs[c * n + n - 1])
+                     : smake<T>(0.0, 0.0);
+  T t = tau[n - 2];
   for (int j = n - 2; j >= 0; --j) {
-    const double2 t = tau_all[job.lam_off + j];
-    if (t.x == 0.0 && t.y == 0.0) continue;
-    const int m = n - j - 1;
-    for (int r = threadIdx.x; r < m; r += blockDim.x)
-      v[r] = r == 0 ? make_double2(1.0, 0.0) : A[(int64_t)j * n + j + 1 + r];
-    __syncthreads();
-    double2 s = make_double2(0.0, 0.0);
-    if (col)
-      for (int r = ty; r < m; r += 8) s = cadd(s, cmulc(v[r], z[(int64_t)(j + 1 + r) * ch.ld + tx]));
-    part[ty][tx] = s;
-    __syncthreads();
-    double2 w = make_double2(0.0, 0.0);
-    for (int g = 0; g < 8; ++g) w = cadd(w, part[g][tx]);
-    w = cmul(t, w);
-    if (col)
-      for (int r = ty; r < m; r += 8) {
-        double2 &zz = z[(int64_t)(j + 1 + r) * ch.ld + tx];
-        const double2 q = cmul(v[r], w);
-        zz = make_double2(zz.x - q.x, zz.y - q.y);
+    const T *v = vb + (j & 1) * n, *vn = vb + ((j + 1) & 1) * n;  // vn: step j - 1
+    if (j > 0) fetch(j - 1);
+    const T tn = j > 0 ? tau[j - 1] : t;
+    T w[C];
+    back_weights(s, t, w);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+      s[c] = lane == 0 && j > 0 ? zs[c * n + j] : smake<T>(0.0, 0.0);
+#pragma unroll 4
+    for (int r = j + 1 + lane; r < n; r += 32) {
+      const T x = v[r], y = j > 0 ? cj(vn[r]) : smake<T>(0.0, 0.0);
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        const T a = smsub(zs[c * n + r], x, w[c]);
+        zs[c * n + r] = a;
+        s[c] = smadd(s[c], y, a);
       }
-    __syncthreads();
+    }
+    __syncwarp();
+    t = tn;
   }
+  for (int r = lane; r < n; r += 32)
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+      if (c < ch.cw) z[(int64_t)r * ch.ld + c] = zs[c * n + r];
 }
 
 }  // namespace
 
-constexpr size_t kTriSmemBytes = 200 * 1024;
+// Shared memory a CTA of the reduction may use, and the matrices that leave
+// room for a second CTA on the SM.
+constexpr size_t kTriSmemBytes = 226 * 1024;
+constexpr size_t kTriSmallBytes = 110 * 1024;
+// Time model of the reduction: 5.5 us per step, and n^3 FMAs (four per complex
+// one) at 3e9 per second and CTA (80% of its FP64 pipe).
+constexpr double kTriStep = 5.5e-6, kTriRate = 3e9;
 
-// Reduces the jobs without shared-memory residence with tridiag_mc_kernel.
-// The SMs are shared out in proportion to n^3 (the flop count), at most
-// kTriMaxParts and n / 8 CTAs per matrix; jobs that do not fit one
-// cooperative launch go to the next.
 template <typename T>
-void tridiag_multi_cta(Ctx &ctx, DeviceScratch &scratch, const std::vector<EigJob> &jobs,
-                       const SymEigWork &wk, double *G, int *dstat) {
-  std::vector<int> big;
-  double work = 0.0;
-  int nmax = 0;
-  for (int q = 0; q < (int)jobs.size(); ++q)
-    if (!jobs[q].smem && jobs[q].n > 0) {
-      big.push_back(q);
-      work += std::pow((double)jobs[q].n, 3);
-      nmax = std::max(nmax, jobs[q].n);
-    }
-  if (big.empty()) return;
-  std::sort(big.begin(), big.end(), [&](int a, int b) { return jobs[a].n > jobs[b].n; });
-  const void *kern = (const void *)tridiag_mc_kernel<T>;
-  const size_t msmem = (4 * (size_t)nmax + kTriThreads / 32) * sizeof(T);
-  UDMRG_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)msmem));
-  int per_sm = 0;
-  UDMRG_CHECK_CUDA(
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTriThreads, msmem));
-  const int budget = std::min(ctx.num_sms, per_sm * ctx.num_sms);
-  UDMRG_REQUIRE(budget >= 1, "eigensolver: the reduction kernel does not fit an SM");
-  size_t at = 0;
-  while (at < big.size()) {
-    std::vector<TriPart> parts;
-    int64_t wb_tot = 0;
-    int slot = 0;
-    for (; at < big.size(); ++at) {
-      const int q = big[at], n = jobs[q].n;
-      const double share = std::pow((double)n, 3) / work;
-      int P = std::max(1, (int)(budget * share));
-      P = std::min({P, kTriMaxParts, std::max(1, n / 8)});
-      if (!parts.empty() && (int)parts.size() + P > budget) break;
-      P = std::min(P, budget);
-      for (int p = 0; p < P; ++p) parts.push_back(TriPart{q, p, P, slot, wb_tot});
-      wb_tot += 2 * (int64_t)n;
-      ++slot;
-    }
-    TriPart *dparts = scratch.get<TriPart>(parts.size());
-    TriSlot *dslots = scratch.get<TriSlot>(slot);
-    T *dwb = scratch.get<T>(wb_tot);
-    T *dred = scratch.get<T>((int64_t)slot * 2 * kTriMaxParts);
-    UDMRG_CHECK_CUDA(cudaMemcpyAsync(dparts, parts.data(), parts.size() * sizeof(TriPart),
-                                     cudaMemcpyHostToDevice, ctx.stream));
-    UDMRG_CHECK_CUDA(cudaMemsetAsync(dslots, 0, slot * sizeof(TriSlot), ctx.stream));
-    const EigJob *djobs = wk.jobs;
-    T *g = (T *)G, *tau = (T *)wk.tau;
-    double *d = wk.d, *e = wk.e, *sc = wk.scale;
-    void *args[] = {&djobs, &dparts, &g, &d, &e, &tau, &sc, &dslots, &dwb, &dred, &dstat};
-    UDMRG_CHECK_CUDA(cudaLaunchCooperativeKernel(kern, dim3((unsigned)parts.size()),
-                                                 dim3(kTriThreads), args, msmem, ctx.stream));
-    ctx.launches++;
-    ctx.sync();  // `parts` must outlive the upload
-  }
+static size_t tri_smem(int n, int P) {  // with the own rows resident
+  return (4 * (size_t)n + tri_parts(n, P) + (size_t)((n + P - 1) / P) * tri_ld<T>(n)) * sizeof(T);
 }
 
-// Lower triangle of each job's matrix from its upper one: G[i][j] = conj(G[j][i]).
-// One block per job walks the 32 x 32 tiles on and below the diagonal; each
-// tile is read transposed from the upper triangle through shared memory, so
-// both the reads and the writes are coalesced rows.
+// Householder reduction of every job.  Matrices of which two fit one SM's
+// shared memory run on one CTA each, on the side stream; the larger ones run in
+// one cooperative launch (more if they do not fit), the SMs shared out so that
+// all are expected to end together.
 template <typename T>
-__global__ void __launch_bounds__(256)
-    sym_mirror_kernel(const EigJob *__restrict__ jobs, T *__restrict__ G) {
-  __shared__ T tile[32][33];
-  const EigJob job = jobs[blockIdx.x];
-  const int n = job.n;
-  const int nt = (n + 31) / 32;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
-  T *A = G + job.g_off;
-  for (int t = 0; t < nt * (nt + 1) / 2; ++t) {
-    // tile (bi, bj) with bi >= bj: row block bi of the lower triangle
-    int bi = 0;
-    while ((bi + 1) * (bi + 2) / 2 <= t) ++bi;
-    const int bj = t - bi * (bi + 1) / 2;
-    // source: rows bj*32.., columns bi*32.. (upper triangle)
-    for (int r = ty; r < 32; r += 8) {
-      const int i = bj * 32 + r, j = bi * 32 + tx;
-      if (i < n && j < n) tile[r][tx] = A[(int64_t)i * n + j];
-    }
-    __syncthreads();
-    for (int r = ty; r < 32; r += 8) {
-      const int i = bi * 32 + r, j = bj * 32 + tx;  // destination (i, j), i > j
-      if (i < n && j < n && i > j) A[(int64_t)i * n + j] = cj(tile[tx][r]);
-    }
-    __syncthreads();
+static void tridiag_all(Ctx &ctx, DeviceScratch &scratch, const std::vector<EigJob> &jobs,
+                        const SymEigWork &wk, double *G, int *dstat) {
+  std::vector<int> big, small;
+  for (int q = 0; q < (int)jobs.size(); ++q) {
+    if (jobs[q].n == 0) continue;
+    (tri_smem<T>(jobs[q].n, 1) <= kTriSmallBytes ? small : big).push_back(q);
   }
+  auto larger = [&](int x, int y) { return jobs[x].n > jobs[y].n; };
+  std::stable_sort(big.begin(), big.end(), larger);
+  std::stable_sort(small.begin(), small.end(), larger);
+  const void *kern = (const void *)tridiag_mc_kernel<T>;
+  size_t max_smem = kTriSmemBytes;
+  if (!big.empty()) max_smem = std::max(max_smem, 4 * (size_t)jobs[big[0]].n * sizeof(T));
+  UDMRG_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)max_smem));
+  const int reserve = std::min((int)(small.size() + 1) / 2, ctx.num_sms / 6);
+  const int budget = ctx.num_sms - (big.empty() ? 0 : reserve);
+  // the parts of every launch, their slots and buffers in one upload
+  std::vector<TriPart> parts;
+  struct Launch {
+    size_t part0, nparts, smem;
+    bool coop;
+  };
+  std::vector<Launch> launches;
+  int64_t wb_tot = 0;
+  int slot = 0;
+  // returns the shared memory of the job's CTAs
+  auto add = [&](int q, int P) {
+    const int n = jobs[q].n;
+    const bool resident = tri_smem<T>(n, P) <= kTriSmemBytes;
+    const int64_t np = tri_parts(n, P), wb = wb_tot;
+    wb_tot += 4 * (int64_t)n;
+    size_t bytes = tri_smem<T>(n, P);
+    if (!resident) bytes = (4 * (size_t)n + np) * sizeof(T);
+    const bool gpart = bytes > kTriSmemBytes;
+    if (gpart) bytes = 4 * (size_t)n * sizeof(T);
+    for (int p = 0; p < P; ++p) {
+      parts.push_back(TriPart{q, p, P, slot, wb, gpart ? wb_tot : -1, resident ? 1 : 0, 0});
+      if (gpart) wb_tot += np;
+    }
+    ++slot;
+    return bytes;
+  };
+  const double rate = kTriRate / (sizeof(T) / sizeof(double) == 2 ? 4.0 : 1.0);
+  for (size_t at = 0; at < big.size();) {
+    // as many matrices as fit with the fewest CTAs that keep their rows resident
+    std::vector<int> pmin, cap;
+    size_t end = at;
+    int sum = 0;
+    for (; end < big.size(); ++end) {
+      const int n = jobs[big[end]].n;
+      const int c = std::min({kTriMaxParts, std::max(1, n / 8), budget});
+      int P = 1;
+      while (P < c && tri_smem<T>(n, P) > kTriSmemBytes) ++P;
+      if (end > at && sum + P > budget) break;
+      sum += P;
+      pmin.push_back(P);
+      cap.push_back(c);
+    }
+    auto share = [&](double t, size_t i) {
+      const double n = jobs[big[at + i]].n, left = t - n * kTriStep;
+      const double P = left > 0 ? std::ceil(n * n * n / rate / left) : 1e9;
+      return (int)std::min<double>(cap[i], std::max<double>(pmin[i], P));
+    };
+    double lo = 0.0, hi = 10.0;  // seconds
+    for (int it = 0; it < 60; ++it) {
+      const double t = 0.5 * (lo + hi);
+      int s = 0;
+      for (size_t i = 0; i < pmin.size(); ++i) s += share(t, i);
+      (s <= budget ? hi : lo) = t;
+    }
+    Launch L{parts.size(), 0, 0, true};
+    for (size_t i = 0; i < pmin.size(); ++i) {
+      L.smem = std::max(L.smem, add(big[at + i], share(hi, i)));
+    }
+    L.nparts = parts.size() - L.part0;
+    launches.push_back(L);
+    at = end;
+  }
+  if (!small.empty()) {
+    Launch L{parts.size(), small.size(), 0, false};
+    for (int q : small) L.smem = std::max(L.smem, add(q, 1));
+    launches.push_back(L);
+  }
+  if (parts.empty()) return;
+  TriPart *dparts = scratch.get<TriPart>(parts.size());
+  TriSlot *dslots = scratch.get<TriSlot>(slot);
+  T *dwb = scratch.get<T>(wb_tot);
+  T *dred = scratch.get<T>((int64_t)slot * 2 * kTriMaxParts);
+  UDMRG_CHECK_CUDA(cudaMemcpyAsync(dparts, parts.data(), parts.size() * sizeof(TriPart),
+                                   cudaMemcpyHostToDevice, ctx.stream));
+  UDMRG_CHECK_CUDA(cudaMemsetAsync(dslots, 0, slot * sizeof(TriSlot), ctx.stream));
+  // the side stream starts after the uploads and the Gram products, and the
+  // main stream goes on after it
+  struct Events {
+    cudaEvent_t a = nullptr, b = nullptr;
+    ~Events() {
+      if (a) cudaEventDestroy(a);
+      if (b) cudaEventDestroy(b);
+    }
+  } ev;
+  const bool side = launches.size() > 1 && !launches.back().coop;
+  if (side) {
+    UDMRG_CHECK_CUDA(cudaEventCreateWithFlags(&ev.a, cudaEventDisableTiming));
+    UDMRG_CHECK_CUDA(cudaEventCreateWithFlags(&ev.b, cudaEventDisableTiming));
+    UDMRG_CHECK_CUDA(cudaEventRecord(ev.a, ctx.stream));
+  }
+  const EigJob *djobs = wk.jobs;
+  T *g = (T *)G, *tau = (T *)wk.tau;
+  double *d = wk.d, *e = wk.e, *sc = wk.scale;
+  auto launch = [&](const Launch &L, cudaStream_t st) {
+    const TriPart *dp = dparts + L.part0;
+    void *args[] = {&djobs, &dp, &g, &d, &e, &tau, &sc, &dslots, &dwb, &dred, &dstat};
+    if (L.coop)
+      UDMRG_CHECK_CUDA(cudaLaunchCooperativeKernel(kern, dim3((unsigned)L.nparts),
+                                                   dim3(kTriThreads), args, L.smem, st));
+    else
+      UDMRG_CHECK_CUDA(
+          cudaLaunchKernel(kern, dim3((unsigned)L.nparts), dim3(kTriThreads), args, L.smem, st));
+    ctx.launches++;
+  };
+  launch(launches[0], ctx.stream);
+  if (side) {
+    UDMRG_CHECK_CUDA(cudaStreamWaitEvent(ctx.side, ev.a, 0));
+    launch(launches.back(), ctx.side);
+    UDMRG_CHECK_CUDA(cudaEventRecord(ev.b, ctx.side));
+  }
+  for (size_t i = 1; i + (side ? 1 : 0) < launches.size(); ++i) launch(launches[i], ctx.stream);
+  if (side) UDMRG_CHECK_CUDA(cudaStreamWaitEvent(ctx.stream, ev.b, 0));
+  ctx.sync();  // `parts` must outlive the upload
 }
 
 int sym_eig_values(Ctx &ctx, DeviceScratch &scratch, std::vector<EigJob> &jobs, double *G,
                    double *lam, SymEigWork &wk, bool cplx, int64_t need, int64_t floor,
-                   const std::vector<int64_t> *rank_cap, bool mirror) {
+                   const std::vector<int64_t> *rank_cap) {
   const int nj = (int)jobs.size();
   if (nj == 0) return 0;
   int64_t ltot = 0;
@@ -1171,44 +1171,15 @@ int sym_eig_values(Ctx &ctx, DeviceScratch &scratch, std::vector<EigJob> &jobs, 
   wk.tau = scratch.get<double>((cplx ? 2 : 1) * std::max<int64_t>(ltot, 1));
   wk.scale = scratch.get<double>(nj);
   wk.cplx = cplx;
-  const size_t es = (cplx ? 2 : 1) * sizeof(double);
-  size_t smem = 0;
-  for (auto &j : jobs) {
-    const size_t base = 2 * (size_t)j.n * es;
-    const size_t full = base + (size_t)j.n * j.n * es;
-    j.smem = full <= kTriSmemBytes ? 1 : 0;
-    if (j.smem) smem = std::max(smem, full);
-  }
-  UDMRG_CHECK_CUDA(cudaFuncSetAttribute(tridiag_kernel,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)kTriSmemBytes));
-  UDMRG_CHECK_CUDA(cudaFuncSetAttribute(tridiag_c_kernel,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)kTriSmemBytes));
   wk.jobs = scratch.get<EigJob>(nj);
   int *dstat = scratch.get<int>(1);
   UDMRG_CHECK_CUDA(cudaMemsetAsync(dstat, 0, sizeof(int), ctx.stream));
   UDMRG_CHECK_CUDA(cudaMemcpyAsync(wk.jobs, jobs.data(), nj * sizeof(EigJob),
                                    cudaMemcpyHostToDevice, ctx.stream));
-  if (mirror) {
-    if (cplx)
-      sym_mirror_kernel<double2><<<nj, 256, 0, ctx.stream>>>(wk.jobs, (double2 *)G);
-    else
-      sym_mirror_kernel<double><<<nj, 256, 0, ctx.stream>>>(wk.jobs, G);
-    UDMRG_CHECK_CUDA(cudaGetLastError());
-    ctx.launches++;
-  }
   if (cplx)
-    tridiag_c_kernel<<<nj, kTriThreads, smem, ctx.stream>>>(
-        wk.jobs, (double2 *)G, wk.d, wk.e, (double2 *)wk.tau, wk.scale, dstat);
+    tridiag_all<double2>(ctx, scratch, jobs, wk, G, dstat);
   else
-    tridiag_kernel<<<nj, kTriThreads, smem, ctx.stream>>>(wk.jobs, G, wk.d, wk.e, wk.tau,
-                                                          wk.scale, dstat);
-  UDMRG_CHECK_CUDA(cudaGetLastError());
-  if (cplx)
-    tridiag_multi_cta<double2>(ctx, scratch, jobs, wk, G, dstat);
-  else
-    tridiag_multi_cta<double>(ctx, scratch, jobs, wk, G, dstat);
+    tridiag_all<double>(ctx, scratch, jobs, wk, G, dstat);
   const size_t bsmem = 2 * (size_t)nmax * sizeof(double);
   if (bsmem > 48 * 1024) {
     UDMRG_CHECK_CUDA(cudaFuncSetAttribute(bisect_kernel,
@@ -1332,7 +1303,7 @@ void sym_eig_vectors(Ctx &ctx, DeviceScratch &scratch, const std::vector<EigJob>
     double *work = scratch.get<double>(6 * (int64_t)nmax * ncl);
     UDMRG_CHECK_CUDA(cudaMemcpyAsync(dcl, cl.data(), ncl * sizeof(EigCluster),
                                      cudaMemcpyHostToDevice, ctx.stream));
-    invit_kernel<<<(ncl + 63) / 64, 64, 0, ctx.stream>>>(dcl, ncl, wk.jobs, wk.d, wk.e, wk.scale,
+    invit_kernel<<<(ncl + 31) / 32, 32, 0, ctx.stream>>>(dcl, ncl, wk.jobs, wk.d, wk.e, wk.scale,
                                                         lam, Z, work, nmax);
     UDMRG_CHECK_CUDA(cudaGetLastError());
     ctx.launches++;
@@ -1350,31 +1321,27 @@ void sym_eig_vectors(Ctx &ctx, DeviceScratch &scratch, const std::vector<EigJob>
     if (stot > 0) {
       DeviceScratch ns(ctx);
       double *S = ns.get<double>(stot), *Zc = ns.get<double>(ztot);
-      GemmPlan gs, gz, gc;
-      gs.ctx = gz.ctx = gc.ctx = &ctx;
-      gz.may_slice = false;  // accumulates into Zc
+      GemmPlan gs, gz;
+      gs.ctx = gz.ctx = &ctx;
       for (int q = 0; q < nj; ++q) {
         if (k[q] == 0) continue;
         const int64_t n = jobs[q].n, kk = k[q];
         // S = Z^T Z (k x k): A = Z^T (ms 1, ks ld), B = Z (ks ld, ns 1)
         gemm_add_simple(gs, soff[q], kk, kk, n, z_off[q], 1, z_ld[q], z_off[q], z_ld[q], 1, false);
-        // Zc = Z S (n x k, packed): accumulated as Zc = -0.5 Z S + 1.5 Zc
+        // Zc = Z S (n x k, packed)
         gemm_add_simple(gz, zc_off[q], n, kk, kk, z_off[q], z_ld[q], 1, soff[q], kk, 1, false);
       }
       gemm_finalize(gs);
       gemm_finalize(gz);
-      std::vector<Copy2D> to_c, from_c;
-      for (int q = 0; q < nj; ++q) {
-        if (k[q] == 0) continue;
-        to_c.push_back(Copy2D{z_off[q], zc_off[q], jobs[q].n, (int32_t)k[q], z_ld[q], 1, k[q], 1});
-        from_c.push_back(
-            Copy2D{zc_off[q], z_off[q], jobs[q].n, (int32_t)k[q], k[q], 1, z_ld[q], 1});
-      }
+      std::vector<Copy2D> upd;  // Z = 1.5 Z - 0.5 Zc
+      for (int q = 0; q < nj; ++q)
+        if (k[q] > 0)
+          upd.push_back(
+              Copy2D{zc_off[q], z_off[q], jobs[q].n, (int32_t)k[q], k[q], 1, z_ld[q], 1});
       for (int it = 0; it < 2; ++it) {
         (ctx.svd_dw ? run_gemm_dw : run_gemm)(ctx, gs, kF64, Z, Z, S, 1.0, 0.0);
-        run_copy2d(ctx, to_c, Z, Zc, false);
-        (ctx.svd_dw ? run_gemm_dw : run_gemm)(ctx, gz, kF64, Z, S, Zc, -0.5, 1.5);
-        run_copy2d(ctx, from_c, Zc, Z, false);
+        (ctx.svd_dw ? run_gemm_dw : run_gemm)(ctx, gz, kF64, Z, S, Zc, 1.0, 0.0);
+        run_axpby2d(ctx, upd, Zc, Z, 1.5, -0.5);
       }
     }
   }
@@ -1388,13 +1355,15 @@ void sym_eig_vectors(Ctx &ctx, DeviceScratch &scratch, const std::vector<EigJob>
                              z_ld_out[q], 1});
     run_copy2d(ctx, ops, Zc, Zout, true);
   }
-  // back-transformation by the reflectors: complex data 32 columns per block,
-  // real data kBackCols columns per block (the chunk in shared memory)
+  // back-transformation by the reflectors, the largest matrices first
   {
-    const int narrow = nmax * 8 * (int)sizeof(double) <= 218 * 1024 ? 8 : 4;
-    const int width = wk.cplx ? 32 : narrow;
+    const int width = wk.cplx ? BackShape<double2>::kCols : BackShape<double>::kCols;
+    std::vector<int> order(nj);
+    for (int q = 0; q < nj; ++q) order[q] = q;
+    std::stable_sort(order.begin(), order.end(),
+                     [&](int x, int y) { return jobs[x].n > jobs[y].n; });
     std::vector<BackChunk> bt;
-    for (int q = 0; q < nj; ++q)
+    for (int q : order)
       for (int64_t c0 = 0; c0 < k[q]; c0 += width)
         bt.push_back(BackChunk{z_off_out[q], z_ld_out[q], q, (int32_t)c0,
                                (int32_t)std::min<int64_t>(width, k[q] - c0), 0});
@@ -1402,29 +1371,21 @@ void sym_eig_vectors(Ctx &ctx, DeviceScratch &scratch, const std::vector<EigJob>
       BackChunk *dbt = scratch.get<BackChunk>(bt.size());
       UDMRG_CHECK_CUDA(cudaMemcpyAsync(dbt, bt.data(), bt.size() * sizeof(BackChunk),
                                        cudaMemcpyHostToDevice, ctx.stream));
-      const size_t smem = wk.cplx ? (size_t)nmax * 2 * sizeof(double)
-                                  : (size_t)nmax * narrow * sizeof(double);
+      const size_t smem = wk.cplx
+                              ? (size_t)nmax * (BackShape<double2>::kCols + 2) * sizeof(double2)
+                              : (size_t)nmax * (BackShape<double>::kCols + 2) * sizeof(double);
       UDMRG_REQUIRE(smem <= 227 * 1024, "back transformation: matrix too large");
-      if (smem > 48 * 1024) {
-        UDMRG_CHECK_CUDA(cudaFuncSetAttribute(backtransform_narrow_kernel<8>,
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
+      const void *kern = wk.cplx ? (const void *)backtransform_kernel<double2>
+                                 : (const void *)backtransform_kernel<double>;
+      if (smem > 48 * 1024)
+        UDMRG_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               (int)smem));
-        UDMRG_CHECK_CUDA(cudaFuncSetAttribute(backtransform_narrow_kernel<4>,
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)smem));
-        UDMRG_CHECK_CUDA(cudaFuncSetAttribute(backtransform_c_kernel,
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)smem));
-      }
       if (wk.cplx)
-        backtransform_c_kernel<<<(int)bt.size(), kBackThreads, smem, ctx.stream>>>(
+        backtransform_kernel<double2><<<(int)bt.size(), 32, smem, ctx.stream>>>(
             wk.jobs, dbt, (const double2 *)G, (const double2 *)wk.tau, (double2 *)Zout);
-      else if (narrow == 8)
-        backtransform_narrow_kernel<8><<<(int)bt.size(), kBackThreads, smem, ctx.stream>>>(
-            wk.jobs, dbt, G, wk.tau, Zout);
       else
-        backtransform_narrow_kernel<4><<<(int)bt.size(), kBackThreads, smem, ctx.stream>>>(
-            wk.jobs, dbt, G, wk.tau, Zout);
+        backtransform_kernel<double><<<(int)bt.size(), 32, smem, ctx.stream>>>(wk.jobs, dbt, G,
+                                                                              wk.tau, Zout);
       UDMRG_CHECK_CUDA(cudaGetLastError());
       ctx.launches++;
     }

@@ -419,7 +419,7 @@ SvdResult svd_trunc(Ctx &ctx, const BTensor &T, int ldims, const QN &ldiv, doubl
       gemm_add_simple(g, jobs[q].g_off, x.xr, x.xr, x.xc, x.off, x.sr, x.sc, x.off, x.sc, x.sr,
                       cplx);
     }
-    gemm_finalize(g, cplx, true);  // the eigensolver mirrors the upper triangle
+    gemm_finalize(g, cplx, true);  // the eigensolver reads the upper triangles
     run_gemm(ctx, g, cplx ? kC128 : kF64, Mbuf, Mc, G, 1.0, 0.0);
   }
   // at most Dmax states are kept: only the leading eigenvalues of the sectors
@@ -430,7 +430,7 @@ SvdResult svd_trunc(Ctx &ctx, const BTensor &T, int ldims, const QN &ldiv, doubl
   for (int q = 0; q < nsec; ++q) rank_cap[q] = std::min(secs[q].rows, secs[q].cols);
   check_eig_status(sym_eig_values(ctx, scratch, jobs, G, lam, wk, cplx,
                                   Dmax > 0 ? std::max(Dmax, Dmin) + 64 : 0,
-                                  spectrum_floor, &rank_cap, true));
+                                  spectrum_floor, &rank_cap));
   const std::vector<double> hlam = download_vec(ctx, lam, ltot);
   std::vector<std::vector<double>> sv(nsec);
   double rest = 0.0;

@@ -15,8 +15,7 @@ struct Copy2D {
 struct EigJob {
   int64_t g_off;    // offset of the n x n matrix in the G / V / W buffers
   int64_t lam_off;  // offset of the n eigenvalues
-  int32_t n;
-  int32_t smem;     // set by sym_eig_values (matrix held in shared memory)
+  int32_t n, pad;
 };
 
 // Batched symmetric eigen-solver (Householder tridiagonalisation, bisection,
@@ -45,6 +44,9 @@ struct ScaleJob {
 
 void run_copy2d(Ctx &ctx, const std::vector<Copy2D> &ops, const double *src, double *dst,
                 bool cplx);
+// dst = fd dst + fs src over the ops (real data, fs != 0)
+void run_axpby2d(Ctx &ctx, const std::vector<Copy2D> &ops, const double *src, double *dst,
+                 double fd, double fs);
 void run_scale(Ctx &ctx, const std::vector<ScaleJob> &jobs, double *X, const double *f, bool cplx);
 
 // Kept-state selection over all bond sectors (the rule of the oracle):
@@ -54,7 +56,7 @@ void run_scale(Ctx &ctx, const std::vector<ScaleJob> &jobs, double *X, const dou
 // Phase 1: reduce every job's symmetric n x n matrix in G to tridiagonal form
 // (G keeps the reflectors) and put its eigenvalues, descending, at
 // lam[lam_off ...].  Returns 0, 2 for non-finite input, 3 if the multi-CTA
-// reduction timed out.  jobs[].smem is set.  With cplx, G holds complex
+// reduction timed out.  Only the upper triangles are read.  With cplx, G holds complex
 // Hermitian matrices (offsets in complex elements) and phase 2 returns
 // complex eigenvectors.
 // need > 0 (positive semi-definite matrices, e.g. Gram matrices): only the
@@ -64,12 +66,9 @@ void run_scale(Ctx &ctx, const std::vector<ScaleJob> &jobs, double *X, const dou
 // trace, so the weight of the rest is known exactly.  rank_cap (optional, one
 // per job): the caller uses at most that many of the job's eigenvalues (a Gram
 // matrix of rank min(rows, cols)), so no more of them count towards `need`.
-// mirror: only the upper triangles of the matrices hold data; the lower ones
-// are filled from them first (conjugated for complex data).
 int sym_eig_values(Ctx &ctx, DeviceScratch &scratch, std::vector<EigJob> &jobs, double *G,
                    double *lam, SymEigWork &wk, bool cplx = false, int64_t need = 0,
-                   int64_t floor = 0, const std::vector<int64_t> *rank_cap = nullptr,
-                   bool mirror = false);
+                   int64_t floor = 0, const std::vector<int64_t> *rank_cap = nullptr);
 // Phase 2: the leading k[q] eigenvectors of job q (hlam: host copy of lam) as
 // the columns of Z (row-major n x k[q], leading dimension z_ld[q], at z_off[q]),
 // orthonormal to FP64 accuracy.
@@ -77,7 +76,7 @@ void sym_eig_vectors(Ctx &ctx, DeviceScratch &scratch, const std::vector<EigJob>
                      const double *G, const double *lam, const std::vector<double> &hlam,
                      const std::vector<int64_t> &k, const std::vector<int64_t> &z_off,
                      const std::vector<int64_t> &z_ld, double *Z, const SymEigWork &wk,
-                     uint64_t seed = 0x5EED5EEDull);
+                     uint64_t seed = 1);
 
 void select_kept(const std::vector<std::vector<double>> &svals, double trunc_err, int64_t Dmin,
                  int64_t Dmax, std::vector<int64_t> &kept, int64_t &D, double &err,
