@@ -41,7 +41,10 @@ __global__ void __launch_bounds__(32 * kMpoWarps, 2)
   tc::pdl_wait();  // T1 from the L.psi GEMM
   for (int t = blockIdx.x * kMpoWarps + warp; t < ntasks; t += gridDim.x * kMpoWarps) {
     const MpoTask tk = tasks[t];
-    const MpoPair pr = pairs[tk.pair];
+    MpoPair pr = pairs[tk.pair];
+    pr.out0 += tk.o0;  // the task's output channels
+    pr.row0 += tk.o0;
+    pr.nout = tk.nout;
     const int nch = pr.dbp >> 3;
     const int u = tk.u0 + lane;
     const bool valid = u < pr.da * nch;

@@ -466,20 +466,52 @@ std::unique_ptr<SgMatvecPlan> plan_sg_tables(const BTensor &L, const BTensor &R,
         p->tgtref[gm.tgt0 + ((int64_t)gm.nrb + lc.i) * gm.nkb + lc.j] = {
             p->pairs[nreal + q].row0 + tgt_out[t], p->targets[t].dw2};
     }
-    // warp tasks: 32 units (a', 8-wide chunk of b) each, the pairs with the
-    // most work per unit (nonzeros and output channels) first
-    std::vector<int> order(p->pairs.size());
-    for (size_t q = 0; q < order.size(); ++q) order[q] = (int)q;
-    auto cost = [&](int q) {
-      const MpoPair &pr = p->pairs[q];
-      return 2 * (p->rowptr[pr.row0 + pr.nout] - p->rowptr[pr.row0]) + 3 * pr.nout;
+    // warp tasks: 32 units (a', 8-wide chunk of b) of a run of output channels,
+    // the most expensive first.  A task walks its nonzeros serially (a load
+    // latency per four), so where whole pairs would give the resident warps
+    // fewer than four tasks each, the pairs' channels are cut into runs of
+    // about 1/16 of one warp's share of the step, at least 24 nonzeros: MPO
+    // step of the Hubbard D = 701 bond 34.8 -> 18.4 us (1/4: 26.6, 1/8: 22.5),
+    // ladder D = 512 20.5 -> 16.4.  With more tasks than that the step is bound
+    // by HBM and a run's inputs are read again by its pair's other runs (D =
+    // 2000: 110 us whole, 114.7 us in runs).
+    constexpr double kResidentWarps = 152 * 16, kMpoTaskShare = 16;
+    double work = 0, whole = 0;
+    for (const MpoPair &pr : p->pairs) {
+      const double t = (double)(((int64_t)pr.da * (pr.dbp / 8) + 31) / 32);
+      whole += t;
+      work += t * (p->rowptr[pr.row0 + pr.nout] - p->rowptr[pr.row0] + pr.nout);
+    }
+    const int target = whole >= 4 * kResidentWarps
+                           ? INT32_MAX
+                           : (int)std::max(24.0, work / (kResidentWarps * kMpoTaskShare));
+    struct Run {
+      int q, o0, nout, cost;
     };
-    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost(x) > cost(y); });
-    for (int q : order) {
+    std::vector<Run> runs;
+    for (size_t q = 0; q < p->pairs.size(); ++q) {
       const MpoPair &pr = p->pairs[q];
-      const int64_t units = (int64_t)pr.da * (pr.dbp / 8);
-      UDMRG_REQUIRE(units < (1LL << 31), "mixed matvec: sector pair too large");
-      for (int64_t u0 = 0; u0 < units; u0 += 32) p->tasks.push_back({q, (int32_t)u0});
+      const int32_t *rp = p->rowptr.data() + pr.row0;
+      UDMRG_REQUIRE((int64_t)pr.da * (pr.dbp / 8) < (1LL << 31),
+                    "mixed matvec: sector pair too large");
+      const int total = rp[pr.nout] - rp[0] + pr.nout;  // a channel counts one for its store
+      const int parts = (int)std::max<int64_t>(1, ((int64_t)total + target / 2) / target);
+      for (int o = 0, k = 0; o < pr.nout; ++k) {
+        int e = o;
+        const int64_t until = (int64_t)total * (k + 1) / parts;
+        do
+          ++e;
+        while (e < pr.nout && rp[e] - rp[0] + e < until);
+        runs.push_back({(int)q, o, e - o, 2 * (rp[e] - rp[o]) + 3 * (e - o)});
+        o = e;
+      }
+    }
+    std::stable_sort(runs.begin(), runs.end(),
+                     [](const Run &x, const Run &y) { return x.cost > y.cost; });
+    for (const Run &r : runs) {
+      const MpoPair &pr = p->pairs[r.q];
+      const int32_t units = pr.da * (pr.dbp / 8);
+      for (int32_t u0 = 0; u0 < units; u0 += 32) p->tasks.push_back({r.q, u0, r.o0, r.nout});
     }
   }
   p->host_sec = std::chrono::duration<double>(std::chrono::steady_clock::now() - tstart).count();

@@ -79,9 +79,10 @@ struct MpoNzRec {
   int32_t astride;
   float v;
 };
-// Work of one warp: 32 consecutive units (a', 8-wide b chunk) of one pair.
+// Work of one warp: output channels o0 .. o0 + nout - 1 of one pair at 32
+// consecutive units (a', 8-wide b chunk).
 struct MpoTask {
-  int32_t pair, u0;
+  int32_t pair, u0, o0, nout;
 };
 struct MpoOut {
   int64_t img_off;  // byte offset of the step-3 A image of the target's group
@@ -133,7 +134,7 @@ struct SgMatvecPlan {
   std::vector<MpoOut> outs;
   std::vector<int32_t> rowptr;  // CSR row pointers over all output channels (+1)
   std::vector<MpoNzRec> nz;
-  std::vector<MpoTask> tasks;   // warp tasks, most expensive pair first
+  std::vector<MpoTask> tasks;   // warp tasks, most expensive first
   MpoPair *d_pairs = nullptr;
   MpoOut *d_outs = nullptr;
   int32_t *d_rowptr = nullptr;

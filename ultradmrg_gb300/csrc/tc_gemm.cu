@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t tmem = tc_setup<BN>(b, 1, 0);
   tc::pdl_wait();  // the images (and outputs) of the previous kernel
   if (warp == 0) {
-    if (lane == 0) {  // producer: one bulk copy per operand unit and chunk
+    if (lane == 0) {  // producer: one bulk copy per operand unit and chunk (per plane at K's end)
       uint32_t G = 0;
       for (int t = blockIdx.x; t < ntiles && !*b.abort_flag; t += gridDim.x) {
         const TcTile tile = tiles[t];
@@ -117,10 +117,22 @@ __global__ void __launch_bounds__(kThreads, 1)
             break;
           }
           uint8_t *st = smem + s * S::kStageBytes;
-          tc::mbar_expect_tx(&b.full[s], (uint32_t)(kTcUnitA + S::kUnitB));
-          tc::bulk_g2s(st, abase + (int64_t)c * kTcUnitA, (uint32_t)kTcUnitA, &b.full[s]);
-          tc::bulk_g2s(st + kTcUnitA, bbase + (int64_t)c * S::kUnitB, (uint32_t)S::kUnitB,
-                       &b.full[s]);
+          const uint8_t *as = abase + (int64_t)c * kTcUnitA, *bs = bbase + (int64_t)c * S::kUnitB;
+          const int kk = c + 1 < g.kc ? kTcBK : tc_chunk_k(g, c);
+          if (kk == kTcBK) {
+            tc::mbar_expect_tx(&b.full[s], (uint32_t)(kTcUnitA + S::kUnitB));
+            tc::bulk_g2s(st, as, (uint32_t)kTcUnitA, &b.full[s]);
+            tc::bulk_g2s(st + kTcUnitA, bs, (uint32_t)S::kUnitB, &b.full[s]);
+          } else {  // the leading K columns of each plane are contiguous
+            constexpr int planeA = kTcBM * kTcBK * 2, planeB = BN * kTcBK * 2;
+            const uint32_t ab = (uint32_t)(kTcBM * kk * 2), bb = (uint32_t)(BN * kk * 2);
+            tc::mbar_expect_tx(&b.full[s], 3 * (ab + bb));
+#pragma unroll
+            for (int p = 0; p < 3; ++p) {
+              tc::bulk_g2s(st + p * planeA, as + p * planeA, ab, &b.full[s]);
+              tc::bulk_g2s(st + kTcUnitA + p * planeB, bs + p * planeB, bb, &b.full[s]);
+            }
+          }
         }
       }
     }

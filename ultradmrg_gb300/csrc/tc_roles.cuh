@@ -113,27 +113,23 @@ __device__ __forceinline__ float narrow_f64(double x) {
 __device__ __forceinline__ float to_f32(float x) { return x; }
 __device__ __forceinline__ float to_f32(double x) { return narrow_f64(x); }
 
-__device__ __forceinline__ uint32_t pack_bf16x2(__nv_bfloat16 a, __nv_bfloat16 b) {
-  return (uint32_t)__bfloat16_as_ushort(a) | ((uint32_t)__bfloat16_as_ushort(b) << 16);
-}
-
 // x = hi + mid + lo, each the BF16 rounding of the remainder (exact
-// differences in FP32), eight values into three 16-byte plane segments.
+// differences in FP32), eight values into three 16-byte plane segments: two
+// values per conversion, widened back by a shift or a mask.
+__device__ __forceinline__ uint32_t bf16x2_rn(float lo, float hi) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t *>(&v);
+}
 __device__ __forceinline__ void split8(const float (&x)[8], uint4 &h, uint4 &m, uint4 &l) {
   uint32_t ph[4], pm[4], pl[4];
 #pragma unroll
-  for (int j = 0; j < 8; j += 2) {
-    __nv_bfloat16 hv[2], mv[2], lv[2];
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
-      hv[t] = __float2bfloat16_rn(x[j + t]);
-      const float r1 = x[j + t] - __bfloat162float(hv[t]);
-      mv[t] = __float2bfloat16_rn(r1);
-      lv[t] = __float2bfloat16_rn(r1 - __bfloat162float(mv[t]));
-    }
-    ph[j >> 1] = pack_bf16x2(hv[0], hv[1]);
-    pm[j >> 1] = pack_bf16x2(mv[0], mv[1]);
-    pl[j >> 1] = pack_bf16x2(lv[0], lv[1]);
+  for (int j = 0; j < 4; ++j) {
+    const float x0 = x[2 * j], x1 = x[2 * j + 1];
+    ph[j] = bf16x2_rn(x0, x1);
+    const float r0 = x0 - __uint_as_float(ph[j] << 16);
+    const float r1 = x1 - __uint_as_float(ph[j] & 0xFFFF0000u);
+    pm[j] = bf16x2_rn(r0, r1);
+    pl[j] = bf16x2_rn(r0 - __uint_as_float(pm[j] << 16), r1 - __uint_as_float(pm[j] & 0xFFFF0000u));
   }
   h = make_uint4(ph[0], ph[1], ph[2], ph[3]);
   m = make_uint4(pm[0], pm[1], pm[2], pm[3]);
@@ -211,6 +207,13 @@ __device__ __forceinline__ void tc_fail(const TcBars &b, int *err, int code) {
   *b.abort_flag = 1;
 }
 
+// K columns of chunk c that hold data, in whole 16-deep steps (the rest of the
+// chunk's image is zero): the last chunk of a group is neither staged nor
+// multiplied beyond them.
+__device__ __forceinline__ int tc_chunk_k(const TcGroup &g, int c) {
+  return min(kTcBK, (g.K - c * kTcBK + 15) & ~15);
+}
+
 // MMA issue (one thread) over the CTA's tiles (static schedule
 // t = blockIdx.x + i * gridDim.x): for each K chunk, wait for its stage,
 // issue the six split products per 16-deep K step, release the stage; after
@@ -242,17 +245,22 @@ __device__ __forceinline__ void tc_mma_role(const TcTile *__restrict__ tiles, in
       const uint32_t sa = tc::smem_u32(smem + s * S::kStageBytes);
       const uint32_t sb = sa + (uint32_t)kTcUnitA;
       constexpr uint32_t planeA = kTcBM * kTcBK * 2, planeB = BN * kTcBK * 2;
-#pragma unroll
-      for (int ks = 0; ks < kTcBK / 16; ++ks) {
+      auto step = [&](int ks) {  // K step ks covers core-matrix columns 2ks, 2ks+1
 #pragma unroll
         for (int p = 0; p < 6; ++p) {
-          // K step ks covers core-matrix columns 2ks, 2ks+1
           const uint64_t ad = tc::make_desc(
               sa + kProdA[p] * planeA + ks * 2 * (kTcBM / 8) * 128, (kTcBM / 8) * 128, 128);
           const uint64_t bd = tc::make_desc(
               sb + kProdB[p] * planeB + ks * 2 * (BN / 8) * 128, (BN / 8) * 128, 128);
           tc::mma_bf16(dcol, ad, bd, idesc, (c > 0 || ks > 0 || p > 0) ? 1u : 0u);
         }
+      };
+      if (c + 1 < g.kc) {
+#pragma unroll
+        for (int ks = 0; ks < kTcBK / 16; ++ks) step(ks);
+      } else {
+        const int nks = tc_chunk_k(g, c) >> 4;
+        for (int ks = 0; ks < nks; ++ks) step(ks);
       }
       tc::mma_commit(&b.empty[s]);  // the stage is free once these MMAs completed
     }
