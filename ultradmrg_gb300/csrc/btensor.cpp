@@ -29,6 +29,44 @@ Ctx::~Ctx() {
     cudaStreamDestroy(side);
   }
   if (pinned) cudaFreeHost(pinned);
+  if (stage) cudaFreeHost(stage);
+}
+
+uint8_t *Ctx::stage_room(size_t bytes) {
+  bytes = (bytes + 255) & ~(size_t)255;
+  if (bytes > kStage) return nullptr;
+  if (!stage) UDMRG_CHECK_CUDA(cudaMallocHost((void **)&stage, kStage));
+  if (stage_off + bytes > kStage) {
+    sync();  // the ring's copies have left it
+    stage_off = 0;
+  }
+  uint8_t *p = stage + stage_off;
+  stage_off += bytes;
+  return p;
+}
+
+void Ctx::upload(void *dst, const void *src, size_t bytes) {
+  if (bytes == 0) return;
+  uint8_t *p = stage_room(bytes);
+  if (p) std::memcpy(p, src, bytes);
+  UDMRG_CHECK_CUDA(cudaMemcpyAsync(dst, p ? p : src, bytes, cudaMemcpyHostToDevice, stream));
+  if (!p) sync();
+}
+
+uint8_t *UploadBatch::commit() {
+  if (total == 0) return nullptr;
+  uint8_t *dev = (uint8_t *)ctx.alloc(total);
+  size_t used = 0;
+  for (const Item &i : items) used = std::max(used, i.off + i.bytes);
+  uint8_t *p = ctx.stage_room(used);
+  if (!p) {
+    for (const Item &i : items) ctx.upload(dev + i.off, i.src, i.bytes);
+    return dev;
+  }
+  for (const Item &i : items) std::memcpy(p + i.off, i.src, i.bytes);
+  if (used)
+    UDMRG_CHECK_CUDA(cudaMemcpyAsync(dev, p, used, cudaMemcpyHostToDevice, ctx.stream));
+  return dev;
 }
 
 void *Ctx::alloc(size_t bytes) {

@@ -91,8 +91,20 @@ struct Ctx {
   bool closing = false;
   void *owner = nullptr;  // the C-ABI object that holds this context
 
+  // Page-locked staging ring of upload(): host tables reach the device without
+  // waiting, and the caller's memory is free when upload returns.  At most
+  // kStage bytes, given back with the context; it wraps after a
+  // synchronisation.
+  static constexpr size_t kStage = 16u << 20;
+  uint8_t *stage = nullptr;
+  size_t stage_off = 0;
+
   explicit Ctx(int dev);
   ~Ctx();
+  // Stream-ordered copy of host memory to the device.
+  void upload(void *dst, const void *src, size_t bytes);
+  // Room for `bytes` in the ring (null: more than it holds).
+  uint8_t *stage_room(size_t bytes);
   void *alloc(size_t bytes);
   void free(void *p);
   void sync();
@@ -174,6 +186,30 @@ struct DeviceScratch {
     ptrs.push_back(p);
     return (T *)p;
   }
+};
+
+// Host tables copied to the device in one allocation and one copy.
+struct UploadBatch {
+  Ctx &ctx;
+  struct Item {
+    const void *src;
+    size_t bytes, off;
+  };
+  std::vector<Item> items;
+  size_t total = 0;
+  explicit UploadBatch(Ctx &c) : ctx(c) {}
+  size_t reserve(size_t bytes) {  // offset of `bytes` that are not copied
+    const size_t off = total;
+    total += (bytes + 255) & ~(size_t)255;
+    return off;
+  }
+  template <typename V>
+  size_t add(const std::vector<V> &v) {
+    const size_t off = reserve(v.size() * sizeof(V));
+    if (!v.empty()) items.push_back({v.data(), v.size() * sizeof(V), off});
+    return off;
+  }
+  uint8_t *commit();  // the device block (the caller frees it)
 };
 
 // Sort + deduplicate a flat key list (rank-sized tuples).

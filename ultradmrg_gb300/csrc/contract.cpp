@@ -7,28 +7,20 @@
 namespace udmrg {
 
 GemmPlan::~GemmPlan() {
-  if (!ctx) return;
-  ctx->free(d_segs);
-  ctx->free(d_probs);
-  for (auto &p : d_tiles) ctx->free(p);
-}
-
-template <typename V>
-static V *upload_vec(Ctx *ctx, const std::vector<V> &v) {
-  if (v.empty()) return nullptr;
-  V *d = (V *)ctx->alloc(v.size() * sizeof(V));
-  UDMRG_CHECK_CUDA(
-      cudaMemcpyAsync(d, v.data(), v.size() * sizeof(V), cudaMemcpyHostToDevice, ctx->stream));
-  return d;
+  if (ctx) ctx->free(d_block);
 }
 
 void GemmPlan::upload() {
-  d_segs = upload_vec(ctx, segs);
-  d_probs = upload_vec(ctx, probs);
-  for (int c = 0; c < kNumCfg; ++c) d_tiles[c] = upload_vec(ctx, tiles[c]);
-  if (sl) sl->upload();
-  // host vectors stay: the descriptors are read before the upload completes
-  ctx->sync();
+  UploadBatch up(*ctx);
+  const size_t os = up.add(segs), op = up.add(probs);
+  size_t ot[kNumCfg];
+  for (int c = 0; c < kNumCfg; ++c) ot[c] = up.add(tiles[c]);
+  ctx->free(d_block);
+  d_block = up.commit();
+  d_segs = (GSeg *)(d_block + os);
+  d_probs = (GProb *)(d_block + op);
+  for (int c = 0; c < kNumCfg; ++c) d_tiles[c] = (GTile *)(d_block + ot[c]);
+  if (sl && !sl->d_block) sl->upload();
 }
 
 static const int kCfgBM[kNumCfg] = {64, 256, 16, 32};
@@ -396,7 +388,7 @@ std::unique_ptr<SlicePlan> slice_contract(const BTensor &A, const BTensor &B,
 // Both are sums over padded work, so ragged sectors, short K and narrow blocks
 // (the MPO tensors' few channels) stay on the FMAs.
 template <typename Build>
-std::unique_ptr<SlicePlan> slice_worth(const GemmPlan &g, bool cplx, Build build) {
+std::unique_ptr<SlicePlan> slice_worth(GemmPlan &g, bool cplx, bool upper, Build build) {
   const int form = g.ctx ? g.ctx->gemm_form : 0;
   if (form == 0 || g.probs.empty()) return nullptr;
   double t64 = 0.0;
@@ -407,6 +399,13 @@ std::unique_ptr<SlicePlan> slice_worth(const GemmPlan &g, bool cplx, Build build
   }
   auto sp = build();
   if (sp && form < 0 && sp->seconds() >= t64) sp.reset();
+  if (sp) {  // the FP64 tiles of operands outside its range: one launch, 64 x 64
+    for (auto &t : g.tiles) t.clear();
+    for (size_t p = 0; p < g.probs.size(); ++p)
+      for (int32_t m = 0; m < g.probs[p].M; m += 64)
+        for (int32_t n = upper ? m / 64 * 64 : 0; n < g.probs[p].N; n += 64)
+          g.tiles[kCfg64x64].push_back({(int32_t)p, m, n, 0});
+  }
   return sp;
 }
 
@@ -630,7 +629,7 @@ static std::unique_ptr<ContractPlan> plan_impl(const BTensor &A, const BTensor &
   if (!ca.empty()) {
     std::vector<int64_t> coff(nout);
     for (size_t o = 0; o < nout; ++o) coff[o] = C->offs[dest[o]];
-    g.sl = slice_worth(g, A.dtype == kC128, [&] {
+    g.sl = slice_worth(g, A.dtype == kC128, false, [&] {
       return slice_contract(A, B, ca, cb, fa, fb, matches, mstart, coff);
     });
   }
@@ -690,7 +689,7 @@ void gemm_finalize(GemmPlan &g, bool cplx, bool upper) {
               t.end());
     }
   sort_tiles(g);
-  g.sl = slice_worth(g, cplx, [&] { return slice_simple(g, cplx, upper); });
+  g.sl = slice_worth(g, cplx, upper, [&] { return slice_simple(g, cplx, upper); });
   g.upload();
 }
 
@@ -703,11 +702,7 @@ void gemm_retile(GemmPlan &g, int policy) {
   for (size_t p = 0; p < g.probs.size(); ++p)
     add_tiles(g, (int32_t)p, g.probs[p].M, g.probs[p].N, policy);
   sort_tiles(g);
-  for (int c = 0; c < kNumCfg; ++c) {
-    g.ctx->free(g.d_tiles[c]);
-    g.d_tiles[c] = upload_vec(g.ctx, g.tiles[c]);
-  }
-  g.ctx->sync();
+  g.upload();
 }
 
 TensorPtr contract_struct(const BTensor &A, const BTensor &B, const std::vector<int> &ca,

@@ -12,9 +12,9 @@ namespace udmrg {
 static_assert(kSpectrumFloor == kRankSv, "the SVD keeps the spectrum the rank model reads");
 
 TensorPtr contract_axes(Ctx &ctx, const BTensor &A, const BTensor &B, const std::vector<int> &ca,
-                        const std::vector<int> &cb, bool dw) {
+                        const std::vector<int> &cb) {
   auto p = plan_contract_axes(A, B, ca, cb);
-  return run_contract(ctx, *p, A, B, dw);
+  return run_contract(ctx, *p, A, B);
 }
 
 TensorPtr contract_cyclic(Ctx &ctx, const BTensor &A, const BTensor &B, int a_start, int b_start,
@@ -411,12 +411,16 @@ void MatvecPlan::apply_fp64(const double *in, double *out, bool dw) {
 // Bowdler, Martin, Reinsch and Wilkinson, Numer. Math. 11 (1968) 293).
 // ---------------------------------------------------------------------------
 
-void tridiag_eig(const std::vector<double> &a, const std::vector<double> &b, int64_t n,
-                 std::vector<double> &w, std::vector<double> &z) {
+// z: the eigenvectors too (null: eigenvalues only, n^2 work, the same values)
+static void tridiag_ql(const std::vector<double> &a, const std::vector<double> &b, int64_t n,
+                       std::vector<double> &w, std::vector<double> *zp) {
   std::vector<double> d(a.begin(), a.begin() + n), e(n, 0.0);
   for (int64_t i = 0; i + 1 < n; ++i) e[i] = b[i];
-  z.assign(n * n, 0.0);
-  for (int64_t i = 0; i < n; ++i) z[i * n + i] = 1.0;
+  std::vector<double> none, &z = zp ? *zp : none;
+  if (zp) {
+    z.assign(n * n, 0.0);
+    for (int64_t i = 0; i < n; ++i) z[i * n + i] = 1.0;
+  }
   const double eps = 2.220446049250313e-16;
   for (int64_t l = 0; l < n; ++l) {
     int iter = 0;
@@ -451,7 +455,7 @@ void tridiag_eig(const std::vector<double> &a, const std::vector<double> &b, int
         p = s * r;
         d[i + 1] = g + p;
         g = c * r - bb;
-        for (int64_t k = 0; k < n; ++k) {  // accumulate the rotation into z
+        for (int64_t k = 0; zp && k < n; ++k) {  // accumulate the rotation into z
           const double zk1 = z[k * n + i + 1];
           z[k * n + i + 1] = s * z[k * n + i] + c * zk1;
           z[k * n + i] = c * z[k * n + i] - s * zk1;
@@ -468,18 +472,23 @@ void tridiag_eig(const std::vector<double> &a, const std::vector<double> &b, int
   for (int64_t i = 0; i < n; ++i) ord[i] = i;
   std::stable_sort(ord.begin(), ord.end(), [&](int64_t x, int64_t y) { return d[x] < d[y]; });
   w.resize(n);
+  for (int64_t j = 0; j < n; ++j) w[j] = d[ord[j]];
+  if (!zp) return;
   std::vector<double> zs(n * n);
-  for (int64_t j = 0; j < n; ++j) {
-    w[j] = d[ord[j]];
+  for (int64_t j = 0; j < n; ++j)
     for (int64_t k = 0; k < n; ++k) zs[k * n + j] = z[k * n + ord[j]];
-  }
   z.swap(zs);
+}
+
+void tridiag_eig(const std::vector<double> &a, const std::vector<double> &b, int64_t n,
+                 std::vector<double> &w, std::vector<double> &z) {
+  tridiag_ql(a, b, n, w, &z);
 }
 
 double tridiag_lowest(const std::vector<double> &a, const std::vector<double> &b, int64_t n,
                       std::vector<double> *vec) {
   std::vector<double> w, z;
-  tridiag_eig(a, b, n, w, z);
+  tridiag_ql(a, b, n, w, vec ? &z : nullptr);
   if (vec) {
     vec->resize(n);
     for (int64_t k = 0; k < n; ++k) (*vec)[k] = z[k * n];
@@ -805,29 +814,63 @@ ExpmvResult lanczos_expmv(Ctx &ctx, MatvecPlan &mv, const BTensor &init_state, d
 // Environments
 // ---------------------------------------------------------------------------
 
-// T (a, x1, x2, b) through the MPO tensor W: (a, y1, y2, b).  Null where W has
-// imaginary coefficients or the context asks for plain FP64 GEMMs.
-static TensorPtr mpo_apply(Ctx &ctx, const BTensor &T, const BTensor &W, int x1, int x2) {
+// An environment update with the MPO tensor as a channel map: first . second
+// over one pair of axes gives T (a, x1, x2, b), W takes it to (a, y1, y2, b),
+// and `close` names the last contraction.  The three plans need block
+// structures only, so they are built on host threads and the device starts on
+// the first while the others are under way.  Null where W has imaginary
+// coefficients or the context asks for plain FP64 GEMMs.
+struct EnvClose {
+  bool map_left;  // the mapped tensor is the last contraction's first operand
+  const BTensor &other;
+  std::vector<int> ca, cb;
+};
+static TensorPtr mapped_env(Ctx &ctx, const BTensor &first, const BTensor &second, int ax_a,
+                            int ax_b, const BTensor &W, int x1, int x2, const EnvClose &close,
+                            bool dw) {
   if (ctx.gemm_form == 0) return nullptr;
-  auto out = mpo_map_struct(T, W, x1, x2);
   bool real = true;
   const std::vector<double> wh = mpo_data(ctx, W, &real);
   if (!real) return nullptr;
-  auto m = build_mpo_map(T, W, wh, x1, x2, *out);
+  std::vector<int> ca, cb, fa, fb;
+  cyclic_axes(first.rank(), second.rank(), ax_a, ax_b, 1, ca, cb, fa, fb);
+  UDMRG_REQUIRE(first.dtype == second.dtype, "contract: operands must have the same element type");
+  auto T = contract_struct(first, second, ca, cb, fa, fb);
+  auto M = mpo_map_struct(*T, W, x1, x2);
+  auto map = std::async(std::launch::async,
+                        [&] { return build_mpo_map(*T, W, wh, x1, x2, *M); });
+  auto last = std::async(std::launch::async, [&] {
+    return close.map_left ? plan_contract_axes(*M, close.other, close.ca, close.cb, false)
+                          : plan_contract_axes(close.other, *M, close.ca, close.cb, false);
+  });
+  std::exception_ptr err;  // both threads end before this scope does
+  TensorPtr t;
+  try {
+    auto p1 = plan_contract_cyclic(first, second, ax_a, ax_b, 1);
+    t = run_contract(ctx, *p1, first, second, dw);
+  } catch (...) {
+    err = std::current_exception();
+  }
+  map.wait();
+  last.wait();
+  if (err) std::rethrow_exception(err);
+  auto m = map.get();
   upload_mpo_step64(ctx, *m);
-  out->alloc_data();
-  run_mpo_step64(ctx, *m, T.data, out->data);
-  return out;
+  M->alloc_data();
+  run_mpo_step64(ctx, *m, t->data, M->data);
+  t.reset();
+  auto p2 = last.get();
+  gemm_upload(p2->gemm);
+  return close.map_left ? run_contract(ctx, *p2, *M, close.other, dw)
+                        : run_contract(ctx, *p2, close.other, *M, dw);
 }
 
 TensorPtr update_site_lenv(Ctx &ctx, const BTensor &lenv, const BTensor &A, const BTensor &W,
                            bool dw) {
   auto Ad = dag(ctx, A);
-  auto t = contract_cyclic(ctx, lenv, A, 2, 0, 1, dw);  // (a', w, s, b)
-  if (auto t2 = mpo_apply(ctx, *t, W, 0, 1)) {          // (a', s', w', b)
-    t.reset();
-    return contract_axes(ctx, *Ad, *t2, {0, 1}, {0, 1}, dw);
-  }
+  // T (a', w, s, b) -> (a', s', w', b), closed with A*(a', s', b')
+  if (auto r = mapped_env(ctx, lenv, A, 2, 0, W, 0, 1, {false, *Ad, {0, 1}, {0, 1}}, dw)) return r;
+  auto t = contract_cyclic(ctx, lenv, A, 2, 0, 1, dw);
   auto t2 = contract_cyclic(ctx, *t, W, 1, 0, 2, dw);
   t.reset();
   return contract_cyclic(ctx, *Ad, *t2, 0, 1, 2, dw);
@@ -836,11 +879,9 @@ TensorPtr update_site_lenv(Ctx &ctx, const BTensor &lenv, const BTensor &A, cons
 TensorPtr update_site_renv(Ctx &ctx, const BTensor &renv, const BTensor &A, const BTensor &W,
                            bool dw) {
   auto Ad = dag(ctx, A);
-  auto t = contract_cyclic(ctx, *Ad, renv, 2, 0, 1, dw);  // (a', s', w, b)
-  if (auto t2 = mpo_apply(ctx, *t, W, 2, 3)) {            // (a', w', s, b)
-    t.reset();
-    return contract_axes(ctx, *t2, A, {2, 3}, {1, 2}, dw);
-  }
+  // T (a', s', w, b) -> (a', w', s, b), closed with A(a, s, b)
+  if (auto r = mapped_env(ctx, *Ad, renv, 2, 0, W, 2, 3, {true, A, {2, 3}, {1, 2}}, dw)) return r;
+  auto t = contract_cyclic(ctx, *Ad, renv, 2, 0, 1, dw);
   auto t2 = contract_cyclic(ctx, *t, W, 1, 2, 2, dw);
   t.reset();
   return contract_cyclic(ctx, *t2, A, 3, 1, 2, dw);

@@ -14,7 +14,7 @@ enum Precision : int { kPrecFP64 = 0, kPrecMixed = 1 };
 
 // Block-sparse ops built on plan + run.
 TensorPtr contract_axes(Ctx &ctx, const BTensor &A, const BTensor &B, const std::vector<int> &ca,
-                        const std::vector<int> &cb, bool dw = false);
+                        const std::vector<int> &cb);
 TensorPtr contract_cyclic(Ctx &ctx, const BTensor &A, const BTensor &B, int a_start, int b_start,
                           int n, bool dw = false);
 TensorPtr dag(Ctx &ctx, const BTensor &A);

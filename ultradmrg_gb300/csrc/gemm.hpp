@@ -53,7 +53,8 @@ struct GemmPlan {
   // the digit-sliced tensor-core form of the same problems, where it is the
   // faster one (slice_worth); the tiles then only run on operands outside its range
   std::unique_ptr<SlicePlan> sl;
-  // device copies
+  // device copies, in one block
+  uint8_t *d_block = nullptr;
   GSeg *d_segs = nullptr;
   GProb *d_probs = nullptr;
   GTile *d_tiles[kNumCfg] = {nullptr, nullptr, nullptr, nullptr};

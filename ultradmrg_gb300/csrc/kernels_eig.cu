@@ -1111,8 +1111,7 @@ static void tridiag_all(Ctx &ctx, DeviceScratch &scratch, const std::vector<EigJ
   TriSlot *dslots = scratch.get<TriSlot>(slot);
   T *dwb = scratch.get<T>(wb_tot);
   T *dred = scratch.get<T>((int64_t)slot * 2 * kTriMaxParts);
-  UDMRG_CHECK_CUDA(cudaMemcpyAsync(dparts, parts.data(), parts.size() * sizeof(TriPart),
-                                   cudaMemcpyHostToDevice, ctx.stream));
+  ctx.upload(dparts, parts.data(), parts.size() * sizeof(TriPart));
   UDMRG_CHECK_CUDA(cudaMemsetAsync(dslots, 0, slot * sizeof(TriSlot), ctx.stream));
   // the side stream starts after the uploads and the Gram products, and the
   // main stream goes on after it
@@ -1151,7 +1150,6 @@ static void tridiag_all(Ctx &ctx, DeviceScratch &scratch, const std::vector<EigJ
   }
   for (size_t i = 1; i + (side ? 1 : 0) < launches.size(); ++i) launch(launches[i], ctx.stream);
   if (side) UDMRG_CHECK_CUDA(cudaStreamWaitEvent(ctx.stream, ev.b, 0));
-  ctx.sync();  // `parts` must outlive the upload
 }
 
 int sym_eig_values(Ctx &ctx, DeviceScratch &scratch, std::vector<EigJob> &jobs, double *G,
@@ -1174,8 +1172,7 @@ int sym_eig_values(Ctx &ctx, DeviceScratch &scratch, std::vector<EigJob> &jobs, 
   wk.jobs = scratch.get<EigJob>(nj);
   int *dstat = scratch.get<int>(1);
   UDMRG_CHECK_CUDA(cudaMemsetAsync(dstat, 0, sizeof(int), ctx.stream));
-  UDMRG_CHECK_CUDA(cudaMemcpyAsync(wk.jobs, jobs.data(), nj * sizeof(EigJob),
-                                   cudaMemcpyHostToDevice, ctx.stream));
+  ctx.upload(wk.jobs, jobs.data(), nj * sizeof(EigJob));
   if (cplx)
     tridiag_all<double2>(ctx, scratch, jobs, wk, G, dstat);
   else
@@ -1245,8 +1242,7 @@ int sym_eig_values(Ctx &ctx, DeviceScratch &scratch, std::vector<EigJob> &jobs, 
     for (int i0 = jobs[q].n - (int)wk.computed[q]; i0 < jobs[q].n; i0 += kBisectEigs)
       chunks.push_back(make_int2(q, i0));
   int2 *dch = scratch.get<int2>(chunks.size());
-  UDMRG_CHECK_CUDA(cudaMemcpyAsync(dch, chunks.data(), chunks.size() * sizeof(int2),
-                                   cudaMemcpyHostToDevice, ctx.stream));
+  ctx.upload(dch, chunks.data(), chunks.size() * sizeof(int2));
   if (!chunks.empty())
     bisect_kernel<<<(int)chunks.size(), 32, bsmem, ctx.stream>>>(
         wk.jobs, dch, wk.d, wk.e, wk.scale, lam, dtop, dcnt);
@@ -1301,8 +1297,7 @@ void sym_eig_vectors(Ctx &ctx, DeviceScratch &scratch, const std::vector<EigJob>
     const int ncl = (int)cl.size();
     EigCluster *dcl = scratch.get<EigCluster>(ncl);
     double *work = scratch.get<double>(6 * (int64_t)nmax * ncl);
-    UDMRG_CHECK_CUDA(cudaMemcpyAsync(dcl, cl.data(), ncl * sizeof(EigCluster),
-                                     cudaMemcpyHostToDevice, ctx.stream));
+    ctx.upload(dcl, cl.data(), ncl * sizeof(EigCluster));
     invit_kernel<<<(ncl + 31) / 32, 32, 0, ctx.stream>>>(dcl, ncl, wk.jobs, wk.d, wk.e, wk.scale,
                                                         lam, Z, work, nmax);
     UDMRG_CHECK_CUDA(cudaGetLastError());
@@ -1369,8 +1364,7 @@ void sym_eig_vectors(Ctx &ctx, DeviceScratch &scratch, const std::vector<EigJob>
                                (int32_t)std::min<int64_t>(width, k[q] - c0), 0});
     if (!bt.empty()) {
       BackChunk *dbt = scratch.get<BackChunk>(bt.size());
-      UDMRG_CHECK_CUDA(cudaMemcpyAsync(dbt, bt.data(), bt.size() * sizeof(BackChunk),
-                                       cudaMemcpyHostToDevice, ctx.stream));
+      ctx.upload(dbt, bt.data(), bt.size() * sizeof(BackChunk));
       const size_t smem = wk.cplx
                               ? (size_t)nmax * (BackShape<double2>::kCols + 2) * sizeof(double2)
                               : (size_t)nmax * (BackShape<double>::kCols + 2) * sizeof(double);
@@ -1390,7 +1384,6 @@ void sym_eig_vectors(Ctx &ctx, DeviceScratch &scratch, const std::vector<EigJob>
       ctx.launches++;
     }
   }
-  ctx.sync();  // host vectors above must outlive the uploads
 }
 
 }  // namespace udmrg

@@ -76,14 +76,12 @@ static void launch_copy2d(Ctx &ctx, const std::vector<Copy2D> &blocks, const dou
   const std::vector<Copy2D> ops = split_rows(blocks);
   if (ops.empty()) return;
   Copy2D *d = (Copy2D *)ctx.alloc(ops.size() * sizeof(Copy2D));
-  UDMRG_CHECK_CUDA(cudaMemcpyAsync(d, ops.data(), ops.size() * sizeof(Copy2D),
-                                   cudaMemcpyHostToDevice, ctx.stream));
+  ctx.upload(d, ops.data(), ops.size() * sizeof(Copy2D));
   const int grid = (int)std::min<size_t>(ops.size(), 8 * (size_t)ctx.num_sms);
   copy2d_kernel<<<grid, 256, 0, ctx.stream>>>(d, (int)ops.size(), src, dst, cplx ? 1 : 0, fd, fs);
   UDMRG_CHECK_CUDA(cudaGetLastError());
   ctx.launches++;
   ctx.free(d);
-  ctx.sync();  // host vector `ops` must outlive the upload
 }
 
 void run_copy2d(Ctx &ctx, const std::vector<Copy2D> &ops, const double *src, double *dst,
@@ -100,13 +98,11 @@ void run_scale(Ctx &ctx, const std::vector<ScaleJob> &jobs, double *X, const dou
                bool cplx) {
   if (jobs.empty()) return;
   ScaleJob *d = (ScaleJob *)ctx.alloc(jobs.size() * sizeof(ScaleJob));
-  UDMRG_CHECK_CUDA(cudaMemcpyAsync(d, jobs.data(), jobs.size() * sizeof(ScaleJob),
-                                   cudaMemcpyHostToDevice, ctx.stream));
+  ctx.upload(d, jobs.data(), jobs.size() * sizeof(ScaleJob));
   const int grid = (int)std::min<size_t>(jobs.size(), 8 * (size_t)ctx.num_sms);
   scale_cols_kernel<<<grid, 256, 0, ctx.stream>>>(d, (int)jobs.size(), X, f, cplx ? 1 : 0);
   UDMRG_CHECK_CUDA(cudaGetLastError());
   ctx.launches++;
-  ctx.sync();
   ctx.free(d);
 }
 

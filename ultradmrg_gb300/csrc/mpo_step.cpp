@@ -4,19 +4,6 @@
 
 namespace udmrg {
 
-namespace {
-
-template <typename V>
-V *upload(Ctx &ctx, const std::vector<V> &v) {
-  if (v.empty()) return nullptr;
-  V *d = (V *)ctx.alloc(v.size() * sizeof(V));
-  UDMRG_CHECK_CUDA(
-      cudaMemcpyAsync(d, v.data(), v.size() * sizeof(V), cudaMemcpyHostToDevice, ctx.stream));
-  return d;
-}
-
-}  // namespace
-
 std::vector<double> mpo_data(Ctx &ctx, const BTensor &t, bool *real) {
   const int es = elem_doubles(t.dtype);
   std::vector<double> h(t.size() * es);
@@ -96,8 +83,7 @@ const std::vector<FusedMpo::Entry> &FusedMpo::get(int32_t S1p, int32_t S2p, int3
 
 MpoStep64::~MpoStep64() {
   if (!ctx) return;
-  for (void *p : {(void *)d_pairs, (void *)d_outs, (void *)d_rowptr, (void *)d_nz, (void *)d_tasks})
-    ctx->free(p);
+  ctx->free(d_block);
 }
 
 namespace {
@@ -261,12 +247,15 @@ std::unique_ptr<MpoStep64> build_mpo_map(const BTensor &T, const BTensor &W,
 
 void upload_mpo_step64(Ctx &ctx, MpoStep64 &m) {
   m.ctx = &ctx;
-  m.d_pairs = upload(ctx, m.pairs);
-  m.d_outs = upload(ctx, m.outs);
-  m.d_rowptr = upload(ctx, m.rowptr);
-  m.d_nz = upload(ctx, m.nz);
-  m.d_tasks = upload(ctx, m.tasks);
-  ctx.sync();  // host vectors stay, but the uploads finish before they could move
+  UploadBatch up(ctx);
+  const size_t o0 = up.add(m.pairs), o1 = up.add(m.outs), o2 = up.add(m.rowptr), o3 = up.add(m.nz),
+               o4 = up.add(m.tasks);
+  m.d_block = up.commit();
+  m.d_pairs = (MpoPair64 *)(m.d_block + o0);
+  m.d_outs = (MpoOut64 *)(m.d_block + o1);
+  m.d_rowptr = (int32_t *)(m.d_block + o2);
+  m.d_nz = (MpoNz64 *)(m.d_block + o3);
+  m.d_tasks = (MpoTask64 *)(m.d_block + o4);
 }
 
 }  // namespace udmrg

@@ -68,6 +68,7 @@ struct MpoStep64 {
   std::vector<int32_t> rowptr;
   std::vector<MpoNz64> nz;
   std::vector<MpoTask64> tasks;
+  uint8_t *d_block = nullptr;
   MpoPair64 *d_pairs = nullptr;
   MpoOut64 *d_outs = nullptr;
   int32_t *d_rowptr = nullptr;

@@ -23,8 +23,7 @@ template <typename V>
 V *upload_vec(Ctx &ctx, const std::vector<V> &v) {
   if (v.empty()) return nullptr;
   V *d = (V *)ctx.alloc(v.size() * sizeof(V));
-  UDMRG_CHECK_CUDA(
-      cudaMemcpyAsync(d, v.data(), v.size() * sizeof(V), cudaMemcpyHostToDevice, ctx.stream));
+  ctx.upload(d, v.data(), v.size() * sizeof(V));
   return d;
 }
 
@@ -549,7 +548,6 @@ void plan_sg_device(Ctx &ctx, SgMatvecPlan &plan, const BTensor &L, const BTenso
   p->d_kchunks = upload_vec(ctx, p->kchunks);
   p->d_tgtref = upload_vec(ctx, p->tgtref);
   p->mixed_flops = 6.0 * (p->g1.flops + p->g3.flops);
-  ctx.sync();
   std::vector<PackOp>().swap(p->l_ops);  // packed; the host copies go
   std::vector<PackOp>().swap(p->r_ops);
   p->dev_sec = std::chrono::duration<double>(std::chrono::steady_clock::now() - tstart).count();

@@ -420,22 +420,12 @@ __global__ void __launch_bounds__(kSlThreads, 1)
   if (warp == 0) tc::tmem_dealloc(tmem, 512);
 }
 
-template <typename V>
-V *up(Ctx *ctx, const std::vector<V> &v) {
-  if (v.empty()) return nullptr;
-  V *d = (V *)ctx->alloc(v.size() * sizeof(V));
-  UDMRG_CHECK_CUDA(
-      cudaMemcpyAsync(d, v.data(), v.size() * sizeof(V), cudaMemcpyHostToDevice, ctx->stream));
-  return d;
-}
-
 }  // namespace
 
 SlicePlan::~SlicePlan() {
   if (!ctx) return;
-  for (void *p : {(void *)d_ops, (void *)d_items, (void *)d_groups, (void *)d_tiles,
-                  (void *)d_lines, (void *)d_cblk, (void *)img, (void *)scale})
-    ctx->free(p);
+  ctx->free(d_block);
+  ctx->free(img);
 }
 
 int SlicePlan::add_group(const Dims &d, const std::vector<SlLine> &rows,
@@ -508,14 +498,19 @@ void SlicePlan::finalize() {
 }
 
 void SlicePlan::upload() {
-  d_ops = up(ctx, ops);
-  d_items = up(ctx, items);
-  d_groups = up(ctx, groups);
-  d_tiles = up(ctx, tiles);
-  d_lines = up(ctx, lines);
-  d_cblk = up(ctx, cblk);
+  UploadBatch up(*ctx);
+  const size_t o0 = up.add(ops), o1 = up.add(items), o2 = up.add(groups), o3 = up.add(tiles),
+               o4 = up.add(lines), o5 = up.add(cblk),
+               o6 = up.reserve((lines.size() + 2) * sizeof(int));
+  d_block = up.commit();
+  d_ops = (SlOp *)(d_block + o0);
+  d_items = (SlItem *)(d_block + o1);
+  d_groups = (SlGroup *)(d_block + o2);
+  d_tiles = (SlTile *)(d_block + o3);
+  d_lines = (SlLine *)(d_block + o4);
+  d_cblk = (int64_t *)(d_block + o5);
+  scale = (int *)(d_block + o6);
   img = (uint8_t *)ctx->alloc(std::max<int64_t>(img_bytes, 1));
-  scale = (int *)ctx->alloc((lines.size() + 2) * sizeof(int));
   if (holes) UDMRG_CHECK_CUDA(cudaMemsetAsync(img, 0, img_bytes, ctx->stream));
 }
 
@@ -540,8 +535,12 @@ void run_slice(Ctx &ctx, const SlicePlan &p, const double *a, const double *b, d
     slice_pack_kernel<<<pg, kPackThreads, 0, ctx.stream>>>(p.d_ops, p.d_items, ni, a, b, p.scale,
                                                            p.img);
   }
-  UDMRG_CHECK_CUDA(cudaFuncSetAttribute(slice_gemm_kernel,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, kSlSmem));
+  static bool attr_set = false;
+  if (!attr_set) {
+    UDMRG_CHECK_CUDA(cudaFuncSetAttribute(slice_gemm_kernel,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, kSlSmem));
+    attr_set = true;
+  }
   const int nt = (int)p.tiles.size();
   slice_gemm_kernel<<<std::min(nt, ctx.num_sms), kSlThreads, kSlSmem, ctx.stream>>>(
       p.d_tiles, nt, p.d_groups, p.d_lines, p.d_cblk, p.scale, p.img, c, p.scale);

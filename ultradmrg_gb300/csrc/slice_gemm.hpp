@@ -87,6 +87,7 @@ struct SlicePlan {
   std::vector<int64_t> cblk;
   int64_t img_bytes = 0;
   bool holes = false;  // image entries no op writes
+  uint8_t *d_block = nullptr;  // the tables and scale
   SlOp *d_ops = nullptr;
   SlItem *d_items = nullptr;
   SlGroup *d_groups = nullptr;

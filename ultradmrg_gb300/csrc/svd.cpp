@@ -238,10 +238,7 @@ void build_outputs(Ctx &ctx, DeviceScratch &scratch, const BTensor &T, int ldims
         if (p > 0) res.ee += -p * std::log(p);
       }
     }
-    if (!hs.empty())
-      UDMRG_CHECK_CUDA(cudaMemcpyAsync(s->data, hs.data(), hs.size() * sizeof(double),
-                                       cudaMemcpyHostToDevice, ctx.stream));
-    ctx.sync();
+    ctx.upload(s->data, hs.data(), hs.size() * sizeof(double));
   }
   // centre factor: C_q = U_q^T M_q (k x cols) on the left side, M_q V_q (rows x k) on the right
   int64_t ctot = 0;
@@ -294,8 +291,7 @@ void build_outputs(Ctx &ctx, DeviceScratch &scratch, const BTensor &T, int ldims
       for (int64_t i = 0; i < kept[q]; ++i) inv.push_back(sv[q][i] > 0 ? 1.0 / sv[q][i] : 0.0);
     }
     double *dinv = scratch.get<double>(std::max<size_t>(inv.size(), 1));
-    UDMRG_CHECK_CUDA(cudaMemcpyAsync(dinv, inv.data(), inv.size() * sizeof(double),
-                                     cudaMemcpyHostToDevice, ctx.stream));
+    ctx.upload(dinv, inv.data(), inv.size() * sizeof(double));
     run_scale(ctx, sj, Cbuf, dinv, cplx);
   }
   std::vector<Copy2D> uops, vops;

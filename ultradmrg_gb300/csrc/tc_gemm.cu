@@ -227,8 +227,7 @@ template <typename V>
 static V *upload(Ctx *ctx, const std::vector<V> &v) {
   if (v.empty()) return nullptr;
   V *d = (V *)ctx->alloc(v.size() * sizeof(V));
-  UDMRG_CHECK_CUDA(
-      cudaMemcpyAsync(d, v.data(), v.size() * sizeof(V), cudaMemcpyHostToDevice, ctx->stream));
+  ctx->upload(d, v.data(), v.size() * sizeof(V));
   return d;
 }
 
@@ -241,7 +240,6 @@ void TcPlan::finalize() {
   d_rowaddr = upload(ctx, rowaddr);
   d_err = (int *)ctx->alloc(sizeof(int));
   UDMRG_CHECK_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int), ctx->stream));
-  ctx->sync();
 }
 
 std::vector<PackTile> pack_tiles(const std::vector<PackOp> &ops, int kstep) {
@@ -299,7 +297,6 @@ void run_pack(Ctx &ctx, const std::vector<PackOp> &ops, const void *src, bool sr
   pl.ops = ops;
   pl.upload(ctx);
   launch_pack(ctx, pl.d_ops, pl.d_tiles, (int)pl.tiles.size(), src, src_f64, img, pl.rows_src);
-  ctx.sync();  // the lists are freed on return
 }
 
 template <int BN>
