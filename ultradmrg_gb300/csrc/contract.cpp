@@ -65,11 +65,10 @@ struct Match {
   int64_t a, b;
 };
 
-// Choose the tile configuration with the least padded work and emit the tiles.
-// Policy 1 charges 32 x 32 tiles (four outputs per thread) twice their padded
-// work, so they are taken only where the larger tiles would pad more than
-// twice as much.
-void add_tiles(GemmPlan &g, int32_t pid, int64_t M, int64_t N, int policy) {
+// The tile configuration with the least padded work.  Policy 1 charges 32 x 32
+// tiles (four outputs per thread) twice their padded work, so they are taken
+// only where the larger tiles would pad more than twice as much.
+int tile_cfg(int64_t M, int64_t N, int policy, double *padded = nullptr) {
   int best = 0;
   double bestw = 1e300;
   for (int c = 0; c < kNumCfg; ++c) {
@@ -81,6 +80,12 @@ void add_tiles(GemmPlan &g, int32_t pid, int64_t M, int64_t N, int policy) {
       best = c;
     }
   }
+  if (padded) *padded = bestw;
+  return best;
+}
+
+void add_tiles(GemmPlan &g, int32_t pid, int64_t M, int64_t N, int policy) {
+  const int best = tile_cfg(M, N, policy);
   for (int64_t m0 = 0; m0 < M; m0 += kCfgBM[best])
     for (int64_t n0 = 0; n0 < N; n0 += kCfgBN[best])
       g.tiles[best].push_back({pid, (int32_t)m0, (int32_t)n0, 0});
@@ -88,23 +93,24 @@ void add_tiles(GemmPlan &g, int32_t pid, int64_t M, int64_t N, int policy) {
 
 }  // namespace
 
-static void sort_tiles(GemmPlan &g);
+static void tile_all(GemmPlan &g);
 
 namespace {
 
 constexpr int64_t up8(int64_t x) { return (x + 7) & ~(int64_t)7; }
 
-// Estimated time of a plan's FP64 tiles: multiply-adds of the padded tiles at
-// 0.5e12 per second (80% of the FP64 pipe), four per complex one.
-double fp64_seconds(const GemmPlan &g, bool cplx) {
-  std::vector<double> k(g.probs.size(), 0.0);
-  for (size_t p = 0; p < g.probs.size(); ++p)
-    for (int s = 0; s < g.probs[p].nseg; ++s)
-      k[p] += (double)((g.segs[g.probs[p].seg0 + s].K + 15) / 16 * 16);
+// Estimated time of a plan's FP64 tiles: multiply-adds of the padded tiles
+// (half of them for an upper triangle) at 0.5e12 per second (80% of the FP64
+// pipe), four per complex one.
+double fp64_seconds(const GemmPlan &g, bool cplx, bool upper) {
   double macs = 0;
-  for (int c = 0; c < kNumCfg; ++c)
-    for (const GTile &t : g.tiles[c]) macs += k[t.prob] * kCfgBM[c] * kCfgBN[c];
-  return 4e-6 + macs * (cplx ? 4.0 : 1.0) / 0.5e12;
+  for (const GProb &p : g.probs) {
+    double k = 0, area = 0;
+    for (int s = 0; s < p.nseg; ++s) k += (double)((g.segs[p.seg0 + s].K + 15) / 16 * 16);
+    tile_cfg(p.M, p.N, 0, &area);
+    macs += k * area;
+  }
+  return 4e-6 + macs * (cplx ? 4.0 : 1.0) * (upper ? 0.5 : 1.0) / 0.5e12;
 }
 
 // Below this estimate the sliced form's three launches and its passes over
@@ -185,10 +191,14 @@ void add_ops(SlicePlan &sp, int group, SlOp base, bool cplx, int32_t kh) {
 // Lines of C's rows (blk, m) and columns (blk, n, block width; two per complex
 // column).
 void push_rows(std::vector<SlLine> &v, int blk, int64_t M) {
-  for (int64_t m = 0; m < M; ++m) v.push_back({blk, (int32_t)m, 0, 0});
+  const size_t n0 = v.size();
+  v.resize(n0 + M);
+  for (int64_t m = 0; m < M; ++m) v[n0 + m] = {blk, (int32_t)m, 0, 0};
 }
 void push_cols(std::vector<SlLine> &v, int blk, int64_t N, int es) {
-  for (int64_t n = 0; n < N * es; ++n) v.push_back({blk, (int32_t)n, (int32_t)(N * es), 0});
+  const size_t n0 = v.size();
+  v.resize(n0 + N * es);
+  for (int64_t n = 0; n < N * es; ++n) v[n0 + n] = {blk, (int32_t)n, (int32_t)(N * es), 0};
 }
 
 // The sliced form of gemm_add_simple's problems: one group each.
@@ -394,13 +404,12 @@ std::unique_ptr<SlicePlan> slice_worth(GemmPlan &g, bool cplx, bool upper, Build
   double t64 = 0.0;
   if (form < 0) {
     if (mean_k(g) < kSliceMinK) return nullptr;
-    t64 = fp64_seconds(g, cplx);
+    t64 = fp64_seconds(g, cplx, upper);
     if (t64 < kSliceMin) return nullptr;
   }
   auto sp = build();
   if (sp && form < 0 && sp->seconds() >= t64) sp.reset();
   if (sp) {  // the FP64 tiles of operands outside its range: one launch, 64 x 64
-    for (auto &t : g.tiles) t.clear();
     for (size_t p = 0; p < g.probs.size(); ++p)
       for (int32_t m = 0; m < g.probs[p].M; m += 64)
         for (int32_t n = upper ? m / 64 * 64 : 0; n < g.probs[p].N; n += 64)
@@ -622,10 +631,8 @@ static std::unique_ptr<ContractPlan> plan_impl(const BTensor &A, const BTensor &
       g.segs.push_back(sg);
     }
     g.flops += 2.0 * cplx * (double)M * (double)N * kflops;
-    add_tiles(g, (int32_t)g.probs.size(), M, N, g.policy);
     g.probs.push_back(p);
   }
-  sort_tiles(g);
   if (!ca.empty()) {
     std::vector<int64_t> coff(nout);
     for (size_t o = 0; o < nout; ++o) coff[o] = C->offs[dest[o]];
@@ -633,6 +640,7 @@ static std::unique_ptr<ContractPlan> plan_impl(const BTensor &A, const BTensor &
       return slice_contract(A, B, ca, cb, fa, fb, matches, mstart, coff);
     });
   }
+  if (!g.sl) tile_all(g);
   if (upload) g.upload();
   plan->out = std::move(out);
   return plan;
@@ -665,11 +673,14 @@ void gemm_add_simple(GemmPlan &g, int64_t c_off, int64_t M, int64_t N, int64_t K
   s.b_ks[0] = b_ks;
   g.segs.push_back(s);
   g.flops += 2.0 * (cplx ? 4.0 : 1.0) * (double)M * (double)N * (double)K;
-  add_tiles(g, (int32_t)g.probs.size(), M, N, g.policy);
   g.probs.push_back(p);
 }
 
-static void sort_tiles(GemmPlan &g) {
+// Every problem's tiles under the plan's policy.
+static void tile_all(GemmPlan &g) {
+  for (auto &t : g.tiles) t.clear();
+  for (size_t p = 0; p < g.probs.size(); ++p)
+    add_tiles(g, (int32_t)p, g.probs[p].M, g.probs[p].N, g.policy);
   // largest K first for load balance
   std::vector<int64_t> ktot(g.probs.size(), 0);
   for (size_t i = 0; i < g.probs.size(); ++i)
@@ -681,15 +692,17 @@ static void sort_tiles(GemmPlan &g) {
 }
 
 void gemm_finalize(GemmPlan &g, bool cplx, bool upper) {
-  if (upper)
-    for (int c = 0; c < kNumCfg; ++c) {
-      auto &t = g.tiles[c];
-      t.erase(std::remove_if(t.begin(), t.end(),
-                             [&](const GTile &x) { return x.m0 > x.n0 + kCfgBN[c] - 1; }),
-              t.end());
-    }
-  sort_tiles(g);
   g.sl = slice_worth(g, cplx, upper, [&] { return slice_simple(g, cplx, upper); });
+  if (!g.sl) {
+    tile_all(g);
+    if (upper)
+      for (int c = 0; c < kNumCfg; ++c) {
+        auto &t = g.tiles[c];
+        t.erase(std::remove_if(t.begin(), t.end(),
+                               [&](const GTile &x) { return x.m0 > x.n0 + kCfgBN[c] - 1; }),
+                t.end());
+      }
+  }
   g.upload();
 }
 
@@ -698,10 +711,7 @@ void gemm_upload(GemmPlan &g) { g.upload(); }
 void gemm_retile(GemmPlan &g, int policy) {
   if (policy == g.policy) return;
   g.policy = policy;
-  for (auto &t : g.tiles) t.clear();
-  for (size_t p = 0; p < g.probs.size(); ++p)
-    add_tiles(g, (int32_t)p, g.probs[p].M, g.probs[p].N, policy);
-  sort_tiles(g);
+  tile_all(g);
   g.upload();
 }
 

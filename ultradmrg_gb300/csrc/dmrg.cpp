@@ -816,10 +816,9 @@ ExpmvResult lanczos_expmv(Ctx &ctx, MatvecPlan &mv, const BTensor &init_state, d
 
 // An environment update with the MPO tensor as a channel map: first . second
 // over one pair of axes gives T (a, x1, x2, b), W takes it to (a, y1, y2, b),
-// and `close` names the last contraction.  The three plans need block
-// structures only, so they are built on host threads and the device starts on
-// the first while the others are under way.  Null where W has imaginary
-// coefficients or the context asks for plain FP64 GEMMs.
+// and `close` names the last contraction.  Each plan needs block structures
+// only, so the next one is built while the device runs the one before.  Null
+// where W has imaginary coefficients or the context asks for plain FP64 GEMMs.
 struct EnvClose {
   bool map_left;  // the mapped tensor is the last contraction's first operand
   const BTensor &other;
@@ -832,35 +831,15 @@ static TensorPtr mapped_env(Ctx &ctx, const BTensor &first, const BTensor &secon
   bool real = true;
   const std::vector<double> wh = mpo_data(ctx, W, &real);
   if (!real) return nullptr;
-  std::vector<int> ca, cb, fa, fb;
-  cyclic_axes(first.rank(), second.rank(), ax_a, ax_b, 1, ca, cb, fa, fb);
-  UDMRG_REQUIRE(first.dtype == second.dtype, "contract: operands must have the same element type");
-  auto T = contract_struct(first, second, ca, cb, fa, fb);
-  auto M = mpo_map_struct(*T, W, x1, x2);
-  auto map = std::async(std::launch::async,
-                        [&] { return build_mpo_map(*T, W, wh, x1, x2, *M); });
-  auto last = std::async(std::launch::async, [&] {
-    return close.map_left ? plan_contract_axes(*M, close.other, close.ca, close.cb, false)
-                          : plan_contract_axes(close.other, *M, close.ca, close.cb, false);
-  });
-  std::exception_ptr err;  // both threads end before this scope does
-  TensorPtr t;
-  try {
-    auto p1 = plan_contract_cyclic(first, second, ax_a, ax_b, 1);
-    t = run_contract(ctx, *p1, first, second, dw);
-  } catch (...) {
-    err = std::current_exception();
-  }
-  map.wait();
-  last.wait();
-  if (err) std::rethrow_exception(err);
-  auto m = map.get();
+  auto t = contract_cyclic(ctx, first, second, ax_a, ax_b, 1, dw);
+  auto M = mpo_map_struct(*t, W, x1, x2);
+  auto m = build_mpo_map(*t, W, wh, x1, x2, *M);
   upload_mpo_step64(ctx, *m);
   M->alloc_data();
   run_mpo_step64(ctx, *m, t->data, M->data);
   t.reset();
-  auto p2 = last.get();
-  gemm_upload(p2->gemm);
+  auto p2 = close.map_left ? plan_contract_axes(*M, close.other, close.ca, close.cb)
+                           : plan_contract_axes(close.other, *M, close.ca, close.cb);
   return close.map_left ? run_contract(ctx, *p2, *M, close.other, dw)
                         : run_contract(ctx, *p2, close.other, *M, dw);
 }

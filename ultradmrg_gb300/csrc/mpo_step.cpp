@@ -99,7 +99,25 @@ struct PairMap {
   };
   std::vector<In> ins;
   std::vector<MpoOut64> outs;
-  std::vector<Nz> nz;
+  std::vector<Nz> nz, sorted;
+  std::vector<int32_t> start, at;
+  std::vector<std::pair<int64_t, int32_t>> in_first;  // input block -> its first channel
+  void clear() {
+    ins.clear();
+    outs.clear();
+    nz.clear();
+    in_first.clear();
+  }
+  // first channel of input block b, appended with `n` channels of `db` columns
+  // from offset off if it is new
+  int32_t input(int64_t b, int64_t off, int64_t n, int64_t db) {
+    for (const auto &f : in_first)
+      if (f.first == b) return f.second;
+    const int32_t c0 = (int32_t)ins.size();
+    in_first.push_back({b, c0});
+    for (int64_t c = 0; c < n; ++c) ins.push_back({off + c * db, n * db});
+    return c0;
+  }
 };
 
 // Appends the pair in CSR form (couplings of one (o, i) summed, by ascending i).
@@ -111,16 +129,22 @@ void push_pair(MpoStep64 &p, PairMap &m, int64_t da, int64_t db, int es) {
   pr.da = (int32_t)da;
   pr.db = (int32_t)(db * es);
   for (MpoOut64 o : m.outs) p.outs.push_back({o.base * es, o.astride * es, 0});
-  std::stable_sort(m.nz.begin(), m.nz.end(), [](const PairMap::Nz &x, const PairMap::Nz &y) {
-    return x.o != y.o ? x.o < y.o : x.i < y.i;
-  });
+  // couplings by output channel (counting sort, stable), then by input
+  m.start.assign(pr.nout + 1, 0);
+  for (const PairMap::Nz &z : m.nz) m.start[z.o + 1]++;
+  for (int o = 0; o < pr.nout; ++o) m.start[o + 1] += m.start[o];
+  m.sorted.resize(m.nz.size());
+  m.at.assign(m.start.begin(), m.start.end() - 1);
+  for (const PairMap::Nz &z : m.nz) m.sorted[m.at[z.o]++] = z;
   const size_t n0 = p.nz.size();
-  size_t q = 0;
   for (int o = 0; o < pr.nout; ++o) {
-    for (; q < m.nz.size() && m.nz[q].o == o;) {
+    auto b = m.sorted.begin() + m.start[o], e = m.sorted.begin() + m.start[o + 1];
+    auto less = [](const PairMap::Nz &x, const PairMap::Nz &y) { return x.i < y.i; };
+    if (!std::is_sorted(b, e, less)) std::stable_sort(b, e, less);
+    for (auto q = b; q != e;) {
       double v = 0.0;
-      const int i = m.nz[q].i;
-      for (; q < m.nz.size() && m.nz[q].o == o && m.nz[q].i == i; ++q) v += m.nz[q].v;
+      const int i = q->i;
+      for (; q != e && q->i == i; ++q) v += q->v;
       if (v == 0.0) continue;
       UDMRG_REQUIRE(m.ins[i].astride * es < (1ll << 31), "MPO step: block too large");
       p.nz.push_back({m.ins[i].base * es, v, (int32_t)(m.ins[i].astride * es), 0});
@@ -134,12 +158,33 @@ void push_pair(MpoStep64 &p, PairMap &m, int64_t da, int64_t db, int es) {
   p.pairs.push_back(pr);
 }
 
-// Blocks grouped by the sectors of their first and last axes.
-std::map<std::pair<int32_t, int32_t>, std::vector<int64_t>> by_ends(const BTensor &t) {
-  std::map<std::pair<int32_t, int32_t>, std::vector<int64_t>> m;
-  for (int64_t b = 0; b < t.nblocks(); ++b)
-    m[{t.key(b)[0], t.key(b)[t.rank() - 1]}].push_back(b);
-  return m;
+// Blocks with the sectors of their first and last axes, grouped by them
+// (ascending; block order within a pair).
+struct Ends {
+  int32_t a, b;
+  int64_t blk;
+};
+std::vector<Ends> by_ends(const BTensor &t) {
+  std::vector<Ends> v(t.nblocks());
+  for (int64_t b = 0; b < t.nblocks(); ++b) v[b] = {t.key(b)[0], t.key(b)[t.rank() - 1], b};
+  std::sort(v.begin(), v.end(), [](const Ends &x, const Ends &y) {
+    return x.a != y.a ? x.a < y.a : x.b != y.b ? x.b < y.b : x.blk < y.blk;
+  });
+  return v;
+}
+
+// Block of t with the given sector ids (blocks are sorted), or -1.
+int64_t find_block(const BTensor &t, const int32_t *k) {
+  const int r = t.rank();
+  int64_t lo = 0, hi = t.nblocks();
+  while (lo < hi) {
+    const int64_t mid = (lo + hi) / 2;
+    if (std::lexicographical_compare(t.key(mid), t.key(mid) + r, k, k + r))
+      lo = mid + 1;
+    else
+      hi = mid;
+  }
+  return lo < t.nblocks() && std::equal(k, k + r, t.key(lo)) ? lo : -1;
 }
 
 }  // namespace
@@ -148,18 +193,15 @@ std::unique_ptr<MpoStep64> build_mpo_step64(FusedMpo &fm, const BTensor &T1, con
   UDMRG_REQUIRE(T1.rank() == 5 && T3.rank() == 5, "MPO step: rank-5 intermediates expected");
   auto p = std::make_unique<MpoStep64>();
   const int es = elem_doubles(T1.dtype);
-  std::map<std::array<int32_t, 5>, int64_t> t1blk;  // (A', W, S1, S2, B)
-  for (int64_t b = 0; b < T1.nblocks(); ++b) {
-    const int32_t *k = T1.key(b);
-    t1blk[{k[0], k[1], k[2], k[3], k[4]}] = b;
-  }
   p->rowptr.push_back(0);
-  for (auto &kv : by_ends(T3)) {
-    const int32_t Ap = kv.first.first, Bs = kv.first.second;
+  const std::vector<Ends> ends = by_ends(T3);
+  PairMap m;
+  for (size_t g = 0; g < ends.size();) {
+    const int32_t Ap = ends[g].a, Bs = ends[g].b;
     const int64_t da = T3.idx[0].dims[Ap], db = T3.idx[4].dims[Bs];
-    PairMap m;
-    std::map<int64_t, int32_t> in_first;  // T1 block -> its first input channel
-    for (int64_t ob : kv.second) {
+    m.clear();
+    for (; g < ends.size() && ends[g].a == Ap && ends[g].b == Bs; ++g) {
+      const int64_t ob = ends[g].blk;
       const int32_t *k = T3.key(ob);
       const int64_t nout =
           T3.idx[1].dims[k[1]] * T3.idx[2].dims[k[2]] * T3.idx[3].dims[k[3]];
@@ -167,19 +209,16 @@ std::unique_ptr<MpoStep64> build_mpo_step64(FusedMpo &fm, const BTensor &T1, con
       for (int64_t c = 0; c < nout; ++c)
         m.outs.push_back({T3.offs[ob] + c * db, (int32_t)(nout * db), 0});
       for (const FusedMpo::Entry &e : fm.get(k[1], k[2], k[3])) {
-        auto tb = t1blk.find({Ap, e.src[0], e.src[1], e.src[2], Bs});
-        if (tb == t1blk.end()) continue;
+        const int32_t tk[5] = {Ap, e.src[0], e.src[1], e.src[2], Bs};
+        const int64_t tb = find_block(T1, tk);
+        if (tb < 0) continue;
         const int64_t nin = T1.idx[1].dims[e.src[0]] * T1.idx[2].dims[e.src[1]] *
                             T1.idx[3].dims[e.src[2]];
-        auto f = in_first.emplace(tb->second, (int32_t)m.ins.size());
-        if (f.second)
-          for (int64_t c = 0; c < nin; ++c)
-            m.ins.push_back({T1.offs[tb->second] + c * db, nin * db});
+        const int32_t ifirst = m.input(tb, T1.offs[tb], nin, db);
         for (int64_t ic = 0; ic < nin; ++ic)
           for (int64_t oc = 0; oc < nout; ++oc) {
             const double v = e.coef[ic * nout + oc];
-            if (v != 0.0)
-              m.nz.push_back({(int32_t)(ofirst + oc), (int32_t)(f.first->second + ic), v});
+            if (v != 0.0) m.nz.push_back({(int32_t)(ofirst + oc), (int32_t)(ifirst + ic), v});
           }
       }
     }
@@ -197,47 +236,62 @@ std::unique_ptr<MpoStep64> build_mpo_map(const BTensor &T, const BTensor &W,
   int y[2], ny = 0;
   for (int ax = 0; ax < 4; ++ax)
     if (ax != x1 && ax != x2) y[ny++] = ax;
-  std::map<std::array<int32_t, 4>, int64_t> tblk;
-  for (int64_t b = 0; b < T.nblocks(); ++b) {
-    const int32_t *k = T.key(b);
-    tblk[{k[0], k[1], k[2], k[3]}] = b;
+  // W's blocks by their output sectors, with the nonzeros of each
+  struct WNz {
+    int32_t i, o;
+    double v;
+  };
+  struct WBlk {
+    int32_t y1, y2, k1, k2;
+    int64_t nin;
+    std::vector<WNz> nz;
+  };
+  std::vector<WBlk> wb;
+  for (int64_t b = 0; b < W.nblocks(); ++b) {
+    const int32_t *kw = W.key(b);
+    const int64_t e1 = W.idx[x1].dims[kw[x1]], e2 = W.idx[x2].dims[kw[x2]];
+    const int64_t d1 = W.idx[y[0]].dims[kw[y[0]]], d2 = W.idx[y[1]].dims[kw[y[1]]];
+    int64_t st[4];
+    st[3] = 1;
+    for (int ax = 2; ax >= 0; --ax) st[ax] = st[ax + 1] * W.idx[ax + 1].dims[kw[ax + 1]];
+    WBlk w{kw[y[0]], kw[y[1]], kw[x1], kw[x2], e1 * e2, {}};
+    for (int64_t i1 = 0; i1 < e1; ++i1)
+      for (int64_t i2 = 0; i2 < e2; ++i2)
+        for (int64_t o1 = 0; o1 < d1; ++o1)
+          for (int64_t o2 = 0; o2 < d2; ++o2) {
+            const double v =
+                wh[W.offs[b] + i1 * st[x1] + i2 * st[x2] + o1 * st[y[0]] + o2 * st[y[1]]];
+            if (v != 0.0) w.nz.push_back({(int32_t)(i1 * e2 + i2), (int32_t)(o1 * d2 + o2), v});
+          }
+    wb.push_back(std::move(w));
   }
-  std::map<std::pair<int32_t, int32_t>, std::vector<int64_t>> w_by_y;
-  for (int64_t b = 0; b < W.nblocks(); ++b) w_by_y[{W.key(b)[y[0]], W.key(b)[y[1]]}].push_back(b);
+  std::stable_sort(wb.begin(), wb.end(), [](const WBlk &u, const WBlk &v) {
+    return u.y1 != v.y1 ? u.y1 < v.y1 : u.y2 < v.y2;
+  });
   p->rowptr.push_back(0);
-  for (auto &kv : by_ends(out)) {
-    const int32_t Ap = kv.first.first, Bs = kv.first.second;
+  const std::vector<Ends> ends = by_ends(out);
+  PairMap m;
+  for (size_t g = 0; g < ends.size();) {
+    const int32_t Ap = ends[g].a, Bs = ends[g].b;
     const int64_t da = out.idx[0].dims[Ap], db = out.idx[3].dims[Bs];
-    PairMap m;
-    std::map<int64_t, int32_t> in_first;
-    for (int64_t ob : kv.second) {
+    m.clear();
+    for (; g < ends.size() && ends[g].a == Ap && ends[g].b == Bs; ++g) {
+      const int64_t ob = ends[g].blk;
       const int32_t *k = out.key(ob);
       const int64_t d1 = out.idx[1].dims[k[1]], d2 = out.idx[2].dims[k[2]];
       const int32_t ofirst = (int32_t)m.outs.size();
       for (int64_t c = 0; c < d1 * d2; ++c)
         m.outs.push_back({out.offs[ob] + c * db, (int32_t)(d1 * d2 * db), 0});
-      for (int64_t wb : w_by_y[{k[1], k[2]}]) {
-        const int32_t *kw = W.key(wb);
-        auto tb = tblk.find({Ap, kw[x1], kw[x2], Bs});
-        if (tb == tblk.end()) continue;
-        const int64_t e1 = W.idx[x1].dims[kw[x1]], e2 = W.idx[x2].dims[kw[x2]];
-        auto f = in_first.emplace(tb->second, (int32_t)m.ins.size());
-        if (f.second)
-          for (int64_t c = 0; c < e1 * e2; ++c)
-            m.ins.push_back({T.offs[tb->second] + c * db, e1 * e2 * db});
-        int64_t st[4];
-        st[3] = 1;
-        for (int ax = 2; ax >= 0; --ax) st[ax] = st[ax + 1] * W.idx[ax + 1].dims[kw[ax + 1]];
-        for (int64_t i1 = 0; i1 < e1; ++i1)
-          for (int64_t i2 = 0; i2 < e2; ++i2)
-            for (int64_t o1 = 0; o1 < d1; ++o1)
-              for (int64_t o2 = 0; o2 < d2; ++o2) {
-                const double v = wh[W.offs[wb] + i1 * st[x1] + i2 * st[x2] + o1 * st[y[0]] +
-                                    o2 * st[y[1]]];
-                if (v != 0.0)
-                  m.nz.push_back({(int32_t)(ofirst + o1 * d2 + o2),
-                                  (int32_t)(f.first->second + i1 * e2 + i2), v});
-              }
+      auto it = std::lower_bound(wb.begin(), wb.end(), std::make_pair(k[1], k[2]),
+                                 [](const WBlk &u, const std::pair<int32_t, int32_t> &q) {
+                                   return u.y1 != q.first ? u.y1 < q.first : u.y2 < q.second;
+                                 });
+      for (; it != wb.end() && it->y1 == k[1] && it->y2 == k[2]; ++it) {
+        const int32_t tk[4] = {Ap, it->k1, it->k2, Bs};
+        const int64_t tb = find_block(T, tk);
+        if (tb < 0) continue;
+        const int32_t ifirst = m.input(tb, T.offs[tb], it->nin, db);
+        for (const WNz &z : it->nz) m.nz.push_back({ofirst + z.o, ifirst + z.i, z.v});
       }
     }
     push_pair(*p, m, da, db, es);

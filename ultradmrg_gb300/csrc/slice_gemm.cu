@@ -458,15 +458,6 @@ int SlicePlan::add_group(const Dims &d, const std::vector<SlLine> &rows,
   g.v_img = img_bytes;
   img_bytes += vt * g.kc * kSlUnitV;
   const int32_t id = (int32_t)groups.size();
-  for (int64_t i = 0; i < ut; ++i)
-    for (int64_t j = 0; j < vt; ++j) {
-      if (upper) {  // rows m, columns n: drop tiles with every n < m
-        const int64_t n1 = (g.lanes_n ? i * kSlU + kSlU - 1 : j * kSlV + kSlV - 1) * d.M / d.N;
-        const int64_t m0 = g.lanes_n ? j * kSlV : i * kSlU;
-        if (m0 > n1) continue;
-      }
-      tiles.push_back({id, (int32_t)i, (int32_t)j, 0});
-    }
   if (d.K % kSlK) holes = true;
   groups.push_back(g);
   return id;
@@ -492,9 +483,24 @@ void SlicePlan::finalize() {
     for (int32_t r = 0; r < ops[o].rows; r += 32)
       for (int32_t k = 0; k < ops[o].cols; k += 64) items.push_back({(int32_t)o, r, k, 0});
   // largest K first (longest processing time first over the persistent grid)
-  std::stable_sort(tiles.begin(), tiles.end(), [&](const SlTile &x, const SlTile &y) {
-    return groups[x.group].kc > groups[y.group].kc;
-  });
+  std::vector<int> order(groups.size());
+  for (size_t g = 0; g < order.size(); ++g) order[g] = (int)g;
+  std::stable_sort(order.begin(), order.end(),
+                   [&](int x, int y) { return groups[x].kc > groups[y].kc; });
+  tiles.clear();
+  for (int id : order) {
+    const SlGroup &g = groups[id];
+    const int es = g.upper && g.lanes_n ? g.nu / std::max(g.nv, 1) : g.nv / std::max(g.nu, 1);
+    for (int32_t i = 0; i * kSlU < g.nu; ++i)
+      for (int32_t j = 0; j * kSlV < g.nv; ++j) {
+        if (g.upper) {  // rows m, columns n: drop tiles with every n < m
+          const int n1 = (g.lanes_n ? i * kSlU + kSlU - 1 : j * kSlV + kSlV - 1) / std::max(es, 1);
+          const int m0 = g.lanes_n ? j * kSlV : i * kSlU;
+          if (m0 > n1) continue;
+        }
+        tiles.push_back({id, i, j, 0});
+      }
+  }
 }
 
 void SlicePlan::upload() {
