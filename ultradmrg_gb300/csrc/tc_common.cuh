@@ -127,6 +127,14 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
          | ((uint32_t)(M >> 4) << 24); // M / 16
 }
 
+// Tile of round i of a persistent block over a list sorted by descending work:
+// rounds alternate in direction, so that the block with the longest tile of one
+// round gets the shortest of the next.
+__device__ __forceinline__ int snake_tile(int i) {
+  const int g = gridDim.x, b = blockIdx.x;
+  return i * g + (i & 1 ? g - 1 - b : b);
+}
+
 // Programmatic dependent launch.  A kernel launched with launch_pdl may
 // start while its predecessor on the stream is still running: it calls
 // pdl_wait() before it touches anything the predecessor writes (a no-op when

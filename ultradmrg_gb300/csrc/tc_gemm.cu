@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(256)
 }
 
 // Warp-specialised persistent kernel over the tile list (static schedule
-// t = blockIdx.x + i * gridDim.x): warp 0 stages both operands by bulk copies
+// tc::snake_tile): warp 0 stages both operands by bulk copies
 // from their images, warp 1 issues the MMAs, warps 2-5 drain the
 // accumulators.
 template <int BN>
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (warp == 0) {
     if (lane == 0) {  // producer: one bulk copy per operand unit and chunk (per plane at K's end)
       uint32_t G = 0;
-      for (int t = blockIdx.x; t < ntiles && !*b.abort_flag; t += gridDim.x) {
+      for (int i = 0, t; (t = tc::snake_tile(i)) < ntiles && !*b.abort_flag; ++i) {
         const TcTile tile = tiles[t];
         const TcGroup g = groups[tile.group];
         const uint8_t *abase = aimg + g.a_img + (int64_t)tile.mtile * g.kc * kTcUnitA;

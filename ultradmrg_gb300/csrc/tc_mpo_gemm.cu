@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
     constexpr int64_t planeA = (int64_t)kTcBM * kTcBK * 2;
     uint32_t G = 0;
     bool ok = true;
-    for (int t = blockIdx.x; ok && t < ntiles && !*b.abort_flag; t += gridDim.x) {
+    for (int i = 0, t; ok && (t = tc::snake_tile(i)) < ntiles && !*b.abort_flag; ++i) {
       const TcTile tile = tiles[t];
       const TcGroup g = groups[tile.group];
       const MpoGroupMap gm = gmap[tile.group];

@@ -215,7 +215,7 @@ __device__ __forceinline__ int tc_chunk_k(const TcGroup &g, int c) {
 }
 
 // MMA issue (one thread) over the CTA's tiles (static schedule
-// t = blockIdx.x + i * gridDim.x): for each K chunk, wait for its stage,
+// tc::snake_tile): for each K chunk, wait for its stage,
 // issue the six split products per 16-deep K step, release the stage; after
 // the last chunk, hand the accumulator to the epilogue.
 template <int BN>
@@ -225,7 +225,7 @@ __device__ __forceinline__ void tc_mma_role(const TcTile *__restrict__ tiles, in
   using S = TcShape<BN>;
   constexpr uint32_t idesc = tc::idesc_bf16_f32(kTcBM, BN);
   uint32_t G = 0, i = 0;
-  for (int t = blockIdx.x; t < ntiles && !*b.abort_flag; t += gridDim.x, ++i) {
+  for (int t; (t = tc::snake_tile((int)i)) < ntiles && !*b.abort_flag; ++i) {
     const TcGroup g = groups[tiles[t].group];
     const uint32_t acc = i & 1;
     if (i >= kAcc && !wait_phase(&b.tempty[acc], ((i >> 1) - 1) & 1)) {
@@ -285,7 +285,7 @@ __device__ __forceinline__ void tc_epilogue_role(int q, int lane,
                                                  uint32_t tmem, int *err) {
     const int m = q * 32 + lane;
     uint32_t i = 0;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++i) {
+    for (int t; (t = tc::snake_tile((int)i)) < ntiles; ++i) {
       const TcTile tile = tiles[t];
       const TcGroup g = groups[tile.group];
       const uint32_t acc = i & 1;
