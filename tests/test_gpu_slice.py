@@ -60,6 +60,14 @@ def test_tile_edges(ctx, m, n, k, cplx):
     check(product(ctx, a, b), a, b)
 
 
+@pytest.mark.parametrize("k", [376, 384, 400, 2047, 2305, 5001])
+def test_k_parts(ctx, k):
+    """Few tiles of a long contraction: split over K parts of at least 256."""
+    rng = np.random.default_rng(k)
+    a, b = rng.standard_normal((130, k)), rng.standard_normal((k, 33))
+    check(product(ctx, a, b), a, b)
+
+
 @pytest.mark.parametrize("kind", ["ones", "graded", "scaled", "zero_rows", "powers"])
 def test_values(ctx, kind):
     rng = np.random.default_rng(5)

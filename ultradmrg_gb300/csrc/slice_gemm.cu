@@ -105,12 +105,42 @@ __device__ __forceinline__ int64_t slice_bits(double x, int be, bool neg) {
   return v + 0x80808080808080ll;
 }
 
+// Eight consecutive columns of one row into their eight 16-byte plane segments: a
+// byte of slice_bits becomes a float by the 2^23 + byte pattern (one byte
+// permute and one FP32 add per digit), two floats' upper halves a BF16 pair.
+__device__ __forceinline__ void store_digits(const double (&x)[8], int be, bool neg, uint8_t *o,
+                                             int64_t plane) {
+  uint32_t p[kSlDigits][4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    float f[2][kSlDigits];
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      const int64_t v = slice_bits(x[2 * j + t], be, neg);
+      const uint32_t lo = (uint32_t)v, hi = (uint32_t)(v >> 32);
+      f[t][0] = __uint_as_float(0x4B000000u + 128u + (uint32_t)((int32_t)hi >> 24));
+      f[t][1] = __uint_as_float(__byte_perm(hi, 0x4B000000u, 0x7652));
+      f[t][2] = __uint_as_float(__byte_perm(hi, 0x4B000000u, 0x7651));
+      f[t][3] = __uint_as_float(__byte_perm(hi, 0x4B000000u, 0x7650));
+      f[t][4] = __uint_as_float(__byte_perm(lo, 0x4B000000u, 0x7653));
+      f[t][5] = __uint_as_float(__byte_perm(lo, 0x4B000000u, 0x7652));
+      f[t][6] = __uint_as_float(__byte_perm(lo, 0x4B000000u, 0x7651));
+      f[t][7] = __uint_as_float(__byte_perm(lo, 0x4B000000u, 0x7650));
+    }
+#pragma unroll
+    for (int d = 0; d < kSlDigits; ++d)
+      p[d][j] = __byte_perm(__float_as_uint(f[0][d] - 8388736.0f),
+                            __float_as_uint(f[1][d] - 8388736.0f), 0x7632);
+  }
+#pragma unroll
+  for (int d = 0; d < kSlDigits; ++d)
+    *(uint4 *)(o + d * plane) = make_uint4(p[d][0], p[d][1], p[d][2], p[d][3]);
+}
+
 // Digits of the operands into their images.  A work item is 32 rows x 64
 // columns of one op, staged in shared memory along the source's contiguous
-// direction; then a thread cuts one row's 8 consecutive columns into eight
-// 16-byte plane segments (a byte of slice_bits becomes a float by the
-// 2^23 + byte pattern: one byte permute and one FP32 add per digit), and the
-// 32 rows of a warp fill 512 contiguous bytes per plane.  HBM bound: 8 B read
+// direction; then a thread cuts one row's 8 consecutive columns, and the 32
+// rows of a warp fill 512 contiguous bytes per plane.  HBM bound: 8 B read
 // and 16 B written per element.  Ops start at columns that are multiples of 8; the
 // columns from an op's edge to the next one are written as zeros.  A line whose
 // largest element is non-finite or outside the sliced range raises the flag.
@@ -147,45 +177,74 @@ __global__ void __launch_bounds__(kPackThreads)
     const int64_t plane = (int64_t)tr * kSlK * 2;
     const int64_t tbase = op.img_off + (int64_t)(row >> ts) * op.kc * kSlDigits * plane;
     const int rin = row & (tr - 1);
-    const int n = min(8, op.cols - ks);
-    float f[kSlDigits][8];
+    double x[8];  // (zeros past the op's columns)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int64_t v = j < n ? slice_bits(tile[g * 8 + j][r], be, op.neg != 0)
-                              : 0x80808080808080ll;
-      const uint32_t lo = (uint32_t)v, hi = (uint32_t)(v >> 32);
-      f[0][j] = __uint_as_float(0x4B000000u + 128u + (uint32_t)((int32_t)hi >> 24)) - 8388736.0f;
-      f[1][j] = __uint_as_float(__byte_perm(hi, 0x4B000000u, 0x7652)) - 8388736.0f;
-      f[2][j] = __uint_as_float(__byte_perm(hi, 0x4B000000u, 0x7651)) - 8388736.0f;
-      f[3][j] = __uint_as_float(__byte_perm(hi, 0x4B000000u, 0x7650)) - 8388736.0f;
-      f[4][j] = __uint_as_float(__byte_perm(lo, 0x4B000000u, 0x7653)) - 8388736.0f;
-      f[5][j] = __uint_as_float(__byte_perm(lo, 0x4B000000u, 0x7652)) - 8388736.0f;
-      f[6][j] = __uint_as_float(__byte_perm(lo, 0x4B000000u, 0x7651)) - 8388736.0f;
-      f[7][j] = __uint_as_float(__byte_perm(lo, 0x4B000000u, 0x7650)) - 8388736.0f;
+    for (int j = 0; j < 8; ++j) x[j] = tile[g * 8 + j][r];
+    store_digits(x, be, op.neg != 0,
+                 img + tbase + (int64_t)(col >> 4) * kSlDigits * plane +
+                     canon_off(rin, col & 15, tr), plane);
+  }
+}
+
+// The same for ops whose columns are contiguous (or every second double:
+// complex parts): no shared memory.  A warp takes 8 rows x 32 columns at a time,
+// lane = (column group, row): eight loads of its row's 64 bytes (consecutive
+// lanes' rows share no sectors, but each sector is used whole over the eight),
+// then the plane segments of eight rows fill 128 contiguous bytes.
+constexpr int kPackCols = 128;  // columns of a work item
+__global__ void __launch_bounds__(kPackThreads)
+    slice_pack_k_kernel(const SlOp *__restrict__ ops, const SlItem *__restrict__ items, int nitems,
+                        const double *__restrict__ a, const double *__restrict__ b,
+                        int *__restrict__ scale, uint8_t *__restrict__ img) {
+  const int lane = threadIdx.x & 31, r = lane & 7, g = lane >> 3;
+  const int wpb = blockDim.x >> 5;
+  for (int w = blockIdx.x * wpb + (threadIdx.x >> 5); w < nitems; w += gridDim.x * wpb) {
+    const SlItem it = items[w];
+    const SlOp &op = ops[it.op];
+    const int rs = it.r0 + r;
+    if (rs >= op.rows) continue;
+    const double *src = (op.src ? b : a) + op.src_off + sl_off(rs, op.re, op.rs, op.nr);
+    const int es = op.nk ? (int)op.ks[0] : 1;
+    const int row = op.r0 + rs * op.rstep;
+    const int sc = scale[2 + op.sc0 + row];
+    const int be = sc == 0 ? 0x7FF : sc >> 20;
+    if (sc != 0 && (be < kLoExp || be > kHiExp)) atomicExch(scale, 1);
+    const int tr = op.tr, ts = tr == kSlU ? 7 : 6;
+    const int64_t plane = (int64_t)tr * kSlK * 2;
+    uint8_t *orow = img + op.img_off + (int64_t)(row >> ts) * op.kc * kSlDigits * plane;
+    const int rin = row & (tr - 1), end = min(op.cols, it.k0 + kPackCols);
+    const bool neg = op.neg != 0;
+    for (int ks = it.k0 + g * 8; ks < end; ks += 32) {
+      const int n = min(8, op.cols - ks), col = op.k0 + ks;
+      double x[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) x[j] = j < n ? __ldg(src + (ks + j) * es) : 0.0;
+      store_digits(x, be, neg, orow + (int64_t)(col >> 4) * kSlDigits * plane +
+                                   canon_off(rin, col & 15, tr), plane);
     }
-    uint8_t *o = img + tbase + (int64_t)(col >> 4) * kSlDigits * plane +
-                 canon_off(rin, col & 15, tr);
-#pragma unroll
-    for (int p = 0; p < kSlDigits; ++p)
-      *(uint4 *)(o + p * plane) =
-          make_uint4(__byte_perm(__float_as_uint(f[p][0]), __float_as_uint(f[p][1]), 0x7632),
-                     __byte_perm(__float_as_uint(f[p][2]), __float_as_uint(f[p][3]), 0x7632),
-                     __byte_perm(__float_as_uint(f[p][4]), __float_as_uint(f[p][5]), 0x7632),
-                     __byte_perm(__float_as_uint(f[p][6]), __float_as_uint(f[p][7]), 0x7632));
   }
 }
 
 // ---- the GEMM ----
 //
-// Warp-specialised persistent kernel over the tile list (t = blockIdx.x + i *
-// gridDim.x): warp 0 stages the two operands' K steps by bulk copies (four
-// stages of 48 KB), warp 1 issues 36 tcgen05.mma (M 128, N 64, K 16) per step
-// into eight 64-column accumulators (all 512 TMEM columns), warps 2 .. 9 drain
-// them after every kSlChunk steps.  An epilogue thread owns 32 outputs of one
-// lane; it adds the levels into two 64-bit integers per output and frees the
-// accumulators before it rounds and stores, so the next chunk's products
-// overlap the rounding.  Every wait is bounded.
-constexpr int kSlThreads = 320;
+// Warp-specialised persistent kernel over the tile list: warp 0 stages the two
+// operands' K steps by bulk copies (four stages of 48 KB), warp 1 issues 36
+// tcgen05.mma (M 128, N 64, K 16) per step into eight 64-column accumulators
+// (all 512 TMEM columns), warps 2 .. 17 drain them after every kSlChunk steps.
+// An epilogue thread owns 16 outputs of one lane; it adds the levels into a
+// 96-bit integer per output and frees the accumulators before it rounds and
+// stores, so the next chunk's products overlap the rounding.  Every wait is
+// bounded.
+//
+// Bound by the draining: the accumulators take all of TMEM, so the tensor core
+// waits while they are read, and the 64-bit integer sums cost more issue slots
+// than the 36 products of a step.  Sixteen warps of 16 outputs (three registers
+// each: no spills at the 96 registers that 576 threads leave) against eight of
+// 32: Hubbard 4x8, D = 1000, effective Hamiltonian 549 -> 402 us together with
+// the K parts and slice_pack_k_kernel.
+constexpr int kSlParts = 4;  // epilogue warps per lane quarter
+constexpr int kSlCols = kSlV / kSlParts;
+constexpr int kSlThreads = 64 + 128 * kSlParts;
 constexpr int kSlStages = 4;
 constexpr int kSlStageBytes = (int)(kSlUnitU + kSlUnitV);
 constexpr int kSlBarOffset = kSlStages * kSlStageBytes + kPadBytes;
@@ -204,19 +263,29 @@ __device__ __forceinline__ void sl_fail(SlBars *b, int *flags) {
   b->abort = 1;
 }
 
-// 32 lanes x 32 bit, 4 consecutive columns per thread
-__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+// 32 lanes x 32 bit, 2 consecutive columns per thread
+__device__ __forceinline__ void tmem_ld2(uint32_t taddr, uint32_t (&r)[2]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];"
+               : "=r"(r[0]), "=r"(r[1])
                : "r"(taddr)
                : "memory");
 }
 
-// (hi 2^32 + lo) 2^(e - 68) rounded to nearest FP64; |hi| < 2^62, the sum of
-// the level products with the lowest level's unit 2^-68
-__device__ __forceinline__ double sl_round(int64_t hi, int64_t lo, int e) {
-  hi += lo >> 32;
-  uint32_t w0 = (uint32_t)lo;
+// A sum of level products in units of 2^-68: hi 2^32 + lo, hi signed.
+struct SlSum {
+  int64_t hi;
+  uint32_t lo;
+};
+__device__ __forceinline__ void sl_add(SlSum &s, int64_t hi, int64_t lo) {  // + hi 2^32 + lo
+  lo += s.lo;
+  s.hi += hi + (lo >> 32);
+  s.lo = (uint32_t)lo;
+}
+
+// s 2^(e - 68) rounded to nearest FP64; |hi| < 2^62
+__device__ __forceinline__ double sl_round(const SlSum &s, int e) {
+  const int64_t hi = s.hi;
+  uint32_t w0 = s.lo;
   const bool neg = hi < 0;
   uint64_t h = (uint64_t)hi;
   if (neg) {
@@ -250,7 +319,8 @@ __global__ void __launch_bounds__(kSlThreads, 1)
     slice_gemm_kernel(const SlTile *__restrict__ tiles, int ntiles,
                       const SlGroup *__restrict__ groups, const SlLine *__restrict__ lines,
                       const int64_t *__restrict__ cblk, const int *__restrict__ scale,
-                      const uint8_t *__restrict__ img, double *__restrict__ C, int *flags) {
+                      const uint8_t *__restrict__ img, double *__restrict__ C, int *flags,
+                      longlong2 *__restrict__ scratch, int *__restrict__ arrived) {
   extern __shared__ __align__(1024) uint8_t smem[];
   SlBars *b = (SlBars *)(smem + kSlBarOffset);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -261,7 +331,7 @@ __global__ void __launch_bounds__(kSlThreads, 1)
       tc::mbar_init(&b->empty[s], 1);
     }
     tc::mbar_init(&b->tfull, 1);
-    tc::mbar_init(&b->tempty, 8);  // one arrival per epilogue warp
+    tc::mbar_init(&b->tempty, 4 * kSlParts);  // one arrival per epilogue warp
     tc::mbar_init(&b->fin, 1);
     b->abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -278,12 +348,13 @@ __global__ void __launch_bounds__(kSlThreads, 1)
   if (warp == 0) {
     if (lane == 0) {
       uint32_t G = 0;
-      for (int t = blockIdx.x; t < ntiles && !b->abort; t += gridDim.x) {
+      for (int i = 0, t; (t = tc::snake_tile(i)) < ntiles && !b->abort; ++i) {
         const SlTile tile = tiles[t];
         const SlGroup g = groups[tile.group];
         const uint8_t *u = img + g.u_img + (int64_t)tile.ut * g.kc * kSlUnitU;
         const uint8_t *v = img + g.v_img + (int64_t)tile.vt * g.kc * kSlUnitV;
-        for (int c = 0; c < g.kc; ++c, ++G) {
+        const int c0 = tile.part * g.kpart, c1 = min(g.kc, c0 + g.kpart);
+        for (int c = c0; c < c1; ++c, ++G) {
           const uint32_t s = G % kSlStages;
           if (G >= kSlStages && !wait_phase(&b->empty[s], ((G / kSlStages) - 1) & 1)) {
             sl_fail(b, flags);
@@ -304,8 +375,9 @@ __global__ void __launch_bounds__(kSlThreads, 1)
       constexpr uint32_t idesc = tc::idesc_bf16_f32(kSlU, kSlV);
       uint32_t G = 0, n = 0;  // K steps, chunks so far
       bool ok = true;
-      for (int t = blockIdx.x; t < ntiles && ok && !b->abort; t += gridDim.x) {
-        const int kc = groups[tiles[t].group].kc;
+      for (int i = 0, t; (t = tc::snake_tile(i)) < ntiles && ok && !b->abort; ++i) {
+        const SlGroup &g = groups[tiles[t].group];
+        const int kc = min(g.kpart, g.kc - tiles[t].part * g.kpart);
         for (int c = 0; c < kc && ok; ++c, ++G) {
           const bool first = c % kSlChunk == 0;
           if (first) {
@@ -325,16 +397,25 @@ __global__ void __launch_bounds__(kSlThreads, 1)
           const uint32_t sv = su + (uint32_t)kSlUnitU;
           constexpr uint32_t planeU = kSlU * kSlK * 2, planeV = kSlV * kSlK * 2;
 #pragma unroll
-          for (int i = 0; i < kSlDigits; ++i) {
+          for (int u = 0; u < kSlDigits; ++u) {
             const uint64_t ad =
-                tc::make_desc(su + i * planeU, (kSlU / 8) * 128, 128);
+                tc::make_desc(su + u * planeU, (kSlU / 8) * 128, 128);
 #pragma unroll
             for (int j = 0; j < kSlDigits; ++j) {
-              if (i + j >= kSlLevels) break;
+              if (u + j >= kSlLevels) break;
               const uint64_t bd =
                   tc::make_desc(sv + j * planeV, (kSlV / 8) * 128, 128);
               // digit pair (0, l) is the first product of level l
-              tc::mma_bf16(tmem + (i + j) * kSlV, ad, bd, idesc, first && i == 0 ? 0u : 1u);
+              const uint32_t d = tmem + (u + j) * kSlV, acc = first && u == 0 ? 0u : 1u;
+              // U plane u stays in the collector over its products
+              if (u + 1 == kSlDigits)
+                tc::mma_bf16(d, ad, bd, idesc, acc);
+              else if (j == 0)
+                tc::mma_bf16_a<tc::kCollectFill>(d, ad, bd, idesc, acc);
+              else if (u + j + 1 == kSlLevels)
+                tc::mma_bf16_a<tc::kCollectLast>(d, ad, bd, idesc, acc);
+              else
+                tc::mma_bf16_a<tc::kCollectUse>(d, ad, bd, idesc, acc);
             }
           }
           tc::mma_commit(&b->empty[s]);
@@ -346,37 +427,53 @@ __global__ void __launch_bounds__(kSlThreads, 1)
       if (!wait_phase(&b->fin, 0)) sl_fail(b, flags);
     }
   } else {
-    const int q = warp & 3, half = (warp - 2) >> 2;
+    const int q = warp & 3, part = (warp - 2) >> 2;  // lane quarter, column part
     uint32_t n = 0;  // chunks so far
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    for (int i = 0, t; (t = tc::snake_tile(i)) < ntiles; ++i) {
       const SlTile tile = tiles[t];
       const SlGroup g = groups[tile.group];
-      int64_t hi[32], lo[32];
+      // the lane's own line, and lane j's register line j
+      const int64_t ui = (int64_t)tile.ut * kSlU + q * 32 + lane;
+      const bool uok = ui < g.nu;
+      const SlLine ul = uok ? lines[g.u0 + ui] : SlLine{0, 0, 0, 0};
+      const int64_t vi = (int64_t)tile.vt * kSlV + part * kSlCols + lane;
+      const bool vok = lane < kSlCols && vi < g.nv;
+      const SlLine vl = vok ? lines[g.v0 + vi] : SlLine{-1, 0, 0, 0};
+      // a line without nonzero elements has scale 0: its sums are zero
+      const int ue = (uok ? scale[2 + g.u0 + ui] >> 20 : 0) - 1022;
+      const int ve = (vok ? scale[2 + g.v0 + vi] >> 20 : 0) - 1022;
+      SlSum sum[kSlCols];
 #pragma unroll
-      for (int j = 0; j < 32; ++j) hi[j] = lo[j] = 0;
+      for (int j = 0; j < kSlCols; ++j) sum[j] = SlSum{0, 0};
       bool ok = true;
-      for (int c0 = 0; c0 < g.kc; c0 += kSlChunk, ++n) {
+      // pieces entirely past the result's edge are neither read nor rounded
+      const bool live = tile.ut * kSlU + q * 32 < g.nu &&
+                        tile.vt * kSlV + part * kSlCols < g.nv;
+      const int kc = min(g.kpart, g.kc - tile.part * g.kpart);
+      for (int c0 = 0; c0 < kc; c0 += kSlChunk, ++n) {
         if (b->abort || !wait_phase(&b->tfull, n & 1)) {
           ok = false;
           break;
         }
         tc::fence_after_sync();
-        const uint32_t base = tmem + ((uint32_t)(q * 32) << 16) + half * 32;
+        const uint32_t base = tmem + ((uint32_t)(q * 32) << 16) + part * kSlCols;
+        if (live)
 #pragma unroll
-        for (int cb = 0; cb < 8; ++cb) {
-          uint32_t r[kSlLevels][4];
+        for (int cb = 0; cb < kSlCols / 2; ++cb) {
+          uint32_t r[kSlLevels][2];
 #pragma unroll
-          for (int l = 0; l < kSlLevels; ++l) tmem_ld4(base + l * kSlV + cb * 4, r[l]);
+          for (int l = 0; l < kSlLevels; ++l) tmem_ld2(base + l * kSlV + cb * 2, r[l]);
           tc::tmem_wait_ld();
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
+          for (int j = 0; j < 2; ++j) {
             int v[kSlLevels];
 #pragma unroll
             for (int l = 0; l < kSlLevels; ++l) v[l] = __float2int_rn(__uint_as_float(r[l][j]));
-            hi[cb * 4 + j] += (int64_t)v[0] * (1 << 24) + (int64_t)v[1] * (1 << 16) +
-                              (int64_t)v[2] * (1 << 8) + (int64_t)v[3];
-            lo[cb * 4 + j] += (int64_t)v[4] * (1 << 24) + (int64_t)v[5] * (1 << 16) +
-                              (int64_t)v[6] * (1 << 8) + (int64_t)v[7];
+            sl_add(sum[cb * 2 + j],
+                   (int64_t)v[0] * (1 << 24) + (int64_t)v[1] * (1 << 16) +
+                       (int64_t)v[2] * (1 << 8) + (int64_t)v[3],
+                   (int64_t)v[4] * (1 << 24) + (int64_t)v[5] * (1 << 16) +
+                       (int64_t)v[6] * (1 << 8) + (int64_t)v[7]);
           }
         }
         tc::fence_before_sync();
@@ -387,30 +484,54 @@ __global__ void __launch_bounds__(kSlThreads, 1)
         if (lane == 0) sl_fail(b, flags);
         break;
       }
-      const int64_t ui = (int64_t)tile.ut * kSlU + q * 32 + lane;
-      const bool uok = ui < g.nu;
-      const SlLine ul = uok ? lines[g.u0 + ui] : SlLine{0, 0, 0, 0};
-      // a line without nonzero elements has scale 0: its sums are zero
-      const int ue = uok ? (scale[2 + g.u0 + ui] >> 20) - 1022 : 0;
-      int64_t cb = -1;
-      int blk = -1;
-      const int64_t vi0 = (int64_t)tile.vt * kSlV + half * 32;
+      if (!live) continue;
+      if (tile.part0 >= 0) {
+        // the integer sums of this K part; the warp that arrives last for its
+        // piece of the tile adds the others' (exact, so the order is free)
+        const int w = q * kSlParts + part;
+        auto slot = [&](int p) {
+          return scratch + ((int64_t)(tile.part0 + p) * kSlU * kSlV + w * (32 * kSlCols) + lane);
+        };
+        longlong2 *mine = slot(tile.part);
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const int64_t vi = vi0 + j;
-        if (vi >= g.nv) break;
-        const SlLine vl = lines[g.v0 + vi];
-        const int ve = (scale[2 + g.v0 + vi] >> 20) - 1022;
-        if (vl.blk != blk) {
-          blk = vl.blk;
-          cb = !uok ? -1
-                    : cblk[g.cb0 + (g.lanes_n ? (int64_t)vl.blk * g.ncb + ul.blk
-                                              : (int64_t)ul.blk * g.ncb + vl.blk)];
+        for (int j = 0; j < kSlCols; ++j) __stcg(mine + 32 * j, make_longlong2(sum[j].hi, sum[j].lo));
+        __threadfence();
+        __syncwarp();
+        int before = 0;
+        if (lane == 0) before = atomicAdd(arrived + (int64_t)tile.part0 * 16 + w, 1);
+        if (__shfl_sync(0xffffffffu, before, 0) != g.parts - 1) continue;
+        __threadfence();
+        for (int p = 0; p < g.parts; ++p) {
+          if (p == tile.part) continue;
+          const longlong2 *o = slot(p);
+#pragma unroll
+          for (int j = 0; j < kSlCols; ++j) {
+            const longlong2 x = __ldcg(o + 32 * j);
+            sl_add(sum[j], x.x, x.y);
+          }
         }
-        if (cb < 0) continue;
-        const int64_t at = cb + (g.lanes_n ? (int64_t)vl.loc * ul.w + ul.loc
-                                           : (int64_t)ul.loc * vl.w + vl.loc);
-        C[at] = sl_round(hi[j], lo[j], ue + ve);
+      }
+      // within a block consecutive register lines are a fixed stride apart
+      int64_t at = -1;
+      int blk = -1;
+      const int64_t step = g.lanes_n ? ul.w : 1;
+#pragma unroll
+      for (int j = 0; j < kSlCols; ++j) {
+        const double x = sl_round(sum[j], ue + __shfl_sync(0xffffffffu, ve, j));
+        const int bj = __shfl_sync(0xffffffffu, vl.blk, j);
+        at += step;
+        if (bj != blk) {  // warp-uniform
+          blk = bj;
+          const int loc = __shfl_sync(0xffffffffu, vl.loc, j);
+          const int w = __shfl_sync(0xffffffffu, vl.w, j);
+          const int64_t cb =
+              bj < 0 || !uok ? -1
+                             : cblk[g.cb0 + (g.lanes_n ? (int64_t)bj * g.ncb + ul.blk
+                                                       : (int64_t)ul.blk * g.ncb + bj)];
+          at = cb < 0 ? INT64_MIN / 2
+                      : cb + (g.lanes_n ? (int64_t)loc * ul.w + ul.loc : (int64_t)ul.loc * w + loc);
+        }
+        if (at >= 0) C[at] = x;
       }
     }
   }
@@ -479,68 +600,121 @@ void SlicePlan::add_op(int group, SlOp op) {
 
 void SlicePlan::finalize() {
   items.clear();
-  for (size_t o = 0; o < ops.size(); ++o)
-    for (int32_t r = 0; r < ops[o].rows; r += 32)
-      for (int32_t k = 0; k < ops[o].cols; k += 64) items.push_back({(int32_t)o, r, k, 0});
-  // largest K first (longest processing time first over the persistent grid)
-  std::vector<int> order(groups.size());
-  for (size_t g = 0; g < order.size(); ++g) order[g] = (int)g;
-  std::stable_sort(order.begin(), order.end(),
-                   [&](int x, int y) { return groups[x].kc > groups[y].kc; });
-  tiles.clear();
-  for (int id : order) {
-    const SlGroup &g = groups[id];
-    const int es = g.upper && g.lanes_n ? g.nu / std::max(g.nv, 1) : g.nv / std::max(g.nu, 1);
-    for (int32_t i = 0; i * kSlU < g.nu; ++i)
-      for (int32_t j = 0; j * kSlV < g.nv; ++j) {
-        if (g.upper) {  // rows m, columns n: drop tiles with every n < m
-          const int n1 = (g.lanes_n ? i * kSlU + kSlU - 1 : j * kSlV + kSlV - 1) / std::max(es, 1);
-          const int m0 = g.lanes_n ? j * kSlV : i * kSlU;
-          if (m0 > n1) continue;
-        }
-        tiles.push_back({id, i, j, 0});
-      }
+  items_k.clear();
+  items_t.clear();
+  for (size_t o = 0; o < ops.size(); ++o) {
+    const SlOp &op = ops[o];
+    for (int32_t r = 0; r < op.rows; r += 32)
+      for (int32_t k = 0; k < op.cols; k += 64) items.push_back({(int32_t)o, r, k, 0});
+    if (!op.rows_fast && op.nk <= 1 && (op.nk == 0 || op.ks[0] <= 2)) {
+      for (int32_t r = 0; r < op.rows; r += 8)
+        for (int32_t k = 0; k < op.cols; k += kPackCols) items_k.push_back({(int32_t)o, r, k, 0});
+    } else {
+      for (int32_t r = 0; r < op.rows; r += 32)
+        for (int32_t k = 0; k < op.cols; k += 64) items_t.push_back({(int32_t)o, r, k, 0});
+    }
   }
+  // K parts: a unit of work is at most about a third of one SM's share of the
+  // K steps, so that few large tiles (long contractions with small results)
+  // still fill the chip; parts cost 16 B per output and part of L2 traffic.
+  // Last stage of the effective Hamiltonian without parts / halves / thirds /
+  // sixths: ladder D = 300 174 / 105 / 106 / 106 us, D = 512 299 / 205 / 197 /
+  // 221 us, Hubbard D = 1000 209 / 184 / 201 / 201 us.
+  auto of_group = [&](auto &&fn) {
+    for (size_t id = 0; id < groups.size(); ++id) {
+      const SlGroup &g = groups[id];
+      const int es = std::max(1, g.lanes_n ? g.nu / std::max(g.nv, 1) : g.nv / std::max(g.nu, 1));
+      for (int32_t i = 0; i * kSlU < g.nu; ++i)
+        for (int32_t j = 0; j * kSlV < g.nv; ++j) {
+          if (g.upper) {  // rows m, columns n: drop tiles with every n < m
+            const int n1 = (g.lanes_n ? i * kSlU + kSlU - 1 : j * kSlV + kSlV - 1) / es;
+            if ((g.lanes_n ? j * kSlV : i * kSlU) > n1) continue;
+          }
+          fn((int32_t)id, i, j);
+        }
+    }
+  };
+  double steps = 0;
+  of_group([&](int32_t id, int32_t, int32_t) { steps += groups[id].kc; });
+  const int unit = std::max<int>(
+      kSlChunk, ((int)(steps / (ctx ? ctx->num_sms : 152) / 3) + kSlChunk - 1) / kSlChunk * kSlChunk);
+  for (SlGroup &g : groups) {
+    g.parts = std::max(1, std::min(8, (g.kc + unit / 2) / unit));
+    const int per = (g.kc + g.parts - 1) / g.parts;
+    g.kpart = std::max(kSlChunk, (per + kSlChunk - 1) / kSlChunk * kSlChunk);
+    g.parts = std::max(1, (g.kc + g.kpart - 1) / g.kpart);
+  }
+  tiles.clear();
+  slots = 0;
+  of_group([&](int32_t id, int32_t i, int32_t j) {
+    const int32_t p0 = groups[id].parts > 1 ? (int32_t)slots : -1;
+    for (int32_t p = 0; p < groups[id].parts; ++p) tiles.push_back({id, i, j, p, p0, 0});
+    if (p0 >= 0) slots += groups[id].parts;
+  });
+  // most K steps first (longest processing time first over the persistent grid)
+  auto cost = [&](const SlTile &t) {
+    const SlGroup &g = groups[t.group];
+    return std::min(g.kpart, g.kc - t.part * g.kpart);
+  };
+  std::vector<int> count;
+  for (const SlTile &t : tiles) {
+    const int c = cost(t);
+    if ((int)count.size() <= c) count.resize(c + 1, 0);
+    count[c]++;
+  }
+  std::vector<int> at(count.size(), 0);
+  for (int c = (int)count.size() - 1, sum = 0; c >= 0; sum += count[c], --c) at[c] = sum;
+  std::vector<SlTile> sorted(tiles.size());
+  for (const SlTile &t : tiles) sorted[at[cost(t)]++] = t;
+  tiles.swap(sorted);
 }
 
 void SlicePlan::upload() {
   UploadBatch up(*ctx);
-  const size_t o0 = up.add(ops), o1 = up.add(items), o2 = up.add(groups), o3 = up.add(tiles),
+  const size_t o0 = up.add(ops), o1 = up.add(items), o1k = up.add(items_k),
+               o1t = up.add(items_t), o2 = up.add(groups), o3 = up.add(tiles),
                o4 = up.add(lines), o5 = up.add(cblk),
-               o6 = up.reserve((lines.size() + 2) * sizeof(int));
+               o6 = up.reserve(nscale() * sizeof(int)),
+               o7 = up.reserve(slots * kSlU * kSlV * sizeof(longlong2));
   d_block = up.commit();
   d_ops = (SlOp *)(d_block + o0);
   d_items = (SlItem *)(d_block + o1);
+  d_items_k = (SlItem *)(d_block + o1k);
+  d_items_t = (SlItem *)(d_block + o1t);
   d_groups = (SlGroup *)(d_block + o2);
   d_tiles = (SlTile *)(d_block + o3);
   d_lines = (SlLine *)(d_block + o4);
   d_cblk = (int64_t *)(d_block + o5);
   scale = (int *)(d_block + o6);
+  scratch = (longlong2 *)(d_block + o7);
   img = (uint8_t *)ctx->alloc(std::max<int64_t>(img_bytes, 1));
   if (holes) UDMRG_CHECK_CUDA(cudaMemsetAsync(img, 0, img_bytes, ctx->stream));
 }
 
 size_t SlicePlan::workspace() const {
-  return (size_t)img_bytes + (lines.size() + 2) * sizeof(int);
+  return (size_t)img_bytes + nscale() * sizeof(int) + slots * kSlU * kSlV * sizeof(longlong2);
 }
 
 double SlicePlan::seconds() const {
   double steps = 0, elems = 0;
-  for (const SlTile &t : tiles) steps += groups[t.group].kc + 2.0;
+  for (const SlTile &t : tiles) steps += std::min(groups[t.group].kpart, groups[t.group].kc) + 2.0;
   for (const SlOp &o : ops) elems += (double)o.rows * o.cols;
   return 30e-6 + steps * 0.7e-6 / 152 + elems * 30.0 / 3e12;
 }
 
 void run_slice(Ctx &ctx, const SlicePlan &p, const double *a, const double *b, double *c) {
   if (p.tiles.empty()) return;
-  UDMRG_CHECK_CUDA(cudaMemsetAsync(p.scale, 0, (p.lines.size() + 2) * sizeof(int), ctx.stream));
-  const int ni = (int)p.items.size();
-  const int pg = std::min(ni, 8 * ctx.num_sms);
-  if (ni) {
-    slice_scale_kernel<<<pg, kPackThreads, 0, ctx.stream>>>(p.d_ops, p.d_items, ni, a, b, p.scale);
-    slice_pack_kernel<<<pg, kPackThreads, 0, ctx.stream>>>(p.d_ops, p.d_items, ni, a, b, p.scale,
-                                                           p.img);
-  }
+  UDMRG_CHECK_CUDA(cudaMemsetAsync(p.scale, 0, p.nscale() * sizeof(int), ctx.stream));
+  const int ni = (int)p.items.size(), nk = (int)p.items_k.size(), nx = (int)p.items_t.size();
+  if (ni)
+    slice_scale_kernel<<<std::min(ni, 8 * ctx.num_sms), kPackThreads, 0, ctx.stream>>>(
+        p.d_ops, p.d_items, ni, a, b, p.scale);
+  if (nk)
+    slice_pack_k_kernel<<<std::min((nk + 7) / 8, 16 * ctx.num_sms), kPackThreads, 0,
+                          ctx.stream>>>(p.d_ops, p.d_items_k, nk, a, b, p.scale, p.img);
+  if (nx)
+    slice_pack_kernel<<<std::min(nx, 8 * ctx.num_sms), kPackThreads, 0, ctx.stream>>>(
+        p.d_ops, p.d_items_t, nx, a, b, p.scale, p.img);
   static bool attr_set = false;
   if (!attr_set) {
     UDMRG_CHECK_CUDA(cudaFuncSetAttribute(slice_gemm_kernel,
@@ -549,9 +723,10 @@ void run_slice(Ctx &ctx, const SlicePlan &p, const double *a, const double *b, d
   }
   const int nt = (int)p.tiles.size();
   slice_gemm_kernel<<<std::min(nt, ctx.num_sms), kSlThreads, kSlSmem, ctx.stream>>>(
-      p.d_tiles, nt, p.d_groups, p.d_lines, p.d_cblk, p.scale, p.img, c, p.scale);
+      p.d_tiles, nt, p.d_groups, p.d_lines, p.d_cblk, p.scale, p.img, c, p.scale, p.scratch,
+      p.scale + 2 + p.lines.size());
   UDMRG_CHECK_CUDA(cudaGetLastError());
-  ctx.launches += ni ? 3 : 1;
+  ctx.launches += 1 + (ni > 0) + (nk > 0) + (nx > 0);
 }
 
 }  // namespace udmrg

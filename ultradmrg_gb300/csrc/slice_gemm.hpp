@@ -53,7 +53,7 @@ struct SlOp {
   int32_t neg;      // negated values
   int32_t rows_fast;  // rows are the contiguous direction of the source
 };
-struct SlItem {  // work item of the scale and pack kernels: 32 rows x 64 columns
+struct SlItem {  // work item of the scale and pack kernels: rows from r0, columns from k0
   int32_t op, r0, k0, pad;
 };
 
@@ -72,24 +72,30 @@ struct SlGroup {
   int32_t ncb;           // columns of the block table (C column blocks)
   int32_t lanes_n;       // lanes along C's columns
   int32_t upper;         // square: entries below the diagonal are not needed
+  int32_t parts, kpart;  // K parts of a tile, K steps of each (a multiple of kSlChunk)
 };
+// One K part of an output tile.  Tiles of several parts leave their integer
+// sums at part0 in the scratch; the part that arrives last adds them up.
 struct SlTile {
-  int32_t group, ut, vt, pad;
+  int32_t group, ut, vt, part;
+  int32_t part0, pad;  // first of the tile's slots in the scratch (-1: one part)
 };
 
 struct SlicePlan {
   Ctx *ctx = nullptr;
   std::vector<SlOp> ops;
-  std::vector<SlItem> items;
+  std::vector<SlItem> items;             // scale pass
+  std::vector<SlItem> items_k, items_t;  // pack: contiguous columns, the others
   std::vector<SlGroup> groups;
   std::vector<SlTile> tiles;
   std::vector<SlLine> lines;
   std::vector<int64_t> cblk;
+  int64_t slots = 0;  // scratch slots (one per part of a tile with several)
   int64_t img_bytes = 0;
   bool holes = false;  // image entries no op writes
   uint8_t *d_block = nullptr;  // the tables and scale
   SlOp *d_ops = nullptr;
-  SlItem *d_items = nullptr;
+  SlItem *d_items = nullptr, *d_items_k = nullptr, *d_items_t = nullptr;
   SlGroup *d_groups = nullptr;
   SlTile *d_tiles = nullptr;
   SlLine *d_lines = nullptr;
@@ -97,8 +103,9 @@ struct SlicePlan {
   uint8_t *img = nullptr;
   // flags[0]: an operand is out of the sliced range (non-finite, or a row
   // maximum outside 2^-500 .. 2^500), flags[1]: a bounded wait ran out; then
-  // one scale entry per line
+  // one scale entry per line, then the arrival counters of the scratch slots
   int *scale = nullptr;
+  longlong2 *scratch = nullptr;
   SlicePlan() = default;
   SlicePlan(const SlicePlan &) = delete;
   SlicePlan &operator=(const SlicePlan &) = delete;
@@ -115,9 +122,10 @@ struct SlicePlan {
   // op: strides, extents, rows, cols, src, r0, k0, rstep, neg set by the caller
   void add_op(int group, SlOp op);
   double seconds() const;  // the cost model's estimate
-  void finalize();         // items and tile order (host)
+  void finalize();         // items, K parts and tile order (host)
   void upload();           // device tables and workspaces
   size_t workspace() const;
+  size_t nscale() const { return 2 + lines.size() + 16 * (size_t)slots; }
 };
 
 // C = A B for every group; sets the plan's flags where the sliced form does
