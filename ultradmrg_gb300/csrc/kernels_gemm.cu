@@ -21,6 +21,7 @@
 // below what the mixed solver's FP64 anchor needs.  Operands below 2^-102 in
 // magnitude keep only their high part, below 2^-126 they count as zero.
 #include "gemm.hpp"
+#include "tc_common.cuh"
 
 namespace udmrg {
 
@@ -149,6 +150,7 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
                         const In *__restrict__ A, const In *__restrict__ B, In *__restrict__ C,
                         double alpha, double beta, const int *__restrict__ gate) {
   // gate: the sliced form's flags; the tiles run only where it did not apply
+  tc::pdl_wait();  // the sliced form's kernel (a no-op in an ordinary launch)
   if (gate && gate[0] == 0 && gate[1] == 0) return;
   constexpr int NT = (BM / TM) * (BN / TN);
   // rows padded by one element: the staging stores of a warp walk K (the
@@ -255,9 +257,16 @@ void launch_cfg(Ctx &ctx, const GemmPlan &plan, int cfg, const In *a, const In *
     UDMRG_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         &per_sm, grouped_gemm_kernel<T, In, BM, BN, TM, TN, BK>, NT, 0));
   const int grid = std::min(ntiles, std::max(1, per_sm) * ctx.num_sms);
-  grouped_gemm_kernel<T, In, BM, BN, TM, TN, BK><<<grid, NT, 0, ctx.stream>>>(
-      plan.d_tiles[cfg], ntiles, plan.d_probs, plan.d_segs, a, b, c, alpha, beta, gate);
-  UDMRG_CHECK_CUDA(cudaGetLastError());
+  auto kernel = grouped_gemm_kernel<T, In, BM, BN, TM, TN, BK>;
+  if (gate) {
+    UDMRG_CHECK_CUDA(tc::launch_pdl(kernel, dim3(grid), dim3(NT), 0, ctx.stream,
+                                    plan.d_tiles[cfg], ntiles, plan.d_probs, plan.d_segs, a, b, c,
+                                    alpha, beta, gate));
+  } else {
+    kernel<<<grid, NT, 0, ctx.stream>>>(plan.d_tiles[cfg], ntiles, plan.d_probs, plan.d_segs, a,
+                                        b, c, alpha, beta, gate);
+    UDMRG_CHECK_CUDA(cudaGetLastError());
+  }
   ctx.launches++;
 }
 

@@ -145,6 +145,7 @@ __global__ void __launch_bounds__(256)
                      const double *__restrict__ t1, double *__restrict__ t3) {
   constexpr int kB = 4;  // couplings whose loads are in flight together
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  tc::pdl_wait();  // T1 from the L.psi GEMM
   for (int t = blockIdx.x * 8 + warp; t < ntasks; t += gridDim.x * 8) {
     const MpoTask64 tk = tasks[t];
     const MpoPair64 pr = pairs[tk.pair];
@@ -197,9 +198,9 @@ void run_mpo_step64(Ctx &ctx, const MpoStep64 &p, const double *t1, double *t3) 
   const int ntasks = (int)p.tasks.size();
   if (ntasks == 0) return;
   const int grid = std::min((ntasks + 7) / 8, 16 * ctx.num_sms);
-  mpo_map64_kernel<<<grid, 256, 0, ctx.stream>>>(p.d_tasks, ntasks, p.d_pairs, p.d_outs,
-                                                 p.d_rowptr, p.d_nz, t1, t3);
-  UDMRG_CHECK_CUDA(cudaGetLastError());
+  UDMRG_CHECK_CUDA(tc::launch_pdl(mpo_map64_kernel, dim3(grid), dim3(256), 0, ctx.stream,
+                                  p.d_tasks, ntasks, p.d_pairs, p.d_outs, p.d_rowptr, p.d_nz, t1,
+                                  t3));
   ctx.launches++;
 }
 

@@ -10,7 +10,8 @@ namespace udmrg {
 
 namespace {
 
-constexpr int kPackThreads = 256;
+constexpr int kPackThreads = 256, kPackWarps = kPackThreads / 32;
+constexpr int kPackRows = 8, kPackCols = 128;  // item of the warps with contiguous columns
 constexpr int kLoExp = 1023 - 500, kHiExp = 1023 + 500;  // biased exponents of the sliced range
 
 __device__ __forceinline__ int64_t sl_off(int64_t i, const int32_t *ext, const int64_t *str, int n) {
@@ -38,18 +39,64 @@ __device__ __forceinline__ void tile_offsets(const SlOp &op, const SlItem &it, i
   }
 }
 
-// scale[line] = max over the line's elements of the high word of |x| (bit 0
-// set where the low word alone is nonzero): its exponent bounds the line.
-// HBM bound: 8 B per element, read once; lanes walk the contiguous direction.
+// high word of |x|, bit 0 set where the low word alone is nonzero
+__device__ __forceinline__ int abs_high(double x) {
+  const uint64_t d = (uint64_t)__double_as_longlong(x);
+  return (int)((uint32_t)(d >> 32) & 0x7FFFFFFFu) | ((uint32_t)d ? 1 : 0);
+}
+
+// scale[line] = max over the line's elements of abs_high: its exponent bounds
+// the line.  HBM bound: 8 B per element, read once.  The first nbk blocks take
+// the items with contiguous columns (or every second double: complex parts), a
+// warp 8 rows at a time with sixteen loads per lane in flight; the others an
+// item of 32 rows x 64 columns per block, lanes along the contiguous direction.
 __global__ void __launch_bounds__(kPackThreads)
-    slice_scale_kernel(const SlOp *__restrict__ ops, const SlItem *__restrict__ items, int nitems,
+    slice_scale_kernel(const SlOp *__restrict__ ops, const SlItem *__restrict__ items_k, int nk,
+                       int nbk, const SlItem *__restrict__ items_t, int nt,
                        const double *__restrict__ a, const double *__restrict__ b,
                        int *__restrict__ scale) {
   __shared__ int64_t roff[32], koff[64];
   __shared__ int mx[32];
   const int tid = threadIdx.x;
-  for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
-    const SlItem it = items[w];
+  tc::pdl_launch_dependents();
+  if (blockIdx.x < nbk) {
+    const int lane = tid & 31;
+    for (int w = blockIdx.x * kPackWarps + (tid >> 5); w < nk; w += nbk * kPackWarps) {
+      const SlItem it = items_k[w];
+      const SlOp &op = ops[it.op];
+      const int es = op.nk ? (int)op.ks[0] : 1, nr = min(kPackRows, op.rows - it.r0);
+      const int n = min(op.cols - it.k0, it.width);
+      const double *src = (op.src ? b : a) + op.src_off + (int64_t)it.k0 * es;
+      const long long off = lane < nr ? sl_off(it.r0 + lane, op.re, op.rs, op.nr) : 0;
+      int best = 0;  // of row it.r0 + lane
+#pragma unroll
+      for (int r0 = 0; r0 < kPackRows; r0 += 4) {
+        double x[4][kPackCols / 32];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const long long o = __shfl_sync(0xffffffffu, off, r0 + r);
+#pragma unroll
+          for (int c = 0; c < kPackCols / 32; ++c) {
+            const int k = lane + 32 * c;
+            x[r][c] = r0 + r < nr && k < n ? __ldg(src + o + (int64_t)k * es) : 0.0;
+          }
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          int v = 0;
+#pragma unroll
+          for (int c = 0; c < kPackCols / 32; ++c) v = max(v, abs_high(x[r][c]));
+          v = __reduce_max_sync(0xffffffffu, v);
+          if (lane == r0 + r) best = v;
+        }
+      }
+      if (best)
+        atomicMax(scale + 2 + op.sc0 + op.r0 + (int64_t)(it.r0 + lane) * op.rstep, best);
+    }
+    return;
+  }
+  for (int w = blockIdx.x - nbk; w < nt; w += gridDim.x - nbk) {
+    const SlItem it = items_t[w];
     const SlOp &op = ops[it.op];
     const double *src = op.src ? b : a;
     const bool rows_fast = op.rows_fast != 0;
@@ -62,12 +109,7 @@ __global__ void __launch_bounds__(kPackThreads)
     for (int q = 0; q < 8; ++q) {
       const int e = tid + q * kPackThreads;
       const int r = rows_fast ? e & 31 : e >> 6, k = rows_fast ? e >> 5 : e & 63;
-      int v = 0;
-      if (roff[r] >= 0 && koff[k] >= 0) {
-        const uint64_t d = (uint64_t)__double_as_longlong(__ldg(src + roff[r] + koff[k]));
-        v = (int)((uint32_t)(d >> 32) & 0x7FFFFFFFu) | ((uint32_t)d ? 1 : 0);
-      }
-      best[q] = v;
+      best[q] = roff[r] >= 0 && koff[k] >= 0 ? abs_high(__ldg(src + roff[r] + koff[k])) : 0;
     }
     if (rows_fast) {  // a thread's eight elements share its row
       int v = 0;
@@ -137,22 +179,67 @@ __device__ __forceinline__ void store_digits(const double (&x)[8], int be, bool 
     *(uint4 *)(o + d * plane) = make_uint4(p[d][0], p[d][1], p[d][2], p[d][3]);
 }
 
-// Digits of the operands into their images.  A work item is 32 rows x 64
-// columns of one op, staged in shared memory along the source's contiguous
-// direction; then a thread cuts one row's 8 consecutive columns, and the 32
-// rows of a warp fill 512 contiguous bytes per plane.  HBM bound: 8 B read
-// and 16 B written per element.  Ops start at columns that are multiples of 8; the
-// columns from an op's edge to the next one are written as zeros.  A line whose
-// largest element is non-finite or outside the sliced range raises the flag.
+// Image address of row `row`, K step and column follow; be: the row's biased
+// exponent (0x7FF for a line of zeros: every digit zero).  A line whose largest
+// element is non-finite or outside the sliced range raises the flag.
+__device__ __forceinline__ uint8_t *image_row(const SlOp &op, int row, int *scale, uint8_t *img,
+                                              int &be) {
+  const int sc = scale[2 + op.sc0 + row];
+  be = sc == 0 ? 0x7FF : sc >> 20;
+  if (sc != 0 && (be < kLoExp || be > kHiExp)) atomicExch(scale, 1);
+  const int64_t plane = (int64_t)op.tr * kSlK * 2;
+  return img + op.img_off + (int64_t)(row >> (op.tr == kSlU ? 7 : 6)) * op.kc * kSlDigits * plane;
+}
+
+// Digits of the operands into their images.  HBM bound: 8 B read and 16 B
+// written per element.  Ops start at columns that are multiples of 8; the columns
+// from an op's edge to the next one are written as zeros.
+//
+// The first nbk blocks take the items with contiguous columns (or every second
+// double), without shared memory: a warp takes 8 rows x 32 columns at a time, lane =
+// (column group, row): eight loads of its row's 64 bytes (consecutive lanes' rows
+// share no sectors, but each sector is used whole over the eight), then the
+// plane segments of eight rows fill 128 contiguous bytes.  The other blocks'
+// items are 32 rows x 64 columns, staged in shared memory along the source's
+// contiguous direction; then a thread cuts one row's 8 consecutive columns, and
+// the 32 rows of a warp fill 512 contiguous bytes per plane.
 __global__ void __launch_bounds__(kPackThreads)
-    slice_pack_kernel(const SlOp *__restrict__ ops, const SlItem *__restrict__ items, int nitems,
+    slice_pack_kernel(const SlOp *__restrict__ ops, const SlItem *__restrict__ items_k, int nk,
+                      int nbk, const SlItem *__restrict__ items_t, int nt,
                       const double *__restrict__ a, const double *__restrict__ b,
                       int *__restrict__ scale, uint8_t *__restrict__ img) {
   __shared__ int64_t roff[32], koff[64];
   __shared__ double tile[64][33];
   const int tid = threadIdx.x;
-  for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
-    const SlItem it = items[w];
+  tc::pdl_launch_dependents();
+  tc::pdl_wait();  // the scales
+  if (blockIdx.x < nbk) {
+    const int lane = tid & 31, r = lane % kPackRows, g = lane / kPackRows;
+    for (int w = blockIdx.x * kPackWarps + (tid >> 5); w < nk; w += nbk * kPackWarps) {
+      const SlItem it = items_k[w];
+      const SlOp &op = ops[it.op];
+      const int rs = it.r0 + r;
+      if (rs >= op.rows) continue;
+      const double *src = (op.src ? b : a) + op.src_off + sl_off(rs, op.re, op.rs, op.nr);
+      const int es = op.nk ? (int)op.ks[0] : 1, row = op.r0 + rs * op.rstep;
+      int be;
+      uint8_t *orow = image_row(op, row, scale, img, be);
+      const int64_t plane = (int64_t)op.tr * kSlK * 2;
+      const int rin = row & (op.tr - 1), end = min(op.cols, it.k0 + it.width);
+      const bool neg = op.neg != 0;
+      for (int ks = it.k0 + g * 8; ks < end; ks += 32) {
+        const int n = min(8, op.cols - ks), col = op.k0 + ks;
+        double x[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) x[j] = j < n ? __ldg(src + (int64_t)(ks + j) * es) : 0.0;
+        store_digits(x, be, neg, orow + (int64_t)(col >> 4) * kSlDigits * plane +
+                                     canon_off(rin, col & 15, op.tr), plane);
+      }
+    }
+    return;
+  }
+  for (int w = blockIdx.x - nbk; w < nt; w += gridDim.x - nbk) {
+    const SlItem it = items_t[w];
     const SlOp &op = ops[it.op];
     const double *src = op.src ? b : a;
     const bool rows_fast = op.rows_fast != 0;
@@ -170,58 +257,15 @@ __global__ void __launch_bounds__(kPackThreads)
     const int rs = it.r0 + r, ks = it.k0 + g * 8;
     if (rs >= op.rows || ks >= op.cols) continue;
     const int row = op.r0 + rs * op.rstep, col = op.k0 + ks;
-    const int sc = scale[2 + op.sc0 + row];
-    const int be = sc == 0 ? 0x7FF : sc >> 20;  // a line of zeros: every digit zero
-    if (sc != 0 && (be < kLoExp || be > kHiExp)) atomicExch(scale, 1);
-    const int tr = op.tr, ts = tr == kSlU ? 7 : 6;
-    const int64_t plane = (int64_t)tr * kSlK * 2;
-    const int64_t tbase = op.img_off + (int64_t)(row >> ts) * op.kc * kSlDigits * plane;
-    const int rin = row & (tr - 1);
+    int be;
+    uint8_t *orow = image_row(op, row, scale, img, be);
+    const int64_t plane = (int64_t)op.tr * kSlK * 2;
     double x[8];  // (zeros past the op's columns)
 #pragma unroll
     for (int j = 0; j < 8; ++j) x[j] = tile[g * 8 + j][r];
     store_digits(x, be, op.neg != 0,
-                 img + tbase + (int64_t)(col >> 4) * kSlDigits * plane +
-                     canon_off(rin, col & 15, tr), plane);
-  }
-}
-
-// The same for ops whose columns are contiguous (or every second double:
-// complex parts): no shared memory.  A warp takes 8 rows x 32 columns at a time,
-// lane = (column group, row): eight loads of its row's 64 bytes (consecutive
-// lanes' rows share no sectors, but each sector is used whole over the eight),
-// then the plane segments of eight rows fill 128 contiguous bytes.
-constexpr int kPackCols = 128;  // columns of a work item
-__global__ void __launch_bounds__(kPackThreads)
-    slice_pack_k_kernel(const SlOp *__restrict__ ops, const SlItem *__restrict__ items, int nitems,
-                        const double *__restrict__ a, const double *__restrict__ b,
-                        int *__restrict__ scale, uint8_t *__restrict__ img) {
-  const int lane = threadIdx.x & 31, r = lane & 7, g = lane >> 3;
-  const int wpb = blockDim.x >> 5;
-  for (int w = blockIdx.x * wpb + (threadIdx.x >> 5); w < nitems; w += gridDim.x * wpb) {
-    const SlItem it = items[w];
-    const SlOp &op = ops[it.op];
-    const int rs = it.r0 + r;
-    if (rs >= op.rows) continue;
-    const double *src = (op.src ? b : a) + op.src_off + sl_off(rs, op.re, op.rs, op.nr);
-    const int es = op.nk ? (int)op.ks[0] : 1;
-    const int row = op.r0 + rs * op.rstep;
-    const int sc = scale[2 + op.sc0 + row];
-    const int be = sc == 0 ? 0x7FF : sc >> 20;
-    if (sc != 0 && (be < kLoExp || be > kHiExp)) atomicExch(scale, 1);
-    const int tr = op.tr, ts = tr == kSlU ? 7 : 6;
-    const int64_t plane = (int64_t)tr * kSlK * 2;
-    uint8_t *orow = img + op.img_off + (int64_t)(row >> ts) * op.kc * kSlDigits * plane;
-    const int rin = row & (tr - 1), end = min(op.cols, it.k0 + kPackCols);
-    const bool neg = op.neg != 0;
-    for (int ks = it.k0 + g * 8; ks < end; ks += 32) {
-      const int n = min(8, op.cols - ks), col = op.k0 + ks;
-      double x[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) x[j] = j < n ? __ldg(src + (ks + j) * es) : 0.0;
-      store_digits(x, be, neg, orow + (int64_t)(col >> 4) * kSlDigits * plane +
-                                   canon_off(rin, col & 15, tr), plane);
-    }
+                 orow + (int64_t)(col >> 4) * kSlDigits * plane +
+                     canon_off(row & (op.tr - 1), col & 15, op.tr), plane);
   }
 }
 
@@ -324,7 +368,6 @@ __global__ void __launch_bounds__(kSlThreads, 1)
   extern __shared__ __align__(1024) uint8_t smem[];
   SlBars *b = (SlBars *)(smem + kSlBarOffset);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (scale[0]) return;  // the sliced form does not apply (uniform over the grid)
   if (tid == 0) {
     for (int s = 0; s < kSlStages; ++s) {
       tc::mbar_init(&b->full[s], 1);
@@ -344,6 +387,12 @@ __global__ void __launch_bounds__(kSlThreads, 1)
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = b->tmem;
+  tc::pdl_wait();  // the images and scales
+  if (scale[0]) {  // the sliced form does not apply (uniform over the grid)
+    __syncthreads();
+    if (warp == 0) tc::tmem_dealloc(tmem, 512);
+    return;
+  }
 
   if (warp == 0) {
     if (lane == 0) {
@@ -535,6 +584,7 @@ __global__ void __launch_bounds__(kSlThreads, 1)
       }
     }
   }
+  tc::pdl_launch_dependents();
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
@@ -599,19 +649,27 @@ void SlicePlan::add_op(int group, SlOp op) {
 }
 
 void SlicePlan::finalize() {
-  items.clear();
   items_k.clear();
   items_t.clear();
+  // fewer columns per item where the items of a warp's full width would leave
+  // SMs without work
+  auto by_cols = [](const SlOp &op) {
+    return !op.rows_fast && op.nk <= 1 && (op.nk == 0 || op.ks[0] <= 2);
+  };
+  int64_t wide = 0;
+  for (const SlOp &op : ops)
+    if (by_cols(op))
+      wide += (int64_t)((op.rows + kPackRows - 1) / kPackRows) *
+              ((op.cols + kPackCols - 1) / kPackCols);
+  const int width = wide < 4 * kPackWarps * (ctx ? ctx->num_sms : 152) ? 32 : kPackCols;
   for (size_t o = 0; o < ops.size(); ++o) {
     const SlOp &op = ops[o];
-    for (int32_t r = 0; r < op.rows; r += 32)
-      for (int32_t k = 0; k < op.cols; k += 64) items.push_back({(int32_t)o, r, k, 0});
-    if (!op.rows_fast && op.nk <= 1 && (op.nk == 0 || op.ks[0] <= 2)) {
-      for (int32_t r = 0; r < op.rows; r += 8)
-        for (int32_t k = 0; k < op.cols; k += kPackCols) items_k.push_back({(int32_t)o, r, k, 0});
+    if (by_cols(op)) {
+      for (int32_t r = 0; r < op.rows; r += kPackRows)
+        for (int32_t k = 0; k < op.cols; k += width) items_k.push_back({(int32_t)o, r, k, width});
     } else {
       for (int32_t r = 0; r < op.rows; r += 32)
-        for (int32_t k = 0; k < op.cols; k += 64) items_t.push_back({(int32_t)o, r, k, 0});
+        for (int32_t k = 0; k < op.cols; k += 64) items_t.push_back({(int32_t)o, r, k, 64});
     }
   }
   // K parts: a unit of work is at most about a third of one SM's share of the
@@ -671,15 +729,14 @@ void SlicePlan::finalize() {
 
 void SlicePlan::upload() {
   UploadBatch up(*ctx);
-  const size_t o0 = up.add(ops), o1 = up.add(items), o1k = up.add(items_k),
-               o1t = up.add(items_t), o2 = up.add(groups), o3 = up.add(tiles),
+  const size_t o0 = up.add(ops), o1 = up.add(items_k), o1t = up.add(items_t),
+               o2 = up.add(groups), o3 = up.add(tiles),
                o4 = up.add(lines), o5 = up.add(cblk),
                o6 = up.reserve(nscale() * sizeof(int)),
                o7 = up.reserve(slots * kSlU * kSlV * sizeof(longlong2));
   d_block = up.commit();
   d_ops = (SlOp *)(d_block + o0);
-  d_items = (SlItem *)(d_block + o1);
-  d_items_k = (SlItem *)(d_block + o1k);
+  d_items_k = (SlItem *)(d_block + o1);
   d_items_t = (SlItem *)(d_block + o1t);
   d_groups = (SlGroup *)(d_block + o2);
   d_tiles = (SlTile *)(d_block + o3);
@@ -705,16 +762,17 @@ double SlicePlan::seconds() const {
 void run_slice(Ctx &ctx, const SlicePlan &p, const double *a, const double *b, double *c) {
   if (p.tiles.empty()) return;
   UDMRG_CHECK_CUDA(cudaMemsetAsync(p.scale, 0, p.nscale() * sizeof(int), ctx.stream));
-  const int ni = (int)p.items.size(), nk = (int)p.items_k.size(), nx = (int)p.items_t.size();
-  if (ni)
-    slice_scale_kernel<<<std::min(ni, 8 * ctx.num_sms), kPackThreads, 0, ctx.stream>>>(
-        p.d_ops, p.d_items, ni, a, b, p.scale);
-  if (nk)
-    slice_pack_k_kernel<<<std::min((nk + 7) / 8, 16 * ctx.num_sms), kPackThreads, 0,
-                          ctx.stream>>>(p.d_ops, p.d_items_k, nk, a, b, p.scale, p.img);
-  if (nx)
-    slice_pack_kernel<<<std::min(nx, 8 * ctx.num_sms), kPackThreads, 0, ctx.stream>>>(
-        p.d_ops, p.d_items_t, nx, a, b, p.scale, p.img);
+  const int nk = (int)p.items_k.size(), nx = (int)p.items_t.size();
+  const int nbk = std::min((nk + kPackWarps - 1) / kPackWarps, 16 * ctx.num_sms);
+  const int grid = nbk + std::min(nx, 8 * ctx.num_sms);
+  if (grid) {
+    slice_scale_kernel<<<grid, kPackThreads, 0, ctx.stream>>>(p.d_ops, p.d_items_k, nk, nbk,
+                                                              p.d_items_t, nx, a, b, p.scale);
+    UDMRG_CHECK_CUDA(cudaGetLastError());
+    UDMRG_CHECK_CUDA(tc::launch_pdl(slice_pack_kernel, dim3(grid), dim3(kPackThreads), 0,
+                                    ctx.stream, p.d_ops, p.d_items_k, nk, nbk, p.d_items_t, nx, a,
+                                    b, p.scale, p.img));
+  }
   static bool attr_set = false;
   if (!attr_set) {
     UDMRG_CHECK_CUDA(cudaFuncSetAttribute(slice_gemm_kernel,
@@ -722,11 +780,11 @@ void run_slice(Ctx &ctx, const SlicePlan &p, const double *a, const double *b, d
     attr_set = true;
   }
   const int nt = (int)p.tiles.size();
-  slice_gemm_kernel<<<std::min(nt, ctx.num_sms), kSlThreads, kSlSmem, ctx.stream>>>(
-      p.d_tiles, nt, p.d_groups, p.d_lines, p.d_cblk, p.scale, p.img, c, p.scale, p.scratch,
-      p.scale + 2 + p.lines.size());
-  UDMRG_CHECK_CUDA(cudaGetLastError());
-  ctx.launches += 1 + (ni > 0) + (nk > 0) + (nx > 0);
+  UDMRG_CHECK_CUDA(tc::launch_pdl(slice_gemm_kernel, dim3(std::min(nt, ctx.num_sms)),
+                                  dim3(kSlThreads), kSlSmem, ctx.stream, p.d_tiles, nt,
+                                  p.d_groups, p.d_lines, p.d_cblk, p.scale, p.img, c, p.scale,
+                                  p.scratch, p.scale + 2 + p.lines.size()));
+  ctx.launches += grid ? 3 : 1;
 }
 
 }  // namespace udmrg

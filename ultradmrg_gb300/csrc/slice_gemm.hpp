@@ -53,8 +53,8 @@ struct SlOp {
   int32_t neg;      // negated values
   int32_t rows_fast;  // rows are the contiguous direction of the source
 };
-struct SlItem {  // work item of the scale and pack kernels: rows from r0, columns from k0
-  int32_t op, r0, k0, pad;
+struct SlItem {  // work item of the scale and pack kernels: rows from r0, width columns from k0
+  int32_t op, r0, k0, width;
 };
 
 // Output address of (lane line u, register line v): with lanes along C's
@@ -84,8 +84,7 @@ struct SlTile {
 struct SlicePlan {
   Ctx *ctx = nullptr;
   std::vector<SlOp> ops;
-  std::vector<SlItem> items;             // scale pass
-  std::vector<SlItem> items_k, items_t;  // pack: contiguous columns, the others
+  std::vector<SlItem> items_k, items_t;  // of ops with contiguous columns, of the others
   std::vector<SlGroup> groups;
   std::vector<SlTile> tiles;
   std::vector<SlLine> lines;
@@ -95,7 +94,7 @@ struct SlicePlan {
   bool holes = false;  // image entries no op writes
   uint8_t *d_block = nullptr;  // the tables and scale
   SlOp *d_ops = nullptr;
-  SlItem *d_items = nullptr, *d_items_k = nullptr, *d_items_t = nullptr;
+  SlItem *d_items_k = nullptr, *d_items_t = nullptr;
   SlGroup *d_groups = nullptr;
   SlTile *d_tiles = nullptr;
   SlLine *d_lines = nullptr;
