@@ -131,3 +131,36 @@ def test_block_sparse_forms_agree(ctx, dtype):
         scale = max(np.abs(v).max() for v in x.blocks.values())
         for k in x.blocks:
             assert np.abs(x.blocks[k] - y.blocks[k]).max() <= 1e-13 * scale
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.complex128])
+def test_scales_from_the_mpo_step(ctx, dtype):
+    """The product on a plan, where the MPO step finds the scales of the last
+    GEMM's operand: against the FP64 form, and linear in the state bit for bit
+    under powers of two (scales left over from a larger state would show)."""
+    mpo, pb = M.hubbard_cylinder_mpo(3, 2, t=1.0, U=8.0, dtype=dtype)
+    mps = M.random_canonical_mps([pb] * 6, (5, 1), 60, 2, seed=3, dtype=dtype)
+    out = {}
+    for form in (0, 1):
+        ctx.set_gemm_form(form)
+        ten = [[api.DeviceTensor.from_data(ctx, t) for t in x] for x in (mps, mpo)]
+        L, R = (api.DeviceTensor.from_data(ctx, api.trivial_env_data(mps[i], mpo[i], s))
+                for i, s in ((0, "l"), (5, "r")))
+        for i in (0, 1):
+            L = api.update_site_lenvs(ctx, L, ten[0][i], ten[1][i])
+            R = api.update_site_renvs(ctx, R, ten[0][5 - i], ten[1][5 - i])
+        psi = api.contract(ctx, ten[0][2], ten[0][3], [2], [0])
+        plan = api.MatvecPlan(ctx, [L, ten[1][2], ten[1][3], R], psi)
+        for p in (0, -40, 7):
+            data = psi.to_data()
+            data.blocks = {k: v * 2.0 ** p for k, v in data.blocks.items()}
+            x = plan.embed(api.DeviceTensor.from_data(ctx, data))
+            y = plan.embed(psi)
+            plan.apply(x, y)
+            out[form, p] = y.to_data().blocks
+    ctx.set_gemm_form(1)
+    scale = max(np.abs(v).max() for v in out[0, 0].values())
+    for k, v in out[1, 0].items():
+        assert np.abs(v - out[0, 0][k]).max() <= 1e-13 * scale
+        for p in (-40, 7):
+            assert np.array_equal(out[1, p][k], v * 2.0 ** p)

@@ -1147,7 +1147,7 @@ int udmrg_matvec_plan_stage_times(udmrg_matvec_plan *p, const double *d_in, doub
       run_gemm(ctx, m.p1->gemm, dt, m.L->data, d_in, m.t1, 1.0, 0.0);
       cudaEventRecord(ev[1], ctx.stream);
       if (m.m64) {  // both MPO steps in one channel map (stage 2; stage 3 empty)
-        run_mpo_step64(ctx, *m.m64, m.t1, m.t3);
+        run_mpo_step64(ctx, *m.m64, m.t1, m.t3, m.p4->gemm.sl.get());
         cudaEventRecord(ev[2], ctx.stream);
       } else {
         run_gemm(ctx, m.p2->gemm, dt, m.t1, m.W1->data, m.t2, 1.0, 0.0);

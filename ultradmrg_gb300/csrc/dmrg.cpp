@@ -302,6 +302,7 @@ std::unique_ptr<MatvecPlan> plan_matvec2(Ctx &ctx, const BTensor &L, const BTens
   mv->build_sec[1] = lap();
   gemm_upload(mv->p1->gemm);
   if (mv->m64) {
+    link_scales(*mv->m64, mv->p4->gemm.sl.get());
     upload_mpo_step64(ctx, *mv->m64);
   } else {
     gemm_upload(mv->p2->gemm);
@@ -366,8 +367,9 @@ std::unique_ptr<MatvecPlan> plan_matvec1(Ctx &ctx, const BTensor &L, const BTens
     const BTensor &t1 = *mv->p1->out;
     auto t2 = mpo_map_struct(t1, W, 0, 1);
     mv->m64 = build_mpo_map(t1, W, wh, 0, 1, *t2);
-    upload_mpo_step64(ctx, *mv->m64);
     mv->p4 = plan_contract_into(*t2, R, {2, 3}, {1, 2}, {0, 1}, {0}, *S, &mv->missing);
+    link_scales(*mv->m64, mv->p4->gemm.sl.get());
+    upload_mpo_step64(ctx, *mv->m64);
   } else {
     gemm_upload(mv->p2->gemm);
     mv->p4 = plan_contract_into(*mv->p2->out, R, ca, cb, fa, fb, *S, &mv->missing);
@@ -394,7 +396,7 @@ void MatvecPlan::apply_fp64(const double *in, double *out, bool dw) {
   auto gemm = dw ? run_gemm_dw : run_gemm;
   gemm(*ctx, p1->gemm, dt, L->data, in, t1, 1.0, 0.0);
   if (m64) {
-    run_mpo_step64(*ctx, *m64, t1, sites == 2 ? t3 : t2);
+    run_mpo_step64(*ctx, *m64, t1, sites == 2 ? t3 : t2, p4->gemm.sl.get());
   } else {
     gemm(*ctx, p2->gemm, dt, t1, W1->data, t2, 1.0, 0.0);
     if (sites == 2) gemm(*ctx, p3->gemm, dt, t2, W2->data, t3, 1.0, 0.0);

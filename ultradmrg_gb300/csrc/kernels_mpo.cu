@@ -142,7 +142,8 @@ __global__ void __launch_bounds__(256)
     mpo_map64_kernel(const MpoTask64 *__restrict__ tasks, int ntasks,
                      const MpoPair64 *__restrict__ pairs, const MpoOut64 *__restrict__ outs,
                      const int32_t *__restrict__ rowptr, const MpoNz64 *__restrict__ nz,
-                     const double *__restrict__ t1, double *__restrict__ t3) {
+                     const double *__restrict__ t1, double *__restrict__ t3,
+                     int *__restrict__ scale) {
   constexpr int kB = 4;  // couplings whose loads are in flight together
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   tc::pdl_wait();  // T1 from the L.psi GEMM
@@ -153,16 +154,56 @@ __global__ void __launch_bounds__(256)
     const bool v0 = u0 < n, v1 = u1 < n;
     const int a0 = v0 ? u0 / pr.db : 0, b0 = v0 ? u0 - a0 * pr.db : 0;
     const int a1 = v1 ? u1 / pr.db : 0, b1 = v1 ? u1 - a1 * pr.db : 0;
-    const int kbeg = __ldg(rowptr + pr.row0), kend = __ldg(rowptr + pr.row0 + pr.nout);
-    int o = 0;
-    int next = __ldg(rowptr + pr.row0 + 1);  // end of output channel o's couplings
+    const int kbeg = __ldg(rowptr + pr.row0 + tk.o0), kend = __ldg(rowptr + pr.row0 + tk.o1);
+    // scales: few a' over the task, or runs of lanes of one a' (bit i of run:
+    // lane + 2^i belongs to the lane's run; bit 5: first of its run)
+    const int alo = tk.u0 / pr.db, na = (min(tk.u0 + 64, n) - 1) / pr.db - alo + 1;
+    uint32_t run0 = 0, run1 = 0;
+    if (scale && na > 4) {
+#pragma unroll
+      for (int i = 0; i < 5; ++i) {
+        const int d = 1 << i;
+        const int p = __shfl_down_sync(kFull, a0, d), q = __shfl_down_sync(kFull, a1, d);
+        run0 |= (lane + d < 32 && p == a0) << i;
+        run1 |= (lane + d < 32 && q == a1) << i;
+      }
+      const int p = __shfl_up_sync(kFull, a0, 1), q = __shfl_up_sync(kFull, a1, 1);
+      run0 |= (lane == 0 || p != a0) << 5;
+      run1 |= (lane == 0 || q != a1) << 5;
+    }
+    auto run_max = [&](int v, uint32_t run, int *at) {
+#pragma unroll
+      for (int i = 0; i < 5; ++i) {
+        const int w = __shfl_down_sync(kFull, v, 1 << i);
+        if (run >> i & 1) v = max(v, w);
+      }
+      if ((run >> 5 & 1) && v) atomicMax(at, v);
+    };
+    int o = tk.o0;
+    int next = __ldg(rowptr + pr.row0 + o + 1);  // end of output channel o's couplings
     double s0 = 0.0, s1 = 0.0;
     auto finish = [&]() {  // warp-uniform: write channel o, move to o + 1
       const MpoOut64 ot = outs[pr.out0 + o];
       if (v0) t3[ot.base + (int64_t)a0 * ot.astride + b0] = s0;
       if (v1) t3[ot.base + (int64_t)a1 * ot.astride + b1] = s1;
+      if (scale && ot.line >= 0) {
+        const int h0 = v0 ? tc::abs_high(s0) : 0, h1 = v1 ? tc::abs_high(s1) : 0;
+        int *at = scale + 2 + ot.line;
+        if (na <= 4) {
+          int best = 0;  // of a' = alo + lane
+          for (int i = 0; i < na; ++i) {
+            const int v = __reduce_max_sync(
+                kFull, max(a0 == alo + i ? h0 : 0, a1 == alo + i ? h1 : 0));
+            if (lane == i) best = v;
+          }
+          if (best) atomicMax(at + (int64_t)(alo + lane) * ot.step, best);
+        } else {
+          run_max(h0, run0, at + (int64_t)a0 * ot.step);
+          run_max(h1, run1, at + (int64_t)a1 * ot.step);
+        }
+      }
       s0 = s1 = 0.0;
-      if (++o < pr.nout) next = __ldg(rowptr + pr.row0 + 1 + o);
+      if (++o < tk.o1) next = __ldg(rowptr + pr.row0 + 1 + o);
     };
     for (int kb = kbeg; kb < kend; kb += 32) {
       const int nb = min(32, kend - kb);
@@ -188,19 +229,22 @@ __global__ void __launch_bounds__(256)
         }
       }
     }
-    while (o < pr.nout) finish();  // the last channel and channels without couplings
+    while (o < tk.o1) finish();  // the last channel and channels without couplings
   }
 }
 
 }  // namespace
 
-void run_mpo_step64(Ctx &ctx, const MpoStep64 &p, const double *t1, double *t3) {
+void run_mpo_step64(Ctx &ctx, const MpoStep64 &p, const double *t1, double *t3,
+                    const SlicePlan *next) {
   const int ntasks = (int)p.tasks.size();
+  const bool scales = next && next->prescaled;
+  if (scales) next->clear_scales();
   if (ntasks == 0) return;
   const int grid = std::min((ntasks + 7) / 8, 16 * ctx.num_sms);
   UDMRG_CHECK_CUDA(tc::launch_pdl(mpo_map64_kernel, dim3(grid), dim3(256), 0, ctx.stream,
                                   p.d_tasks, ntasks, p.d_pairs, p.d_outs, p.d_rowptr, p.d_nz, t1,
-                                  t3));
+                                  t3, scales ? next->scale : nullptr));
   ctx.launches++;
 }
 

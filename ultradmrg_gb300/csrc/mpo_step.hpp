@@ -16,6 +16,7 @@
 #include <map>
 
 #include "btensor.hpp"
+#include "slice_gemm.hpp"
 
 namespace udmrg {
 
@@ -51,14 +52,15 @@ struct MpoNz64 {
 };
 struct MpoOut64 {
   int64_t base;
-  int32_t astride, pad;
+  int32_t astride;
+  int32_t line, step, pad;  // scale entry at a' = 0 (-1: none), entries between a'
 };
 struct MpoPair64 {
   int32_t out0, nout;
   int32_t row0, da, db, pad;  // row0: first CSR row of the pair; db in doubles
 };
-struct MpoTask64 {  // 64 consecutive (a', b) entries of a pair
-  int32_t pair, u0;
+struct MpoTask64 {  // 64 consecutive (a', b) entries of a pair, channels o0 .. o1 - 1
+  int32_t pair, u0, o0, o1;
 };
 
 struct MpoStep64 {
@@ -90,6 +92,12 @@ std::unique_ptr<MpoStep64> build_mpo_map(const BTensor &T, const BTensor &W,
 // Host copy of an MPO tensor's real parts; *real = no nonzero imaginary part.
 std::vector<double> mpo_data(Ctx &ctx, const BTensor &w, bool *real);
 void upload_mpo_step64(Ctx &ctx, MpoStep64 &p);
-void run_mpo_step64(Ctx &ctx, const MpoStep64 &p, const double *t1, double *t3);
+// Lets the step find the scales of T3, the next sliced GEMM's first operand: its
+// scale pass need not read T3 again.  Before upload_mpo_step64; true where every
+// channel's row of b lies within one line of the operand (its rows of b are K
+// runs); p then runs with next, before it.
+bool link_scales(MpoStep64 &p, SlicePlan *next);
+void run_mpo_step64(Ctx &ctx, const MpoStep64 &p, const double *t1, double *t3,
+                    const SlicePlan *next = nullptr);
 
 }  // namespace udmrg

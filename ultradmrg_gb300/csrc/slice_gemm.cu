@@ -39,13 +39,7 @@ __device__ __forceinline__ void tile_offsets(const SlOp &op, const SlItem &it, i
   }
 }
 
-// high word of |x|, bit 0 set where the low word alone is nonzero
-__device__ __forceinline__ int abs_high(double x) {
-  const uint64_t d = (uint64_t)__double_as_longlong(x);
-  return (int)((uint32_t)(d >> 32) & 0x7FFFFFFFu) | ((uint32_t)d ? 1 : 0);
-}
-
-// scale[line] = max over the line's elements of abs_high: its exponent bounds
+// scale[line] = max over the line's elements of tc::abs_high: its exponent bounds
 // the line.  HBM bound: 8 B per element, read once.  The first nbk blocks take
 // the items with contiguous columns (or every second double: complex parts), a
 // warp 8 rows at a time with sixteen loads per lane in flight; the others an
@@ -85,7 +79,7 @@ __global__ void __launch_bounds__(kPackThreads)
         for (int r = 0; r < 4; ++r) {
           int v = 0;
 #pragma unroll
-          for (int c = 0; c < kPackCols / 32; ++c) v = max(v, abs_high(x[r][c]));
+          for (int c = 0; c < kPackCols / 32; ++c) v = max(v, tc::abs_high(x[r][c]));
           v = __reduce_max_sync(0xffffffffu, v);
           if (lane == r0 + r) best = v;
         }
@@ -109,7 +103,7 @@ __global__ void __launch_bounds__(kPackThreads)
     for (int q = 0; q < 8; ++q) {
       const int e = tid + q * kPackThreads;
       const int r = rows_fast ? e & 31 : e >> 6, k = rows_fast ? e >> 5 : e & 63;
-      best[q] = roff[r] >= 0 && koff[k] >= 0 ? abs_high(__ldg(src + roff[r] + koff[k])) : 0;
+      best[q] = roff[r] >= 0 && koff[k] >= 0 ? tc::abs_high(__ldg(src + roff[r] + koff[k])) : 0;
     }
     if (rows_fast) {  // a thread's eight elements share its row
       int v = 0;
@@ -662,14 +656,22 @@ void SlicePlan::finalize() {
       wide += (int64_t)((op.rows + kPackRows - 1) / kPackRows) *
               ((op.cols + kPackCols - 1) / kPackCols);
   const int width = wide < 4 * kPackWarps * (ctx ? ctx->num_sms : 152) ? 32 : kPackCols;
-  for (size_t o = 0; o < ops.size(); ++o) {
-    const SlOp &op = ops[o];
-    if (by_cols(op)) {
-      for (int32_t r = 0; r < op.rows; r += kPackRows)
-        for (int32_t k = 0; k < op.cols; k += width) items_k.push_back({(int32_t)o, r, k, width});
-    } else {
-      for (int32_t r = 0; r < op.rows; r += 32)
-        for (int32_t k = 0; k < op.cols; k += 64) items_t.push_back({(int32_t)o, r, k, 64});
+  for (int src = 0; src < 2; ++src) {
+    for (size_t o = 0; o < ops.size(); ++o) {
+      const SlOp &op = ops[o];
+      if (op.src != src) continue;
+      if (by_cols(op)) {
+        for (int32_t r = 0; r < op.rows; r += kPackRows)
+          for (int32_t k = 0; k < op.cols; k += width)
+            items_k.push_back({(int32_t)o, r, k, width});
+      } else {
+        for (int32_t r = 0; r < op.rows; r += 32)
+          for (int32_t k = 0; k < op.cols; k += 64) items_t.push_back({(int32_t)o, r, k, 64});
+      }
+    }
+    if (src == 0) {
+      first_k = (int)items_k.size();
+      first_t = (int)items_t.size();
     }
   }
   // K parts: a unit of work is at most about a third of one SM's share of the
@@ -759,19 +761,31 @@ double SlicePlan::seconds() const {
   return 30e-6 + steps * 0.7e-6 / 152 + elems * 30.0 / 3e12;
 }
 
+void SlicePlan::clear_scales() const {
+  UDMRG_CHECK_CUDA(cudaMemsetAsync(scale, 0, nscale() * sizeof(int), ctx->stream));
+}
+
 void run_slice(Ctx &ctx, const SlicePlan &p, const double *a, const double *b, double *c) {
   if (p.tiles.empty()) return;
-  UDMRG_CHECK_CUDA(cudaMemsetAsync(p.scale, 0, p.nscale() * sizeof(int), ctx.stream));
+  if (!p.prescaled) p.clear_scales();
   const int nk = (int)p.items_k.size(), nx = (int)p.items_t.size();
-  const int nbk = std::min((nk + kPackWarps - 1) / kPackWarps, 16 * ctx.num_sms);
-  const int grid = nbk + std::min(nx, 8 * ctx.num_sms);
-  if (grid) {
-    slice_scale_kernel<<<grid, kPackThreads, 0, ctx.stream>>>(p.d_ops, p.d_items_k, nk, nbk,
-                                                              p.d_items_t, nx, a, b, p.scale);
+  const int k0 = p.prescaled ? p.first_k : 0, t0 = p.prescaled ? p.first_t : 0;
+  auto k_blocks = [&](int n) {
+    return std::min((n + kPackWarps - 1) / kPackWarps, 16 * ctx.num_sms);
+  };
+  auto grid = [&](int n, int m) { return k_blocks(n) + std::min(m, 8 * ctx.num_sms); };
+  if (grid(nk - k0, nx - t0)) {
+    slice_scale_kernel<<<grid(nk - k0, nx - t0), kPackThreads, 0, ctx.stream>>>(
+        p.d_ops, p.d_items_k + k0, nk - k0, k_blocks(nk - k0), p.d_items_t + t0, nx - t0, a, b,
+        p.scale);
     UDMRG_CHECK_CUDA(cudaGetLastError());
-    UDMRG_CHECK_CUDA(tc::launch_pdl(slice_pack_kernel, dim3(grid), dim3(kPackThreads), 0,
-                                    ctx.stream, p.d_ops, p.d_items_k, nk, nbk, p.d_items_t, nx, a,
-                                    b, p.scale, p.img));
+    ctx.launches++;
+  }
+  if (grid(nk, nx)) {
+    UDMRG_CHECK_CUDA(tc::launch_pdl(slice_pack_kernel, dim3(grid(nk, nx)), dim3(kPackThreads), 0,
+                                    ctx.stream, p.d_ops, p.d_items_k, nk, k_blocks(nk),
+                                    p.d_items_t, nx, a, b, p.scale, p.img));
+    ctx.launches++;
   }
   static bool attr_set = false;
   if (!attr_set) {
@@ -784,7 +798,7 @@ void run_slice(Ctx &ctx, const SlicePlan &p, const double *a, const double *b, d
                                   dim3(kSlThreads), kSlSmem, ctx.stream, p.d_tiles, nt,
                                   p.d_groups, p.d_lines, p.d_cblk, p.scale, p.img, c, p.scale,
                                   p.scratch, p.scale + 2 + p.lines.size()));
-  ctx.launches += grid ? 3 : 1;
+  ctx.launches++;
 }
 
 }  // namespace udmrg

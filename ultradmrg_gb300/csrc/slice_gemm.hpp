@@ -84,13 +84,16 @@ struct SlTile {
 struct SlicePlan {
   Ctx *ctx = nullptr;
   std::vector<SlOp> ops;
-  std::vector<SlItem> items_k, items_t;  // of ops with contiguous columns, of the others
+  // of ops with contiguous columns, of the others; the first operand's first
+  std::vector<SlItem> items_k, items_t;
+  int first_k = 0, first_t = 0;  // the first operand's
   std::vector<SlGroup> groups;
   std::vector<SlTile> tiles;
   std::vector<SlLine> lines;
   std::vector<int64_t> cblk;
   int64_t slots = 0;  // scratch slots (one per part of a tile with several)
   int64_t img_bytes = 0;
+  bool prescaled = false;  // the first operand's scales are found by its producer
   bool holes = false;  // image entries no op writes
   uint8_t *d_block = nullptr;  // the tables and scale
   SlOp *d_ops = nullptr;
@@ -124,6 +127,7 @@ struct SlicePlan {
   void finalize();         // items, K parts and tile order (host)
   void upload();           // device tables and workspaces
   size_t workspace() const;
+  void clear_scales() const;  // device: flags, scales, counters to zero
   size_t nscale() const { return 2 + lines.size() + 16 * (size_t)slots; }
 };
 

@@ -156,6 +156,13 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
          | ((uint32_t)(M >> 4) << 24); // M / 16
 }
 
+// High word of |x|, bit 0 set where the low word alone is nonzero: the maximum over
+// a line of a sliced GEMM's operand is the line's scale.
+__device__ __forceinline__ int abs_high(double x) {
+  const uint64_t d = (uint64_t)__double_as_longlong(x);
+  return (int)((uint32_t)(d >> 32) & 0x7FFFFFFFu) | ((uint32_t)d ? 1 : 0);
+}
+
 // Tile of round i of a persistent block over a list sorted by descending work:
 // rounds alternate in direction, so that the block with the longest tile of one
 // round gets the shortest of the next.
