@@ -255,12 +255,15 @@ __device__ __forceinline__ void tc_mma_role(const TcTile *__restrict__ tiles, in
           tc::mma_bf16(dcol, ad, bd, idesc, (c > 0 || ks > 0 || p > 0) ? 1u : 0u);
         }
       };
+      // (unrolled twice: constant descriptors in the tail, no branches before it)
       if (c + 1 < g.kc) {
 #pragma unroll
         for (int ks = 0; ks < kTcBK / 16; ++ks) step(ks);
       } else {
         const int nks = tc_chunk_k(g, c) >> 4;
-        for (int ks = 0; ks < nks; ++ks) step(ks);
+#pragma unroll
+        for (int ks = 0; ks < kTcBK / 16; ++ks)
+          if (ks < nks) step(ks);
       }
       tc::mma_commit(&b.empty[s]);  // the stage is free once these MMAs completed
     }
