@@ -148,7 +148,7 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
     grouped_gemm_kernel(const GTile *__restrict__ tiles, int ntiles,
                         const GProb *__restrict__ probs, const GSeg *__restrict__ segs,
                         const In *__restrict__ A, const In *__restrict__ B, In *__restrict__ C,
-                        double alpha, double beta, const int *__restrict__ gate) {
+                        double alpha, double beta, const int *gate) {
   // gate: the sliced form's flags; the tiles run only where it did not apply
   tc::pdl_wait();  // the sliced form's kernel (a no-op in an ordinary launch)
   if (gate && gate[0] == 0 && gate[1] == 0) return;

@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(kPackThreads)
 // than the 36 products of a step.  Sixteen warps of 16 outputs (three registers
 // each: no spills at the 96 registers that 576 threads leave) against eight of
 // 32: Hubbard 4x8, D = 1000, effective Hamiltonian 549 -> 402 us together with
-// the K parts and slice_pack_k_kernel.
+// the K parts and the direct pack of contiguous columns.
 constexpr int kSlParts = 4;  // epilogue warps per lane quarter
 constexpr int kSlCols = kSlV / kSlParts;
 constexpr int kSlThreads = 64 + 128 * kSlParts;
@@ -356,7 +356,7 @@ __device__ __forceinline__ double sl_round(const SlSum &s, int e) {
 __global__ void __launch_bounds__(kSlThreads, 1)
     slice_gemm_kernel(const SlTile *__restrict__ tiles, int ntiles,
                       const SlGroup *__restrict__ groups, const SlLine *__restrict__ lines,
-                      const int64_t *__restrict__ cblk, const int *__restrict__ scale,
+                      const int64_t *__restrict__ cblk, const int *scale,
                       const uint8_t *__restrict__ img, double *__restrict__ C, int *flags,
                       longlong2 *__restrict__ scratch, int *__restrict__ arrived) {
   extern __shared__ __align__(1024) uint8_t smem[];

@@ -176,7 +176,8 @@ __device__ __forceinline__ int snake_tile(int i) {
 // pdl_wait() before it touches anything the predecessor writes (a no-op when
 // nothing is pending), and pdl_launch_dependents() once its own main loop
 // is done, so that its successor's blocks can be scheduled as the last
-// blocks drain.
+// blocks drain.  What is read right behind pdl_wait() is not declared
+// __restrict__: a load from a read-only argument could be moved above it.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
