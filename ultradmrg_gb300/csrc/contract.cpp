@@ -114,13 +114,16 @@ double fp64_seconds(const GemmPlan &g, bool cplx, bool upper) {
 }
 
 // Below this estimate the sliced form's three launches and its passes over
-// the operands cannot pay, and its tables are not built.
+// the operands hardly pay (96^3: 43 us in FP64, 36 sliced; 64^3 takes 35), and
+// its tables are not built.
 constexpr double kSliceMin = 50e-6;
 
-// Contractions over an MPO tensor's few channels stay on the FMAs: their K
-// fills one or two steps, and packing the large operand costs more than its
-// products.
-constexpr double kSliceMinK = 28;
+// Shorter contractions stay on the FMAs: their K fills less than half of one
+// step, and cutting the large operand into digits costs what the products
+// save.  FP64 / sliced form, device time: 40000 x 8 x 8 (rows, columns, K)
+// 48 / 43 us, 40000 x 20 x 20 89 / 49, 40000 x 64 x 16 103 / 64; T1 with an MPO
+// tensor, Hubbard D = 500 870 / 321 us, complex ladder D = 300 464 / 193.
+constexpr double kSliceMinK = 8;
 double mean_k(const GemmPlan &g) {  // mean summed K, weighted with the work
   double w = 0, wk = 0;
   for (const GProb &p : g.probs) {

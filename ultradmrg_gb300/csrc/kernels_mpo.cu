@@ -134,10 +134,13 @@ __global__ void __launch_bounds__(32 * kMpoWarps, 2)
 }
 
 // FP64 form.  A warp takes 64 consecutive (a', b) entries of one pair, two per
-// lane, and walks the pair's couplings (32 records held one per lane, handed
-// out by shuffles; the loads of four couplings' two entries in flight).  HBM
-// bound: 8 B read per T1 entry and written per T3 entry, both in contiguous
-// runs of db.
+// lane, and walks a run of the pair's couplings (32 records held one per lane,
+// handed out by shuffles; the loads of four couplings' two entries in flight).
+// 8 B read per T1 entry and written per T3 entry, both in contiguous runs of db;
+// bound by the latency of the loads (Hubbard 4x8, D = 1000: 66 us, 2.2 TB/s).
+// With scale, the maxima of T3's rows too: one per a' and channel where the
+// task spans at most four a', else over runs of lanes of one a' (against a
+// pass of its own over T3: 44 us).
 __global__ void __launch_bounds__(256)
     mpo_map64_kernel(const MpoTask64 *__restrict__ tasks, int ntasks,
                      const MpoPair64 *__restrict__ pairs, const MpoOut64 *__restrict__ outs,
