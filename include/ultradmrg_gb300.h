@@ -114,8 +114,9 @@ int udmrg_ctx_launches(udmrg_ctx *ctx, uint64_t *out);
  * (lanczos_vmps_solver_impl.h:148, 213). */
 int udmrg_ctx_set_krylov_graph(udmrg_ctx *ctx, int enable);
 /* The mixed-precision Lanczos ends with a refinement run whose first step is
- * one FP64-accurate matvec (the anchor).  dw != 0 (the default): its two
- * block-GEMM stages, and the mixed-precision sweep's environment updates, in
+ * one FP64-accurate matvec (the anchor).  For the contractions of it, and of
+ * the mixed-precision sweep's environment updates, that do not take digit
+ * slices (udmrg_ctx_set_gemm_form), dw != 0 (the default): in
  * double-word FP32 arithmetic (each FP64 operand split into two floats, 48
  * significant bits, error-free products and sums; about 2^-48 relative per
  * product, on this GPU's FP32 pipe instead of its narrow FP64 pipe) for real
@@ -405,8 +406,9 @@ int udmrg_matvec_plan_apply(udmrg_matvec_plan *p, const double *d_in, double *d_
  * copies.  The host-facing form of eff_ham_mul_two_site_state
  * (lanczos_vmps_solver_impl.h:250-289). */
 int udmrg_matvec_plan_apply_host(udmrg_matvec_plan *p, const double *h_in, double *h_out);
-/* The same product in the mixed solver's anchor form (FP64 pipe or
- * double-word FP32, per udmrg_ctx_set_anchor_dw), whatever the plan's
+/* The same product in the mixed solver's anchor form (digit slices, or where
+ * they do not apply the FP64 pipe or double-word FP32, per
+ * udmrg_ctx_set_anchor_dw), whatever the plan's
  * precision. */
 int udmrg_matvec_plan_apply_anchor(udmrg_matvec_plan *p, const double *d_in, double *d_out);
 int udmrg_matvec_plan_destroy(udmrg_matvec_plan *p);
