@@ -114,13 +114,15 @@ int udmrg_ctx_launches(udmrg_ctx *ctx, uint64_t *out);
  * (lanczos_vmps_solver_impl.h:148, 213). */
 int udmrg_ctx_set_krylov_graph(udmrg_ctx *ctx, int enable);
 /* The mixed-precision Lanczos ends with a refinement run whose first step is
- * one FP64-accurate matvec (the anchor).  For the contractions of it, and of
- * the mixed-precision sweep's environment updates, that do not take digit
- * slices (udmrg_ctx_set_gemm_form), dw != 0 (the default): in
+ * one FP64-accurate matvec (the anchor).  For real data it runs, with
+ * dw != 0 (the default), in
  * double-word FP32 arithmetic (each FP64 operand split into two floats, 48
  * significant bits, error-free products and sums; about 2^-48 relative per
- * product, on this GPU's FP32 pipe instead of its narrow FP64 pipe) for real
- * data; 0: on the FP64 pipe.  Complex data always uses the FP64 pipe.  The
+ * product, on this GPU's FP32 pipe instead of its narrow FP64 pipe);
+ * 0: on the FP64 pipe.  So do those contractions of the mixed-precision
+ * sweep's environment updates that do not take digit slices
+ * (udmrg_ctx_set_gemm_form).  The anchor takes slices only with gemm form 1,
+ * or for complex data, which has no double-word form.  The
  * plain FP64 form is not affected.  Replaces nothing in qlmps (its matvec
  * is FP64 throughout). */
 int udmrg_ctx_set_anchor_dw(udmrg_ctx *ctx, int dw);
@@ -406,10 +408,9 @@ int udmrg_matvec_plan_apply(udmrg_matvec_plan *p, const double *d_in, double *d_
  * copies.  The host-facing form of eff_ham_mul_two_site_state
  * (lanczos_vmps_solver_impl.h:250-289). */
 int udmrg_matvec_plan_apply_host(udmrg_matvec_plan *p, const double *h_in, double *h_out);
-/* The same product in the mixed solver's anchor form (digit slices, or where
- * they do not apply the FP64 pipe or double-word FP32, per
- * udmrg_ctx_set_anchor_dw), whatever the plan's
- * precision. */
+/* The same product in the mixed solver's anchor form
+ * (udmrg_ctx_set_anchor_dw), whatever the plan's precision (a plan of the
+ * plain FP64 form takes its own GEMM form). */
 int udmrg_matvec_plan_apply_anchor(udmrg_matvec_plan *p, const double *d_in, double *d_out);
 int udmrg_matvec_plan_destroy(udmrg_matvec_plan *p);
 /* One matvec with CUDA events between its four stages (device ms, written to

@@ -1,0 +1,67 @@
+"""What the choice of a form must not change: results that a mixed Krylov run
+amplifies keep one summation order whatever the cost rule takes elsewhere."""
+import numpy as np
+import pytest
+
+from ultradmrg_gb300 import api
+from ultradmrg_gb300 import models as M
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from ultradmrg_gb300 import build
+    build.build()
+    c = api.Context(0)
+    yield c
+    c.close()
+
+
+@pytest.fixture(scope="module")
+def problem(ctx):
+    """Centre bond of a Hubbard cylinder, large enough that the cost rule slices."""
+    mpo, pb = M.hubbard_cylinder_mpo(4, 4, t=1.0, U=8.0, builder="reference")
+    mps = M.random_mps([pb] * 16, (14, 0), 400, seed=5, sigma=2.0)
+    L, R = api.build_envs(ctx, mpo, mps, 7)
+    ten = [api.DeviceTensor.from_data(ctx, t) for t in (mps[7], mps[8], mpo[7], mpo[8])]
+    psi = api.contract(ctx, ten[0], ten[1], [2], [0])
+    return [L, ten[2], ten[3], R], psi, ten[:2]
+
+
+def in_form(ctx, form, fn):
+    old = ctx.gemm_form()
+    ctx.set_gemm_form(form)
+    try:
+        return fn()
+    finally:
+        ctx.set_gemm_form(old)
+
+
+def test_mixed_anchor_keeps_its_order(ctx, problem):
+    """The double-word anchor under the cost rule is the FMA form's, bit for bit,
+    at a size where the rule slices the plain product."""
+    eff, psi, _ = problem
+
+    def products(precision, anchor):
+        plan = api.MatvecPlan(ctx, eff, psi, precision=precision)
+        x, y = plan.embed(psi), plan.embed(psi)
+        (plan.apply_anchor if anchor else plan.apply)(x, y)
+        return y.download_packed()
+
+    rule, fma = (in_form(ctx, f, lambda: products(api.PREC_MIXED, True)) for f in (-1, 0))
+    assert np.array_equal(rule, fma)
+    rule, fma = (in_form(ctx, f, lambda: products(api.PREC_FP64, False)) for f in (-1, 0))
+    assert not np.array_equal(rule, fma)  # (the rule does slice here)
+
+
+def test_mixed_solve_keeps_its_order(ctx, problem):
+    """So a whole mixed solve does not depend on the rule."""
+    eff, psi, _ = problem
+
+    def solve():
+        r = api.lanczos_solver(ctx, eff, psi, 1e-9, 100, precision=api.PREC_MIXED)
+        return r.gs_eng, r.gs_vec.download_packed()
+
+    (e0, v0), (e1, v1) = (in_form(ctx, f, solve) for f in (-1, 0))
+    assert e0 == e1 and np.array_equal(v0, v1)

@@ -72,9 +72,10 @@ class Context:
         return t.value, c.value
 
     def set_anchor_dw(self, dw: bool):
-        """The mixed solver's FP64-accurate anchor matvec, where its contractions
-        do not take digit slices (``set_gemm_form``): in double-word FP32
-        arithmetic (default) or on the FP64 pipe."""
+        """The mixed solver's FP64-accurate anchor matvec of real data, and the
+        mixed sweep's environment contractions that take no digit slices
+        (``set_gemm_form``): in double-word FP32 arithmetic (default) or on the
+        FP64 pipe."""
         call("udmrg_ctx_set_anchor_dw", self.h, 1 if dw else 0)
 
     def set_host_mapped(self, mode: int):
@@ -720,8 +721,8 @@ class MatvecPlan:
              C.cast(C.c_void_p(d_in), _lib.c_double_p), C.cast(C.c_void_p(d_out), _lib.c_double_p))
 
     def apply_anchor(self, x: DeviceTensor, y: DeviceTensor):
-        """The mixed solver's FP64-accurate anchor product (digit
-        slices, FP64 pipe or double-word FP32, per ``Context.set_anchor_dw``)."""
+        """The mixed solver's FP64-accurate anchor product
+        (``Context.set_anchor_dw``)."""
         self.apply_anchor_ptr(x.device_ptr(), y.device_ptr())
 
     def stage_times(self, d_in: int, d_out: int):

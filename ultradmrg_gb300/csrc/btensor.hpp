@@ -188,6 +188,21 @@ struct DeviceScratch {
   }
 };
 
+// Plans built in its lifetime keep their GEMMs on the FMAs (gemm_form 0) unless
+// the caller chose a form: what a mixed Krylov run starts from (the two-site
+// state, the double-word anchor) decides its result beyond the last bit, because
+// the run amplifies a change of its inputs ten-thousandfold.
+struct FmaGemms {
+  Ctx &c;
+  const int form;
+  FmaGemms(Ctx &x, bool on) : c(x), form(x.gemm_form) {
+    if (on && form < 0) c.gemm_form = 0;
+  }
+  ~FmaGemms() { c.gemm_form = form; }
+  FmaGemms(const FmaGemms &) = delete;
+  FmaGemms &operator=(const FmaGemms &) = delete;
+};
+
 // Host tables copied to the device in one allocation and one copy.
 struct UploadBatch {
   Ctx &ctx;

@@ -428,7 +428,8 @@ static std::unique_ptr<ContractPlan> plan_impl(const BTensor &A, const BTensor &
                                                const std::vector<int> &cb,
                                                const std::vector<int> &fa,
                                                const std::vector<int> &fb, const BTensor *dst,
-                                               std::vector<int64_t> *missing, bool upload) {
+                                               std::vector<int64_t> *missing, bool upload,
+                                               const std::vector<int> &seg_axes = {}) {
   UDMRG_REQUIRE(ca.size() == cb.size(), "contract: axis lists differ in length");
   UDMRG_REQUIRE(A.dtype == B.dtype, "contract: operands must have the same element type");
   UDMRG_REQUIRE(fa.size() + ca.size() == (size_t)A.rank(), "contract: bad A axes");
@@ -476,8 +477,10 @@ static std::unique_ptr<ContractPlan> plan_impl(const BTensor &A, const BTensor &
       matches.push_back({ok, a, it->second});
     }
   }
-  std::sort(matches.begin(), matches.end(), [](const Match &x, const Match &y) {
+  std::sort(matches.begin(), matches.end(), [&](const Match &x, const Match &y) {
     if (x.okey != y.okey) return x.okey < y.okey;
+    for (int ax : seg_axes)
+      if (A.key(x.a)[ax] != A.key(y.a)[ax]) return A.key(x.a)[ax] < A.key(y.a)[ax];
     if (x.a != y.a) return x.a < y.a;
     return x.b < y.b;
   });
@@ -783,8 +786,9 @@ std::unique_ptr<ContractPlan> plan_contract_into(const BTensor &A, const BTensor
                                                  const std::vector<int> &cb,
                                                  const std::vector<int> &fa,
                                                  const std::vector<int> &fb, const BTensor &dst,
-                                                 std::vector<int64_t> *missing, bool upload) {
-  return plan_impl(A, B, ca, cb, fa, fb, &dst, missing, upload);
+                                                 std::vector<int64_t> *missing, bool upload,
+                                                 const std::vector<int> &seg_axes) {
+  return plan_impl(A, B, ca, cb, fa, fb, &dst, missing, upload, seg_axes);
 }
 
 std::unique_ptr<ContractPlan> plan_contract_axes(const BTensor &A, const BTensor &B,

@@ -279,6 +279,9 @@ std::unique_ptr<MatvecPlan> plan_matvec2(Ctx &ctx, const BTensor &L, const BTens
   // tables.  Device work (uploads, packing) follows on this thread.
   S->prepare_lookup();
   {
+    // the mixed solver's anchor on real data keeps its double-word (or FP64)
+    // arithmetic and one summation order (segments by b, then w2)
+    FmaGemms fma(ctx, mixed && psi0.dtype == kF64);
     using Fut = std::future<void>;
     std::vector<Fut> jobs;
     auto run = [&](auto fn) { jobs.push_back(std::async(std::launch::async, fn)); };
@@ -287,7 +290,7 @@ std::unique_ptr<MatvecPlan> plan_matvec2(Ctx &ctx, const BTensor &L, const BTens
     run([&] { mv->p3 = plan_contract_cyclic(*s2, W2, 4, 0, 2, false); });
     run([&] {
       mv->p4 = map ? plan_contract_into(*t3s, R, {3, 4}, {1, 2}, {0, 1, 2}, {0}, *S, &mv->missing,
-                                        false)
+                                        false, {4, 3})
                    : plan_contract_into(*s3, R, ca, cb, fa, fb, *S, &mv->missing, false);
     });
     if (map) run([&] { mv->m64 = build_mpo_step64(*fm, *s1, *t3s); });
@@ -1023,12 +1026,7 @@ LocalUpdate two_site_update_local(Ctx &ctx, const BTensor &lenv, const BTensor &
   // two-site state is formed by the FP64 kernels in either form of the solve.
   TensorPtr init_state;
   {
-    struct FmaForm {
-      Ctx &c;
-      const int form;
-      explicit FmaForm(Ctx &x) : c(x), form(x.gemm_form) { c.gemm_form = 0; }
-      ~FmaForm() { c.gemm_form = form; }
-    } fma(ctx);
+    FmaGemms fma(ctx, true);
     init_state = contract_axes(ctx, mps_l, mps_r, {2}, {0});
   }
   auto mv = plan_matvec2(ctx, lenv, mpo_l, mpo_r, renv, *init_state, p.lancz.precision);

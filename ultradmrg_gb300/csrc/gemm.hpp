@@ -113,7 +113,8 @@ std::unique_ptr<ContractPlan> plan_contract(const BTensor &A, const BTensor &B,
 // Plan whose output is written into an existing structure `dst` (every block
 // the contraction produces must exist in dst).  Blocks of dst that receive no
 // contribution are listed in `missing` (block ids) and must be zeroed by the
-// caller.
+// caller.  seg_axes: an output block sums its segments by ascending sectors of
+// these axes of A (default: by A's block order).
 std::unique_ptr<ContractPlan> plan_contract_into(const BTensor &A, const BTensor &B,
                                                  const std::vector<int> &ca,
                                                  const std::vector<int> &cb,
@@ -121,7 +122,8 @@ std::unique_ptr<ContractPlan> plan_contract_into(const BTensor &A, const BTensor
                                                  const std::vector<int> &b_free_order,
                                                  const BTensor &dst,
                                                  std::vector<int64_t> *missing,
-                                                 bool upload = true);
+                                                 bool upload = true,
+                                                 const std::vector<int> &seg_axes = {});
 
 // Plain-axes contraction (qlten's Contract(A, B, {axes_a, axes_b}, C)).
 std::unique_ptr<ContractPlan> plan_contract_axes(const BTensor &A, const BTensor &B,
