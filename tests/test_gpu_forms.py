@@ -1,9 +1,12 @@
 """What the choice of a form must not change: results that a mixed Krylov run
 amplifies keep one summation order whatever the cost rule takes elsewhere."""
+import json
+import os
+
 import numpy as np
 import pytest
 
-from ultradmrg_gb300 import api
+from ultradmrg_gb300 import _lib, api
 from ultradmrg_gb300 import models as M
 
 pytestmark = pytest.mark.gpu
@@ -65,3 +68,43 @@ def test_mixed_solve_keeps_its_order(ctx, problem):
 
     (e0, v0), (e1, v1) = (in_form(ctx, f, solve) for f in (-1, 0))
     assert e0 == e1 and np.array_equal(v0, v1)
+
+
+# ---- small sectors of the SVD ---------------------------------------------------
+
+def exact_gram(n, rank):
+    """Z D Z^T of small integers and powers of two: exact in FP64, its smallest
+    eigenvalues up to 2^-32 of the largest."""
+    rng = np.random.default_rng(100 * n + rank)
+    z = rng.integers(-64, 65, (n, rank)) * 2.0 ** -np.sort(rng.integers(0, 17, rank))
+    return z @ z.T
+
+
+def sym_eig(ctx, mats):
+    ns = np.array([m.shape[0] for m in mats], np.int32)
+    flat = np.concatenate([m.ravel() for m in mats])
+    lam, vec = np.zeros(int(ns.sum())), np.zeros(flat.size)
+    ptr = lambda a, t: a.ctypes.data_as(t)  # noqa: E731
+    _lib.call("udmrg_selftest_sym_eig", ctx.h, len(mats), ptr(ns, _lib.c_int32_p),
+              ptr(flat, _lib.c_double_p), ptr(ns, _lib.c_int32_p), ptr(lam, _lib.c_double_p),
+              ptr(vec, _lib.c_double_p))
+    cut = np.cumsum(ns)[:-1]
+    return [(w, v.reshape(len(w), -1)) for w, v in
+            zip(np.split(lam, cut), np.split(vec, np.cumsum(ns.astype(int) ** 2)[:-1]))]
+
+
+def test_small_sectors_keep_their_order(ctx):
+    """Up to 32 rows the eigenvalues are the one-CTA reduction's bit for bit
+    (recorded from it), and so is, up to the rounding of the projection itself,
+    the space of the leading vectors.  The lowest of these eigenvalues lie 2^-32
+    below the largest: another order of any sum in the reduction turns the space
+    by about 2^-53 2^32."""
+    path = os.path.join(os.path.dirname(__file__), "golden", "sym_eig_ordered.json")
+    gold = json.load(open(path))
+    sizes = [tuple(map(int, k.split())) for k in gold]
+    for (n, rank), (lam, z), g in zip(sizes, sym_eig(ctx, [exact_gram(*s) for s in sizes]),
+                                      gold.values()):
+        assert np.array_equal(lam, [float.fromhex(v) for v in g["lam"]]), n
+        z, x = z[:, :rank], np.arange(1, n + 1) / n
+        px = np.array([float.fromhex(v) for v in g["px"]])
+        assert np.abs(z @ (z.T @ x) - px).max() <= 1e-13 * np.linalg.norm(x), n

@@ -42,9 +42,11 @@ __device__ __forceinline__ double exp_shift(double x, int k) {
 // and scaling run on the integer pipes (64 sectors of a D = 2000 bond: 4.6 ->
 // 1.4 ms).  A zero minor counts as a sign change and goes on as -1e-30 of its
 // predecessor.  Up to 32 rows the quotients q_k = d_k - x - e2_{k-1} / q_{k-1}
-// themselves (Barth, Martin and Wilkinson): the chain is short either way, and
-// the few-state sectors of short chains keep their rounding, on whose last bit
-// a noised sweep's adaptation can turn.
+// themselves (Barth, Martin and Wilkinson).  The product form is the faster one
+// there too (64 matrices of 32 rows, values and vectors: 1.48 against 1.66 ms; of
+// 8 rows: 0.43 against 0.47), but with the ordered reduction the quotients give a
+// few-state sector's eigenvalues bit for bit, and a noised sweep adapts its noise
+// by the sign of an energy difference that can be rounding alone.
 constexpr int kSturmQuotient = 32;
 __device__ __forceinline__ int sturm_count(const double *d, const double *e2, int n, double x) {
   if (n <= kSturmQuotient) {
@@ -283,8 +285,9 @@ __device__ __forceinline__ double start_entry(uint64_t seed, int i) {
 // Bound: a serial chain of about 40 FP64 instructions per row, 64 clocks each
 // (a few hundred warps cannot fill the chip).  The factors of eight rows are
 // loaded together, ahead of the recurrences that use them, so the chain does
-// not wait for L2; one division per row; the norm is summed in the back
-// substitution and its factor applied by the next pass.
+// not wait for L2; two divisions per row (a multiplier from the pivot's reciprocal
+// would be rounded twice); the norm is summed from the first row on, its factor
+// applied by the next pass.
 constexpr int kInvB = 8;
 __global__ void __launch_bounds__(32)
     invit_kernel(const EigCluster *__restrict__ cl, int ncl, const EigJob *__restrict__ jobs,
@@ -332,7 +335,7 @@ __global__ void __launch_bounds__(32)
       }
       const bool keep = fabs(a) >= fabs(s0);
       const double r = rinv(keep ? a : s0);
-      const double f = (keep ? s0 : a) * r;
+      const double f = (keep ? s0 : a) / (keep ? (a != 0.0 ? a : tiny) : s0);
       const int64_t at = i * T;
       u0[at] = r;
       u1[at] = keep ? b : dl;
@@ -371,11 +374,9 @@ __global__ void __launch_bounds__(32)
           }
         }
       }
-      // back substitution with U, summing the norm
-      double y1 = 0.0, y2 = 0.0, nrm = 0.0;
-      y1 = cur * u0[(n - 1) * T];
+      // back substitution with U
+      double y1 = cur * u0[(n - 1) * T], y2 = 0.0;
       y[(n - 1) * T] = y1;
-      nrm = y1 * y1;
       for (int i0 = n - 2; i0 >= 0; i0 -= kInvB) {
         double av[kInvB], bv[kInvB], cv[kInvB], yv[kInvB];
 #pragma unroll
@@ -394,7 +395,6 @@ __global__ void __launch_bounds__(32)
           if (i >= 0) {
             const double s = fma(-cv[q], y2, fma(-bv[q], y1, yv[q])) * av[q];
             y[i * T] = s;
-            nrm = fma(s, s, nrm);
             y2 = y1;
             y1 = s;
           }
@@ -404,13 +404,11 @@ __global__ void __launch_bounds__(32)
       for (int q = c.first; q < p; ++q) {
         double s = 0.0;
         for (int i = 0; i < n; ++i) s += zc[(int64_t)i * c.ld + q] * y[i * T];
-        nrm = 0.0;
-        for (int i = 0; i < n; ++i) {
-          const double v = y[i * T] - s * zc[(int64_t)i * c.ld + q];
-          y[i * T] = v;
-          nrm = fma(v, v, nrm);
-        }
+        for (int i = 0; i < n; ++i) y[i * T] -= s * zc[(int64_t)i * c.ld + q];
       }
+      double nrm = 0.0;
+#pragma unroll 8
+      for (int i = 0; i < n; ++i) nrm = fma(y[i * T], y[i * T], nrm);
       nrm = sqrt(nrm);
       fac = nrm > 0.0 ? 1.0 / nrm : 0.0;
     }
@@ -453,6 +451,14 @@ __device__ __forceinline__ double2 cadd(double2 a, double2 b) {
 // next reflector.  The barrier gives up after kTriTimeoutNs and sets status 3.
 // Partial sums are added in CTA order, so the result does not depend on timing.
 //
+// A matrix of at most tri_one() rows is one CTA's, and ordered: every sum and
+// every entry's update has the order of a row per warp (32 interleaved chains and
+// their tree), whatever the lanes that compute it, and nothing fused across the
+// two terms of an update.  A Gram matrix's small sectors hold kept vectors whose
+// eigenvalue is near the rounding of the largest (a 9 x 9 one with s_7 / s_1 =
+// 5e-6: 4e-6 of the vector), so a state's small parts follow this kernel's last
+// bit.  Costs four FP64 instructions per entry and step instead of three.
+//
 // Bound: 3 m^2 FP64 FMAs per step at two per clock and SM (n^3 in all, shared
 // out over the CTAs), plus about 5.5 us per step of barrier, L2 and scalar
 // latency.  A warp's FP64 instruction holds its quarter's pipe for
@@ -463,7 +469,7 @@ struct TriPart {
   int32_t job, p, P, slot;
   int64_t wb_off;  // 4 n scalars: w entries and pivot rows (double-buffered by step parity)
   int64_t part_off;  // slice sums in the w buffer (-1: in shared memory)
-  int32_t resident, pad;  // the own rows are kept in shared memory
+  int32_t resident, ordered;  // the own rows are kept in shared memory; one CTA, fixed order
 };
 struct TriSlot {  // one per matrix, zeroed before the launch
   unsigned int arrive;
@@ -507,6 +513,16 @@ __device__ __forceinline__ double rank2(double a, double v, double w, double u, 
 __device__ __forceinline__ double2 rank2(double2 a, double2 v, double2 w, double2 u, double2 x) {
   const double2 p = cadd(cmul(v, w), cmul(u, x));
   return make_double2(a.x - p.x, a.y - p.y);
+}
+// The same in the fixed order: a - (v w + u x), real data with the first product
+// fused into the second's rounding, complex data (a - v w) - u x.
+__device__ __forceinline__ double rank2_ordered(double a, double v, double w, double u, double x) {
+  return __dsub_rn(a, fma(v, w, __dmul_rn(u, x)));
+}
+__device__ __forceinline__ double2 rank2_ordered(double2 a, double2 v, double2 w, double2 u,
+                                                 double2 x) {
+  const double2 p = cmul(v, w), q = cmul(u, x);
+  return make_double2(a.x - p.x - q.x, a.y - p.y - q.y);
 }
 __device__ __forceinline__ double sinv(double a) { return 1.0 / a; }
 __device__ __forceinline__ double2 sinv(double2 a) {
@@ -587,6 +603,12 @@ template <typename T>
 __host__ __device__ constexpr int tri_ld(int n) {
   return sizeof(T) == 8 ? (n + 7) / 16 * 16 + 8 : (n | 1);
 }
+// Largest matrix of the ordered one-CTA reduction (square and two rows within
+// 200 KB; the resident rows then fit an SM).
+template <typename T>
+__host__ __device__ constexpr int tri_one() {
+  return sizeof(T) == 8 ? 159 : 112;
+}
 // Slice sums of the row pass: one per own row of the full rounds, at most eight
 // for each of the 4 x 7 rows left over.
 __host__ __device__ constexpr int tri_parts(int n, int P) { return 224 + (n + P - 1) / P + 4; }
@@ -620,6 +642,9 @@ __global__ void __launch_bounds__(kTriThreads)
   const int64_t rld = pt.resident ? tri_ld<T>(n) : (int64_t)P * n;
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
   const int nwarp = nt >> 5;
+  const bool ordered = pt.ordered != 0;
+  // the thread's first vector entry: the ordered sums start at entry 2
+  const int r0 = ordered ? (tid + 2) & (kTriThreads - 1) : tid;
   unsigned nbar = 0;
 
   // 1. max-abs and finiteness of the upper triangle of the own rows; partials
@@ -708,15 +733,21 @@ __global__ void __launch_bounds__(kTriThreads)
 
   // Reflector of step j from the pivot row in rb (rb[c - j] = A[j][c]; its
   // entries rb[2 ..] already squared into x2): v (v_0 = 1) into v[0 .. m), tau
-  // into sh_t.  Same formulas as the single-CTA kernels.
+  // into sh_t.
   auto reflector = [&](int j, double x2, T *v) {
     for (int o = 16; o > 0; o >>= 1) x2 += __shfl_down_sync(0xffffffffu, x2, o);
     if (lane == 0) red[warp] = x2;
     __syncthreads();
     const int m = n - j - 1;
     if (warp == 0) {
-      double s = lane < nwarp ? red[lane] : 0.0;
-      for (int o = kTriThreads / 64; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      double s;
+      if (ordered) {
+        s = red[0];
+        for (int q = 1; q < (tri_one<T>() + 31) / 32; ++q) s += red[q];
+      } else {
+        s = lane < nwarp ? red[lane] : 0.0;
+        for (int o = kTriThreads / 64; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      }
       const T alpha = cj(rb[1]);
       const bool refl = s > 0.0 || sim(alpha) != 0.0;
       double beta = sre(alpha);
@@ -753,7 +784,7 @@ __global__ void __launch_bounds__(kTriThreads)
     constexpr int W = kTriThreads / 32;
     const int k0 = lo <= p ? 0 : (lo - p + P - 1) / P;
     const int cnt = kown - k0, g4 = (cnt + 3) >> 2;
-    const int gfull = g4 / W * W, rem = g4 - gfull;
+    const int gfull = ordered ? g4 : g4 / W * W, rem = g4 - gfull;
     int lq = 0;  // log2 Q: the smallest with rem Q a multiple of the warps
     while (((rem << lq) & (W - 1)) != 0) ++lq;
     const int Q = 1 << lq, len = n - lo;
@@ -766,8 +797,25 @@ __global__ void __launch_bounds__(kTriThreads)
       const bool ok = k < kown, first = i == lo;
       T s = smake<T>(0.0, 0.0);
       T *ar = rows + (ok ? k : k0) * rld + lo;
-      if (upd) {
-        const T vi = ok ? va[i - lo] : s, wi = ok ? wa[i - lo] : s;
+      const T vi = ok && upd ? va[i - lo] : s, wi = ok && upd ? wa[i - lo] : s;
+      if (ordered) {  // chains over columns 32 apart, four per lane, then their tree
+        T sq[4] = {s, s, s, s};
+        for (int c0 = lane & 7; c0 < len; c0 += 32) {
+#pragma unroll
+          for (int b = 0; b < 4; ++b) {
+            const int c = c0 + 8 * b;
+            if (c >= len) break;
+            T a = ar[c];
+            if (upd) {
+              a = rank2_ordered(a, vi, cj(wa[c]), wi, cj(va[c]));
+              if (ok) ar[c] = a;
+            }
+            if (first) prow[c] = a;
+            sq[b] = smadd(sq[b], a, vn[c]);
+          }
+        }
+        s = sadd(sadd(sq[0], sq[2]), sadd(sq[1], sq[3]));
+      } else if (upd) {
 #pragma unroll 4
         for (int c = q * 8 + (lane & 7); c < len; c += step) {
           const T a = rank2(ar[c], vi, cj(wa[c]), wi, cj(va[c]));
@@ -827,7 +875,7 @@ __global__ void __launch_bounds__(kTriThreads)
   // step 0: reflector and products of the own rows
   {
     double x2 = 0.0;
-    for (int c = tid; c < n; c += nt) {
+    for (int c = r0; c < n; c += nt) {
       rb[c] = __ldcg(&pb[n + c]);
       if (c >= 2) x2 += sabs2(rb[c]);
     }
@@ -845,7 +893,7 @@ __global__ void __launch_bounds__(kTriThreads)
     const T w0raw = __ldcg(&wj[0]);
 #pragma unroll
     for (int q = 0; q < kPer; ++q) {
-      const int r = tid + q * nt;
+      const int r = r0 + q * nt;
       if (r < m) {
         we[q] = __ldcg(&wj[r]);
         pe[q] = __ldcg(&pj[r]);
@@ -870,16 +918,18 @@ __global__ void __launch_bounds__(kTriThreads)
       const T v = vA[r];
       const T w = smadd(wr, K, v);
       wA[r] = w;
-      const T a = rank2(ar, smake<T>(1.0, 0.0), cj(w), w0, cj(v));
+      const T one = smake<T>(1.0, 0.0);
+      const T a = ordered ? rank2_ordered(ar, one, cj(w), w0, cj(v))
+                          : rank2(ar, one, cj(w), w0, cj(v));
       rb[r] = a;
       if (r >= 2) x2 += sabs2(a);
     };
 #pragma unroll
     for (int q = 0; q < kPer; ++q)
-      if (tid + q * nt < m) entry(tid + q * nt, we[q], pe[q]);
-    for (int r = tid + kPer * nt; r < m; r += nt) entry(r, __ldcg(&wj[r]), __ldcg(&pj[r]));
+      if (r0 + q * nt < m) entry(r0 + q * nt, we[q], pe[q]);
+    for (int r = r0 + kPer * nt; r < m; r += nt) entry(r, __ldcg(&wj[r]), __ldcg(&pj[r]));
     if (j + 2 == n) {  // the trailing block is the last diagonal entry
-      if (p == 0 && tid == 0) {
+      if (p == 0 && r0 == 0) {  // the thread that wrote it
         d[n - 1] = sre(rb[0]);
         e[n - 1] = 0.0;
         tau[n - 1] = smake<T>(0.0, 0.0);
@@ -902,7 +952,9 @@ __global__ void __launch_bounds__(kTriThreads)
 // forms the products with reflector j - 1, whose vector was copied to shared
 // memory meanwhile (cp.async), so neither L2 nor a block barrier is waited for.
 // FP64 bound: a warp's FP64 instruction holds its quarter's pipe for 64 clocks,
-// four per row of C columns and five additions per reflector.
+// four per row of C columns and nine additions per reflector.  A column's
+// product is summed over rows 32 apart in two chains, over the lanes by fours
+// and then over these: small sectors' vectors keep this order.
 template <typename T>
 struct BackShape;
 template <>
@@ -913,17 +965,26 @@ template <>
 struct BackShape<double2> {
   static constexpr int kCols = 1;
 };
-// sum of x over the warp in lanes 0 .. 15, of y in lanes 16 .. 31
+// sum of x over the warp in lanes 0 .. 15, of y in lanes 16 .. 31 (the parts of a
+// complex column)
 __device__ __forceinline__ double pair_sum(double x, double y) {
   const bool up = threadIdx.x & 16;
   double v = (up ? y : x) + __shfl_xor_sync(0xffffffffu, up ? x : y, 16);
   for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
+// Two real columns: sums over four lanes (x in the even ones, y in the odd ones),
+// then over the eight quads in order.
 __device__ __forceinline__ void back_weights(const double (&s)[2], double t, double (&w)[2]) {
-  const double v = pair_sum(s[0], s[1]) * t;
-  w[0] = __shfl_sync(0xffffffffu, v, 0);
-  w[1] = __shfl_sync(0xffffffffu, v, 16);
+  const bool odd = threadIdx.x & 1;
+  double v = (odd ? s[1] : s[0]) + __shfl_xor_sync(0xffffffffu, odd ? s[0] : s[1], 1);
+  v += __shfl_xor_sync(0xffffffffu, v, 2);
+  double sum = __shfl_sync(0xffffffffu, v, odd);
+#pragma unroll
+  for (int q = 1; q < 8; ++q) sum += __shfl_sync(0xffffffffu, v, 4 * q + odd);
+  sum *= t;
+  w[0] = __shfl_sync(0xffffffffu, sum, 0);
+  w[1] = __shfl_sync(0xffffffffu, sum, 1);
 }
 __device__ __forceinline__ void back_weights(const double2 (&s)[1], double2 t, double2 (&w)[1]) {
   const double v = pair_sum(s[0].x, s[0].y);
@@ -980,20 +1041,29 @@ __global__ void __launch_bounds__(32)
     back_weights(s, t, w);
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncwarp();
+    T s2[C][2];  // rows from j on, 32 apart, in two chains
 #pragma unroll
-    for (int c = 0; c < C; ++c)
-      s[c] = lane == 0 && j > 0 ? zs[c * n + j] : smake<T>(0.0, 0.0);
-#pragma unroll 4
-    for (int r = j + 1 + lane; r < n; r += 32) {
-      const T x = v[r], y = j > 0 ? cj(vn[r]) : smake<T>(0.0, 0.0);
+    for (int c = 0; c < C; ++c) s2[c][0] = s2[c][1] = smake<T>(0.0, 0.0);
+#pragma unroll 2
+    for (int r0 = j + lane; r0 < n; r0 += 64) {
 #pragma unroll
-      for (int c = 0; c < C; ++c) {
-        const T a = smsub(zs[c * n + r], x, w[c]);
-        zs[c * n + r] = a;
-        s[c] = smadd(s[c], y, a);
+      for (int h = 0; h < 2; ++h) {
+        const int r = r0 + 32 * h;
+        if (r >= n) break;
+        // row j takes part in the products only
+        const T x = r > j ? v[r] : smake<T>(0.0, 0.0);
+        const T y = j > 0 ? cj(vn[r]) : smake<T>(0.0, 0.0);
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          const T a = smsub(zs[c * n + r], x, w[c]);
+          zs[c * n + r] = a;
+          s2[c][h] = smadd(s2[c][h], y, a);
+        }
       }
     }
     __syncwarp();
+#pragma unroll
+    for (int c = 0; c < C; ++c) s[c] = sadd(s2[c][0], s2[c][1]);
     t = tn;
   }
   for (int r = lane; r < n; r += 32)
@@ -1003,6 +1073,10 @@ __global__ void __launch_bounds__(32)
 }
 
 }  // namespace
+
+bool eig_ordered(int64_t n, bool cplx) {
+  return n <= (cplx ? tri_one<double2>() : tri_one<double>());
+}
 
 // Shared memory a CTA of the reduction may use, and the matrices that leave
 // room for a second CTA on the SM.
@@ -1020,7 +1094,7 @@ static size_t tri_smem(int n, int P) {  // with the own rows resident
 // Householder reduction of every job.  Matrices of which two fit one SM's
 // shared memory run on one CTA each, on the side stream; the larger ones run in
 // one cooperative launch (more if they do not fit), the SMs shared out so that
-// all are expected to end together.
+// all are expected to end together (ordered ones: one CTA).
 template <typename T>
 static void tridiag_all(Ctx &ctx, DeviceScratch &scratch, const std::vector<EigJob> &jobs,
                         const SymEigWork &wk, double *G, int *dstat) {
@@ -1059,7 +1133,8 @@ static void tridiag_all(Ctx &ctx, DeviceScratch &scratch, const std::vector<EigJ
     const bool gpart = bytes > kTriSmemBytes;
     if (gpart) bytes = 4 * (size_t)n * sizeof(T);
     for (int p = 0; p < P; ++p) {
-      parts.push_back(TriPart{q, p, P, slot, wb, gpart ? wb_tot : -1, resident ? 1 : 0, 0});
+      parts.push_back(TriPart{q, p, P, slot, wb, gpart ? wb_tot : -1, resident ? 1 : 0,
+                              n <= tri_one<T>() ? 1 : 0});
       if (gpart) wb_tot += np;
     }
     ++slot;
@@ -1073,7 +1148,7 @@ static void tridiag_all(Ctx &ctx, DeviceScratch &scratch, const std::vector<EigJ
     int sum = 0;
     for (; end < big.size(); ++end) {
       const int n = jobs[big[end]].n;
-      const int c = std::min({kTriMaxParts, std::max(1, n / 8), budget});
+      const int c = n <= tri_one<T>() ? 1 : std::min({kTriMaxParts, n / 8, budget});
       int P = 1;
       while (P < c && tri_smem<T>(n, P) > kTriSmemBytes) ++P;
       if (end > at && sum + P > budget) break;

@@ -408,15 +408,23 @@ SvdResult svd_trunc(Ctx &ctx, const BTensor &T, int ldims, const QN &ldiv, doubl
   double *G = scratch.get<double>(es * std::max<int64_t>(gtot, 1));
   double *lam = scratch.get<double>(std::max<int64_t>(ltot, 1));
   {
-    GemmPlan g;
-    g.ctx = &ctx;
+    // Sectors that the reduction takes in one fixed order keep theirs on the FMAs
+    // too: their small singular values' vectors carry the product's last bit over
+    // (s / s_1)^2 (and a product this small gains nothing in slices).
+    GemmPlan g, gs;
+    g.ctx = gs.ctx = &ctx;
     for (int q = 0; q < nsec; ++q) {
       const XView x = xview(secs[q], left);  // G = X X^T (X X^H)
-      gemm_add_simple(g, jobs[q].g_off, x.xr, x.xr, x.xc, x.off, x.sr, x.sc, x.off, x.sc, x.sr,
-                      cplx);
+      gemm_add_simple(eig_ordered(jobs[q].n, cplx) ? gs : g, jobs[q].g_off, x.xr, x.xr, x.xc,
+                      x.off, x.sr, x.sc, x.off, x.sc, x.sr, cplx);
     }
     gemm_finalize(g, cplx, true);  // the eigensolver reads the upper triangles
-    run_gemm(ctx, g, cplx ? kC128 : kF64, Mbuf, Mc, G, 1.0, 0.0);
+    {
+      FmaGemms fma(ctx, true);
+      gemm_finalize(gs, cplx, true);
+    }
+    for (const GemmPlan *x : {&g, &gs})
+      run_gemm(ctx, *x, cplx ? kC128 : kF64, Mbuf, Mc, G, 1.0, 0.0);
   }
   // at most Dmax states are kept: only the leading eigenvalues of the sectors
   // (a margin of 64 below the Dmax-th largest) are computed; the weight of

@@ -69,6 +69,8 @@ void run_scale(Ctx &ctx, const std::vector<ScaleJob> &jobs, double *X, const dou
 int sym_eig_values(Ctx &ctx, DeviceScratch &scratch, std::vector<EigJob> &jobs, double *G,
                    double *lam, SymEigWork &wk, bool cplx = false, int64_t need = 0,
                    int64_t floor = 0, const std::vector<int64_t> *rank_cap = nullptr);
+// Whether a matrix of n rows is reduced in one fixed order (kernels_eig.cu).
+bool eig_ordered(int64_t n, bool cplx);
 // Phase 2: the leading k[q] eigenvectors of job q (hlam: host copy of lam) as
 // the columns of Z (row-major n x k[q], leading dimension z_ld[q], at z_off[q]),
 // orthonormal to FP64 accuracy.
@@ -76,7 +78,7 @@ void sym_eig_vectors(Ctx &ctx, DeviceScratch &scratch, const std::vector<EigJob>
                      const double *G, const double *lam, const std::vector<double> &hlam,
                      const std::vector<int64_t> &k, const std::vector<int64_t> &z_off,
                      const std::vector<int64_t> &z_ld, double *Z, const SymEigWork &wk,
-                     uint64_t seed = 1);
+                     uint64_t seed = 0x5EED5EEDull);
 
 void select_kept(const std::vector<std::vector<double>> &svals, double trunc_err, int64_t Dmin,
                  int64_t Dmax, std::vector<int64_t> &kept, int64_t &D, double &err,
