@@ -12,7 +12,11 @@ namespace {
 
 constexpr int kPackThreads = 256, kPackWarps = kPackThreads / 32;
 constexpr int kPackRows = 8, kPackCols = 128;  // item of the warps with contiguous columns
-constexpr int kLoExp = 1023 - 500, kHiExp = 1023 + 500;  // biased exponents of the sliced range
+// Biased exponents of the sliced range.  Two lines from its lower end have sums in
+// units of 2^-1018: no result is below the normal range.
+constexpr int kLoExp = 1023 - 476, kHiExp = 1023 + 476;
+static_assert(2 * (kLoExp - 1022) - 68 >= -1022, "sliced GEMM: sl_round makes no denormals");
+static_assert(2 * (kHiExp - 1022) + 30 <= 1023, "sliced GEMM: sums of 2^30 products stay finite");
 
 __device__ __forceinline__ int64_t sl_off(int64_t i, const int32_t *ext, const int64_t *str, int n) {
   int64_t off = 0;
@@ -320,7 +324,8 @@ __device__ __forceinline__ void sl_add(SlSum &s, int64_t hi, int64_t lo) {  // +
   s.lo = (uint32_t)lo;
 }
 
-// s 2^(e - 68) rounded to nearest FP64; |hi| < 2^62
+// s 2^(e - 68) rounded to nearest FP64; |hi| < 2^62, e within twice the sliced
+// range (the result is zero or normal)
 __device__ __forceinline__ double sl_round(const SlSum &s, int e) {
   const int64_t hi = s.hi;
   uint32_t w0 = s.lo;

@@ -104,7 +104,7 @@ struct SlicePlan {
   int64_t *d_cblk = nullptr;
   uint8_t *img = nullptr;
   // flags[0]: an operand is out of the sliced range (non-finite, or a row
-  // maximum outside 2^-500 .. 2^500), flags[1]: a bounded wait ran out; then
+  // maximum outside 2^-476 .. 2^476), flags[1]: a bounded wait ran out; then
   // one scale entry per line, then the arrival counters of the scratch slots
   int *scale = nullptr;
   longlong2 *scratch = nullptr;
