@@ -150,7 +150,11 @@ int udmrg_ctx_tc_tuning(udmrg_ctx *ctx, int64_t *trials, int64_t *classes);
  * MPO tensor as a GEMM too), 1 digit slices on the
  * tensor cores (exact integer products, one rounding), -1 the one a cost rule
  * on the padded work expects to be faster (default).  Plans built afterwards
- * follow it.  No counterpart in the reference. */
+ * follow it.  A slice keeps 62 bits below its row's (column's) largest element:
+ * errors are relative to row maximum x column maximum, so a result made of small
+ * terms alone (a graded row whose large entries meet zeros) has fewer correct
+ * digits than with FMAs, at most K 2^-57 of those maxima; choose 0 where such
+ * components count by themselves.  No counterpart in the reference. */
 int udmrg_ctx_set_gemm_form(udmrg_ctx *ctx, int form);
 int udmrg_ctx_gemm_form(udmrg_ctx *ctx, int *form);
 /* Tile policy of the grouped FP64 (and double-word) block GEMMs of a

@@ -32,3 +32,23 @@ def test_ends_of_the_range(ctx, ea, eb):  # noqa: F811
     tiny = np.ldexp(np.longdouble(1), -1074)
     assert np.all(np.isfinite(got))
     assert np.all(np.abs(got - ref) <= 2.0 ** -53 * np.abs(ref) + k * (2.0 ** -52 * top + tiny))
+
+
+@pytest.mark.parametrize("k", [256, 512, 1040])
+def test_coherent_low_digits(ctx, k):  # noqa: F811
+    """Leading digits that cancel over lower ones of one sign: the largest sums of
+    the lower levels, beyond 2^24 in level 5.  Bound: one rounding of the result and
+    four units of level 5 (2^-50 of the lines' scales, here 1) per product."""
+    s, t = (np.where(np.arange(k) // w % 2, -1, 1) for w in (1, 2))
+    low = sum(127 * 2.0 ** -(6 + 8 * d) for d in range(1, 5))
+    a = s * 63 / 64 + low + t * 127 * 2.0 ** -46
+    b = t * 63 / 64 + low + s * 127 * 2.0 ** -46
+    a, b = np.tile(a, (130, 1)), np.tile(b[:, None], (1, 66))
+    b[:, 1] *= -1.0
+    got = product(ctx, a, b)
+    ref = np.array([[sum(int(x) * int(y) for x, y in zip(a[0] * 2.0 ** 46, b[:, j] * 2.0 ** 46))
+                     for j in (0, 1)]], dtype=object)
+    for j in (0, 1):
+        exact = np.longdouble(float(ref[0, j] >> 40)) * np.ldexp(np.longdouble(1), 40 - 92)
+        cols = got[:, j::2] if j == 0 else got[:, 1:2]
+        assert np.all(np.abs(cols - exact) <= 2.0 ** -52 * np.abs(exact) + k * 2.0 ** -50)

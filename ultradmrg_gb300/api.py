@@ -51,7 +51,9 @@ class Context:
     def set_gemm_form(self, form: int = -1):
         """FP64-accurate grouped GEMMs of plans built afterwards: 0 FP64 (or
         double-word) FMAs, 1 digit slices on the tensor cores, -1 the one the
-        cost rule expects to be faster (default)."""
+        cost rule expects to be faster (default).  A sliced result's error is
+        relative to row maximum x column maximum, not to its own terms: choose 0
+        where small components count by themselves."""
         call("udmrg_ctx_set_gemm_form", self.h, int(form))
 
     def gemm_form(self) -> int:

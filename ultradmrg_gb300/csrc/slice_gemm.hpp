@@ -8,13 +8,25 @@
 // of 6: 62 bits below the row's power of two), each exact in BF16.  The products
 // of digit s of one operand and digit t of the other have weight
 // 2^-(12 + 8 (s + t)); those with s + t <= 7 (36 of the 64 pairs) are summed in
-// FP32 TMEM accumulators, one per level s + t.  The sums of levels 0 .. 3 are
-// integers below 2^24 for 256-deep K, so they are exact; those of levels 4 .. 7
-// are exact too or rounded below 2^-58 of the largest products.  The epilogue
+// FP32 TMEM accumulators, one per level s + t.  The sums of levels 0 .. 4 are
+// integers of at most 2^24 for 256-deep K, so they are exact.  The epilogue
 // adds the eight levels of an output in 64-bit integers (over all 256-deep K
-// chunks) and rounds once to FP64, without an FP64 instruction.  An output's
-// error is one FP64 rounding and about 2^-61 of (row maximum) x (column
-// maximum) per product.
+// chunks) and rounds once to FP64, without an FP64 instruction.
+//
+// Error: one FP64 rounding of the result, and per product of the two lines' scales
+// 2^-62 for the operands' last digits and 2^-59.2 for the dropped pairs (seven of
+// level 8, below 2^14 each): K 2^-57 rowmax colmax, since a scale is at most twice
+// its line's maximum.  Sums of levels 5 .. 7 can reach 1.75 2^24, where FP32 has
+// units of two; only where nearly all digits of a 256-deep run agree in sign and
+// size, and then by at most four units of level 5 (2^-50 of the scales) per
+// product.
+// The bound is to the lines' maxima, not to the terms of the sum as that of FP64
+// FMAs: elements more than 2^9 below their line's maximum keep fewer than 53
+// bits, so a small term that meets no large one (a product with an identity, an
+// output of graded lines whose large parts meet zeros) is not correct to its own
+// last bit.  In norm the form is the more accurate one: 1.0e-16 against the
+// FMAs' 7.5e-16 for an effective-Hamiltonian product (Heisenberg, D = 308, in
+// extended precision).
 //
 // The GEMMs of a block contraction are merged into one dense GEMM per set of
 // blocks that share contracted sectors (a quantum-number flow); sub-matrices
