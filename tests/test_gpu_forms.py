@@ -108,3 +108,49 @@ def test_small_sectors_keep_their_order(ctx):
         z, x = z[:, :rank], np.arange(1, n + 1) / n
         px = np.array([float.fromhex(v) for v in g["px"]])
         assert np.abs(z @ (z.T @ x) - px).max() <= 1e-13 * np.linalg.norm(x), n
+
+
+# ---- environments ---------------------------------------------------------------
+
+def _chain():
+    mpo, pb = M.hubbard_cylinder_mpo(4, 4, t=1.0, U=8.0, builder="reference")
+    return mpo, M.random_mps([pb] * 16, (14, 0), 250, seed=6, sigma=2.0)
+
+
+def test_build_envs_keeps_a_chosen_form(ctx):
+    """build_envs: FMAs under the rule, the caller's form where one is set (the
+    context's own updates, one by one)."""
+    mpo, mps = _chain()
+
+    def built():
+        return [t.download_packed() for t in api.build_envs(ctx, mpo, mps, 7, normalize=False)]
+
+    def grown():
+        out = []
+        for side, sites, grow in (("l", range(7), api.update_site_lenvs),
+                                  ("r", range(15, 8, -1), api.update_site_renvs)):
+            end = 0 if side == "l" else 15
+            e = api.DeviceTensor.from_data(ctx, api.trivial_env_data(mps[end], mpo[end], side))
+            for i in sites:
+                e = grow(ctx, e, *(api.DeviceTensor.from_data(ctx, t) for t in (mps[i], mpo[i])))
+            out.append(e.download_packed())
+        return out
+
+    for form, like in ((-1, 0), (0, 0), (1, 1)):
+        for x, y in zip(in_form(ctx, form, built), in_form(ctx, like, grown)):
+            assert np.array_equal(x, y), form
+
+
+def test_mixed_solve_from_either_environments(ctx):
+    """A mixed solve from environments of FMAs and of slices: Ritz values that move
+    less than 1e-10 in their last step, so the energies agree to a hundred such
+    steps."""
+    mpo, mps = _chain()
+    ten = [api.DeviceTensor.from_data(ctx, t) for t in (mps[7], mps[8], mpo[7], mpo[8])]
+    psi = in_form(ctx, 0, lambda: api.contract(ctx, ten[0], ten[1], [2], [0]))
+    e = []
+    for form in (0, 1):
+        L, R = in_form(ctx, form, lambda: api.build_envs(ctx, mpo, mps, 7, normalize=False))
+        e.append(api.lanczos_solver(ctx, [L, ten[2], ten[3], R], psi, 1e-10, 100,
+                                    precision=api.PREC_MIXED).gs_eng)
+    assert abs(e[0] - e[1]) <= 1e-8

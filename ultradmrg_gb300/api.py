@@ -641,11 +641,13 @@ def build_envs(ctx, mpo: Sequence[BlockTensorData], mps: Sequence[BlockTensorDat
     """Left environment of sites [0, l) and right environment of sites (l+1, N)
     by device environment updates (each one normalised when ``normalize``).
 
-    They use the plain FP64 GEMMs, whose summation order is fixed: a mixed
-    Krylov run follows the last bit of the environments it starts from, so
-    these do not depend on the form rule."""
+    Under the default form rule they use the plain FP64 GEMMs, whose summation
+    order is fixed: a mixed Krylov run follows the last bit of the environments
+    it starts from.  (A sweep grows its own under the rule; solves from either
+    agree to the solver's tolerance.)  A form chosen with ``set_gemm_form`` is
+    kept."""
     form = ctx.gemm_form()
-    ctx.set_gemm_form(0)
+    ctx.set_gemm_form(max(form, 0))
     try:
         return _grow_envs(ctx, mpo, mps, l, normalize)
     finally:
