@@ -32,6 +32,22 @@ Ctx::~Ctx() {
   if (stage) cudaFreeHost(stage);
 }
 
+void Ctx::allow_smem(const void *kernel, size_t bytes) {
+  if (std::find(smem_set.begin(), smem_set.end(), kernel) != smem_set.end()) return;
+  UDMRG_CHECK_CUDA(
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  smem_set.push_back(kernel);
+}
+
+int Ctx::blocks_per_sm(const void *kernel, int threads) {
+  for (const auto &o : occupancy)
+    if (o.first == kernel) return o.second;
+  int n = 0;
+  UDMRG_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, 0));
+  occupancy.push_back({kernel, n});
+  return n;
+}
+
 uint8_t *Ctx::stage_room(size_t bytes) {
   bytes = (bytes + 255) & ~(size_t)255;
   if (bytes > kStage) return nullptr;

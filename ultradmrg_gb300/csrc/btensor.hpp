@@ -99,8 +99,17 @@ struct Ctx {
   uint8_t *stage = nullptr;
   size_t stage_off = 0;
 
+  // Launch set-up of kernels on this context's device, asked for once each (the
+  // driver keeps both per device, so nothing here belongs to the process).
+  std::vector<const void *> smem_set;
+  std::vector<std::pair<const void *, int>> occupancy;
+
   explicit Ctx(int dev);
   ~Ctx();
+  // Lets the kernel use `bytes` of dynamic shared memory (one size per kernel).
+  void allow_smem(const void *kernel, size_t bytes);
+  // Resident blocks per SM of a kernel without dynamic shared memory.
+  int blocks_per_sm(const void *kernel, int threads);
   // Stream-ordered copy of host memory to the device.
   void upload(void *dst, const void *src, size_t bytes);
   // Room for `bytes` in the ring (null: more than it holds).

@@ -252,12 +252,9 @@ void launch_cfg(Ctx &ctx, const GemmPlan &plan, int cfg, const In *a, const In *
   const int ntiles = (int)plan.tiles[cfg].size();
   if (ntiles == 0) return;
   constexpr int NT = (BM / TM) * (BN / TN);
-  static int per_sm = 0;
-  if (per_sm == 0)
-    UDMRG_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &per_sm, grouped_gemm_kernel<T, In, BM, BN, TM, TN, BK>, NT, 0));
-  const int grid = std::min(ntiles, std::max(1, per_sm) * ctx.num_sms);
   auto kernel = grouped_gemm_kernel<T, In, BM, BN, TM, TN, BK>;
+  const int per_sm = ctx.blocks_per_sm((const void *)kernel, NT);
+  const int grid = std::min(ntiles, std::max(1, per_sm) * ctx.num_sms);
   if (gate) {
     UDMRG_CHECK_CUDA(tc::launch_pdl(kernel, dim3(grid), dim3(NT), 0, ctx.stream,
                                     plan.d_tiles[cfg], ntiles, plan.d_probs, plan.d_segs, a, b, c,

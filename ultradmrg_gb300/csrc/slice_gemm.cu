@@ -792,12 +792,7 @@ void run_slice(Ctx &ctx, const SlicePlan &p, const double *a, const double *b, d
                                     p.d_items_t, nx, a, b, p.scale, p.img));
     ctx.launches++;
   }
-  static bool attr_set = false;
-  if (!attr_set) {
-    UDMRG_CHECK_CUDA(cudaFuncSetAttribute(slice_gemm_kernel,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, kSlSmem));
-    attr_set = true;
-  }
+  ctx.allow_smem((const void *)slice_gemm_kernel, kSlSmem);
   const int nt = (int)p.tiles.size();
   UDMRG_CHECK_CUDA(tc::launch_pdl(slice_gemm_kernel, dim3(std::min(nt, ctx.num_sms)),
                                   dim3(kSlThreads), kSlSmem, ctx.stream, p.d_tiles, nt,

@@ -303,13 +303,7 @@ template <int BN>
 static void launch_tc_gemm(Ctx &ctx, const TcPlan &plan, const uint8_t *a_img,
                            const uint8_t *b_img, void *out, int out_kind, double alpha) {
   const int ntiles = (int)plan.tiles.size();
-  static bool attr_set = false;
-  if (!attr_set) {
-    UDMRG_CHECK_CUDA(cudaFuncSetAttribute(tc_gemm_kernel<BN>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          TcShape<BN>::kSmemBytes));
-    attr_set = true;
-  }
+  ctx.allow_smem((const void *)tc_gemm_kernel<BN>, TcShape<BN>::kSmemBytes);
   const int grid = std::min(ntiles, ctx.num_sms);
   UDMRG_CHECK_CUDA(tc::launch_pdl(tc_gemm_kernel<BN>, dim3(grid), dim3(kThreads),
                                   (size_t)TcShape<BN>::kSmemBytes, ctx.stream, plan.d_tiles,

@@ -158,13 +158,7 @@ template <int BN>
 static void launch_tc_mpo_gemm(Ctx &ctx, const SgMatvecPlan &p, double *out) {
   const TcPlan &plan = p.g3;
   const int ntiles = (int)plan.tiles.size();
-  static bool attr_set = false;
-  if (!attr_set) {
-    UDMRG_CHECK_CUDA(cudaFuncSetAttribute(tc_mpo_gemm_kernel<BN>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          TcShape<BN>::kSmemBytes));
-    attr_set = true;
-  }
+  ctx.allow_smem((const void *)tc_mpo_gemm_kernel<BN>, TcShape<BN>::kSmemBytes);
   const int grid = std::min(ntiles, ctx.num_sms);
   tc_mpo_gemm_kernel<BN><<<grid, kFusedThreads, TcShape<BN>::kSmemBytes, ctx.stream>>>(
       plan.d_tiles, ntiles, plan.d_groups, p.d_gmap, p.d_rowinfo, p.d_kchunks, p.d_tgtref,
