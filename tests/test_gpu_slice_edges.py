@@ -5,6 +5,7 @@ import pytest
 
 from test_gpu_slice import ctx, product  # noqa: F401
 from ultradmrg_gb300 import api
+from ultradmrg_gb300.tensor_data import IN, OUT, BlockTensorData, Index
 
 pytestmark = pytest.mark.gpu
 
@@ -52,3 +53,40 @@ def test_coherent_low_digits(ctx, k):  # noqa: F811
         exact = np.longdouble(float(ref[0, j] >> 40)) * np.ldexp(np.longdouble(1), 40 - 92)
         cols = got[:, j::2] if j == 0 else got[:, 1:2]
         assert np.all(np.abs(cols - exact) <= 2.0 ** -52 * np.abs(exact) + k * 2.0 ** -50)
+
+
+def two_sectors(shapes, decades, seed, dtype=np.float64):
+    """A block-diagonal matrix (one block per charge) and its blocks; singular values
+    decay over `decades`."""
+    rng = np.random.default_rng(seed)
+    blocks = {}
+    for q, (r, c) in enumerate(shapes):
+        k = min(r, c)
+        def orth(n):
+            x = rng.standard_normal((n, k))
+            if dtype == np.complex128:
+                x = x + 1j * rng.standard_normal((n, k))
+            return np.linalg.qr(x)[0]
+        s = 10.0 ** (-decades * np.arange(k) / k) / (q + 1)
+        blocks[q, q] = (orth(r) * s) @ orth(c).conj().T
+    idx = [Index.make([((q,), s[i]) for q, s in enumerate(shapes)], (IN, OUT)[i]) for i in (0, 1)]
+    return BlockTensorData(idx, blocks, dtype), blocks
+
+
+def rebuilt(ctx, u, s, vt):  # noqa: F811
+    return api.contract(ctx, api.contract(ctx, u, s, [1], [0]), vt, [1], [0]).to_data().blocks
+
+
+@pytest.mark.parametrize("shapes", [((129, 300), (40, 65)), ((260, 193), (64, 64))])
+def test_randomized_svd(ctx, shapes):  # noqa: F811
+    """Products that add to their result (the residuals) run on the FMAs whatever
+    the form; the truncated matrix is the exact SVD's to the sketch's accuracy."""
+    t, _ = two_sectors(shapes, 8, sum(shapes[0]))
+    d = api.DeviceTensor.from_data(ctx, t)
+    u, s, vt, err, kept = api.svd(ctx, d, 1, (0,), 1e-10, 1, 1000)
+    x, y, z, err2, kept2, _ = api.svd_randomized(ctx, d, 1, (0,), 1e-10, 1, 1000,
+                                                 [((q,), 30) for q in range(2)])
+    assert kept == kept2 and abs(err - err2) <= 1e-12
+    a, b = rebuilt(ctx, u, s, vt), rebuilt(ctx, x, y, z)
+    for k in a:
+        assert np.abs(a[k] - b[k]).max() <= 1e-6

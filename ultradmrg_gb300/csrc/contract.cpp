@@ -697,8 +697,8 @@ static void tile_all(GemmPlan &g) {
     });
 }
 
-void gemm_finalize(GemmPlan &g, bool cplx, bool upper) {
-  g.sl = slice_worth(g, cplx, upper, [&] { return slice_simple(g, cplx, upper); });
+void gemm_finalize(GemmPlan &g, bool cplx, bool upper, bool adds) {
+  if (!adds) g.sl = slice_worth(g, cplx, upper, [&] { return slice_simple(g, cplx, upper); });
   if (!g.sl) {
     tile_all(g);
     if (upper)

@@ -80,13 +80,15 @@ void gemm_add_simple(GemmPlan &g, int64_t c_off, int64_t M, int64_t N, int64_t K
 // cplx: element type of the data (the sliced form's choice depends on it).
 // upper: square problems whose result is symmetric (Hermitian): only the tiles
 // that reach the diagonal or lie above it.
-void gemm_finalize(GemmPlan &g, bool cplx = false, bool upper = false);
+// adds: the plan runs with beta != 0, which only the FMAs do (no sliced form).
+void gemm_finalize(GemmPlan &g, bool cplx = false, bool upper = false, bool adds = false);
 // the descriptors of a plan made with upload = false onto the device
 void gemm_upload(GemmPlan &g);
 // The same problems tiled under another policy (results are bit-identical:
 // every output element sums its segments and K in the same order).
 void gemm_retile(GemmPlan &g, int policy);
-// Run C = alpha * A*B (+ beta * C) for every problem of the plan.
+// Run C = alpha * A*B (+ beta * C) for every problem of the plan (one with a
+// sliced form: alpha = 1 and beta = 0).
 void run_gemm(Ctx &ctx, const GemmPlan &plan, DType dt, const double *a, const double *b,
               double *c, double alpha, double beta);
 // The same GEMMs of real data in double-word FP32 arithmetic (48-bit

@@ -271,7 +271,8 @@ template <typename T, typename In>
 void run_typed(Ctx &ctx, const GemmPlan &plan, const In *a, const In *b, In *c, double alpha,
                double beta) {
   const int *gate = nullptr;
-  if (plan.sl && alpha == 1.0 && beta == 0.0) {
+  if (plan.sl) {
+    UDMRG_REQUIRE(alpha == 1.0 && beta == 0.0, "gemm: a sliced plan computes C = A B only");
     run_slice(ctx, *plan.sl, (const double *)a, (const double *)b, (double *)c);
     gate = plan.sl->scale;
   }

@@ -556,7 +556,7 @@ SvdResult svd_trunc_sketch(Ctx &ctx, const BTensor &T, int ldims, const QN &ldiv
         const int64_t sq = s[act[a]];
         gemm_add_simple(g, yoff[a], x.xr, sq, x.xc, x.off, x.sr, x.sc, zoff[a], sq, 1, false);
       }
-      gemm_finalize(g);
+      gemm_finalize(g, false, false, beta != 0.0);
       run_gemm(ctx, g, kF64, Mbuf, zin, yout, 1.0, beta);
     };
     auto mult_xty = [&](const double *yin, double *zout) {  // Z = X^T Y
