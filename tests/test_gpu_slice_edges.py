@@ -1,9 +1,11 @@
 """The sliced FP64 GEMM at the ends of its range and on the calls that reach it in
 other ways than a plain contraction."""
+import time
+
 import numpy as np
 import pytest
 
-from test_gpu_slice import ctx, product  # noqa: F401
+from test_gpu_slice import ctx, dense, product  # noqa: F401
 from ultradmrg_gb300 import api
 from ultradmrg_gb300.tensor_data import IN, OUT, BlockTensorData, Index
 
@@ -90,3 +92,31 @@ def test_randomized_svd(ctx, shapes):  # noqa: F811
     a, b = rebuilt(ctx, u, s, vt), rebuilt(ctx, x, y, z)
     for k in a:
         assert np.abs(a[k] - b[k]).max() <= 1e-6
+
+
+@pytest.mark.parametrize("m,n", [(60000, 8), (8, 60000)])
+def test_narrow_out_of_range_product(ctx, m, n):  # noqa: F811
+    """An operand outside the range, narrow result: the FMAs' result bit for bit, from
+    tiles of its shape (64 x 64 ones would take four times the work): not three
+    times as long as the FMA form itself, at a K that leaves the plan's host time
+    behind."""
+    rng = np.random.default_rng(9)
+    a, b = rng.standard_normal((m, 1024)), rng.standard_normal((1024, n))
+    (a if m > n else b)[3, 5] = 1e200
+    x, y = (api.DeviceTensor.from_data(ctx, dense(v, (IN, OUT))) for v in (a, b))
+
+    def timed(form):
+        ctx.set_gemm_form(form)
+        best = 1e9
+        for _ in range(8):
+            ctx.sync()
+            t = time.perf_counter()
+            c = api.contract(ctx, x, y, [1], [0])
+            ctx.sync()
+            best = min(best, time.perf_counter() - t)
+        return best, c.download_packed()
+
+    t0, want = timed(0)
+    t1, got = timed(1)
+    assert np.array_equal(got, want)
+    assert t1 <= 3 * t0, (t0, t1)

@@ -97,6 +97,31 @@ static void tile_all(GemmPlan &g);
 
 namespace {
 
+// One tile configuration for all problems: 64 x 64, or the one whose padded work
+// is less by a quarter or more (32 x 32 charged twice: four outputs per thread).
+int one_cfg(const GemmPlan &g) {
+  int best = kCfg64x64;
+  double bestw = 0;
+  for (int c = 0; c < kNumCfg; ++c) {
+    double w = 0;
+    for (const GProb &p : g.probs) {
+      double k = 0;
+      for (int s = 0; s < p.nseg; ++s) k += g.segs[p.seg0 + s].K;
+      w += k * (double)(((int64_t)p.M + kCfgBM[c] - 1) / kCfgBM[c] * kCfgBM[c]) *
+           (double)(((int64_t)p.N + kCfgBN[c] - 1) / kCfgBN[c] * kCfgBN[c]);
+    }
+    if (c == kCfg32x32) w *= 2.0;
+    if (c == 0 || w < 0.75 * bestw) {
+      bestw = w;
+      best = c;
+    }
+  }
+  return best;
+}
+
+// Whether a tile holds entries on or above the diagonal.
+bool reaches_diagonal(int cfg, int32_t m0, int32_t n0) { return m0 <= n0 + kCfgBN[cfg] - 1; }
+
 constexpr int64_t up8(int64_t x) { return (x + 7) & ~(int64_t)7; }
 
 // Estimated time of a plan's FP64 tiles: multiply-adds of the padded tiles
@@ -412,11 +437,13 @@ std::unique_ptr<SlicePlan> slice_worth(GemmPlan &g, bool cplx, bool upper, Build
   }
   auto sp = build();
   if (sp && form < 0 && sp->seconds() >= t64) sp.reset();
-  if (sp) {  // the FP64 tiles of operands outside its range: one launch, 64 x 64
+  if (sp) {  // the FP64 tiles of operands outside its range: one launch
+    const int cfg = one_cfg(g);
     for (size_t p = 0; p < g.probs.size(); ++p)
-      for (int32_t m = 0; m < g.probs[p].M; m += 64)
-        for (int32_t n = upper ? m / 64 * 64 : 0; n < g.probs[p].N; n += 64)
-          g.tiles[kCfg64x64].push_back({(int32_t)p, m, n, 0});
+      for (int32_t m = 0; m < g.probs[p].M; m += kCfgBM[cfg])
+        for (int32_t n = 0; n < g.probs[p].N; n += kCfgBN[cfg])
+          if (!upper || reaches_diagonal(cfg, m, n))
+            g.tiles[cfg].push_back({(int32_t)p, m, n, 0});
   }
   return sp;
 }
@@ -704,8 +731,9 @@ void gemm_finalize(GemmPlan &g, bool cplx, bool upper, bool adds) {
     if (upper)
       for (int c = 0; c < kNumCfg; ++c) {
         auto &t = g.tiles[c];
-        t.erase(std::remove_if(t.begin(), t.end(),
-                               [&](const GTile &x) { return x.m0 > x.n0 + kCfgBN[c] - 1; }),
+        t.erase(std::remove_if(
+                    t.begin(), t.end(),
+                    [&](const GTile &x) { return !reaches_diagonal(c, x.m0, x.n0); }),
                 t.end());
       }
   }
