@@ -5,8 +5,9 @@ import time
 import numpy as np
 import pytest
 
-from test_gpu_slice import ctx, dense, product  # noqa: F401
+from test_gpu_slice import check, ctx, dense, product  # noqa: F401
 from ultradmrg_gb300 import api
+from ultradmrg_gb300 import models as M
 from ultradmrg_gb300.tensor_data import IN, OUT, BlockTensorData, Index
 
 pytestmark = pytest.mark.gpu
@@ -120,3 +121,121 @@ def test_narrow_out_of_range_product(ctx, m, n):  # noqa: F811
     t1, got = timed(1)
     assert np.array_equal(got, want)
     assert t1 <= 3 * t0, (t0, t1)
+
+
+# ---- the calls that reach the form in other ways --------------------------------
+
+@pytest.mark.parametrize("k", [1153, 2501])
+def test_complex_k_parts(ctx, k):  # noqa: F811
+    """Few tiles of a long complex contraction, whose embedded K is cut into parts."""
+    rng = np.random.default_rng(k)
+    a = rng.standard_normal((70, k)) + 1j * rng.standard_normal((70, k))
+    b = rng.standard_normal((k, 33)) + 1j * rng.standard_normal((k, 33))
+    check(product(ctx, a, b), a, b)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.complex128])
+@pytest.mark.parametrize("shapes", [((63, 129), (65, 64)), ((128, 300), (200, 127)),
+                                    ((257, 193), (30, 7)), ((320, 320), (160, 131))])
+@pytest.mark.parametrize("mode", [api.SVD_SPLIT_LEFT, api.SVD_SPLIT_RIGHT])
+def test_svd_products(ctx, shapes, dtype, mode):  # noqa: F811
+    """Gram products of the upper triangle, Newton-Schulz and factor products in the
+    sliced form, at sizes around the tiles' edges and in both orientations.  Bounds
+    of the Gram route: squared singular values to 1e-14 sqrt(n) of the largest, the
+    factors' product (all states kept) to 1e-13 n of it."""
+    t, blocks = two_sectors(shapes, 4, shapes[0][0] + shapes[1][1], dtype)
+    u, s, vt, err, kept = api.svd(ctx, api.DeviceTensor.from_data(ctx, t), 1, (0,), 0.0, 1, 10000,
+                                  mode)
+    assert kept == sum(min(x) for x in shapes)
+    sv = {k[0]: np.diag(b).real for k, b in s.to_data().blocks.items()}
+    state = api.contract(ctx, u, vt, [1], [0]).to_data().blocks
+    top = max(np.linalg.norm(b, 2) for b in blocks.values())
+    got = np.sort(np.concatenate([sv[k] for k in sorted(sv)]))[::-1]
+    want = np.sort(np.concatenate([np.linalg.svd(b, compute_uv=False)
+                                   for b in blocks.values()]))[::-1]
+    n = max(max(x) for x in shapes)
+    assert np.abs(got ** 2 - want ** 2).max() <= 1e-14 * np.sqrt(n) * top ** 2
+    for k, b in blocks.items():
+        assert np.abs(state[k] - b).max() <= 1e-13 * n * top
+
+
+@pytest.fixture(scope="module", params=[np.float64, np.complex128], ids=["real", "complex"])
+def bond(request, ctx):  # noqa: F811
+    """(L, W1, W2, R, two site tensors) at the centre of a 3 x 2 Hubbard cylinder."""
+    dtype = request.param
+    mpo, pb = M.hubbard_cylinder_mpo(3, 2, t=1.0, U=8.0, dtype=dtype)
+    mps = M.random_canonical_mps([pb] * 6, (5, 1), 60, 2, seed=3, dtype=dtype)
+    up = lambda t: api.DeviceTensor.from_data(ctx, t)  # noqa: E731
+    ctx.set_gemm_form(0)
+    L, R = api.build_envs(ctx, mpo, mps, 2)
+    ctx.set_gemm_form(1)
+    return L, up(mpo[2]), up(mpo[3]), R, up(mps[2]), up(mps[3])
+
+
+def scaled(ctx, t, f):  # noqa: F811
+    d = t.to_data()
+    d.blocks = {k: v * f for k, v in d.blocks.items()}
+    return api.DeviceTensor.from_data(ctx, d)
+
+
+def both_forms(ctx, fn):  # noqa: F811
+    out = []
+    for form in (0, 1):
+        ctx.set_gemm_form(form)
+        out.append(fn().to_data().blocks)
+    return out
+
+
+def agree(x, y, tol):
+    scale = max(np.abs(v).max() for v in x.values())
+    assert scale > 0 and sorted(x) == sorted(y)
+    for k in x:
+        assert np.abs(x[k] - y[k]).max() <= tol * scale
+
+
+@pytest.mark.parametrize("p", [0, -60, 300, -430])
+def test_one_site_product(ctx, bond, p):  # noqa: F811
+    """The one-site product, whose MPO step finds the last GEMM's scales, for states
+    of several magnitudes in a row (at 2^-430 the scales that the step finds are
+    outside the range, those of the state are not)."""
+    L, w1, _, R1, a, _ = bond
+    L = scaled(ctx, L, 2.0 ** -60) if p == -430 else L
+    # its right environment: one more update from the two-site one
+    ctx.set_gemm_form(0)
+    R = api.update_site_renvs(ctx, R1, bond[5], bond[2])
+    for q in (p, 0, p):
+        x, y = both_forms(ctx, lambda: api.eff_ham_mul_single_site_state(
+            ctx, [L, w1, R], scaled(ctx, a, 2.0 ** q)))
+        agree(x, y, 1e-13)
+
+
+def test_two_site_scales_out_of_range(ctx, bond):  # noqa: F811
+    """A state and an environment inside the range whose product is not."""
+    L, w1, w2, R, a, b = bond
+    psi = api.contract(ctx, a, b, [2], [0])
+    big = scaled(ctx, L, 2.0 ** -240)
+    x, y = both_forms(ctx, lambda: api.eff_ham_mul_two_site_state(
+        ctx, [big, w1, w2, R], scaled(ctx, psi, 2.0 ** -250)))
+    agree(x, y, 1e-13)
+
+
+def test_double_word_fallback(ctx, bond):  # noqa: F811
+    """A sliced anchor whose operand is not finite: the double-word tiles' result."""
+    L, w1, w2, R, a, b = bond
+    psi = api.contract(ctx, a, b, [2], [0])
+    bad = psi.to_data()
+    k = sorted(bad.blocks)[len(bad.blocks) // 2]
+    bad.blocks[k] = np.full_like(bad.blocks[k], np.inf)
+    bad = api.DeviceTensor.from_data(ctx, bad)
+
+    def run():
+        plan = api.MatvecPlan(ctx, [L, w1, w2, R], psi, precision=api.PREC_MIXED)
+        x, y = plan.embed(bad), plan.embed(psi)
+        plan.apply_anchor(x, y)
+        return y
+
+    x, y = both_forms(ctx, run)
+    for k in x:
+        assert np.array_equal(np.isfinite(x[k]), np.isfinite(y[k]))
+        ok = np.isfinite(x[k])
+        assert np.abs(x[k][ok] - y[k][ok]).max(initial=0.0) <= 1e-12
