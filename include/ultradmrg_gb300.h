@@ -391,7 +391,9 @@ int udmrg_two_site_finite_vmps_noise(udmrg_ctx *ctx, int64_t N, udmrg_tensor **m
 
 /* ---- reusable matvec plan (repeated H_eff * psi on device buffers) -------- */
 /* The plan fixes {L, W_l, W_r, R} and the block structure closed under the
- * matvec that contains psi_struct's blocks (the Krylov structure). */
+ * matvec that contains psi_struct's blocks (the Krylov structure).  L and R are
+ * read at every product (the mixed form: when the plan is made), real MPO
+ * coefficients when the plan is made: a changed MPO needs a new plan. */
 int udmrg_matvec_plan_create(udmrg_ctx *ctx, udmrg_tensor *const *eff_ham,
                              const udmrg_tensor *psi_struct, udmrg_matvec_plan **out);
 /* Same with a matvec precision (UDMRG_PREC_FP64 / UDMRG_PREC_MIXED). */

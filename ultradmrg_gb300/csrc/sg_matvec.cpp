@@ -474,16 +474,17 @@ std::unique_ptr<SgMatvecPlan> plan_sg_tables(const BTensor &L, const BTensor &R,
     // ladder D = 512 20.5 -> 16.4.  With more tasks than that the step is bound
     // by HBM and a run's inputs are read again by its pair's other runs (D =
     // 2000: 110 us whole, 114.7 us in runs).
-    constexpr double kResidentWarps = 152 * 16, kMpoTaskShare = 16;
+    constexpr double kMpoTaskShare = 16;
+    const double resident = 16.0 * L.ctx->num_sms;  // warps
     double work = 0, whole = 0;
     for (const MpoPair &pr : p->pairs) {
       const double t = (double)(((int64_t)pr.da * (pr.dbp / 8) + 31) / 32);
       whole += t;
       work += t * (p->rowptr[pr.row0 + pr.nout] - p->rowptr[pr.row0] + pr.nout);
     }
-    const int target = whole >= 4 * kResidentWarps
+    const int target = whole >= 4 * resident
                            ? INT32_MAX
-                           : (int)std::max(24.0, work / (kResidentWarps * kMpoTaskShare));
+                           : (int)std::max(24.0, work / (resident * kMpoTaskShare));
     struct Run {
       int q, o0, nout, cost;
     };

@@ -660,7 +660,7 @@ void SlicePlan::finalize() {
     if (by_cols(op))
       wide += (int64_t)((op.rows + kPackRows - 1) / kPackRows) *
               ((op.cols + kPackCols - 1) / kPackCols);
-  const int width = wide < 4 * kPackWarps * (ctx ? ctx->num_sms : 152) ? 32 : kPackCols;
+  const int width = wide < 4 * kPackWarps * ctx->num_sms ? 32 : kPackCols;
   for (int src = 0; src < 2; ++src) {
     for (size_t o = 0; o < ops.size(); ++o) {
       const SlOp &op = ops[o];
@@ -702,7 +702,7 @@ void SlicePlan::finalize() {
   double steps = 0;
   of_group([&](int32_t id, int32_t, int32_t) { steps += groups[id].kc; });
   const int unit = std::max<int>(
-      kSlChunk, ((int)(steps / (ctx ? ctx->num_sms : 152) / 3) + kSlChunk - 1) / kSlChunk * kSlChunk);
+      kSlChunk, ((int)(steps / ctx->num_sms / 3) + kSlChunk - 1) / kSlChunk * kSlChunk);
   for (SlGroup &g : groups) {
     g.parts = std::max(1, std::min(8, (g.kc + unit / 2) / unit));
     const int per = (g.kc + g.parts - 1) / g.parts;
@@ -755,15 +755,11 @@ void SlicePlan::upload() {
   if (holes) UDMRG_CHECK_CUDA(cudaMemsetAsync(img, 0, img_bytes, ctx->stream));
 }
 
-size_t SlicePlan::workspace() const {
-  return (size_t)img_bytes + nscale() * sizeof(int) + slots * kSlU * kSlV * sizeof(longlong2);
-}
-
 double SlicePlan::seconds() const {
   double steps = 0, elems = 0;
   for (const SlTile &t : tiles) steps += std::min(groups[t.group].kpart, groups[t.group].kc) + 2.0;
   for (const SlOp &o : ops) elems += (double)o.rows * o.cols;
-  return 30e-6 + steps * 0.7e-6 / 152 + elems * 30.0 / 3e12;
+  return 30e-6 + steps * 0.7e-6 / ctx->num_sms + elems * 30.0 / 3e12;
 }
 
 void SlicePlan::clear_scales() const {

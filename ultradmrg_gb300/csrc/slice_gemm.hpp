@@ -138,7 +138,6 @@ struct SlicePlan {
   double seconds() const;  // the cost model's estimate
   void finalize();         // items, K parts and tile order (host)
   void upload();           // device tables and workspaces
-  size_t workspace() const;
   void clear_scales() const;  // device: flags, scales, counters to zero
   size_t nscale() const { return 2 + lines.size() + 16 * (size_t)slots; }
 };
