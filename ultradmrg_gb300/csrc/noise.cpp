@@ -167,7 +167,11 @@ void noise_update(Ctx &ctx, std::vector<TensorPtr> &mps, std::vector<TensorPtr> 
   }
   const double t0 = wall();
   const BTensor &L = *lenvs[lenv_len], &R = *renvs[renv_len];
-  auto init = contract_axes(ctx, *mps[l], *mps[r], {2}, {0});
+  TensorPtr init;
+  {
+    FmaGemms fma(ctx, true);  // as in two_site_update_local
+    init = contract_axes(ctx, *mps[l], *mps[r], {2}, {0});
+  }
   auto mv = plan_matvec2(ctx, L, *W[l], *W[r], R, *init, p.lancz.precision);
   // energy expectation of the current state, then the noise for this update
   double actual;
