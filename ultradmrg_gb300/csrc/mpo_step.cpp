@@ -159,7 +159,8 @@ void push_pair(MpoStep64 &p, PairMap &m, int64_t da, int64_t db, int es) {
     p.rowptr.push_back((int32_t)p.nz.size());
   }
   p.flops += 2.0 * (double)(p.nz.size() - n0) * pr.da * pr.db;
-  UDMRG_REQUIRE((int64_t)pr.da * pr.db < (1ll << 31), "MPO step: block too large");
+  // (a task counts to 64 past its first entry in 32 bits)
+  UDMRG_REQUIRE((int64_t)pr.da * db * es < (1ll << 31) - 64, "MPO step: block too large");
   // runs of output channels of at most kMpoRun couplings and writes (one channel at least)
   for (int32_t o0 = 0, o1; o0 < pr.nout; o0 = o1) {
     const int32_t *row = p.rowptr.data() + pr.row0;
@@ -218,6 +219,7 @@ std::unique_ptr<MpoStep64> build_mpo_step64(FusedMpo &fm, const BTensor &T1, con
       const int32_t *k = T3.key(ob);
       const int64_t nout =
           T3.idx[1].dims[k[1]] * T3.idx[2].dims[k[2]] * T3.idx[3].dims[k[3]];
+      UDMRG_REQUIRE(nout * db * es < (1ll << 31), "MPO step: block too large");
       const int32_t ofirst = (int32_t)m.outs.size();
       for (int64_t c = 0; c < nout; ++c)
         m.outs.push_back({T3.offs[ob] + c * db, (int32_t)(nout * db), -1, 0, 0});
@@ -292,6 +294,7 @@ std::unique_ptr<MpoStep64> build_mpo_map(const BTensor &T, const BTensor &W,
       const int64_t ob = ends[g].blk;
       const int32_t *k = out.key(ob);
       const int64_t d1 = out.idx[1].dims[k[1]], d2 = out.idx[2].dims[k[2]];
+      UDMRG_REQUIRE(d1 * d2 * db * es < (1ll << 31), "MPO step: block too large");
       const int32_t ofirst = (int32_t)m.outs.size();
       for (int64_t c = 0; c < d1 * d2; ++c)
         m.outs.push_back({out.offs[ob] + c * db, (int32_t)(d1 * d2 * db), -1, 0, 0});
