@@ -100,22 +100,18 @@ namespace {
 // One tile configuration for all problems: 64 x 64, or the one whose padded work
 // is less by a quarter or more (32 x 32 charged twice: four outputs per thread).
 int one_cfg(const GemmPlan &g) {
-  int best = kCfg64x64;
-  double bestw = 0;
-  for (int c = 0; c < kNumCfg; ++c) {
-    double w = 0;
-    for (const GProb &p : g.probs) {
-      double k = 0;
-      for (int s = 0; s < p.nseg; ++s) k += g.segs[p.seg0 + s].K;
-      w += k * (double)(((int64_t)p.M + kCfgBM[c] - 1) / kCfgBM[c] * kCfgBM[c]) *
-           (double)(((int64_t)p.N + kCfgBN[c] - 1) / kCfgBN[c] * kCfgBN[c]);
-    }
-    if (c == kCfg32x32) w *= 2.0;
-    if (c == 0 || w < 0.75 * bestw) {
-      bestw = w;
-      best = c;
-    }
+  double w[kNumCfg] = {0, 0, 0, 0};
+  for (const GProb &p : g.probs) {
+    double k = 0;
+    for (int s = 0; s < p.nseg; ++s) k += g.segs[p.seg0 + s].K;
+    for (int c = 0; c < kNumCfg; ++c)
+      w[c] += k * (double)(((int64_t)p.M + kCfgBM[c] - 1) / kCfgBM[c] * kCfgBM[c]) *
+              (double)(((int64_t)p.N + kCfgBN[c] - 1) / kCfgBN[c] * kCfgBN[c]);
   }
+  w[kCfg32x32] *= 2.0;
+  int best = kCfg64x64;
+  for (int c = 1; c < kNumCfg; ++c)
+    if (w[c] < (best == kCfg64x64 ? 0.75 * w[best] : w[best])) best = c;
   return best;
 }
 
@@ -504,13 +500,20 @@ static std::unique_ptr<ContractPlan> plan_impl(const BTensor &A, const BTensor &
       matches.push_back({ok, a, it->second});
     }
   }
-  std::sort(matches.begin(), matches.end(), [&](const Match &x, const Match &y) {
+  auto before = [](const Match &x, const Match &y) {
     if (x.okey != y.okey) return x.okey < y.okey;
-    for (int ax : seg_axes)
-      if (A.key(x.a)[ax] != A.key(y.a)[ax]) return A.key(x.a)[ax] < A.key(y.a)[ax];
     if (x.a != y.a) return x.a < y.a;
     return x.b < y.b;
-  });
+  };
+  if (seg_axes.empty())
+    std::sort(matches.begin(), matches.end(), before);
+  else
+    std::sort(matches.begin(), matches.end(), [&](const Match &x, const Match &y) {
+      if (x.okey == y.okey)
+        for (int ax : seg_axes)
+          if (A.key(x.a)[ax] != A.key(y.a)[ax]) return A.key(x.a)[ax] < A.key(y.a)[ax];
+      return before(x, y);
+    });
   // output blocks = distinct keys; [mstart[o], mstart[o + 1]) are their matches
   std::vector<int32_t> flat;
   std::vector<size_t> mstart;
